@@ -1,9 +1,10 @@
 // Setup-phase kernels of the solve path (sm_100a):
-//  * FSAI numeric phase: one warp per row gathers the local SPD system
-//    A[P,P], -A[P,i] of its pattern, factors it in shared memory (FP64
-//    Cholesky), solves, and scales the row by 1/sqrt(a_ii - A_iP A_PP^-1 A_Pi)
-//    (cpt_afsai_coef.cpp:440-541).  Rows are bucketed by local size so each
-//    bucket runs with the shared-memory tile that fits it.
+//  * FSAI numeric phase: a group of lanes per row gathers the local SPD system
+//    A[P,P], -A[P,i] of its pattern, factors it in FP64 (LDL' in registers up
+//    to 32 unknowns, Cholesky in shared memory up to 64), solves, and scales
+//    the row by 1/sqrt(a_ii - A_iP A_PP^-1 A_Pi) (cpt_afsai_coef.cpp:440-541).
+//    Rows are bucketed by local size so each bucket runs with the lane group
+//    or shared-memory tile that fits it.
 //  * Galerkin product P'*(A*P) (cpt_aspAMG.m:277) as two row-wise sparse
 //    products with per-row hash tables: symbolic count, then numeric
 //    accumulation in Gustavson order (each output entry summed in the order
@@ -133,18 +134,250 @@ __device__ __forceinline__ void fsai_row(int i, const int *__restrict__ arp,
   if (lane == 0) gval[gs + m] = s;
 }
 
+// Positions of the columns col[u] in the sorted rows [lo[u], hi[u]) of aci, or
+// -1: U binary searches step together, so their dependent loads overlap.
+template <int U>
+__device__ __forceinline__ void find_cols(const int *__restrict__ aci, int (&lo)[U],
+                                          const int (&hi)[U], const int (&col)[U]) {
+  int n[U];
+  bool any = false;
+#pragma unroll
+  for (int u = 0; u < U; ++u) {
+    n[u] = hi[u] - lo[u];
+    any |= n[u] > 0;
+  }
+  while (any) {
+    int c[U];
+#pragma unroll
+    for (int u = 0; u < U; ++u) c[u] = n[u] > 0 ? __ldg(aci + lo[u] + (n[u] >> 1)) : 0;
+    any = false;
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+      const int half = n[u] >> 1;
+      if (n[u] > 0) {
+        if (c[u] < col[u]) {
+          lo[u] += half + 1;
+          n[u] -= half + 1;
+        } else {
+          n[u] = half;
+        }
+      }
+      any |= n[u] > 0;
+    }
+  }
+#pragma unroll
+  for (int u = 0; u < U; ++u)
+    if (lo[u] >= hi[u] || __ldg(aci + lo[u]) != col[u]) lo[u] = -1;
+}
+
+// Row i of G by T lanes (32/T rows per warp; i < 0: an idle group), local
+// systems of up to MMAX <= T unknowns.  Lane j holds row j of the lower
+// triangle in registers, R[0..j], and takes LDL' steps: at step k the pivot is
+// broadcast, every lane scales its own entry by the pivot's reciprocal and
+// leaves it in the group's shared-memory tile, column by column, from where
+// the update reads the whole column two entries at a time (one 16-byte
+// broadcast) and the backward substitution its row of L'.  The forward
+// substitution rides along.  Registers past the diagonal collect products
+// that nothing reads.  Unknowns beyond m are identity rows, so a row's
+// operations do not depend on the T it runs with.
+// One reciprocal per step and no division or square root: with a warp per
+// row, the factor in shared memory and a lane per column walking A's rows
+// this took 1419 us for 227k rows of mostly 15 unknowns (61^3 diffusion),
+// bound by those and by the serial walk; with the column sent round by
+// shuffles 351 us, bound by issue (71 % of the slots); now 297 us.  The
+// entries A[P,P] are found by T lanes taking the pairs (c, c+s mod m) of each
+// distance s, four searches in flight.
+template <int T, int MMAX>
+__device__ __forceinline__ void fsai_row_reg(int i, const int *__restrict__ arp,
+                                             const int *__restrict__ aci,
+                                             const double *__restrict__ av,
+                                             const int *__restrict__ grp,
+                                             const int *__restrict__ gci,
+                                             double *__restrict__ gval, int *flags, double *S) {
+  constexpr unsigned FULL = 0xffffffffu;
+  constexpr int LD = MMAX + 2;                  // columns start on 16 bytes
+  const int j = threadIdx.x & (T - 1);          // lane of the group
+  int gs = 0, m = 0, ib = 0, ie = 0;
+  if (i >= 0) {
+    gs = __ldg(grp + i);
+    m = __ldg(grp + i + 1) - gs - 1;            // strictly-lower entries
+    ib = __ldg(arp + i);
+    ie = __ldg(arp + i + 1);
+  }
+  const int mw = __reduce_max_sync(FULL, m);    // of the warp's rows
+  const bool live = j < m;
+  int pj = 0, rb = 0, re = 0;
+  if (live) {
+    pj = __ldg(gci + gs + j);
+    rb = __ldg(arp + pj);
+    re = __ldg(arp + pj + 1);
+  }
+  // -A[i, P[j]] and a_ii
+  double y = 0.0, aii = 0.0;
+  bool have_diag = false;
+  {
+    int lo[2] = {ib, ib};
+    const int hi[2] = {live ? ie : ib, ie}, col[2] = {pj, i};
+    find_cols<2>(aci, lo, hi, col);
+    if (lo[0] >= 0) y = -__ldg(av + lo[0]);
+    if (lo[1] >= 0) {
+      aii = __ldg(av + lo[1]);
+      have_diag = true;
+    }
+  }
+  const double rhs = y;
+  // A[P[a], P[b]], a <= b, into S[b][a]
+  for (int s0 = 0; 2 * s0 <= mw; s0 += 4) {
+    int lo[4], hi[4], col[4], at[4];
+#pragma unroll
+    for (int u = 0; u < 4; ++u) {
+      const int s = s0 + u;
+      const bool on = live && 2 * s <= m;
+      int b = j + s;
+      if (b >= m) b -= m;
+      if (!on) b = j;
+      const int pb = __shfl_sync(FULL, pj, b, T), rbb = __shfl_sync(FULL, rb, b, T),
+                reb = __shfl_sync(FULL, re, b, T);
+      const bool up = j <= b;                   // row P[j], column P[b]
+      lo[u] = on ? (up ? rb : rbb) : 0;
+      hi[u] = on ? (up ? re : reb) : 0;
+      col[u] = up ? pb : pj;
+      at[u] = on ? (up ? b * LD + j : j * LD + b) : -1;
+    }
+    find_cols<4>(aci, lo, hi, col);
+#pragma unroll
+    for (int u = 0; u < 4; ++u)
+      if (at[u] >= 0) S[at[u]] = lo[u] >= 0 ? __ldg(av + lo[u]) : 0.0;
+  }
+  __syncwarp();
+  double R[MMAX];
+#pragma unroll
+  for (int l = 0; l < MMAX; ++l) R[l] = (live && l <= j) ? S[j * LD + l] : (l == j ? 1.0 : 0.0);
+  __syncwarp();                                 // S becomes the columns of L
+  bool spd = true;
+  double dinv = 1.0;                            // 1 / pivot of this lane's step
+#pragma unroll
+  for (int k = 0; k < MMAX; ++k) {
+    if (k < mw) {                               // warp-uniform
+      const double d = __shfl_sync(FULL, R[k], k, T);
+      if (k < m && !(d > 0.0)) spd = false;
+      const double inv = 1.0 / d;
+      const double mine = R[k];                 // before scaling
+      const double l_jk = mine * inv;
+      const double zk = __shfl_sync(FULL, y, k, T);
+      if (j > k) y = fma(-l_jk, zk, y);
+      if (j == k) dinv = inv;
+      if (j < MMAX) S[k * LD + j] = l_jk;
+      __syncwarp();
+#pragma unroll
+      for (int l = (k + 1) & ~1; l < MMAX; l += 2) {
+        const double2 v = *reinterpret_cast<const double2 *>(S + k * LD + l);
+        if (l > k) R[l] = fma(-mine, v.x, R[l]);
+        R[l + 1] = fma(-mine, v.y, R[l + 1]);
+      }
+    }
+  }
+  y *= dinv;
+#pragma unroll
+  for (int k = MMAX - 1; k > 0; --k) {          // L' y = D^-1 z
+    if (k < mw) {
+      const double yk = __shfl_sync(FULL, y, k, T);
+      if (j < k && k < m) y = fma(-S[j * LD + k], yk, y);
+    }
+  }
+  double part = live ? rhs * y : 0.0;
+#pragma unroll
+  for (int o = T / 2; o > 0; o >>= 1) part += __shfl_xor_sync(FULL, part, o, T);
+  double scal = aii - part;
+  const bool ok = spd && have_diag && scal > 0.0;
+  if (i < 0) return;
+  if (!ok) {
+    if (j == 0) atomicOr(flags, 1);
+    scal = 1.0;
+    if (!spd) y = 0.0;                          // keep a defined row: diagonal scaling only
+  }
+  const double s = 1.0 / sqrt(scal);
+  if (live) gval[gs + j] = s * y;
+  if (j == 0) gval[gs + m] = s;
+}
+
+// Lanes per row of a tile of MMAX unknowns (0: a warp per row with the
+// shared-memory factor of fsai_row), warps per block, and shared memory of
+// the block.
+__host__ __device__ constexpr int fsai_lanes(int mmax) {
+  return mmax <= 4 ? 4 : mmax <= 8 ? 8 : mmax <= 16 ? 16 : mmax <= 32 ? 32 : 0;
+}
+__host__ __device__ constexpr int fsai_warps(int mmax) { return mmax <= 16 ? 8 : mmax <= 32 ? 4 : 2; }
+__host__ __device__ constexpr int fsai_group_doubles(int mmax) {
+  return mmax <= 32 ? mmax * (mmax + 2) : mmax * mmax + 3 * mmax;
+}
+__host__ __device__ constexpr int fsai_rows_per_block(int mmax) {
+  return fsai_lanes(mmax) ? fsai_warps(mmax) * 32 / fsai_lanes(mmax) : fsai_warps(mmax);
+}
+constexpr size_t fsai_smem(int mmax) {
+  return (size_t)fsai_rows_per_block(mmax) * fsai_group_doubles(mmax) * sizeof(double);
+}
+
 template <int MMAX>
-__global__ void k_fsai_numeric(int nb, const int *__restrict__ rows, const int *__restrict__ arp,
-                               const int *__restrict__ aci, const double *__restrict__ av,
-                               const int *__restrict__ grp, const int *__restrict__ gci,
-                               double *__restrict__ gval, int *flags) {
-  extern __shared__ double smem[];
-  constexpr int STRIDE = MMAX * MMAX + 3 * MMAX;
-  const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
-  const int wglob = blockIdx.x * (blockDim.x >> 5) + wib;
-  if (wglob >= nb) return;                      // warp-uniform exit
-  fsai_row<MMAX>(rows[wglob], arp, aci, av, grp, gci, gval, flags, smem + (size_t)wib * STRIDE,
-                 lane);
+__device__ __forceinline__ void fsai_block_row(int i, const int *arp, const int *aci,
+                                               const double *av, const int *grp, const int *gci,
+                                               double *gval, int *flags, double *smem) {
+  constexpr int T = fsai_lanes(MMAX);
+  if constexpr (T > 0)
+    fsai_row_reg<T, MMAX>(i, arp, aci, av, grp, gci, gval, flags,
+                          smem + (threadIdx.x / T) * fsai_group_doubles(MMAX));
+  else if (i >= 0)
+    fsai_row<MMAX>(i, arp, aci, av, grp, gci, gval, flags,
+                   smem + (threadIdx.x >> 5) * fsai_group_doubles(MMAX), threadIdx.x & 31);
+}
+
+// Entry of the list that a thread's group works on, or -1 past its end.
+template <int MMAX> __device__ __forceinline__ int fsai_list_entry(int nb) {
+  constexpr int T = fsai_lanes(MMAX) ? fsai_lanes(MMAX) : 32;
+  const int64_t q = blockIdx.x * (int64_t)fsai_rows_per_block(MMAX) + threadIdx.x / T;
+  return q < nb ? (int)q : -1;
+}
+
+template <int MMAX>
+__global__ void __launch_bounds__(fsai_warps(MMAX) * 32)
+k_fsai_numeric(int nb, const int *__restrict__ rows, const int *__restrict__ arp,
+               const int *__restrict__ aci, const double *__restrict__ av,
+               const int *__restrict__ grp, const int *__restrict__ gci,
+               double *__restrict__ gval, int *flags) {
+  extern __shared__ __align__(16) double smem[];
+  const int q = fsai_list_entry<MMAX>(nb);
+  fsai_block_row<MMAX>(q >= 0 ? rows[q] : -1, arp, aci, av, grp, gci, gval, flags, smem);
+}
+
+template <int MMAX>
+static void launch_fsai(int cnt, const int *rows, const int *arp, const int *aci, const double *av,
+                        const int *grp, const int *gci, double *gval, int *flags,
+                        cudaStream_t st) {
+  if (cnt <= 0) return;
+  CHRONOS_CUDA(cudaFuncSetAttribute(k_fsai_numeric<MMAX>,
+                                    cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                    (int)fsai_smem(MMAX)));
+  k_fsai_numeric<MMAX><<<ceil_div(cnt, fsai_rows_per_block(MMAX)), fsai_warps(MMAX) * 32,
+                         fsai_smem(MMAX), st>>>(cnt, rows, arp, aci, av, grp, gci, gval, flags);
+  CHRONOS_CHECK_LAUNCH();
+}
+
+// The buckets of fsai_numeric_device and fsai_numeric_noalloc: local systems
+// of at most 4, 8, 16, 32 and 64 unknowns.
+constexpr int kFsaiBuckets = 5;
+__host__ __device__ constexpr int fsai_bucket(int m) {
+  return m <= 4 ? 0 : m <= 8 ? 1 : m <= 16 ? 2 : m <= 32 ? 3 : 4;
+}
+static void launch_fsai_bucket(int b, int cnt, const int *rows, const int *arp, const int *aci,
+                               const double *av, const int *grp, const int *gci, double *gval,
+                               int *flags, cudaStream_t st) {
+  switch (b) {
+    case 0: launch_fsai<4>(cnt, rows, arp, aci, av, grp, gci, gval, flags, st); break;
+    case 1: launch_fsai<8>(cnt, rows, arp, aci, av, grp, gci, gval, flags, st); break;
+    case 2: launch_fsai<16>(cnt, rows, arp, aci, av, grp, gci, gval, flags, st); break;
+    case 3: launch_fsai<32>(cnt, rows, arp, aci, av, grp, gci, gval, flags, st); break;
+    default: launch_fsai<64>(cnt, rows, arp, aci, av, grp, gci, gval, flags, st); break;
+  }
 }
 
 // One problem of a batched FSAI numeric launch (device pointers).
@@ -158,47 +391,34 @@ struct FsaiProblemDev {
 // The rows of many problems in one launch: item k = (problem, row); flags
 // per problem.
 template <int MMAX>
-__global__ void k_fsai_numeric_batched(int nb, const int2 *__restrict__ items,
-                                       const FsaiProblemDev *__restrict__ tab, int *flags) {
-  extern __shared__ double smem[];
-  constexpr int STRIDE = MMAX * MMAX + 3 * MMAX;
-  const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
-  const int wglob = blockIdx.x * (blockDim.x >> 5) + wib;
-  if (wglob >= nb) return;                      // warp-uniform exit
-  const int2 it = items[wglob];
+__global__ void __launch_bounds__(fsai_warps(MMAX) * 32)
+k_fsai_numeric_batched(int nb, const int2 *__restrict__ items,
+                       const FsaiProblemDev *__restrict__ tab, int *flags) {
+  extern __shared__ __align__(16) double smem[];
+  const int q = fsai_list_entry<MMAX>(nb);
+  const int2 it = q >= 0 ? items[q] : make_int2(0, -1);
   const FsaiProblemDev pr = tab[it.x];
-  fsai_row<MMAX>(it.y, pr.arp, pr.aci, pr.av, pr.grp, pr.gci, pr.gval, flags + it.x,
-                 smem + (size_t)wib * STRIDE, lane);
+  fsai_block_row<MMAX>(it.y, pr.arp, pr.aci, pr.av, pr.grp, pr.gci, pr.gval, flags + it.x, smem);
 }
 
 int fsai_numeric_device(int n, const int *arp, const int *aci, const double *av, const int *grp,
                         const int *gci, double *gval, const std::vector<int> &rowlen_h,
                         cudaStream_t st) {
   // Bucket rows by local system size m = rowlen - 1.
-  std::vector<int> b16, b32, b64;
+  std::vector<int> rows[kFsaiBuckets];
   for (int i = 0; i < n; ++i) {
     const int m = rowlen_h[i] - 1;
-    if (m <= 16) b16.push_back(i);
-    else if (m <= 32) b32.push_back(i);
-    else if (m <= 64) b64.push_back(i);
-    else throw Error(CHRONOS_ENOTSUP, "FSAI local system larger than 64 (nstep*step_size)");
+    CHRONOS_REQUIRE(m <= 64, CHRONOS_ENOTSUP, "FSAI local system larger than 64 (nstep*step_size)");
+    rows[fsai_bucket(m)].push_back(i);
   }
   DBuf<int> flags(1);
   flags.zero(st);
-  DBuf<int> d16, d32, d64;
-  auto run = [&](auto kern, const std::vector<int> &rows, DBuf<int> &drows, int mmax, int warps) {
-    if (rows.empty()) return;
-    drows.upload(rows, st);
-    const size_t sm = (size_t)warps * (mmax * mmax + 3 * mmax) * sizeof(double);
-    CHRONOS_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm));
-    const unsigned blocks = ceil_div((int64_t)rows.size(), warps);
-    kern<<<blocks, warps * 32, sm, st>>>((int)rows.size(), drows.get(), arp, aci, av, grp, gci,
-                                         gval, flags.get());
-    CHRONOS_CHECK_LAUNCH();
-  };
-  run(k_fsai_numeric<16>, b16, d16, 16, 8);
-  run(k_fsai_numeric<32>, b32, d32, 32, 4);
-  run(k_fsai_numeric<64>, b64, d64, 64, 2);
+  DBuf<int> drows[kFsaiBuckets];
+  for (int b = 0; b < kFsaiBuckets; ++b) {
+    drows[b].upload(rows[b], st);
+    launch_fsai_bucket(b, (int)rows[b].size(), drows[b].get(), arp, aci, av, grp, gci, gval,
+                       flags.get(), st);
+  }
   int fl = 0;
   CHRONOS_CUDA(cudaMemcpyAsync(&fl, flags.get(), sizeof(int), cudaMemcpyDeviceToHost, st));
   CHRONOS_CUDA(cudaStreamSynchronize(st));
@@ -223,19 +443,15 @@ const std::vector<std::vector<int>> &fsai_bucket_sets() {
   return sets;
 }
 
-// warps per block of a tile size (shared memory: warps * (MMAX^2 + 3 MMAX) doubles)
-int fsai_tile_warps(int mmax) { return mmax <= 24 ? 8 : mmax <= 32 ? 4 : 2; }
-
 template <int MMAX>
 void launch_fsai_batched(int cnt, const int2 *items, const FsaiProblemDev *tab, int *flags,
                          cudaStream_t st) {
   if (cnt == 0) return;
-  const int warps = fsai_tile_warps(MMAX);
-  const size_t sm = (size_t)warps * (MMAX * MMAX + 3 * MMAX) * sizeof(double);
   CHRONOS_CUDA(cudaFuncSetAttribute(k_fsai_numeric_batched<MMAX>,
-                                    cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm));
-  k_fsai_numeric_batched<MMAX><<<ceil_div(cnt, warps), warps * 32, sm, st>>>(cnt, items, tab,
-                                                                            flags);
+                                    cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                    (int)fsai_smem(MMAX)));
+  k_fsai_numeric_batched<MMAX><<<ceil_div(cnt, fsai_rows_per_block(MMAX)), fsai_warps(MMAX) * 32,
+                                 fsai_smem(MMAX), st>>>(cnt, items, tab, flags);
   CHRONOS_CHECK_LAUNCH();
 }
 
@@ -1059,7 +1275,7 @@ void adjoint_scatter(int n, const int *rp, const int *ci, const double *lambda, 
 // FSAI numeric phase without allocation (chronos_fsai_numeric_noalloc)
 // =============================================================================
 //
-// Same kernels as fsai_numeric_device, but the scratch they need -- the three
+// Same kernels as fsai_numeric_device, but the scratch they need -- the
 // row-bucket lists and the flag word -- lives in one file-scope device array
 // instead of cudaMalloc'd buffers.  The array is a fixed 12 MiB + 256 B per
 // device that loads the library, held until the process exits.  Every call
@@ -1067,7 +1283,7 @@ void adjoint_scatter(int n, const int *rp, const int *ci, const double *lambda, 
 // race on it and must be serialised by the caller.
 
 constexpr int kNoAllocMaxRows = 1 << 20;
-constexpr int kNoAllocHeader = 64;            // ints: [0..2] bucket counts, [3] flags
+constexpr int kNoAllocHeader = 64;            // ints: [0..4] bucket counts, [5] flags
 static __device__ __align__(256) int g_fsai_noalloc_scratch[kNoAllocHeader + 3 * kNoAllocMaxRows];
 
 // In host code g_fsai_noalloc_scratch names a host-side stand-in, not a device
@@ -1089,7 +1305,15 @@ static int *noalloc_scratch_address() {
   return g_noalloc_addr[dev];
 }
 
-// Checks row i of both patterns and sorts it into the 16 / 32 / 64 buckets of
+// Place of entry pos of bucket b: three lists of kNoAllocMaxRows ints; buckets
+// 3 and 4 fill the first two from their ends (the buckets hold n <=
+// kNoAllocMaxRows rows together, so they never meet).
+__host__ __device__ constexpr int noalloc_slot(int b, int pos) {
+  return kNoAllocHeader + (b < 3 ? b * kNoAllocMaxRows + pos
+                                 : (b - 2) * kNoAllocMaxRows - 1 - pos);
+}
+
+// Checks row i of both patterns and sorts it into the buckets of
 // fsai_numeric_device.  The numeric kernel indexes A's rows by G's columns and
 // writes G's row at gval[grp[i] .. grp[i+1]-1] with the diagonal last, so a
 // malformed row sets flag bit 2 (and is not bucketed): a G row without
@@ -1097,37 +1321,48 @@ static int *noalloc_scratch_address() {
 // or outside [0, i); an A row whose pointers decrease or whose columns are not
 // ascending inside [0, n); row pointers of either that do not start at 0.
 // A row longer than 64 strictly-lower entries sets flag bit 1.
-__global__ void k_fsai_bucket_rows(int n, const int *__restrict__ arp, const int *__restrict__ aci,
-                                   const int *__restrict__ grp, const int *__restrict__ gci,
-                                   int *scratch) {
+// A warp's rows of one bucket take their places with one atomic: an atomic
+// per row on five counters was the whole time of this kernel (227k rows:
+// 155 us).
+__global__ void __launch_bounds__(256)
+k_fsai_bucket_rows(int n, const int *__restrict__ arp, const int *__restrict__ aci,
+                   const int *__restrict__ grp, const int *__restrict__ gci, int *scratch) {
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= n) return;
-  const int gs = grp[i], ge = grp[i + 1];
-  bool bad = ge <= gs || (i == 0 && (gs != 0 || arp[0] != 0));
-  if (!bad) {
-    bad = gci[ge - 1] != i;
-    for (int k = gs, prev = -1; !bad && k < ge - 1; ++k) {
-      const int c = gci[k];
-      bad = c <= prev || c >= i;
+  const int lane = threadIdx.x & 31;
+  int b = -1, flag = 0;
+  if (i < n) {
+    const int gs = grp[i], ge = grp[i + 1];
+    bool bad = ge <= gs || (i == 0 && (gs != 0 || arp[0] != 0));
+    if (!bad) {
+      bad = gci[ge - 1] != i;
+      for (int k = gs, prev = -1; !bad && k < ge - 1; ++k) {
+        const int c = gci[k];
+        bad = c <= prev || c >= i;
+        prev = c;
+      }
+    }
+    const int as = arp[i], ae = arp[i + 1];
+    bad = bad || ae < as;
+    for (int k = as, prev = -1; !bad && k < ae; ++k) {
+      const int c = aci[k];
+      bad = c <= prev || c >= n;
       prev = c;
     }
+    const int m = ge - gs - 1;
+    if (bad) flag = 4;
+    else if (m > 64) flag = 2;
+    else b = fsai_bucket(m);
   }
-  const int as = arp[i], ae = arp[i + 1];
-  bad = bad || ae < as;
-  for (int k = as, prev = -1; !bad && k < ae; ++k) {
-    const int c = aci[k];
-    bad = c <= prev || c >= n;
-    prev = c;
+  if (flag) atomicOr(scratch + kFsaiBuckets, flag);
+#pragma unroll
+  for (int q = 0; q < kFsaiBuckets; ++q) {
+    const unsigned in = __ballot_sync(0xffffffffu, b == q);
+    if (!in) continue;
+    int base = 0;
+    if (lane == __ffs(in) - 1) base = atomicAdd(scratch + q, __popc(in));
+    base = __shfl_sync(0xffffffffu, base, __ffs(in) - 1);
+    if (b == q) scratch[noalloc_slot(q, base + __popc(in & ((1u << lane) - 1u)))] = i;
   }
-  if (bad) { atomicOr(scratch + 3, 4); return; }
-  const int m = ge - gs - 1;
-  int b;
-  if (m <= 16) b = 0;
-  else if (m <= 32) b = 1;
-  else if (m <= 64) b = 2;
-  else { atomicOr(scratch + 3, 2); return; }
-  const int pos = atomicAdd(scratch + b, 1);
-  scratch[kNoAllocHeader + b * kNoAllocMaxRows + pos] = i;
 }
 
 int fsai_numeric_noalloc(int n, const int *arp, const int *aci, const double *av, const int *grp,
@@ -1140,30 +1375,22 @@ int fsai_numeric_noalloc(int n, const int *arp, const int *aci, const double *av
   CHRONOS_CUDA(cudaMemsetAsync(scr, 0, kNoAllocHeader * sizeof(int), st));
   k_fsai_bucket_rows<<<ceil_div(n, 256), 256, 0, st>>>(n, arp, aci, grp, gci, scr);
   CHRONOS_CHECK_LAUNCH();
-  int hdr[4] = {0, 0, 0, 0};
+  int hdr[kFsaiBuckets + 1] = {};
   CHRONOS_CUDA(cudaMemcpyAsync(hdr, scr, sizeof(hdr), cudaMemcpyDeviceToHost, st));
   CHRONOS_CUDA(cudaStreamSynchronize(st));
   // no numeric kernel runs on a malformed pattern: it would read A and write
   // G's values outside the rows the caller's buffers hold
-  CHRONOS_REQUIRE(!(hdr[3] & 4), CHRONOS_EINVAL,
+  CHRONOS_REQUIRE(!(hdr[kFsaiBuckets] & 4), CHRONOS_EINVAL,
                   "malformed CSR: a G row is empty, does not end with its diagonal or has "
                   "strictly-lower columns not ascending in [0, i); or A's row pointers / "
                   "columns are not a sorted 0-based CSR");
-  CHRONOS_REQUIRE(!(hdr[3] & 2), CHRONOS_ENOTSUP,
+  CHRONOS_REQUIRE(!(hdr[kFsaiBuckets] & 2), CHRONOS_ENOTSUP,
                   "FSAI local system larger than 64 (nstep*step_size)");
-  auto run = [&](auto kern, int cnt, int bucket, int mmax, int warps) {
-    if (cnt == 0) return;
-    const size_t sm = (size_t)warps * (mmax * mmax + 3 * mmax) * sizeof(double);
-    CHRONOS_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm));
-    kern<<<ceil_div(cnt, warps), warps * 32, sm, st>>>(
-        cnt, scr + kNoAllocHeader + bucket * kNoAllocMaxRows, arp, aci, av, grp, gci, gval, scr + 3);
-    CHRONOS_CHECK_LAUNCH();
-  };
-  run(k_fsai_numeric<16>, hdr[0], 0, 16, 8);
-  run(k_fsai_numeric<32>, hdr[1], 1, 32, 4);
-  run(k_fsai_numeric<64>, hdr[2], 2, 64, 2);
+  for (int b = 0; b < kFsaiBuckets; ++b)       // a list from the end: its lowest address
+    launch_fsai_bucket(b, hdr[b], scr + (b < 3 ? noalloc_slot(b, 0) : noalloc_slot(b, hdr[b] - 1)),
+                       arp, aci, av, grp, gci, gval, scr + kFsaiBuckets, st);
   int fl = 0;
-  CHRONOS_CUDA(cudaMemcpyAsync(&fl, scr + 3, sizeof(int), cudaMemcpyDeviceToHost, st));
+  CHRONOS_CUDA(cudaMemcpyAsync(&fl, scr + kFsaiBuckets, sizeof(int), cudaMemcpyDeviceToHost, st));
   CHRONOS_CUDA(cudaStreamSynchronize(st));
   return fl;
 }

@@ -1,0 +1,79 @@
+"""Kernel variants at the edges of their ranges, against plain numpy."""
+import numpy as np
+import pytest
+import scipy.sparse as sp
+
+import chronoslab_b200 as cb
+
+pytestmark = pytest.mark.gpu
+
+
+def _banded_spd(n, band, seed):
+    """Diagonally dominant SPD matrix with `band` sub-diagonals, some entries
+    left out (the local systems then hold zeros)."""
+    rng = np.random.default_rng(seed)
+    A = sp.lil_matrix((n, n))
+    for d in range(1, band + 1):
+        v = rng.uniform(-1.0, 1.0, n - d) * (rng.random(n - d) < 0.7)
+        A.setdiag(v, -d)
+    A = sp.csr_matrix(A)
+    A = A + A.T
+    A = A + sp.diags(1.1 * np.asarray(abs(A).sum(1)).ravel() + 1.0)
+    A = sp.csr_matrix(A)
+    A.sort_indices()
+    return A
+
+
+@pytest.mark.parametrize("sizes", [[0, 1, 2, 3, 4], [4, 5, 7, 8], [8, 9, 15, 16], [16, 17, 31, 32],
+                                   [32, 33, 63, 64], list(range(65))])
+def test_fsai_local_systems_of_every_tile(lib, sizes):
+    """Rows of G of the given local sizes, mixed within warps: each row equals
+    y = -A[P,P]^-1 A[P,i] scaled by 1/sqrt(a_ii + A[i,P] y).  The local systems
+    are diagonally dominant (condition below 50), so 64 unknowns give at most
+    about 64 * 50 * 2.2e-16 = 7e-13 of the row's largest entry."""
+    n = 400
+    A = _banded_spd(n, 70, 5)
+    rng = np.random.default_rng(1)
+    rows, cols = [], []
+    for i in range(n):
+        m = min(sizes[int(rng.integers(len(sizes)))], i)
+        P = np.sort(rng.choice(np.arange(max(0, i - 90), i), m, replace=False)) if m else []
+        rows += [i] * (m + 1)
+        cols += list(P) + [i]
+    indptr = np.concatenate([[0], np.cumsum(np.bincount(rows, minlength=n))])
+    G = sp.csr_matrix((np.ones(len(cols)), np.array(cols), indptr), shape=(n, n))
+    vals, ok = cb.fsai_numeric(A, G)
+    assert ok
+    D = A.toarray()
+    for i in range(n):
+        c = G.indices[indptr[i]:indptr[i + 1]]
+        P = c[:-1]
+        y = -np.linalg.solve(D[np.ix_(P, P)], D[P, i])
+        row = np.append(y, 1.0) / np.sqrt(D[i, i] + D[i, P] @ y)
+        got = vals[indptr[i]:indptr[i + 1]]
+        assert np.abs(got - row).max() <= 1e-12 * np.abs(row).max(), (i, len(P))
+
+
+@pytest.mark.parametrize("m", [3, 8, 15, 16, 32, 40])
+def test_fsai_indefinite_local_system(lib, m):
+    """A local system with a negative pivot in its middle: is_posdef 0, that
+    row the unit row, the others as if alone."""
+    n = m + 90
+    A = _banded_spd(n, 70, 9)
+    bad = A.copy()
+    k = m // 2
+    bad[k, k] = -bad[k, k]
+    bad = sp.csr_matrix(bad)
+    bad.sort_indices()
+    # rows before m diagonal only; row m takes all columns before it; the
+    # rows after it the three before them
+    cols = [[i] for i in range(m)] + [list(range(m + 1))]
+    cols += [list(range(i - 3, i + 1)) if i - 3 > k else [i] for i in range(m + 1, n)]
+    indptr = np.concatenate([[0], np.cumsum([len(c) for c in cols])])
+    G = sp.csr_matrix((np.ones(indptr[-1]), np.concatenate(cols), indptr), shape=(n, n))
+    good_vals, good = cb.fsai_numeric(A, G)
+    vals, ok = cb.fsai_numeric(bad, G)
+    assert good and not ok
+    s, e = indptr[m], indptr[m + 1]
+    assert np.array_equal(vals[s:e], np.append(np.zeros(m), 1.0))
+    assert np.array_equal(vals[e:], good_vals[e:])
