@@ -667,13 +667,18 @@ class Hierarchy:
     def pcg_block(self, B, X0=None, itmax=1000, tol=1e-8, stream=None):
         B = np.asarray(B, dtype=np.float64)
         nrhs = B.shape[1]
-        bc = np.ascontiguousarray(B.T).ravel()
-        xc = np.zeros_like(bc) if X0 is None else np.ascontiguousarray(np.asarray(X0).T).ravel()
+        # either memory order goes to the GPU as it lies; blocks of more than
+        # the library's 16 columns a solve by columns
+        rows = nrhs <= 16 and not B.flags.f_contiguous
+        bc = np.ascontiguousarray(B if rows else B.T)
+        x0 = None if X0 is None else np.ascontiguousarray(np.asarray(X0, dtype=np.float64).T)
+        xc = np.empty(nrhs * self.n)
         its = np.zeros(nrhs, np.int32)
         fl = np.zeros(nrhs, np.int32)
         sec = C.c_double()
-        check(self._lib.chronos_pcg_block(self._h, nrhs, _pd(bc), _pd(xc), itmax, tol, _pi(its),
-                                          _pi(fl), C.byref(sec), _stream(stream)))
+        check(self._lib.chronos_pcg_block_rows(
+            self._h, nrhs, _pd(bc), int(rows), None if x0 is None else _pd(x0), _pd(xc), itmax,
+            tol, _pi(its), _pi(fl), C.byref(sec), _stream(stream)))
         return xc.reshape(nrhs, self.n).T, its, fl, sec.value
 
     def sqmr(self, b, tol=1e-6, itmax=100, x0=None, A=None):

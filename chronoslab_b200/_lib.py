@@ -140,6 +140,7 @@ SIGNATURES = {
     "chronos_pcg": [_vp, _pi, _pi, _pd, _pd, _pd, _i, _d, _pi, _pd, _pi, _pd, _vp],
     "chronos_pcg_dev": [_vp, _vp, _vp, _i, _d, _pi, _pd, _pi, _pd, _vp],
     "chronos_pcg_block": [_vp, _i, _pd, _pd, _i, _d, _pi, _pi, _pd, _vp],
+    "chronos_pcg_block_rows": [_vp, _i, _pd, _i, _pd, _pd, _i, _d, _pi, _pi, _pd, _vp],
     "chronos_batch_setup": [C.POINTER(chronos_params), _i, _pi, _pp, _pp, _pp, _pp],
     "chronos_batch_solve": [_vp, _pp, _pp, _i, _d, _pi, _pi, _pd],
     "chronos_batch_info": [_vp, _i, _pi, _pi],

@@ -1,9 +1,9 @@
 // Block of K right-hand sides solved together: SpMM V-cycles and K independent
 // PCG_CJ recurrences (PCG_CJ.m:34-66 per column) in one CUDA graph.
 //
-// Vectors are row-major n x K (X[i*K + j]).  In the SpMM kernel K consecutive
-// lanes own one row, lane j its column j: every stored value and column index
-// is fetched once (a broadcast to the K lanes) and reused K times, and the
+// Vectors are row-major n x K (X[i*K + j]).  In the SpMM kernel K/VEC
+// consecutive lanes own one row, each lane VEC columns: every stored value and
+// column index is fetched once (a broadcast) and reused K times, and the
 // gathers X[c*K + 0..K-1] are K-wide coalesced loads.  Each column keeps its
 // own scalars, iteration count and stopping test; a converged column is frozen
 // (its x, res and p no longer change), so every column returns exactly what a
@@ -19,9 +19,11 @@ namespace chronos {
 
 template <int K> struct StoreK {
   double *dst;
-  __device__ void operator()(const double *t) const {
-    for (int q = 0; q < K; ++q) dst[q] = t[q];
+  __device__ bool operator()(int j, const double *t) const {
+    dst[j] = t[j];
+    return false;
   }
+  __device__ void done(bool) const {}
 };
 
 // VEC consecutive elements as one 8- or 16-byte access (aligned: K is a
@@ -56,34 +58,44 @@ template <> struct Vec<double, 2> {
 };
 
 // Lanes own VEC consecutive right-hand-side columns of one row: K/VEC lanes
-// per row, 32*VEC/K rows per warp; each stored value and column index is
-// fetched once per row group and applied to K columns.
-template <typename VT, typename XT, typename ZT, typename YT, int K, int VEC, int MODE, bool DOT>
+// per row; each stored value and column index is fetched once per row group
+// and applied to K columns.  split (a power of two, K/VEC*split <= 32) lane
+// sets share a row's entries, set s taking entries s, s+split, ...: a coarse
+// level has too few rows to fill the GPU and its time is one row's chain of
+// loads (spmm_split).
+template <typename VT, typename XT, typename ZT, typename YT, int K, int VEC, int MODE, bool DOT,
+          bool SPLIT>
 __global__ void __launch_bounds__(kApplyThreads)
-k_csr_spmm(int n, const int *__restrict__ rp, const int *__restrict__ ci,
+k_csr_spmm(int n, int split_arg, const int *__restrict__ rp, const int *__restrict__ ci,
            const VT *__restrict__ v, const XT *__restrict__ X, const ZT *Z, YT *Y, VT alpha,
            const double *__restrict__ DW, double *part, unsigned *ticket, double *dot_out) {
+  pdl_begin();
   constexpr int LPR = K / VEC;
-  constexpr int R = 32 / LPR;
-  const int lane = threadIdx.x & 31, g = lane / LPR, j0 = (lane % LPR) * VEC;
+  const int split = SPLIT ? split_arg : 1;
+  const int per_row = LPR * split, R = 32 / per_row;
+  const int lane = threadIdx.x & 31, g = lane / per_row, j0 = (lane % LPR) * VEC;
+  const int part_of = (lane / LPR) & (split - 1);
   const int warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   const int nwarps = (gridDim.x * blockDim.x) >> 5;
   double dacc[VEC];
 #pragma unroll
   for (int e = 0; e < VEC; ++e) dacc[e] = 0.0;
-  for (int base = warp * R; base < n; base += nwarps * R) {
+  for (int base = warp * R; base < n; base += nwarps * R) {     // warp-uniform trip count
     const int row = base + g;
-    if (row < n) {
-      VT s[VEC];
+    VT s[VEC];
 #pragma unroll
-      for (int e = 0; e < VEC; ++e) s[e] = VT(0);
+    for (int e = 0; e < VEC; ++e) s[e] = VT(0);
+    if (row < n) {
       const int e1 = __ldg(rp + row + 1);
-      int k = __ldg(rp + row);
-      for (; k + 3 < e1; k += 4) {            // four entries' loads in flight
+      int k = __ldg(rp + row) + part_of;
+      for (; k + 3 * split < e1; k += 4 * split) {   // four entries' loads in flight
         int c[4];
         VT a[4];
 #pragma unroll
-        for (int u = 0; u < 4; ++u) { c[u] = __ldg(ci + k + u); a[u] = __ldg(v + k + u); }
+        for (int u = 0; u < 4; ++u) {
+          c[u] = __ldg(ci + k + u * split);
+          a[u] = __ldg(v + k + u * split);
+        }
         XT xv[4][VEC];
 #pragma unroll
         for (int u = 0; u < 4; ++u) Vec<XT, VEC>::ld(X + (size_t)c[u] * K + j0, xv[u]);
@@ -92,13 +104,31 @@ k_csr_spmm(int n, const int *__restrict__ rp, const int *__restrict__ ci,
 #pragma unroll
           for (int e = 0; e < VEC; ++e) s[e] += a[u] * (VT)xv[u][e];
       }
-      for (; k < e1; ++k) {
-        const VT a = __ldg(v + k);
-        XT xv[VEC];
-        Vec<XT, VEC>::ld(X + (size_t)__ldg(ci + k) * K + j0, xv);
+      if (k < e1) {        // the last 1..3 entries: loads clamped to the first, sums selected
+        int c[3];
+        VT a[3];
 #pragma unroll
-        for (int e = 0; e < VEC; ++e) s[e] += a * (VT)xv[e];
+        for (int u = 0; u < 3; ++u) {
+          const int ku = k + u * split < e1 ? k + u * split : k;
+          c[u] = __ldg(ci + ku);
+          a[u] = __ldg(v + ku);
+        }
+        XT xv[3][VEC];
+#pragma unroll
+        for (int u = 0; u < 3; ++u) Vec<XT, VEC>::ld(X + (size_t)c[u] * K + j0, xv[u]);
+#pragma unroll
+        for (int u = 0; u < 3; ++u)
+#pragma unroll
+          for (int e = 0; e < VEC; ++e) {
+            const VT t = s[e] + a[u] * (VT)xv[u][e];
+            s[e] = k + u * split < e1 ? t : s[e];
+          }
       }
+    }
+    for (int o = LPR; o < per_row; o <<= 1)
+#pragma unroll
+      for (int e = 0; e < VEC; ++e) s[e] += __shfl_xor_sync(0xffffffffu, s[e], o);
+    if (row < n && part_of == 0) {
       const size_t o = (size_t)row * K + j0;
       ZT zv[VEC];
       if (MODE == MODE_RESID || MODE == MODE_AXPY) Vec<ZT, VEC>::ld(Z + o, zv);
@@ -131,6 +161,21 @@ struct SpmmVec {
   static constexpr int value = v4 > K ? K : v4;
 };
 
+// Lane sets sharing a row: doubled while the rows with twice the lanes still
+// fit the GPU's resident threads and every set keeps at least four entries
+// (one batch of loads in flight).  Diffusion 64^3, 16 columns, residual on the
+// levels of 97,128 / 21,463 / 4,851 rows (11-13 entries a row): 6.9 / 6.5 / 5.5 us
+// unsplit, 5.9 / 4.6 / 4.1 us; on the finest level (262,144 rows of 7 entries)
+// the split form's runtime strides cost more than they give (35 against 22 us).
+inline int spmm_split(const DMat &M, int lanes_per_row) {
+  const int64_t resident = (int64_t)num_sms() * 2048;
+  int s = 1;
+  while (2 * s * lanes_per_row <= 32 && (int64_t)M.nrows * lanes_per_row * 2 * s <= resident &&
+         M.nnz >= (int64_t)M.nrows * 4 * s)
+    s *= 2;
+  return s;
+}
+
 template <typename VT, typename XT, typename ZT, typename YT, int K, int MODE, bool DOT>
 static void spmm(cudaStream_t st, const DMat &M, const VT *vals, const XT *X, const ZT *Z, YT *Y,
                  VT alpha, const double *DW = nullptr, double *part = nullptr,
@@ -138,11 +183,14 @@ static void spmm(cudaStream_t st, const DMat &M, const VT *vals, const XT *X, co
   constexpr int VEC = SpmmVec<XT, ZT, YT, K>::value;
   const int n = M.nrows;
   if (n <= 0) return;
-  const int rows_per_block = kApplyThreads * VEC / K;
+  const int split = spmm_split(M, K / VEC);
+  const int rows_per_block = kApplyThreads * VEC / (K * split);
   int blocks = (int)ceil_div(n, rows_per_block);
   blocks = std::min(blocks, num_sms() * 8);
-  k_csr_spmm<VT, XT, ZT, YT, K, VEC, MODE, DOT><<<blocks, kApplyThreads, 0, st>>>(
-      n, M.rp, M.ci, vals, X, Z, Y, alpha, DW, part, tick, dot_out);
+  launch_pdl(split > 1 ? k_csr_spmm<VT, XT, ZT, YT, K, VEC, MODE, DOT, true>
+                       : k_csr_spmm<VT, XT, ZT, YT, K, VEC, MODE, DOT, false>,
+             blocks, kApplyThreads, st, n, split, M.rp.get(), M.ci.get(), vals, X, Z, Y, alpha, DW,
+             part, tick, dot_out);
   CHRONOS_CHECK_LAUNCH();
 }
 
@@ -150,6 +198,7 @@ static void spmm(cudaStream_t st, const DMat &M, const VT *vals, const XT *X, co
 template <typename TI, typename TO, int K>
 __global__ void k_dense_matmat(int n, const double *__restrict__ W, const TI *__restrict__ B,
                                TO *__restrict__ Y) {
+  pdl_begin();
   const int row = blockIdx.x, j = threadIdx.x % K, g = threadIdx.x / K, G = blockDim.x / K;
   __shared__ double red[256];
   double s = 0.0;
@@ -169,7 +218,9 @@ struct BlockState {
   int K = 0, n = 0;
   std::vector<DBuf<float>> b32, x32, r32, t32;
   std::vector<DBuf<double>> b64, x64, r64, t64;
-  DBuf<double> x, res, p, axp, pres;
+  DBuf<double> x, res, p, axp, pres, b;
+  DBuf<double> stage;           // n x K: the host blocks as they come and go
+  DBuf<double> norms;           // ||b||^2 and ||r0||^2 per column
   DBuf<double> sc;              // per-column scalars, see BS_* below
   DBuf<double> part;
   DBuf<unsigned> tickets;
@@ -204,7 +255,7 @@ static void vcycle_block(Hier &h, BlockState &s, int l, const BT *b, OT *out, co
   double *part = s.part.get();
   unsigned *tick = s.tickets.get();
   if (L.coarsest) {
-    k_dense_matmat<BT, OT, K><<<n, 256, 0, st>>>(n, L.W.get(), b, out);
+    launch_pdl(k_dense_matmat<BT, OT, K>, n, 256, st, n, (const double *)L.W.get(), b, out);
     CHRONOS_CHECK_LAUNCH();
     return;
   }
@@ -248,6 +299,7 @@ static void vcycle_block(Hier &h, BlockState &s, int l, const BT *b, OT *out, co
 template <int K>
 __global__ void k_bpcg_p_update(int n, const double *__restrict__ pres, double *__restrict__ p,
                                 const double *__restrict__ sc) {
+  pdl_begin();
   const double *ptap = sc + bs_off(BS_PTAP, K), *pa = sc + bs_off(BS_PRES_AXP, K);
   const double *it = sc + bs_off(BS_ITER, K), *act = sc + bs_off(BS_ACTIVE, K);
   const size_t total = (size_t)n * K;
@@ -262,28 +314,32 @@ __global__ void k_bpcg_p_update(int n, const double *__restrict__ pres, double *
 
 template <int K> struct FinAlphaBlock {
   double *sc;
-  __device__ void operator()(const double *t) const {
-    for (int j = 0; j < K; ++j) {
-      if (sc[bs_off(BS_ACTIVE, K) + j] == 0.0) continue;
-      const double ptap = t[j], pr = t[K + j];
-      sc[bs_off(BS_PTAP, K) + j] = ptap;
-      if (!(ptap > 0.0) || !isfinite(pr)) {
-        sc[bs_off(BS_ALPHA, K) + j] = 0.0;
-        sc[bs_off(BS_FLAG, K) + j] = 2.0;          // breakdown
-      } else {
-        sc[bs_off(BS_ALPHA, K) + j] = pr / ptap;
-      }
+  __device__ bool operator()(int j, const double *t) const {
+    if (sc[bs_off(BS_ACTIVE, K) + j] == 0.0) return false;
+    const double ptap = t[j], pr = t[K + j];
+    sc[bs_off(BS_PTAP, K) + j] = ptap;
+    if (!(ptap > 0.0) || !isfinite(pr)) {
+      sc[bs_off(BS_ALPHA, K) + j] = 0.0;
+      sc[bs_off(BS_FLAG, K) + j] = 2.0;          // breakdown
+    } else {
+      sc[bs_off(BS_ALPHA, K) + j] = pr / ptap;
     }
+    return false;
   }
+  __device__ void done(bool) const {}
 };
 
-// axp = A p (FP64, block) with p'axp and p'res per column.
+// axp = A p (FP64, block) with p'axp and p'res per column.  262,144 rows x 16
+// columns: 83 us with a one-level reduction finished by one thread, 52 us (its
+// vectors and the operator are 122 MB, 19 us; the gathers of p move 235 MB
+// from L2).
 template <int K>
 __global__ void __launch_bounds__(kApplyThreads)
 k_bpcg_spmm(int n, const int *__restrict__ rp, const int *__restrict__ ci,
             const double *__restrict__ v, const double *__restrict__ p,
             const double *__restrict__ res, double *__restrict__ axp, double *part,
             unsigned *ticket, double *sc) {
+  pdl_begin();
   constexpr int LPR = K / 2;                      // two columns per lane (double2)
   constexpr int R = 32 / LPR;
   const int lane = threadIdx.x & 31, g = lane / LPR, j0 = (lane % LPR) * 2;
@@ -309,23 +365,23 @@ k_bpcg_spmm(int n, const int *__restrict__ rp, const int *__restrict__ ci,
           s[1] += a[u] * pv[u][1];
         }
       }
-      if (k < e1) {                            // the last 1..3 entries, loads predicated
+      if (k < e1) {        // the last 1..3 entries: loads clamped to the first, sums selected
         int c[3];
         double a[3], pv[3][2];
 #pragma unroll
         for (int u = 0; u < 3; ++u) {
-          c[u] = -1;
-          a[u] = 0.0;
-          if (k + u < e1) { c[u] = __ldg(ci + k + u); a[u] = __ldg(v + k + u); }
+          const int ku = k + u < e1 ? k + u : k;
+          c[u] = __ldg(ci + ku);
+          a[u] = __ldg(v + ku);
         }
 #pragma unroll
-        for (int u = 0; u < 3; ++u)
-          if (c[u] >= 0) Vec<double, 2>::ld(p + (size_t)c[u] * K + j0, pv[u]);
+        for (int u = 0; u < 3; ++u) Vec<double, 2>::ld(p + (size_t)c[u] * K + j0, pv[u]);
 #pragma unroll
         for (int u = 0; u < 3; ++u)
-          if (c[u] >= 0) {
-            s[0] += a[u] * pv[u][0];
-            s[1] += a[u] * pv[u][1];
+#pragma unroll
+          for (int e = 0; e < 2; ++e) {
+            const double t = s[e] + a[u] * pv[u][e];
+            s[e] = k + u < e1 ? t : s[e];
           }
       }
       const size_t o = (size_t)row * K + j0;
@@ -347,20 +403,19 @@ template <int K> struct FinResidualBlock {
   double *sc;
   cudaGraphConditionalHandle handle;
   int use_cond;
-  __device__ void operator()(const double *t) const {
+  // one column's stop test; true while it goes on
+  __device__ bool operator()(int j, const double *t) const {
+    if (sc[bs_off(BS_ACTIVE, K) + j] == 0.0) return false;
     const double tol = sc[BS_COUNT * K], itmax = sc[BS_COUNT * K + 1];
-    bool any = false;
-    for (int j = 0; j < K; ++j) {
-      if (sc[bs_off(BS_ACTIVE, K) + j] == 0.0) continue;
-      const double it = sc[bs_off(BS_ITER, K) + j] + 1.0;
-      sc[bs_off(BS_ITER, K) + j] = it;
-      const double r = sqrt(t[j]) / sc[bs_off(BS_BNORM, K) + j];
-      sc[bs_off(BS_RESITER, K) + j] = r;
-      const bool stop = r < tol || it >= itmax || sc[bs_off(BS_FLAG, K) + j] != 0.0 ||
-                        !isfinite(r);
-      if (stop) sc[bs_off(BS_ACTIVE, K) + j] = 0.0;
-      else any = true;
-    }
+    const double it = sc[bs_off(BS_ITER, K) + j] + 1.0;
+    const double r = sqrt(t[j]) / sc[bs_off(BS_BNORM, K) + j];
+    const bool stop = r < tol || it >= itmax || sc[bs_off(BS_FLAG, K) + j] != 0.0 || !isfinite(r);
+    sc[bs_off(BS_ITER, K) + j] = it;
+    sc[bs_off(BS_RESITER, K) + j] = r;
+    if (stop) sc[bs_off(BS_ACTIVE, K) + j] = 0.0;
+    return !stop;
+  }
+  __device__ void done(bool any) const {
     sc[BS_COUNT * K + 2] = any ? 1.0 : 0.0;
     if (use_cond) cudaGraphSetConditional(handle, any ? 1u : 0u);
   }
@@ -371,6 +426,7 @@ __global__ void __launch_bounds__(256)
 k_bpcg_xr_update(int n, double *__restrict__ x, double *__restrict__ res,
                  const double *__restrict__ p, const double *__restrict__ axp, double *part,
                  unsigned *ticket, double *sc, cudaGraphConditionalHandle handle, int use_cond) {
+  pdl_begin();
   // K threads of a group of K walk the K columns of consecutive rows
   const int j = threadIdx.x % K;
   const bool act = sc[bs_off(BS_ACTIVE, K) + j] != 0.0;
@@ -395,6 +451,7 @@ k_bpcg_xr_update(int n, double *__restrict__ x, double *__restrict__ res,
 template <int K>
 __global__ void __launch_bounds__(256)
 k_bnorm2(int n, const double *__restrict__ B, double *part, unsigned *ticket, double *dst) {
+  pdl_begin();
   const int j = threadIdx.x % K;
   double s = 0.0;
   const size_t total = (size_t)n * K;
@@ -408,16 +465,47 @@ k_bnorm2(int n, const double *__restrict__ B, double *part, unsigned *ticket, do
 template <int K>
 __global__ void k_bpcg_init(double *sc, const double *b2, const double *r2, double tol,
                             double itmax) {
-  for (int j = 0; j < K; ++j) {
-    const double bn = sqrt(b2[j]);
-    sc[bs_off(BS_BNORM, K) + j] = bn;
-    sc[bs_off(BS_RESITER, K) + j] = bn > 0.0 ? sqrt(r2[j]) / bn : 0.0;
-    sc[bs_off(BS_ITER, K) + j] = 0.0;
-    sc[bs_off(BS_FLAG, K) + j] = 0.0;
-    sc[bs_off(BS_ACTIVE, K) + j] = (bn > 0.0 && itmax > 0.0) ? 1.0 : 0.0;
+  pdl_begin();
+  const int j = threadIdx.x;                      // one block of K threads
+  const double bn = sqrt(b2[j]);
+  sc[bs_off(BS_BNORM, K) + j] = bn;
+  sc[bs_off(BS_RESITER, K) + j] = bn > 0.0 ? sqrt(r2[j]) / bn : 0.0;
+  sc[bs_off(BS_ITER, K) + j] = 0.0;
+  sc[bs_off(BS_FLAG, K) + j] = 0.0;
+  sc[bs_off(BS_ACTIVE, K) + j] = (bn > 0.0 && itmax > 0.0) ? 1.0 : 0.0;
+  if (j == 0) {
+    sc[BS_COUNT * K] = tol;
+    sc[BS_COUNT * K + 1] = itmax;
   }
-  sc[BS_COUNT * K] = tol;
-  sc[BS_COUNT * K + 1] = itmax;
+}
+
+// Between the callers' layouts (element (i, j) at i*ri + j*cj of the n x m
+// staged block) and the solve's row-major n x K block (columns m..K-1 zero
+// going in, dropped coming out): tiles of 32 rows through shared memory, so
+// both sides are read and written along their contiguous dimension.
+template <int K, bool IN>
+__global__ void __launch_bounds__(256)
+k_block_layout(int n, int m, int64_t ri, int64_t cj, double *__restrict__ staged,
+               double *__restrict__ rows) {
+  __shared__ double tile[32][K + 1];
+  const bool col_major = ri == 1;
+  for (int i0 = blockIdx.x * 32; i0 < n; i0 += gridDim.x * 32) {
+    for (int q = threadIdx.x; q < 32 * K; q += blockDim.x) {
+      const int i = IN && col_major ? q % 32 : q / K, j = IN && col_major ? q / 32 : q % K;
+      if (i0 + i < n)
+        tile[i][j] = !IN ? rows[(size_t)(i0 + i) * K + j]
+                     : j < m ? staged[(i0 + i) * ri + j * cj] : 0.0;
+    }
+    __syncthreads();
+    for (int q = threadIdx.x; q < 32 * K; q += blockDim.x) {
+      const int i = !IN && col_major ? q % 32 : q / K, j = !IN && col_major ? q / 32 : q % K;
+      if (i0 + i < n) {
+        if (IN) rows[(size_t)(i0 + i) * K + j] = tile[i][j];
+        else if (j < m) staged[(i0 + i) * ri + j * cj] = tile[i][j];
+      }
+    }
+    __syncthreads();
+  }
 }
 
 // zero columns with b = 0 (PCG_CJ.m:12-16)
@@ -443,23 +531,25 @@ static void capture_block_iteration(Hier &h, BlockState &s, cudaGraphConditional
   else
     vcycle_block<double, double, double, K>(h, s, 0, s.res.get(), s.pres.get(), s.axp.get(),
                                             sc + bs_off(BS_PRES_AXP, K));
-  k_bpcg_p_update<K><<<nb, 256, 0, st>>>(n, s.pres.get(), s.p.get(), sc);
+  launch_pdl(k_bpcg_p_update<K>, nb, 256, st, n, (const double *)s.pres.get(), s.p.get(),
+             (const double *)sc);
   CHRONOS_CHECK_LAUNCH();
   const DMat &A = h.levels[0].A;
   const int blocks = std::min(num_sms() * 8, (int)ceil_div(n, kApplyThreads * 2 / K));
-  k_bpcg_spmm<K><<<blocks, kApplyThreads, 0, st>>>(n, A.rp, A.ci, A.v64, s.p.get(), s.res.get(),
-                                                   s.axp.get(), s.part.get() + 2 * K * 2048,
-                                                   tk + 1, sc);
+  launch_pdl(k_bpcg_spmm<K>, blocks, kApplyThreads, st, n, (const int *)A.rp.get(),
+             (const int *)A.ci.get(), (const double *)A.v64.get(), (const double *)s.p.get(),
+             (const double *)s.res.get(), s.axp.get(), s.part.get() + 2 * K * 2048,
+             tk + kReduceTickets, sc);
   CHRONOS_CHECK_LAUNCH();
-  k_bpcg_xr_update<K><<<nb, 256, 0, st>>>(n, s.x.get(), s.res.get(), s.p.get(), s.axp.get(),
-                                          s.part.get() + 4 * K * 2048, tk + 2, sc, handle,
-                                          use_cond);
+  launch_pdl(k_bpcg_xr_update<K>, nb, 256, st, n, s.x.get(), s.res.get(),
+             (const double *)s.p.get(), (const double *)s.axp.get(),
+             s.part.get() + 4 * K * 2048, tk + 2 * kReduceTickets, sc, handle, use_cond);
   CHRONOS_CHECK_LAUNCH();
 }
 
 template <int K>
-static void block_solve(Hier &h, const double *B_h, double *X_h, int itmax, double tol,
-                        int *iters, int *flags, double *seconds) {
+static void block_solve(Hier &h, int m, const BlockIn &B, const double *X0_h, double *X_h,
+                        int itmax, double tol, int *iters, int *flags, double *seconds) {
   cudaStream_t st = h.st;
   auto &sp = h.block;
   if (!sp || sp->K != K) {
@@ -478,42 +568,51 @@ static void block_solve(Hier &h, const double *B_h, double *X_h, int itmax, doub
     }
     const size_t m0 = (size_t)s.n * K;
     s.x.alloc(m0); s.res.alloc(m0); s.p.alloc(m0); s.axp.alloc(m0); s.pres.alloc(m0);
+    s.b.alloc(m0); s.stage.alloc(m0); s.norms.alloc(2 * K);
     s.p.zero(st);
     s.axp.zero(st);
     s.sc.alloc((size_t)BS_COUNT * K + 8);
     s.part.alloc((size_t)6 * K * 2048);
-    s.tickets.alloc(8);
+    s.tickets.alloc(4 * kReduceTickets);
     s.tickets.zero(st);
   }
   BlockState &s = *sp;
   const int n = s.n;
-  const size_t m0 = (size_t)n * K;
-  DBuf<double> b(m0), r2(K), b2(K);
-  // column-major host blocks -> row-major device blocks
-  {
-    std::vector<double> tmp(m0), tx(m0);
-    for (int j = 0; j < K; ++j)
-      for (int i = 0; i < n; ++i) {
-        tmp[(size_t)i * K + j] = B_h[(size_t)j * n + i];
-        tx[(size_t)i * K + j] = X_h[(size_t)j * n + i];
-      }
-    b.upload(tmp, st);
-    s.x.upload(tx, st);
-  }
+  double *b = s.b.get(), *b2 = s.norms.get(), *r2 = s.norms.get() + K;
+  // host blocks -> row-major device blocks; a row-major host block of exactly
+  // K columns is already in the solve's layout
+  const int lb = std::max(1, std::min(num_sms() * 8, (int)ceil_div(n, 32)));
+  auto pack = [&](const BlockIn &src, double *dst) {
+    if (src.ld > 0) {                              // row-major, rows ld apart
+      double *to = m == K ? dst : s.stage.get();
+      CHRONOS_CUDA(cudaMemcpy2DAsync(to, sizeof(double) * m, src.p, sizeof(double) * src.ld,
+                                     sizeof(double) * m, n, cudaMemcpyHostToDevice, st));
+      if (m == K) return;
+      k_block_layout<K, true><<<lb, 256, 0, st>>>(n, m, m, 1, s.stage.get(), dst);
+    } else {
+      CHRONOS_CUDA(cudaMemcpyAsync(s.stage.get(), src.p, sizeof(double) * n * m,
+                                   cudaMemcpyHostToDevice, st));
+      k_block_layout<K, true><<<lb, 256, 0, st>>>(n, m, 1, n, s.stage.get(), dst);
+    }
+    CHRONOS_CHECK_LAUNCH();
+  };
+  pack(B, b);
+  if (X0_h) pack(BlockIn{X0_h, 0}, s.x.get());
+  else s.x.zero(st);
   cudaEvent_t e0, e1;
   CHRONOS_CUDA(cudaEventCreate(&e0));
   CHRONOS_CUDA(cudaEventCreate(&e1));
   CHRONOS_CUDA(cudaEventRecord(e0, st));
   const DMat &A = h.levels[0].A;
-  spmm<double, double, double, double, K, MODE_RESID, false>(st, A, A.v64.get(), s.x.get(), b.get(),
+  spmm<double, double, double, double, K, MODE_RESID, false>(st, A, A.v64.get(), s.x.get(), b,
                                                              s.res.get(), 1.0);
   const int nb = std::max(1, std::min(num_sms() * 8, (int)ceil_div((int64_t)n * K, 256)));
-  k_bnorm2<K><<<nb, 256, 0, st>>>(n, b.get(), s.part.get(), s.tickets.get() + 3, b2.get());
-  CHRONOS_CHECK_LAUNCH();
-  k_bnorm2<K><<<nb, 256, 0, st>>>(n, s.res.get(), s.part.get(), s.tickets.get() + 3, r2.get());
-  CHRONOS_CHECK_LAUNCH();
-  k_bpcg_init<K><<<1, 1, 0, st>>>(s.sc.get(), b2.get(), r2.get(), tol, (double)itmax);
-  CHRONOS_CHECK_LAUNCH();
+  launch_pdl(k_bnorm2<K>, nb, 256, st, n, (const double *)b, s.part.get(),
+             s.tickets.get() + 3 * kReduceTickets, b2);
+  launch_pdl(k_bnorm2<K>, nb, 256, st, n, (const double *)s.res.get(), s.part.get(),
+             s.tickets.get() + 3 * kReduceTickets, r2);
+  launch_pdl(k_bpcg_init<K>, 1, K, st, s.sc.get(), (const double *)b2, (const double *)r2, tol,
+             (double)itmax);
   if (itmax > 0 && !h.prm.use_graph) {
     // one iteration per graph launch from a host loop (profilers cannot see
     // the kernel nodes of a graph holding a conditional node); same kernels
@@ -577,17 +676,18 @@ static void block_solve(Hier &h, const double *B_h, double *X_h, int itmax, doub
   k_zero_null_columns<K><<<nb, 256, 0, st>>>(n, s.x.get(), s.sc.get());
   CHRONOS_CHECK_LAUNCH();
   CHRONOS_CUDA(cudaEventRecord(e1, st));
-  std::vector<double> sc_h((size_t)BS_COUNT * K + 8), xr(m0);
+  k_block_layout<K, false><<<lb, 256, 0, st>>>(n, m, 1, n, s.stage.get(), s.x.get());
+  CHRONOS_CHECK_LAUNCH();
+  std::vector<double> sc_h((size_t)BS_COUNT * K + 8);
   s.sc.download(sc_h.data(), sc_h.size(), st);
-  s.x.download(xr.data(), m0, st);
+  s.stage.download(X_h, (size_t)n * m, st);
   CHRONOS_CUDA(cudaStreamSynchronize(st));
   float ms = 0.f;
   CHRONOS_CUDA(cudaEventElapsedTime(&ms, e0, e1));
   cudaEventDestroy(e0);
   cudaEventDestroy(e1);
   if (seconds) *seconds = ms * 1e-3;
-  for (int j = 0; j < K; ++j) {
-    for (int i = 0; i < n; ++i) X_h[(size_t)j * n + i] = xr[(size_t)i * K + j];
+  for (int j = 0; j < m; ++j) {
     iters[j] = (int)(sc_h[bs_off(BS_ITER, K) + j] + 0.5);
     const double r = sc_h[bs_off(BS_RESITER, K) + j];
     flags[j] = (sc_h[bs_off(BS_BNORM, K) + j] == 0.0) ? 0
@@ -595,27 +695,17 @@ static void block_solve(Hier &h, const double *B_h, double *X_h, int itmax, doub
   }
 }
 
-void Hier::pcg_block(int nrhs, const double *B_h, double *X_h, int itmax, double tol,
-                     int *iters, int *flags, double *seconds) {
+void Hier::pcg_block(int nrhs, const BlockIn &B, const double *X0_h, double *X_h, int itmax,
+                     double tol, int *iters, int *flags, double *seconds) {
   CHRONOS_REQUIRE(nrhs >= 1 && nrhs <= 16, CHRONOS_EINVAL, "block solve: 1 <= nrhs <= 16");
-  const int n = levels[0].n;
-  int K = 1;
+  int K = 2;                     // padded with zero right-hand sides (they stay at x = 0)
   while (K < nrhs) K <<= 1;
-  if (K < 2) K = 2;
-  // pad to K columns with zero right-hand sides (they stay at x = 0)
-  std::vector<double> B((size_t)n * K, 0.0), X((size_t)n * K, 0.0);
-  std::copy(B_h, B_h + (size_t)n * nrhs, B.begin());
-  std::copy(X_h, X_h + (size_t)n * nrhs, X.begin());
-  std::vector<int> it(K), fl(K);
   switch (K) {
-    case 2: block_solve<2>(*this, B.data(), X.data(), itmax, tol, it.data(), fl.data(), seconds); break;
-    case 4: block_solve<4>(*this, B.data(), X.data(), itmax, tol, it.data(), fl.data(), seconds); break;
-    case 8: block_solve<8>(*this, B.data(), X.data(), itmax, tol, it.data(), fl.data(), seconds); break;
-    default: block_solve<16>(*this, B.data(), X.data(), itmax, tol, it.data(), fl.data(), seconds); break;
+    case 2: block_solve<2>(*this, nrhs, B, X0_h, X_h, itmax, tol, iters, flags, seconds); break;
+    case 4: block_solve<4>(*this, nrhs, B, X0_h, X_h, itmax, tol, iters, flags, seconds); break;
+    case 8: block_solve<8>(*this, nrhs, B, X0_h, X_h, itmax, tol, iters, flags, seconds); break;
+    default: block_solve<16>(*this, nrhs, B, X0_h, X_h, itmax, tol, iters, flags, seconds); break;
   }
-  std::copy(X.begin(), X.begin() + (size_t)n * nrhs, X_h);
-  std::copy(it.begin(), it.begin() + nrhs, iters);
-  std::copy(fl.begin(), fl.begin() + nrhs, flags);
 }
 
 }  // namespace chronos

@@ -996,6 +996,13 @@ int chronos_pcg(chronos_hier *hh, const int *iat_h, const int *ja_h, const doubl
 
 int chronos_pcg_block(chronos_hier *hh, int nrhs, const double *B_h, double *X_h, int itmax,
                       double tol, int *iters_h, int *flags_h, double *seconds, void *stream) {
+  return chronos_pcg_block_rows(hh, nrhs, B_h, 0, X_h, X_h, itmax, tol, iters_h, flags_h, seconds,
+                                stream);
+}
+
+int chronos_pcg_block_rows(chronos_hier *hh, int nrhs, const double *B_h, int b_row_major,
+                           const double *X0_h, double *X_h, int itmax, double tol, int *iters_h,
+                           int *flags_h, double *seconds, void *stream) {
   return guard([&] {
     CallRange range_("chronos_pcg_block");
     CHRONOS_REQUIRE(hh && B_h && X_h && iters_h && flags_h && nrhs >= 1, CHRONOS_EINVAL,
@@ -1008,8 +1015,9 @@ int chronos_pcg_block(chronos_hier *hh, int nrhs, const double *B_h, double *X_h
     for (int c0 = 0; c0 < nrhs; c0 += 16) {
       const int m = std::min(16, nrhs - c0);
       double sec = 0.0;
-      h.pcg_block(m, B_h + (size_t)c0 * n, X_h + (size_t)c0 * n, itmax, tol, iters_h + c0,
-                  flags_h + c0, &sec);
+      const BlockIn B = b_row_major ? BlockIn{B_h + c0, nrhs} : BlockIn{B_h + (size_t)c0 * n, 0};
+      h.pcg_block(m, B, X0_h ? X0_h + (size_t)c0 * n : nullptr, X_h + (size_t)c0 * n, itmax, tol,
+                  iters_h + c0, flags_h + c0, &sec);
       total += sec;
     }
     if (seconds) *seconds = total;

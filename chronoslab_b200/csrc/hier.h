@@ -96,6 +96,13 @@ struct PcgState {
 
 struct BlockState;   // block-of-right-hand-sides solve state (block.cu)
 
+// A host block of right-hand sides: column-major with n rows (ld = 0), or
+// row-major with rows ld elements apart.
+struct BlockIn {
+  const double *p = nullptr;
+  int64_t ld = 0;
+};
+
 struct Hier {
   chronos_params prm{};
   int precision = CHRONOS_FP32;
@@ -137,9 +144,10 @@ struct Hier {
   void apply_A(const double *x, double *y);
   // timings and algorithmic bytes of the hot kernels
   void profile(int reps, chronos_profile *out);
-  // nrhs <= 16 columns (column-major host blocks) solved together
-  void pcg_block(int nrhs, const double *B_h, double *X_h, int itmax, double tol, int *iters,
-                 int *flags, double *seconds);
+  // nrhs <= 16 columns solved together from x0 (column-major, null: zero)
+  // into X_h (column-major)
+  void pcg_block(int nrhs, const BlockIn &B, const double *X0_h, double *X_h, int itmax,
+                 double tol, int *iters, int *flags, double *seconds);
   std::shared_ptr<BlockState> block;
   DBuf<double> stage_b, stage_x;    // host-buffer entry points' device staging
 };

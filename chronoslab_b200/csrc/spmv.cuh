@@ -85,9 +85,38 @@ __device__ __forceinline__ void grid_reduce(double (&v)[K], double *part, unsign
 // Deterministic grid reduction of NQ quantities of K columns (block
 // right-hand sides).  Lane l owns columns (l % (K/VEC))*VEC .. +VEC-1 and
 // v[q][e] is its partial of quantity q for the e-th of them; lanes owning the
-// same columns are combined by shuffles, warps through shared memory, blocks
-// by the last block to arrive (fixed orders throughout).  fin receives the
-// NQ*K totals, quantity-major (t[q*K + j]).  K*NQ <= 32, K/VEC <= 32.
+// same columns are combined by shuffles, warps through shared memory, then
+// the blocks in two levels: the last of each kReduceGroup consecutive blocks
+// to arrive adds their partials, the last of these the groups' (fixed orders
+// throughout; one level left the last block a serial chain of 148 loads per
+// thread at 1184 blocks).  Thread j < K of that block calls fin(j, t) with the
+// NQ*K totals, quantity-major (t[q*K + j]), and thread 0 then fin.done(any of
+// the results); one thread walking all columns was a chain of K dependent
+// rounds of loads.  ticket[0 .. kReduceTickets) and part[0 .. NQ*K*(blocks +
+// groups)) belong to the launch; K*NQ <= 32, K/VEC <= 32, at most
+// kReduceGroup * (kReduceTickets - 1) blocks.
+constexpr int kReduceGroup = 32;
+constexpr int kReduceTickets = 128;
+
+// red[0..rows)[c] of part's rows summed by stripes of threads, in row order
+// within a stripe and then by stripe; thread c < NC returns column c's sum.
+template <int NC>
+__device__ __forceinline__ double sum_partial_rows(const double *part, int rows,
+                                                   double (&red)[32][NC]) {
+  const int stripes = min((int)blockDim.x / NC, 32);
+  const int c = threadIdx.x % NC, s = threadIdx.x / NC;
+  if (s < stripes) {
+    double acc = 0.0;
+    for (int b = s; b < rows; b += stripes) acc += __ldcg(&part[(size_t)b * NC + c]);
+    red[s][c] = acc;
+  }
+  __syncthreads();
+  double t = 0.0;
+  if ((int)threadIdx.x < NC)
+    for (int w = 0; w < stripes; ++w) t += red[w][threadIdx.x];
+  return t;
+}
+
 template <int K, int VEC, int NQ, typename Fin>
 __device__ __forceinline__ void grid_reduce_cols(double (&v)[NQ][VEC], double *part,
                                                  unsigned *ticket, Fin fin) {
@@ -98,6 +127,10 @@ __device__ __forceinline__ void grid_reduce_cols(double (&v)[NQ][VEC], double *p
   __shared__ double tot[NC];
   __shared__ bool last;
   const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, nw = blockDim.x >> 5;
+  const int ngroups = (gridDim.x + kReduceGroup - 1) / kReduceGroup;
+  const int grp = blockIdx.x / kReduceGroup;
+  const int gsize = min(kReduceGroup, (int)gridDim.x - grp * kReduceGroup);
+  double *gpart = part + (size_t)gridDim.x * NC;
 #pragma unroll
   for (int q = 0; q < NQ; ++q)
 #pragma unroll
@@ -117,27 +150,31 @@ __device__ __forceinline__ void grid_reduce_cols(double (&v)[NQ][VEC], double *p
     __threadfence();
   }
   __syncthreads();
-  if (threadIdx.x == 0) last = atomicAdd(ticket, 1u) == gridDim.x - 1;
+  if (threadIdx.x == 0) last = atomicAdd(ticket + 1 + grp, 1u) == (unsigned)gsize - 1;
   __syncthreads();
   if (!last) return;
   __threadfence();
-  const int stripes = min((int)blockDim.x / NC, 32);
-  const int c = threadIdx.x % NC, sidx = threadIdx.x / NC;
-  if (sidx < stripes) {
-    double acc = 0.0;
-    for (int b = sidx; b < (int)gridDim.x; b += stripes) acc += __ldcg(&part[(size_t)b * NC + c]);
-    red[sidx][c] = acc;
-  }
-  __syncthreads();
+  const double gs = sum_partial_rows<NC>(part + (size_t)grp * kReduceGroup * NC, gsize, red);
   if ((int)threadIdx.x < NC) {
-    double s2 = 0.0;
-    for (int w = 0; w < stripes; ++w) s2 += red[w][threadIdx.x];
-    tot[threadIdx.x] = s2;
+    gpart[(size_t)grp * NC + threadIdx.x] = gs;
+    __threadfence();
   }
   __syncthreads();
   if (threadIdx.x == 0) {
+    ticket[1 + grp] = 0u;
+    last = atomicAdd(ticket, 1u) == (unsigned)ngroups - 1;
+  }
+  __syncthreads();
+  if (!last) return;
+  __threadfence();
+  const double ts = sum_partial_rows<NC>(gpart, ngroups, red);
+  if ((int)threadIdx.x < NC) tot[threadIdx.x] = ts;
+  __syncthreads();
+  const bool mine = (int)threadIdx.x < K && fin((int)threadIdx.x, tot);
+  const bool any = __syncthreads_or(mine) != 0;
+  if (threadIdx.x == 0) {
     *ticket = 0u;
-    fin(tot);
+    fin.done(any);
   }
 }
 

@@ -479,6 +479,12 @@ int chronos_pcg_dev(chronos_hier *h, const double *b_d, double *x_d, int itmax, 
  * stopping tests.  iters_h[nrhs], flags_h[nrhs]. */
 int chronos_pcg_block(chronos_hier *h, int nrhs, const double *B_h, double *X_h, int itmax,
                       double tol, int *iters_h, int *flags_h, double *seconds, void *stream);
+/* The same with B_h n x nrhs column-major (b_row_major = 0) or row-major (1),
+ * and the start vectors X0_h (column-major) apart from the result X_h
+ * (column-major); X0_h = NULL starts from zero. */
+int chronos_pcg_block_rows(chronos_hier *h, int nrhs, const double *B_h, int b_row_major,
+                           const double *X0_h, double *X_h, int itmax, double tol, int *iters_h,
+                           int *flags_h, double *seconds, void *stream);
 
 /* ---- Batch of independent problems of uneven sizes ---------------------- */
 /* One hierarchy per problem (each what chronos_amg_setup builds for it with

@@ -77,3 +77,45 @@ def test_fsai_indefinite_local_system(lib, m):
     s, e = indptr[m], indptr[m + 1]
     assert np.array_equal(vals[s:e], np.append(np.zeros(m), 1.0))
     assert np.array_equal(vals[e:], good_vals[e:])
+
+
+@pytest.mark.parametrize("nrhs", [1, 2, 3, 7, 8, 13, 16, 17])
+def test_block_memory_orders_and_start_vectors(lib, nrhs):
+    """Row-major, column-major and sliced blocks of right-hand sides give the
+    same bits; started from its own solution a block stops at once."""
+    from chronoslab_b200 import problems as PB
+    A, _ = PB.diffusion7(15, seed=3)
+    n = A.shape[0]
+    B = np.ascontiguousarray(PB.uniform_rhs(n, 4, 18)[:, :nrhs])
+    with cb.Hierarchy(A, np.ones(n), cb.params(ntv=1)) as h:
+        X, its, flags, _ = h.pcg_block(B, tol=1e-8)
+        assert X.shape == (n, nrhs) and np.all(flags == 0)
+        assert np.all(np.linalg.norm(B - A @ X, axis=0) <= 1e-8 * np.linalg.norm(B, axis=0))
+        wide = np.zeros((n, 2 * nrhs))
+        wide[:, ::2] = B
+        for other in (np.asfortranarray(B), wide[:, ::2]):
+            X2, its2, _, _ = h.pcg_block(other, tol=1e-8)
+            assert np.array_equal(X, X2) and np.array_equal(its, its2)
+        # the block solve's recurrence starts from b - A x0 and always takes a step
+        X3, its3, flags3, _ = h.pcg_block(B, X0=X, tol=1e-8)
+        assert np.all(its3 == 1) and np.all(flags3 == 0)
+        assert np.linalg.norm(X3 - X) <= 1e-6 * np.linalg.norm(X)
+
+
+@pytest.mark.parametrize("nx", [4, 9, 22, 34])
+@pytest.mark.parametrize("nrhs", [2, 5, 16])
+def test_block_of_small_levels_matches_columns(lib, nx, nrhs):
+    """Levels small enough that several lane sets share a row: each column
+    solved to 1e-11 equals the column's own solve to 1e-8 (both residuals
+    bounded, the operator's condition below 1e3 on these grids)."""
+    from chronoslab_b200 import problems as PB
+    A = PB.poisson7(nx)
+    n = A.shape[0]
+    B = PB.uniform_rhs(n, 9, nrhs)
+    with cb.Hierarchy(A, np.ones(n), cb.params(ntv=1, maxCoarseSZ=20)) as h:
+        X, its, flags, _ = h.pcg_block(B, tol=1e-11)
+        assert np.all(flags == 0)
+        for j in range(nrhs):
+            x, it, _, flag, _ = h.pcg(B[:, j], tol=1e-11)
+            assert flag == 0 and abs(int(its[j]) - it) <= 1
+            assert np.linalg.norm(X[:, j] - x) <= 1e-8 * np.linalg.norm(x)
