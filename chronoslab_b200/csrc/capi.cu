@@ -126,6 +126,35 @@ struct ScopedStream {
   ~ScopedStream() { if (st) { cudaStreamSynchronize(st); cudaStreamDestroy(st); } }
 };
 
+// A caller's host CSR in device memory, as the setup kernels read it.
+struct DeviceCsr {
+  int64_t nnz = 0;
+  DBuf<int> rp, ci;
+  DBuf<double> v;
+};
+
+// Uploads a host CSR from the caller's arrays and checks it on the device (the
+// conditions and messages of from_csr0, without its copies: they and the
+// single-threaded checks were most of a Galerkin call's time).
+static void upload_checked(int n, int ncols, const int *iat, const int *ja, const double *v,
+                           DeviceCsr &d, cudaStream_t st) {
+  CHRONOS_REQUIRE(n > 0 && iat && (iat[n] == 0 || (ja && v)), CHRONOS_EINVAL, "null CSR input");
+  CHRONOS_REQUIRE(iat[0] == 0, CHRONOS_EINVAL, "0-based CSR expected (iat[0] == 0)");
+  bool down = false;
+  for (int i = 0; i < n; ++i) down |= iat[i + 1] < iat[i];
+  CHRONOS_REQUIRE(!down, CHRONOS_EINVAL, "decreasing row pointers");
+  d.nnz = iat[n];
+  d.rp.upload(iat, (size_t)n + 1, st);
+  d.ci.alloc(std::max<int64_t>(d.nnz, 1));
+  d.v.alloc(std::max<int64_t>(d.nnz, 1));
+  d.ci.upload(ja, d.nnz, st);
+  d.v.upload(v, d.nnz, st);
+  const int bad = csr_check_device(n, ncols, d.rp, d.ci, st);
+  CHRONOS_REQUIRE(!(bad & 1), CHRONOS_EINVAL, "column index out of range");
+  CHRONOS_REQUIRE(!(bad & 2), CHRONOS_EINVAL,
+                  "CSR columns must be strictly increasing within a row");
+}
+
 // Records an event on `from` and makes `to` wait for it.
 static void stream_wait(cudaStream_t to, cudaStream_t from) {
   cudaEvent_t e;
@@ -614,25 +643,22 @@ int chronos_galerkin_compute(int n, int nc, const int *iat_A_h, const int *ja_A_
                              const double *val_P_h, int64_t *nnz_Ac, chronos_galerkin_plan **plan) {
   return guard([&] {
     CHRONOS_REQUIRE(plan && nnz_Ac && nc > 0, CHRONOS_EINVAL, "bad argument");
-    HostCSR A = from_csr0(n, n, iat_A_h, ja_A_h, val_A_h);
-    HostCSR P = from_csr0(n, nc, iat_P_h, ja_P_h, val_P_h);
-    for (int i = 0; i < n; ++i)
-      for (int64_t k = A.rp[i] + 1; k < A.rp[i + 1]; ++k)
-        CHRONOS_REQUIRE(A.ci[k] > A.ci[k - 1], CHRONOS_EINVAL, "A rows must be sorted");
     ScopedStream s;
-    DMat dA, dP, dPt;
-    upload_csr(A, dA, false, s.st);
-    upload_csr(P, dP, false, s.st);
-    upload_transpose(dP, dPt, false, s.st, &P);
+    DeviceCsr dA, dP;
+    upload_checked(n, n, iat_A_h, ja_A_h, val_A_h, dA, s.st);
+    upload_checked(n, nc, iat_P_h, ja_P_h, val_P_h, dP, s.st);
+    DBuf<int> ptrp, ptci;
+    DBuf<double> ptv;
+    csr_transpose_device(n, nc, dP.nnz, dP.rp, dP.ci, dP.v, ptrp, ptci, ptv, s.st);
     DBuf<int> aprp, apci;
     DBuf<double> apv;
     int64_t nnz_ap = 0;
-    spgemm_device(n, nc, dA.rp, dA.ci, dA.v64, dP.rp, dP.ci, dP.v64, aprp, apci, apv, &nnz_ap, s.st);
+    spgemm_device(n, nc, dA.rp, dA.ci, dA.v, dP.rp, dP.ci, dP.v, aprp, apci, apv, &nnz_ap, s.st);
     auto *pl = new chronos_galerkin_plan();
     try {
       pl->nc = nc;
-      spgemm_device(nc, nc, dPt.rp, dPt.ci, dPt.v64, aprp, apci, apv, pl->rp, pl->ci, pl->v,
-                    &pl->nnz, s.st);
+      spgemm_device(nc, nc, ptrp, ptci, ptv, aprp, apci, apv, pl->rp, pl->ci, pl->v, &pl->nnz,
+                    s.st);
     } catch (...) {
       delete pl;
       throw;

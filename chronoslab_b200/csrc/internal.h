@@ -112,6 +112,9 @@ void convert_f64_to_f32(int64_t n, const double *src, float *dst, cudaStream_t s
 void csr_transpose_device(int nrows, int ncols, int64_t nnz, const int *rp, const int *ci,
                           const double *v, DBuf<int> &trp, DBuf<int> &tci, DBuf<double> &tv,
                           cudaStream_t st);
+// Columns of a device CSR with ascending row pointers: bit 0 one outside
+// [0, ncols), bit 1 not strictly increasing within a row.  Synchronises st.
+int csr_check_device(int nrows, int ncols, const int *rp, const int *ci, cudaStream_t st);
 // 16-bit column offsets from each row's smallest column (rows without
 // entries: base 0), when every row spans fewer than 65536 columns; returns
 // false (nothing kept) otherwise.

@@ -13,6 +13,7 @@
 //  * Coarsest level: dense FP64 Cholesky, inverse from the factor, dense
 //    matvec apply (AMG_Vcycle.m:9-10).
 #include <cub/cub.cuh>
+#include <thrust/iterator/transform_iterator.h>
 
 #include <algorithm>
 #include <cstdio>
@@ -686,129 +687,281 @@ __global__ void k_spgemm_numeric(int r0, int r1, const int *rows, const int *xrp
   if (lane == 0) cnt_out[i] = emitted;
 }
 
-// Shared-memory variants for rows whose distinct columns fit a warp's table
-// of kSpgemmSmSlots: the same insertion order and sums as the global-table
-// kernels (each output column gets its products in X's row order), so the
-// results are bit-identical; only the table's place and size differ.
+// Shared-memory variants for rows whose distinct columns fill at most half of
+// a warp's table (kSpgemmSmSlots at the largest; rows beyond go to the global
+// tables above).  The products of a row are taken 32 at a time across the
+// entries of X's row -- Y's rows (a prolongation's) are often far shorter than
+// a warp -- and the lanes that hold the same column add theirs in lane order,
+// which is X's row order: every output entry is the same sum, rounded at the
+// same places, as a row-wise Gustavson product's.  A row's table is as large as
+// its class needs, so that short rows fill the SM with warps; the numeric
+// kernel sorts its row in the table before it leaves.  A*P and P'*(A*P) of
+// elasticity 26^3 (57k rows, 81 entries times 4 to 5): an entry of X at a time
+// in 4096-slot tables (4 warps per SM) 6.6 ms, then 1.7 ms in the segmented
+// sort; now 1.5 ms together.
 constexpr int kSpgemmSmSlots = 4096;
-constexpr int kSpgemmSmWarps = 4;
 
-__device__ __forceinline__ unsigned spgemm_cap(int64_t prod, int ncols) {
-  const uint64_t want = (uint64_t)2 * (uint64_t)prod + 1, colcap = (uint64_t)2 * (uint64_t)max(ncols, 1);
-  uint64_t p = 32, v = want < colcap ? want : colcap;
-  while (p < v) p <<= 1;
-  return (unsigned)p;
-}
+// One class of rows: table slots, the largest count that may use it, warps per
+// block.
+template <int SLOTS> struct SpgemmClass {
+  static constexpr int warps = SLOTS <= 1024 ? 8 : 4;
+  static constexpr int max_count = SLOTS / 2;
+};
 
-// Symbolic in shared memory: cnt[i] = distinct columns of row i, or -1 when
-// they outgrow half the warp's table (the row then goes to the global table).
-__global__ void __launch_bounds__(32 * kSpgemmSmWarps)
-k_spgemm_symbolic_sm(int m, int ncols, const int *__restrict__ xrp, const int *__restrict__ xci,
-                     const int *__restrict__ yrp, const int *__restrict__ yci,
-                     const int64_t *__restrict__ prod, int *__restrict__ cnt) {
+// Entries [k0, k0 + 32) of row X: lane l holds entry k0 + l's value, the offset
+// of Y's row minus the products before it, and the running product count.
+struct SpgemmChunk {
+  double a = 0.0;
+  int base = 0, inc = 0, total = 0;
+  __device__ __forceinline__ void load(int k, int ke, const int *__restrict__ xci,
+                                       const double *__restrict__ xv,
+                                       const int *__restrict__ yrp) {
+    const int lane = threadIdx.x & 31;
+    int ys = 0, len = 0;
+    a = 0.0;
+    if (k < ke) {
+      const int j = __ldg(xci + k);
+      if (xv) a = __ldg(xv + k);
+      ys = __ldg(yrp + j);
+      len = __ldg(yrp + j + 1) - ys;
+    }
+    inc = len;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const int t = __shfl_up_sync(0xffffffffu, inc, o);
+      if (lane >= o) inc += t;
+    }
+    total = __shfl_sync(0xffffffffu, inc, 31);
+    base = ys - (inc - len);
+  }
+  // lane holding product t's entry of X
+  __device__ __forceinline__ int owner(int t) const {
+    int lo = 0;
+#pragma unroll
+    for (int step = 16; step > 0; step >>= 1)
+      if (__shfl_sync(0xffffffffu, inc, lo + step - 1) <= t) lo += step;
+    return lo;
+  }
+};
+
+// Symbolic: cnt[i] = distinct columns of the rows whose bound (products, at
+// most ncols) is in (lo, SLOTS/2], or for the largest class everything above
+// lo: -1 (and *nbig) when they outgrow half the table.
+template <int SLOTS>
+__global__ void __launch_bounds__(32 * SpgemmClass<SLOTS>::warps)
+k_spgemm_symbolic_sm(int m, int ncols, int lo, const int *__restrict__ xrp,
+                     const int *__restrict__ xci, const int *__restrict__ yrp,
+                     const int *__restrict__ yci, const int64_t *__restrict__ prod,
+                     int *__restrict__ cnt, int *nbig) {
+  constexpr int W = SpgemmClass<SLOTS>::warps;
+  constexpr bool TOP = SLOTS == kSpgemmSmSlots;
   extern __shared__ int spg_keys[];
-  const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
-  int *tk = spg_keys + wib * kSpgemmSmSlots;
-  const int gw = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-  const int nw = (gridDim.x * blockDim.x) >> 5;
-  for (int i = gw; i < m; i += nw) {
-    const unsigned cap = spgemm_cap(prod[i], ncols);
-    const unsigned tsz = cap < (unsigned)kSpgemmSmSlots ? cap : (unsigned)kSpgemmSmSlots;
-    const unsigned mask = tsz - 1;
+  const int lane = threadIdx.x & 31;
+  int *tk = spg_keys + (threadIdx.x >> 5) * SLOTS;
+  const int nw = gridDim.x * W;
+  for (int i = blockIdx.x * W + (threadIdx.x >> 5); i < m; i += nw) {
+    const int64_t p = __ldg(prod + i);
+    const int bound = (int)(p < ncols ? p : ncols);
+    if (bound <= lo || (!TOP && bound > SLOTS / 2)) continue;
+    unsigned tsz = 32;
+    while (tsz < SLOTS && tsz < 2u * bound) tsz <<= 1;
     for (unsigned s = lane; s < tsz; s += 32) tk[s] = -1;
     __syncwarp();
     int count = 0;
     bool over = false;
-    for (int k = xrp[i]; k < xrp[i + 1] && !over; ++k) {
-      const int j = xci[k];
-      for (int kk0 = yrp[j]; kk0 < yrp[j + 1]; kk0 += 32) {
-        const int kk = kk0 + lane;
-        int fresh_n = 0;
-        if (kk < yrp[j + 1]) {
-          bool fresh;
-          hash_insert(tk, mask, yci[kk], &fresh);
-          fresh_n = fresh;
-        }
-        count += warp_sum(fresh_n);
-        if (2 * count > (int)tsz) {                    // the same for every lane
-          over = true;
-          break;
-        }
+    const int xs = __ldg(xrp + i), xe = __ldg(xrp + i + 1);
+    for (int k0 = xs; k0 < xe && !over; k0 += 32) {
+      SpgemmChunk c;
+      c.load(k0 + lane, xe, xci, nullptr, yrp);
+      for (int t0 = 0; t0 < c.total && !over; t0 += 32) {
+        const int t = t0 + lane, o = c.owner(t);
+        const int base = __shfl_sync(0xffffffffu, c.base, o);
+        bool fresh = false;
+        if (t < c.total) hash_insert(tk, tsz - 1, __ldg(yci + base + t), &fresh);
+        count += __popc(__ballot_sync(0xffffffffu, fresh));
+        over = TOP && 2 * count > SLOTS;               // the same for every lane
       }
     }
-    if (lane == 0) cnt[i] = over ? -1 : count;
+    if (lane == 0) {
+      cnt[i] = over ? -1 : count;
+      if (over) atomicAdd(nbig, 1);
+    }
     __syncwarp();
   }
 }
 
-// Numeric in shared memory for the rows with 0 <= cnt[i] <= kSpgemmSmSlots/2
-// (others skipped): emits row i's nonzero entries unsorted at crp_sym[i].
-__global__ void __launch_bounds__(32 * kSpgemmSmWarps)
-k_spgemm_numeric_sm(int m, const int *__restrict__ xrp, const int *__restrict__ xci,
+// Numeric for the rows with cnt in (lo, SLOTS/2]: the nonzero entries, columns
+// ascending, at cci/cv[crp_sym[i]..]; cnt_out[i] = number emitted.
+template <int SLOTS>
+__global__ void __launch_bounds__(32 * SpgemmClass<SLOTS>::warps)
+k_spgemm_numeric_sm(int m, int lo, const int *__restrict__ xrp, const int *__restrict__ xci,
                     const double *__restrict__ xv, const int *__restrict__ yrp,
                     const int *__restrict__ yci, const double *__restrict__ yv,
                     const int *__restrict__ cnt, const int64_t *__restrict__ crp_sym,
                     int *__restrict__ cci, double *__restrict__ cv, int *__restrict__ cnt_out) {
+  constexpr int W = SpgemmClass<SLOTS>::warps;
+  constexpr unsigned FULL = 0xffffffffu;
   extern __shared__ double spg_vals[];
   const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
-  double *tv = spg_vals + (size_t)wib * kSpgemmSmSlots;
-  int *tk = reinterpret_cast<int *>(spg_vals + (size_t)kSpgemmSmWarps * kSpgemmSmSlots) +
-            wib * kSpgemmSmSlots;
-  const int gw = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-  const int nw = (gridDim.x * blockDim.x) >> 5;
-  for (int i = gw; i < m; i += nw) {
-    const int c = cnt[i];
-    if (c < 0 || 2 * c > kSpgemmSmSlots) continue;
+  double *tv = spg_vals + (size_t)wib * SLOTS;
+  int *tk = reinterpret_cast<int *>(spg_vals + (size_t)W * SLOTS) + wib * SLOTS;
+  const int nw = gridDim.x * W;
+  for (int i = blockIdx.x * W + wib; i < m; i += nw) {
+    const int n = __ldg(cnt + i);
+    if (n <= lo || n > SLOTS / 2) continue;
     unsigned tsz = 32;
-    while (tsz < (unsigned)(2 * c + 1)) tsz <<= 1;
-    const unsigned mask = tsz - 1;
+    while (tsz < 2u * n) tsz <<= 1;
     for (unsigned s = lane; s < tsz; s += 32) { tk[s] = -1; tv[s] = 0.0; }
     __syncwarp();
-    for (int k = xrp[i]; k < xrp[i + 1]; ++k) {
-      const int j = xci[k];
-      const double a = xv[k];
-      for (int kk = yrp[j] + lane; kk < yrp[j + 1]; kk += 32) {
-        bool fresh;
-        const unsigned s = hash_insert(tk, mask, yci[kk], &fresh);
-        tv[s] = __dadd_rn(tv[s], __dmul_rn(a, yv[kk]));
+    const int xs = __ldg(xrp + i), xe = __ldg(xrp + i + 1);
+    for (int k0 = xs; k0 < xe; k0 += 32) {
+      SpgemmChunk c;
+      c.load(k0 + lane, xe, xci, xv, yrp);
+      for (int t0 = 0; t0 < c.total; t0 += 32) {
+        const int t = t0 + lane, o = c.owner(t);
+        const int base = __shfl_sync(FULL, c.base, o);
+        const double a = __shfl_sync(FULL, c.a, o);
+        const bool on = t < c.total;
+        int col = -1 - lane;                           // idle lanes: alone
+        double prod = 0.0;
+        if (on) {
+          col = __ldg(yci + base + t);
+          prod = __dmul_rn(a, __ldg(yv + base + t));
+        }
+        unsigned same = __match_any_sync(FULL, col);
+        const bool lead = on && (same & ((1u << lane) - 1u)) == 0;
+        unsigned s = 0;
+        double acc = 0.0;
+        if (lead) {
+          bool fresh;
+          s = hash_insert(tk, tsz - 1, col, &fresh);
+          acc = tv[s];
+        }
+        // the column's lanes in ascending order, one a round
+        const int rounds = __reduce_max_sync(FULL, lead ? __popc(same) : 0);
+        for (int q = 0; q < rounds; ++q) {
+          const double v = __shfl_sync(FULL, prod, same ? __ffs(same) - 1 : lane);
+          if (same) {
+            acc = __dadd_rn(acc, v);
+            same &= same - 1;
+          }
+        }
+        if (lead) tv[s] = acc;
+        __syncwarp();
       }
+    }
+    // the kept entries to the table's front (writes never pass the reads) ...
+    int kept = 0;
+    for (unsigned s0 = 0; s0 < tsz; s0 += 32) {
+      const int key = tk[s0 + lane];
+      const double val = tv[s0 + lane];
+      const bool keep = key != -1 && val != 0.0;
+      const unsigned bal = __ballot_sync(FULL, keep);
+      if (keep) {
+        const int at = kept + __popc(bal & ((1u << lane) - 1u));
+        tk[at] = key;
+        tv[at] = val;
+      }
+      kept += __popc(bal);
       __syncwarp();
     }
-    const int64_t base = crp_sym[i];
-    int emitted = 0;
-    for (unsigned s0 = 0; s0 < tsz; s0 += 32) {
-      const unsigned s = s0 + lane;
-      bool keep = false;
-      int key = -1;
-      double val = 0.0;
-      if (s < tsz) {
-        key = tk[s];
-        val = tv[s];
-        keep = key != -1 && val != 0.0;
+    // ... sorted by column (bitonic over the next power of two)
+    int N = 2;
+    while (N < kept) N <<= 1;
+    for (int t = kept + lane; t < N; t += 32) tk[t] = 0x7fffffff;
+    __syncwarp();
+    for (int k = 2; k <= N; k <<= 1)
+      for (int j = k >> 1; j > 0; j >>= 1) {
+        for (int t = lane; t < N / 2; t += 32) {
+          const int p = 2 * t - (t & (j - 1)), q = p + j;
+          const int kp = tk[p], kq = tk[q];
+          if ((kp > kq) == ((p & k) == 0)) {
+            const double vp = tv[p], vq = tv[q];
+            tk[p] = kq; tk[q] = kp;
+            tv[p] = vq; tv[q] = vp;
+          }
+        }
+        __syncwarp();
       }
-      const unsigned bal = __ballot_sync(0xffffffffu, keep);
-      if (keep) {
-        const int off = __popc(bal & ((1u << lane) - 1u));
-        cci[base + emitted + off] = key;
-        cv[base + emitted + off] = val;
-      }
-      emitted += __popc(bal);
+    const int64_t out = __ldg(crp_sym + i);
+    for (int t = lane; t < kept; t += 32) {
+      cci[out + t] = tk[t];
+      cv[out + t] = tv[t];
     }
-    if (lane == 0) cnt_out[i] = emitted;
+    if (lane == 0) cnt_out[i] = kept;
     __syncwarp();
   }
 }
 
-__global__ void k_compact_rows(int m, const int64_t *src_rp, const int *cnt, const int *crp,
-                               const int *sci, const double *sv, int *dci, double *dv) {
-  const int i = blockIdx.x;
-  if (i >= m) return;
-  const int64_t s = src_rp[i];
-  const int d = crp[i], c = cnt[i];
-  for (int k = threadIdx.x; k < c; k += blockDim.x) {
-    dci[d + k] = sci[s + k];
-    dv[d + k] = sv[s + k];
+template <int SLOTS>
+static void spgemm_symbolic(int m, int ncols, int lo, const int *xrp, const int *xci,
+                            const int *yrp, const int *yci, const int64_t *prod, int *cnt,
+                            int *nbig, cudaStream_t st) {
+  using C = SpgemmClass<SLOTS>;
+  const int grid = std::max(1, std::min<int>(ceil_div(m, C::warps), num_sms() * 16));
+  const size_t smem = (size_t)C::warps * SLOTS * sizeof(int);
+  CHRONOS_CUDA(cudaFuncSetAttribute(k_spgemm_symbolic_sm<SLOTS>,
+                                    cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  k_spgemm_symbolic_sm<SLOTS><<<grid, 32 * C::warps, smem, st>>>(m, ncols, lo, xrp, xci, yrp, yci,
+                                                                 prod, cnt, nbig);
+  CHRONOS_CHECK_LAUNCH();
+}
+
+template <int SLOTS>
+static void spgemm_numeric(int m, int lo, const int *xrp, const int *xci, const double *xv,
+                           const int *yrp, const int *yci, const double *yv, const int *cnt,
+                           const int64_t *crp_sym, int *cci, double *cv, int *cnt_out,
+                           cudaStream_t st) {
+  using C = SpgemmClass<SLOTS>;
+  const size_t smem = (size_t)C::warps * SLOTS * (sizeof(int) + sizeof(double));
+  CHRONOS_CUDA(cudaFuncSetAttribute(k_spgemm_numeric_sm<SLOTS>,
+                                    cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  const int grid = std::max(1, std::min<int>(ceil_div(m, C::warps), num_sms() * 16));
+  k_spgemm_numeric_sm<SLOTS><<<grid, 32 * C::warps, smem, st>>>(
+      m, lo, xrp, xci, xv, yrp, yci, yv, cnt, crp_sym, cci, cv, cnt_out);
+  CHRONOS_CHECK_LAUNCH();
+}
+
+// Rows from their places in the symbolic layout to the final one (a warp per
+// row); rows computed in global tables (sym_cnt beyond the largest class) come
+// from the second pair of arrays.
+__global__ void __launch_bounds__(256)
+k_compact_rows(int m, const int64_t *__restrict__ src_rp, const int *__restrict__ sym_cnt,
+               const int *__restrict__ crp, const int *__restrict__ sci,
+               const double *__restrict__ sv, const int *__restrict__ bci,
+               const double *__restrict__ bv, int *__restrict__ dci, double *__restrict__ dv) {
+  const int lane = threadIdx.x & 31;
+  const int nw = (gridDim.x * blockDim.x) >> 5;
+  for (int i = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; i < m; i += nw) {
+    const int64_t s = src_rp[i];
+    const int d = crp[i], c = crp[i + 1] - d;
+    const bool big = sym_cnt[i] > kSpgemmSmSlots / 2;
+    const int *ci = big ? bci : sci;
+    const double *v = big ? bv : sv;
+    for (int k = lane; k < c; k += 32) {
+      dci[d + k] = ci[s + k];
+      dv[d + k] = v[s + k];
+    }
   }
+}
+
+__global__ void k_narrow(int n, const int64_t *__restrict__ a, int *__restrict__ b) {
+  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x)
+    b[i] = (int)a[i];
+}
+
+// Exclusive sums of the n + 1 counts (the last one 0) into offs, 64-bit; the
+// negative marks of rows still to be counted add nothing.
+struct NonNegative {
+  __host__ __device__ int64_t operator()(int c) const { return c > 0 ? c : 0; }
+};
+static void scan_counts(int n, const int *cnt, int64_t *offs, DBuf<unsigned char> &tmp,
+                        cudaStream_t st) {
+  thrust::transform_iterator<NonNegative, const int *> in(cnt, NonNegative{});
+  size_t bytes = 0;
+  CHRONOS_CUDA(cub::DeviceScan::ExclusiveSum(nullptr, bytes, in, offs, n + 1, st));
+  if (tmp.size() < bytes) tmp.alloc(std::max<size_t>(bytes, 1));
+  CHRONOS_CUDA(cub::DeviceScan::ExclusiveSum(tmp.get(), bytes, in, offs, n + 1, st));
 }
 
 static unsigned next_pow2(uint64_t v) {
@@ -826,32 +979,34 @@ void spgemm_device(int m, int ncols, const int *xrp, const int *xci, const doubl
     *nnz_c = 0;
     return;
   }
-  DBuf<int64_t> dprod(m);
+  DBuf<int64_t> dprod((size_t)m + 1), drps((size_t)m + 1);
+  DBuf<unsigned char> tmp;
   k_spgemm_products<<<ceil_div(m, 256), 256, 0, st>>>(m, xrp, xci, yrp, dprod.get());
   CHRONOS_CHECK_LAUNCH();
-  // symbolic: in each warp's shared table first; rows whose distinct columns
-  // outgrow it (cnt = -1) again in global tables sized from their products
-  const size_t sym_smem = (size_t)kSpgemmSmWarps * kSpgemmSmSlots * sizeof(int);
-  const size_t num_smem = (size_t)kSpgemmSmWarps * kSpgemmSmSlots * (sizeof(int) + sizeof(double));
-  static const bool attrs = [&] {
-    CHRONOS_CUDA(cudaFuncSetAttribute(k_spgemm_symbolic_sm,
-                                      cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sym_smem));
-    CHRONOS_CUDA(cudaFuncSetAttribute(k_spgemm_numeric_sm,
-                                      cudaFuncAttributeMaxDynamicSharedMemorySize, (int)num_smem));
-    return true;
-  }();
-  (void)attrs;
-  const int sm_grid = (int)std::max<int64_t>(
-      1, std::min<int64_t>(ceil_div(m, kSpgemmSmWarps), (int64_t)num_sms() * 8));
-  DBuf<int> cnt(m);
-  k_spgemm_symbolic_sm<<<sm_grid, 32 * kSpgemmSmWarps, sym_smem, st>>>(m, ncols, xrp, xci, yrp,
-                                                                       yci, dprod.get(), cnt.get());
-  CHRONOS_CHECK_LAUNCH();
-  std::vector<int> cnt_h = cnt.to_host(st);
+  // symbolic: in each warp's shared table; rows whose distinct columns outgrow
+  // the largest (cnt = -1) again in global tables sized from their products.
+  // counts: cnt (m + 1), emitted (m + 1), rows beyond the tables
+  DBuf<int> counts(2 * ((size_t)m + 1) + 1);
+  int *cnt = counts.get(), *cnt2 = cnt + m + 1, *dnbig = cnt2 + m + 1;
+  counts.zero(st);
+  spgemm_symbolic<256>(m, ncols, 0, xrp, xci, yrp, yci, dprod.get(), cnt, dnbig, st);
+  spgemm_symbolic<1024>(m, ncols, 128, xrp, xci, yrp, yci, dprod.get(), cnt, dnbig, st);
+  spgemm_symbolic<kSpgemmSmSlots>(m, ncols, 512, xrp, xci, yrp, yci, dprod.get(), cnt, dnbig, st);
+  scan_counts(m, cnt, drps.get(), tmp, st);
+  int64_t total = 0;
+  int nbig = 0;
+  CHRONOS_CUDA(cudaMemcpyAsync(&total, drps.get() + m, sizeof(total), cudaMemcpyDeviceToHost, st));
+  CHRONOS_CUDA(cudaMemcpyAsync(&nbig, dnbig, sizeof(nbig), cudaMemcpyDeviceToHost, st));
+  CHRONOS_CUDA(cudaStreamSynchronize(st));
+  std::vector<int> cnt_h;
+  if (nbig > 0) {
+    cnt_h.resize(m);
+    CHRONOS_CUDA(cudaMemcpyAsync(cnt_h.data(), cnt, sizeof(int) * m, cudaMemcpyDeviceToHost, st));
+    CHRONOS_CUDA(cudaStreamSynchronize(st));
+  }
   std::vector<int> big;                                // rows for the global tables
-  for (int i = 0; i < m; ++i)
+  for (int i = 0; i < m && nbig > 0; ++i)
     if (cnt_h[i] < 0) big.push_back(i);
-  const int nbig = (int)big.size();
   DBuf<int> dbig;
   std::vector<int> bounds{0};
   DBuf<int> keys;
@@ -890,62 +1045,76 @@ void spgemm_device(int m, int ncols, const int *xrp, const int *xci, const doubl
       const int t0 = bounds[c], t1 = bounds[c + 1];
       k_spgemm_symbolic<<<ceil_div((int64_t)(t1 - t0) * 32, 256), 256, 0, st>>>(
           t0, t1, dbig.get(), xrp, xci, yrp, yci, toff.get() + t0, tcap.get() + t0, keys.get(),
-          cnt.get());
+          cnt);
       CHRONOS_CHECK_LAUNCH();
     }
-    cnt_h = cnt.to_host(st);
+    scan_counts(m, cnt, drps.get(), tmp, st);
+    CHRONOS_CUDA(cudaMemcpyAsync(&total, drps.get() + m, sizeof(total), cudaMemcpyDeviceToHost,
+                                 st));
+    CHRONOS_CUDA(cudaStreamSynchronize(st));
   }
-  std::vector<int64_t> rps(m + 1, 0);
-  for (int i = 0; i < m; ++i) rps[i + 1] = rps[i] + cnt_h[i];
-  DBuf<int64_t> drps(m + 1);
-  drps.upload(rps, st);
-  DBuf<int> sci(std::max<int64_t>(rps[m], 1));
-  DBuf<double> sv(std::max<int64_t>(rps[m], 1));
-  DBuf<int> cnt2(m);
-  k_spgemm_numeric_sm<<<sm_grid, 32 * kSpgemmSmWarps, num_smem, st>>>(
-      m, xrp, xci, xv, yrp, yci, yv, cnt.get(), drps.get(), sci.get(), sv.get(), cnt2.get());
+  DBuf<int> sci(std::max<int64_t>(total, 1)), sci2;
+  DBuf<double> sv(std::max<int64_t>(total, 1)), sv2;
+  spgemm_numeric<128>(m, 0, xrp, xci, xv, yrp, yci, yv, cnt, drps.get(), sci.get(), sv.get(), cnt2,
+                      st);
+  spgemm_numeric<512>(m, 64, xrp, xci, xv, yrp, yci, yv, cnt, drps.get(), sci.get(), sv.get(),
+                      cnt2, st);
+  spgemm_numeric<2048>(m, 256, xrp, xci, xv, yrp, yci, yv, cnt, drps.get(), sci.get(), sv.get(),
+                       cnt2, st);
+  spgemm_numeric<kSpgemmSmSlots>(m, 1024, xrp, xci, xv, yrp, yci, yv, cnt, drps.get(), sci.get(),
+                                 sv.get(), cnt2, st);
+  if (nbig > 0) {
+    for (size_t c = 0; c + 1 < bounds.size(); ++c) {
+      const int t0 = bounds[c], t1 = bounds[c + 1];
+      k_spgemm_numeric<<<ceil_div((int64_t)(t1 - t0) * 32, 256), 256, 0, st>>>(
+          t0, t1, dbig.get(), xrp, xci, xv, yrp, yci, yv, toff.get() + t0, tcap.get() + t0,
+          keys.get(), vals.get(), drps.get(), sci.get(), sv.get(), cnt2);
+      CHRONOS_CHECK_LAUNCH();
+    }
+    // their segments sorted by column into the second pair of arrays
+    std::vector<int64_t> rps((size_t)m + 1), sb(nbig), se(nbig);
+    std::vector<int> got(m);
+    drps.download(rps.data(), (size_t)m + 1, st);
+    CHRONOS_CUDA(cudaMemcpyAsync(got.data(), cnt2, sizeof(int) * m, cudaMemcpyDeviceToHost, st));
+    CHRONOS_CUDA(cudaStreamSynchronize(st));
+    for (int t = 0; t < nbig; ++t) {
+      sb[t] = rps[big[t]];
+      se[t] = sb[t] + got[big[t]];
+    }
+    DBuf<int64_t> dsb, dse;
+    dsb.upload(sb, st);
+    dse.upload(se, st);
+    sci2.alloc(total);
+    sv2.alloc(total);
+    size_t bytes = 0;
+    CHRONOS_CUDA(cub::DeviceSegmentedSort::SortPairs(nullptr, bytes, sci.get(), sci2.get(),
+                                                     sv.get(), sv2.get(), total, nbig, dsb.get(),
+                                                     dse.get(), st));
+    if (tmp.size() < bytes) tmp.alloc(std::max<size_t>(bytes, 1));
+    CHRONOS_CUDA(cub::DeviceSegmentedSort::SortPairs(tmp.get(), bytes, sci.get(), sci2.get(),
+                                                     sv.get(), sv2.get(), total, nbig, dsb.get(),
+                                                     dse.get(), st));
+    CHRONOS_CUDA(cudaStreamSynchronize(st));   // dsb, dse leave this scope
+  }
+  scan_counts(m, cnt2, dprod.get(), tmp, st);    // the product counts have served
+  int64_t nnz = 0;
+  CHRONOS_CUDA(cudaMemcpyAsync(&nnz, dprod.get() + m, sizeof(nnz), cudaMemcpyDeviceToHost, st));
+  CHRONOS_CUDA(cudaStreamSynchronize(st));
+  CHRONOS_REQUIRE(nnz < INT32_MAX, CHRONOS_ENOTSUP, "sparse product exceeds 2^31 entries");
+  k_narrow<<<std::min<int>(ceil_div(m + 1, 256), num_sms() * 8), 256, 0, st>>>(m + 1, dprod.get(),
+                                                                               crp.get());
   CHRONOS_CHECK_LAUNCH();
-  for (size_t c = 0; c + 1 < bounds.size() && nbig > 0; ++c) {
-    const int t0 = bounds[c], t1 = bounds[c + 1];
-    k_spgemm_numeric<<<ceil_div((int64_t)(t1 - t0) * 32, 256), 256, 0, st>>>(
-        t0, t1, dbig.get(), xrp, xci, xv, yrp, yci, yv, toff.get() + t0, tcap.get() + t0,
-        keys.get(), vals.get(), drps.get(), sci.get(), sv.get(), cnt2.get());
+  if (nnz == total && nbig == 0) {             // nothing dropped: the rows lie where they belong
+    cci = std::move(sci);
+    cv = std::move(sv);
+  } else {
+    cci.alloc(std::max<int64_t>(nnz, 1));
+    cv.alloc(std::max<int64_t>(nnz, 1));
+    k_compact_rows<<<std::min<int>(ceil_div(m, 8), num_sms() * 16), 256, 0, st>>>(
+        m, drps.get(), cnt, crp.get(), sci.get(), sv.get(), nbig ? sci2.get() : sci.get(),
+        nbig ? sv2.get() : sv.get(), cci.get(), cv.get());
     CHRONOS_CHECK_LAUNCH();
   }
-  std::vector<int> cnt2_h = cnt2.to_host(st);
-  // Sort every row segment [rps[i], rps[i]+cnt2[i]) by column.
-  {
-    DBuf<int64_t> seg_end(m);
-    std::vector<int64_t> se(m);
-    for (int i = 0; i < m; ++i) se[i] = rps[i] + cnt2_h[i];
-    seg_end.upload(se, st);
-    const int64_t total = rps[m];
-    DBuf<int> sci2(std::max<int64_t>(total, 1));
-    DBuf<double> sv2(std::max<int64_t>(total, 1));
-    size_t tmp_bytes = 0;
-    CHRONOS_CUDA(cub::DeviceSegmentedSort::SortPairs(nullptr, tmp_bytes, sci.get(), sci2.get(),
-                                                     sv.get(), sv2.get(), total, m, drps.get(),
-                                                     seg_end.get(), st));
-    DBuf<unsigned char> tmp(std::max<size_t>(tmp_bytes, 1));
-    CHRONOS_CUDA(cub::DeviceSegmentedSort::SortPairs(tmp.get(), tmp_bytes, sci.get(), sci2.get(),
-                                                     sv.get(), sv2.get(), total, m, drps.get(),
-                                                     seg_end.get(), st));
-    sci = std::move(sci2);
-    sv = std::move(sv2);
-  }
-  std::vector<int> crp_h(m + 1, 0);
-  for (int i = 0; i < m; ++i) {
-    const int64_t t = (int64_t)crp_h[i] + cnt2_h[i];
-    CHRONOS_REQUIRE(t < INT32_MAX, CHRONOS_ENOTSUP, "sparse product exceeds 2^31 entries");
-    crp_h[i + 1] = (int)t;
-  }
-  crp.upload(crp_h, st);
-  const int64_t nnz = crp_h[m];
-  cci.alloc(std::max<int64_t>(nnz, 1));
-  cv.alloc(std::max<int64_t>(nnz, 1));
-  k_compact_rows<<<m, 128, 0, st>>>(m, drps.get(), cnt2.get(), crp.get(), sci.get(), sv.get(),
-                                    cci.get(), cv.get());
-  CHRONOS_CHECK_LAUNCH();
   CHRONOS_CUDA(cudaStreamSynchronize(st));
   *nnz_c = nnz;
 }
@@ -1155,6 +1324,35 @@ void csr_transpose_device(int nrows, int ncols, int64_t nnz64, const int *rp, co
     CHRONOS_CHECK_LAUNCH();
     CHRONOS_CUDA(cudaStreamSynchronize(st));
   }
+}
+
+// A warp per row, coalesced along the columns.
+__global__ void __launch_bounds__(256)
+k_csr_check(int n, int ncols, const int *__restrict__ rp, const int *__restrict__ ci, int *bad) {
+  const int lane = threadIdx.x & 31;
+  const int nw = (gridDim.x * blockDim.x) >> 5;
+  int f = 0;
+  for (int i = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; i < n; i += nw) {
+    const int s = rp[i], e = rp[i + 1];
+    for (int k = s + lane; k < e; k += 32) {
+      const int c = ci[k];
+      if (c < 0 || c >= ncols) f |= 1;
+      if (k > s && ci[k - 1] >= c) f |= 2;
+    }
+  }
+  if (f) atomicOr(bad, f);
+}
+
+int csr_check_device(int nrows, int ncols, const int *rp, const int *ci, cudaStream_t st) {
+  DBuf<int> bad(1);
+  bad.zero(st);
+  k_csr_check<<<std::max(1, std::min<int>(ceil_div(nrows, 8), num_sms() * 16)), 256, 0, st>>>(
+      nrows, ncols, rp, ci, bad.get());
+  CHRONOS_CHECK_LAUNCH();
+  int h = 0;
+  CHRONOS_CUDA(cudaMemcpyAsync(&h, bad.get(), sizeof(int), cudaMemcpyDeviceToHost, st));
+  CHRONOS_CUDA(cudaStreamSynchronize(st));
+  return h;
 }
 
 __global__ void k_row_span(int n, const int *__restrict__ rp, const int *__restrict__ ci,

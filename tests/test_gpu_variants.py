@@ -119,3 +119,38 @@ def test_block_of_small_levels_matches_columns(lib, nx, nrhs):
             x, it, _, flag, _ = h.pcg(B[:, j], tol=1e-11)
             assert flag == 0 and abs(int(its[j]) - it) <= 1
             assert np.linalg.norm(X[:, j] - x) <= 1e-8 * np.linalg.norm(x)
+
+
+def _random_csr(m, n, lens, rng, lo=-1.0, hi=1.0):
+    indptr = np.concatenate([[0], np.cumsum(lens)])
+    idx = np.concatenate([np.sort(rng.choice(n, k, replace=False)) for k in lens]) if len(lens) else []
+    return sp.csr_matrix((rng.uniform(lo, hi, indptr[-1]), np.asarray(idx, np.int64), indptr),
+                         shape=(m, n))
+
+
+@pytest.mark.parametrize("row_lens", [[0, 1, 2, 3], [5, 31, 32, 33, 64], [60, 130, 300],
+                                      [1, 600, 2100], [2047, 2049, 3000]])
+def test_galerkin_rows_of_every_table_size(lib, row_lens):
+    """A = diagonal blocks coupling P's rows so that rows of the products fill
+    the tables of every class and outgrow the largest: the same bits as a
+    row-wise Gustavson product (scipy's, exact zeros dropped)."""
+    rng = np.random.default_rng(len(row_lens) + sum(row_lens))
+    n, nc = 160, 4000
+    lens = rng.choice(row_lens, n)
+    P = _random_csr(n, nc, lens, rng)
+    P.data[rng.random(P.nnz) < 0.2] = 0.5          # exact cancellations against -0.5
+    P.data[rng.random(P.nnz) < 0.2] = -0.5
+    A = _random_csr(n, n, rng.integers(1, 7, n), rng)
+    A.data[rng.random(A.nnz) < 0.3] = 1.0
+    A = sp.csr_matrix(A + A.T)
+    A.sort_indices()
+    AP = sp.csr_matrix(A @ P)
+    AP.eliminate_zeros()
+    AP.sort_indices()
+    want = sp.csr_matrix(sp.csr_matrix(P.T) @ AP)
+    want.eliminate_zeros()
+    want.sort_indices()
+    got = cb.galerkin(A, P)
+    assert np.array_equal(got.indptr, want.indptr)
+    assert np.array_equal(got.indices, want.indices)
+    assert np.array_equal(got.data, want.data)
