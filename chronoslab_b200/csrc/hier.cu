@@ -778,11 +778,66 @@ static double tridiag_last_component(const std::vector<double> &a, const std::ve
 // largest.  Stops as ARPACK's dsaupd does for eigs(...,opts.tol): once the
 // Ritz pair's residual norm beta_j |s_j| (s the unit eigenvector of the
 // tridiagonal for theta) is at most tol |theta|.
+// The recurrence runs on the device, kLanczosBatch steps queued at a time, and
+// the host tests the steps of a batch in order afterwards: a synchronisation
+// and a host sum for each of a step's two dots were most of the setup's omega
+// phase (Poisson 32^3, three levels: 17 ms; queued 8.0 ms), and the steps
+// past the accepted one that a batch may run cost less than they.
+namespace {
+constexpr int kLanczosBatch = 8;
+
+// alpha = v'w into a[j]
+__global__ void __launch_bounds__(256)
+k_lanczos_alpha(int n, const double *__restrict__ v, const double *__restrict__ w, double *part,
+                unsigned *ticket, double *alpha) {
+  pdl_begin();
+  double s = 0.0;
+  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x)
+    s += v[i] * w[i];
+  double t[1] = {s};
+  grid_reduce<1>(t, part, ticket, StoreScalar{alpha});
+}
+
+// w -= alpha v + beta_prev vp, ||w||^2 into *b2 (b2_prev null on the first step)
+__global__ void __launch_bounds__(256)
+k_lanczos_update(int n, const double *__restrict__ v, const double *__restrict__ vp,
+                 double *__restrict__ w, const double *__restrict__ alpha,
+                 const double *__restrict__ b2_prev, double *part, unsigned *ticket, double *b2) {
+  pdl_begin();
+  const double al = *alpha, be = b2_prev ? sqrt(fmax(*b2_prev, 0.0)) : 0.0;
+  double s = 0.0;
+  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
+    double x = fma(-al, v[i], w[i]);
+    if (b2_prev) x = fma(-be, vp[i], x);
+    w[i] = x;
+    s += x * x;
+  }
+  double t[1] = {s};
+  grid_reduce<1>(t, part, ticket, StoreScalar{b2});
+}
+
+// v = w / beta
+__global__ void __launch_bounds__(256)
+k_lanczos_next(int n, const double *__restrict__ w, const double *__restrict__ b2,
+               double *__restrict__ v) {
+  pdl_begin();
+  const double s = 1.0 / sqrt(fmax(*b2, 0.0));
+  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x)
+    v[i] = s * w[i];
+}
+}  // namespace
+
 double lanczos_lmax(int n, const std::function<void(const double *, double *)> &mv, double tol,
                     int maxit, cudaStream_t st) {
-  DBuf<double> v(n), vp(n), w(n), scratch(256);
-  std::vector<double> v0(n);
+  const int grid = std::max(1, std::min(num_sms() * 4, (int)ceil_div(n, 256)));
+  // three vectors, alpha and beta^2 of every step, block partials
+  DBuf<double> work(3 * (size_t)n + 2 * (size_t)maxit + grid);
+  DBuf<unsigned> ticket(1);
+  ticket.zero(st);
+  double *v = work.get(), *vp = v + n, *w = vp + n, *a_d = w + n, *b2_d = a_d + maxit,
+         *part = b2_d + maxit;
   {
+    std::vector<double> v0(n);
     MT19937 r(5489u);
     double nrm = 0.0;
     for (int i = 0; i < n; ++i) {
@@ -791,25 +846,36 @@ double lanczos_lmax(int n, const std::function<void(const double *, double *)> &
     }
     nrm = std::sqrt(nrm);
     for (int i = 0; i < n; ++i) v0[i] /= nrm;
+    CHRONOS_CUDA(cudaMemcpyAsync(v, v0.data(), sizeof(double) * n, cudaMemcpyHostToDevice, st));
+    CHRONOS_CUDA(cudaStreamSynchronize(st));
   }
-  v.upload(v0, st);
-  vp.zero(st);
-  std::vector<double> a, b;
-  double theta = 0.0, beta = 0.0;
-  for (int j = 0; j < maxit; ++j) {
-    mv(v.get(), w.get());
-    const double alpha = device_dot(n, w.get(), v.get(), scratch.get(), st);
-    device_axpby(n, -alpha, v.get(), 1.0, w.get(), st);
-    if (j > 0) device_axpby(n, -beta, vp.get(), 1.0, w.get(), st);
-    a.push_back(alpha);
-    beta = std::sqrt(std::max(device_dot(n, w.get(), w.get(), scratch.get(), st), 0.0));
-    const double th = tridiag_lmax(a, b);
-    const bool conv = beta * tridiag_last_component(a, b, th) <= tol * std::fabs(th);
-    theta = th;
-    if (conv || beta <= 1e-300 * std::fabs(theta)) break;
-    b.push_back(beta);
-    std::swap(vp, v);                     // vp <- v
-    device_scale_copy(n, 1.0 / beta, w.get(), v.get(), st);
+  std::vector<double> a, b, got(2 * (size_t)maxit);
+  double theta = 0.0;
+  for (int j0 = 0; j0 < maxit; j0 += kLanczosBatch) {
+    const int j1 = std::min(maxit, j0 + kLanczosBatch);
+    for (int j = j0; j < j1; ++j) {
+      mv(v, w);
+      launch_pdl(k_lanczos_alpha, grid, 256, st, n, (const double *)v, (const double *)w, part,
+                 ticket.get(), a_d + j);
+      launch_pdl(k_lanczos_update, grid, 256, st, n, (const double *)v, (const double *)vp, w,
+                 (const double *)(a_d + j), j > 0 ? (const double *)(b2_d + j - 1) : nullptr, part,
+                 ticket.get(), b2_d + j);
+      launch_pdl(k_lanczos_next, grid, 256, st, n, (const double *)w, (const double *)(b2_d + j),
+                 vp);
+      std::swap(v, vp);                   // the new v; vp the one before
+    }
+    CHRONOS_CUDA(cudaMemcpyAsync(got.data(), a_d, sizeof(double) * 2 * maxit,
+                                 cudaMemcpyDeviceToHost, st));
+    CHRONOS_CUDA(cudaStreamSynchronize(st));
+    for (int j = j0; j < j1; ++j) {
+      a.push_back(got[j]);
+      const double beta = std::sqrt(std::max(got[(size_t)maxit + j], 0.0));
+      const double th = tridiag_lmax(a, b);
+      const bool conv = beta * tridiag_last_component(a, b, th) <= tol * std::fabs(th);
+      theta = th;
+      if (conv || beta <= 1e-300 * std::fabs(theta)) return theta;
+      b.push_back(beta);
+    }
   }
   return theta;
 }
@@ -1171,12 +1237,12 @@ void HierBuilder::end_level(int fl) {
     DBuf<double> t1(n), t2(n);
     Level *Lp = &L;
     auto mv = [&](const double *v, double *w) {
-      csr_apply<double, double, double, double, MODE_PLAIN, false>(
-          st, 8, n, Lp->Gt.rp, Lp->Gt.ci, Lp->Gt.v64, v, nullptr, t1.get(), 1.0);
-      csr_apply<double, double, double, double, MODE_PLAIN, false>(
-          st, 8, n, Lp->A.rp, Lp->A.ci, Lp->A.v64, t1.get(), nullptr, t2.get(), 1.0);
-      csr_apply<double, double, double, double, MODE_PLAIN, false>(
-          st, 8, n, Lp->G.rp, Lp->G.ci, Lp->G.v64, t2.get(), nullptr, w, 1.0);
+      mat_apply<double, double, double, double, MODE_PLAIN, false>(
+          st, Lp->Gt, Lp->Gt.v64.get(), v, (const double *)nullptr, t1.get(), 1.0);
+      op_apply<double, double, double, double, MODE_PLAIN, false>(
+          st, Lp->A, t1.get(), (const double *)nullptr, t2.get(), 1.0);
+      mat_apply<double, double, double, double, MODE_PLAIN, false>(
+          st, Lp->G, Lp->G.v64.get(), t2.get(), (const double *)nullptr, w, 1.0);
     };
     L.lambda = lanczos_lmax(n, mv, 5e-4, 200, st);
     L.omega = std::min(1.0, 1.9 / L.lambda);
