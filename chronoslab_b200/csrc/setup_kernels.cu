@@ -1123,38 +1123,172 @@ void spgemm_device(int m, int ncols, const int *xrp, const int *xci, const doubl
 // Dense coarse level
 // =============================================================================
 
-// Single-block right-looking Cholesky on an n x n column-major matrix.
-__global__ void __launch_bounds__(1024) k_dense_cholesky(int n, double *A, int *info) {
-  __shared__ int bad;
-  const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5, nw = blockDim.x >> 5;
-  if (tid == 0) { bad = 0; *info = 0; }
-  __syncthreads();
-  for (int k = 0; k < n; ++k) {
-    if (tid == 0) {
-      const double d = A[(size_t)k * n + k];
-      if (!(d > 0.0)) bad = k + 1;
-      else A[(size_t)k * n + k] = sqrt(d);
+// Blocked right-looking Cholesky, 32-column panels: k_chol_panel factors the
+// diagonal block (every block of the grid for itself, in one warp's registers)
+// and solves its 64 rows of the panel against it, k_chol_update subtracts the
+// panel's outer product from the trailing lower tiles.  The inverse of the
+// factor is put together from its 32 x 32 diagonal blocks' by doubling, and
+// A^-1 = X'X, all on 64 x 64 FP64 tiles.  One thread block for the whole
+// factorisation and a block per column for the inverse, a barrier per column,
+// took 53 ms for the coarsest level of diffusion 36^3 (about 950 rows), its assembly
+// and upload included; now 4.7 ms.
+constexpr int kCholNb = 32;
+
+// c += op(A) op(B) over k in [k0, k1): rows i0 + tx + 16 r, columns
+// j0 + ty + 16 q of a 64 x 64 tile; la(i, k) and lb(k, j) give 0 outside.
+// KA / KB: the operand is contiguous along k.
+template <bool KA, bool KB, typename LA, typename LB>
+__device__ __forceinline__ void tile_gemm(int i0, int j0, int k0, int k1, LA la, LB lb,
+                                          double (&c)[4][4]) {
+  __shared__ double As[16][65], Bs[16][65];
+  const int tid = threadIdx.x, tx = tid & 15, ty = tid >> 4;
+  for (int k = k0; k < k1; k += 16) {
+#pragma unroll
+    for (int u = 0; u < 4; ++u) {
+      const int e = tid + 256 * u;
+      const int ia = KA ? e >> 4 : e & 63, ka = KA ? e & 15 : e >> 6;
+      const int jb = KB ? e >> 4 : e & 63, kb = KB ? e & 15 : e >> 6;
+      As[ka][ia] = k + ka < k1 ? la(i0 + ia, k + ka) : 0.0;
+      Bs[kb][jb] = k + kb < k1 ? lb(k + kb, j0 + jb) : 0.0;
     }
     __syncthreads();
-    if (bad) break;
-    const double dk = A[(size_t)k * n + k];
-    for (int i = k + 1 + tid; i < n; i += blockDim.x) A[(size_t)k * n + i] /= dk;
-    __syncthreads();
-    for (int j = k + 1 + wid; j < n; j += nw) {
-      const double ljk = A[(size_t)k * n + j];
-      for (int i = j + lane; i < n; i += 32) A[(size_t)j * n + i] -= A[(size_t)k * n + i] * ljk;
+#pragma unroll
+    for (int kk = 0; kk < 16; ++kk) {
+      double av[4], bv[4];
+#pragma unroll
+      for (int r = 0; r < 4; ++r) {
+        av[r] = As[kk][tx + 16 * r];
+        bv[r] = Bs[kk][ty + 16 * r];
+      }
+#pragma unroll
+      for (int r = 0; r < 4; ++r)
+#pragma unroll
+        for (int q = 0; q < 4; ++q) c[r][q] = fma(av[r], bv[q], c[r][q]);
     }
     __syncthreads();
   }
-  if (tid == 0) *info = bad;
-  // zero the strict upper triangle
-  for (int j = 1 + wid; j < n; j += nw)
-    for (int i = lane; i < j; i += 32) A[(size_t)j * n + i] = 0.0;
+}
+
+// Panel [k0, k0 + nb): D receives the diagonal block's factor (32 x 32, column
+// by column; the other blocks of the grid still read A's), A the rows below it.
+// *info: the 1-based index of the first non-positive pivot.
+__global__ void __launch_bounds__(256)
+k_chol_panel(int n, int k0, int nb, double *A, double *D, int *info) {
+  constexpr unsigned FULL = 0xffffffffu;
+  __shared__ double Ls[kCholNb][kCholNb + 1], Xs[kCholNb][65];
+  __shared__ int bad;
+  const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
+  if (*info) return;
+  const int r0 = k0 + nb + blockIdx.x * 64;
+  for (int e = tid; e < nb * 64; e += 256) {
+    const int i = e & 63, j = e >> 6;
+    Xs[j][i] = r0 + i < n ? A[(size_t)(k0 + j) * n + r0 + i] : 0.0;
+  }
+  if (wid == 0) {
+    double R[kCholNb];
+#pragma unroll
+    for (int c = 0; c < kCholNb; ++c)
+      R[c] = (lane < nb && c <= lane) ? A[(size_t)(k0 + c) * n + k0 + lane]
+                                      : (c == lane ? 1.0 : 0.0);
+    int first = 0;
+#pragma unroll
+    for (int k = 0; k < kCholNb; ++k) {
+      const double d = __shfl_sync(FULL, R[k], k);
+      if (!(d > 0.0) && first == 0) first = k0 + k + 1;
+      const double s = sqrt(d), l = R[k] / s;
+      R[k] = lane == k ? s : l;
+#pragma unroll
+      for (int c = k + 1; c < kCholNb; ++c) {
+        const double v = __shfl_sync(FULL, l, c);
+        if (lane >= c) R[c] = fma(-l, v, R[c]);
+      }
+    }
+    if (lane == 0) bad = first;
+#pragma unroll
+    for (int c = 0; c < kCholNb; ++c) Ls[lane][c] = c <= lane ? R[c] : 0.0;
+  }
+  __syncthreads();
+  if (blockIdx.x == 0) {
+    for (int e = tid; e < kCholNb * kCholNb; e += 256) D[e] = Ls[e & 31][e >> 5];
+    if (tid == 0 && bad) *info = bad;
+  }
+  if (bad) return;
+  // row x of the panel: x L' = a, lane j its entry j; a warp's eight rows together
+  double L[kCholNb];
+#pragma unroll
+  for (int c = 0; c < kCholNb; ++c) L[c] = Ls[lane][c];
+  const double inv = 1.0 / Ls[lane][lane];
+  double x[8];
+#pragma unroll
+  for (int q = 0; q < 8; ++q) x[q] = lane < nb ? Xs[lane][wid * 8 + q] : 0.0;
+#pragma unroll
+  for (int k = 0; k < kCholNb; ++k) {
+#pragma unroll
+    for (int q = 0; q < 8; ++q) {
+      const double xk = __shfl_sync(FULL, x[q] * inv, k);
+      x[q] = lane == k ? xk : lane > k ? fma(-L[k], xk, x[q]) : x[q];
+    }
+  }
+  if (lane < nb)
+#pragma unroll
+    for (int q = 0; q < 8; ++q) Xs[lane][wid * 8 + q] = x[q];
+  __syncthreads();
+  for (int e = tid; e < nb * 64; e += 256) {
+    const int i = e & 63, j = e >> 6;
+    if (r0 + i < n) A[(size_t)(k0 + j) * n + r0 + i] = Xs[j][i];
+  }
+}
+
+// Lower tiles of the trailing matrix [t0, n)^2 minus the panel's X X'.
+__global__ void __launch_bounds__(256)
+k_chol_update(int n, int k0, int t0, double *A, const int *info) {
+  if (*info || blockIdx.y < blockIdx.x) return;
+  const int i0 = t0 + blockIdx.y * 64, j0 = t0 + blockIdx.x * 64;
+  double c[4][4] = {};
+  tile_gemm<false, false>(
+      i0, j0, k0, t0, [&](int i, int k) { return i < n ? A[(size_t)k * n + i] : 0.0; },
+      [&](int k, int j) { return j < n ? A[(size_t)k * n + j] : 0.0; }, c);
+  const int tx = threadIdx.x & 15, ty = threadIdx.x >> 4;
+#pragma unroll
+  for (int r = 0; r < 4; ++r)
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+      const int i = i0 + tx + 16 * r, j = j0 + ty + 16 * q;
+      if (i < n && j < n) A[(size_t)j * n + i] -= c[r][q];
+    }
+}
+
+// The diagonal blocks' factors into place, the strict upper triangle zero.
+__global__ void __launch_bounds__(256)
+k_chol_finish(int n, double *A, const double *__restrict__ D) {
+  for (int64_t e = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; e < (int64_t)n * n;
+       e += (int64_t)gridDim.x * blockDim.x) {
+    const int i = (int)(e % n), j = (int)(e / n), b = j / kCholNb;
+    if (i < j) A[e] = 0.0;
+    else if (i / kCholNb == b)
+      A[e] = D[(size_t)b * kCholNb * kCholNb + (j % kCholNb) * kCholNb + i % kCholNb];
+  }
 }
 
 int dense_cholesky_device(int n, double *A, cudaStream_t st) {
+  if (n <= 0) return 0;
+  const int np = ceil_div(n, kCholNb);
+  DBuf<double> D((size_t)np * kCholNb * kCholNb);
   DBuf<int> info(1);
-  k_dense_cholesky<<<1, 1024, 0, st>>>(n, A, info.get());
+  info.zero(st);
+  for (int p = 0; p < np; ++p) {
+    const int k0 = p * kCholNb, nb = std::min(kCholNb, n - k0), rest = n - k0 - nb;
+    k_chol_panel<<<std::max(1u, ceil_div(rest, 64)), 256, 0, st>>>(
+        n, k0, nb, A, D.get() + (size_t)p * kCholNb * kCholNb, info.get());
+    CHRONOS_CHECK_LAUNCH();
+    if (rest > 0) {
+      const unsigned t = ceil_div(rest, 64);
+      k_chol_update<<<dim3(t, t), 256, 0, st>>>(n, k0, k0 + nb, A, info.get());
+      CHRONOS_CHECK_LAUNCH();
+    }
+  }
+  k_chol_finish<<<std::min<int64_t>(ceil_div((int64_t)n * n, 256), (int64_t)num_sms() * 8), 256, 0,
+                  st>>>(n, A, D.get());
   CHRONOS_CHECK_LAUNCH();
   int h = 0;
   CHRONOS_CUDA(cudaMemcpyAsync(&h, info.get(), sizeof(int), cudaMemcpyDeviceToHost, st));
@@ -1162,52 +1296,90 @@ int dense_cholesky_device(int n, double *A, cudaStream_t st) {
   return h;
 }
 
-// Column j of L^{-1} by forward substitution (one block per column).
-__global__ void k_tri_inverse(int n, const double *L, double *X) {
-  extern __shared__ double xs[];
-  const int j = blockIdx.x;
-  for (int i = threadIdx.x; i < n; i += blockDim.x) xs[i] = (i == j) ? 1.0 : 0.0;
-  __syncthreads();
-  for (int k = j; k < n; ++k) {
-    const double xk = xs[k] / L[(size_t)k * n + k];
-    __syncthreads();
-    if (threadIdx.x == 0) xs[k] = xk;
-    for (int i = k + 1 + threadIdx.x; i < n; i += blockDim.x) xs[i] -= L[(size_t)k * n + i] * xk;
-    __syncthreads();
+// Inverses of L's 32 x 32 diagonal blocks (a warp each, lane j column j).
+__global__ void __launch_bounds__(32)
+k_tri_inverse_diag(int n, const double *__restrict__ L, double *__restrict__ X) {
+  __shared__ double Ls[kCholNb][kCholNb + 1];
+  const int k0 = blockIdx.x * kCholNb, nb = min(kCholNb, n - k0), lane = threadIdx.x;
+  for (int j = 0; j < kCholNb; ++j)
+    Ls[lane][j] = (lane < nb && j < nb && j <= lane) ? L[(size_t)(k0 + j) * n + k0 + lane]
+                                                     : (lane == j ? 1.0 : 0.0);
+  __syncwarp();
+  double x[kCholNb];
+#pragma unroll
+  for (int i = 0; i < kCholNb; ++i) {
+    double t = i == lane ? 1.0 : 0.0;
+#pragma unroll
+    for (int k = 0; k < i; ++k) t = fma(-Ls[i][k], x[k], t);
+    x[i] = t / Ls[i][i];
   }
-  for (int i = threadIdx.x; i < n; i += blockDim.x) X[(size_t)j * n + i] = xs[i];
+  if (lane < nb)
+#pragma unroll
+    for (int i = 0; i < kCholNb; ++i)
+      if (i < nb) X[(size_t)(k0 + lane) * n + k0 + i] = x[i];
 }
 
-// W = X^T X with X = L^{-1} lower (column-major); 16x16 tiles.
-__global__ void k_gram(int n, const double *X, double *W) {
-  __shared__ double a[16][17], b[16][17];
-  const int tx = threadIdx.x, ty = threadIdx.y;
-  const int i = blockIdx.y * 16 + ty, j = blockIdx.x * 16 + tx;
-  double s = 0.0;
-  const int kstart = max(blockIdx.y * 16, blockIdx.x * 16);
-  for (int k0 = (kstart / 16) * 16; k0 < n; k0 += 16) {
-    const int ka = k0 + tx, kb = k0 + ty;
-    const int ci = blockIdx.y * 16 + ty, cj = blockIdx.x * 16 + tx;
-    a[ty][tx] = (ci < n && ka < n) ? X[(size_t)ci * n + ka] : 0.0;   // X[ka][ci]
-    b[ty][tx] = (cj < n && kb < n) ? X[(size_t)cj * n + kb] : 0.0;   // X[kb][cj]
-    __syncthreads();
+// One doubling of the inverse: with the s x s diagonal blocks of X done, the
+// blocks below them, X21 = -X22 (L21 X11); FIRST computes T = L21 X11.
+template <bool FIRST>
+__global__ void __launch_bounds__(256)
+k_tri_inverse_merge(int n, int s, const double *__restrict__ L, double *X, double *T) {
+  const int c0 = blockIdx.z * 2 * s, b0 = c0 + s, b1 = min(n, b0 + s);
+  const int i0 = b0 + blockIdx.y * 64, j0 = c0 + blockIdx.x * 64;
+  if (i0 >= b1) return;
+  double c[4][4] = {};
+  if (FIRST)
+    tile_gemm<false, true>(
+        i0, j0, j0, b0, [&](int i, int k) { return i < b1 ? L[(size_t)k * n + i] : 0.0; },
+        [&](int k, int j) { return j < b0 ? X[(size_t)j * n + k] : 0.0; }, c);
+  else
+    tile_gemm<false, true>(
+        i0, j0, b0, min(b1, i0 + 64), [&](int i, int k) { return i < b1 ? X[(size_t)k * n + i] : 0.0; },
+        [&](int k, int j) { return j < b0 ? T[(size_t)j * n + k] : 0.0; }, c);
+  const int tx = threadIdx.x & 15, ty = threadIdx.x >> 4;
 #pragma unroll
-    for (int kk = 0; kk < 16; ++kk) s += a[ty][kk] * b[kk][tx];
-    __syncthreads();
-  }
-  if (i < n && j < n) W[(size_t)i * n + j] = s;
+  for (int r = 0; r < 4; ++r)
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+      const int i = i0 + tx + 16 * r, j = j0 + ty + 16 * q;
+      if (i < b1 && j < b0) (FIRST ? T : X)[(size_t)j * n + i] = FIRST ? c[r][q] : -c[r][q];
+    }
+}
+
+// W = X'X with X lower triangular, every tile from its first nonzero row on.
+__global__ void __launch_bounds__(256)
+k_gram(int n, const double *__restrict__ X, double *__restrict__ W) {
+  const int i0 = blockIdx.y * 64, j0 = blockIdx.x * 64;
+  double c[4][4] = {};
+  tile_gemm<true, true>(
+      i0, j0, max(i0, j0), n, [&](int i, int k) { return i < n ? X[(size_t)i * n + k] : 0.0; },
+      [&](int k, int j) { return j < n ? X[(size_t)j * n + k] : 0.0; }, c);
+  const int tx = threadIdx.x & 15, ty = threadIdx.x >> 4;
+#pragma unroll
+  for (int r = 0; r < 4; ++r)
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+      const int i = i0 + tx + 16 * r, j = j0 + ty + 16 * q;
+      if (i < n && j < n) W[(size_t)j * n + i] = c[r][q];
+    }
 }
 
 void dense_inverse_from_chol(int n, const double *L, double *W, cudaStream_t st) {
+  CHRONOS_REQUIRE((size_t)n * sizeof(double) <= 200 * 1024, CHRONOS_ENOTSUP,
+                  "coarsest level too large for the dense solve");
   DBuf<double> X((size_t)n * n);
-  const size_t sm = (size_t)n * sizeof(double);
-  CHRONOS_REQUIRE(sm <= 200 * 1024, CHRONOS_ENOTSUP, "coarsest level too large for the dense solve");
-  if (sm > 48 * 1024)
-    CHRONOS_CUDA(cudaFuncSetAttribute(k_tri_inverse, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm));
-  k_tri_inverse<<<n, 256, sm, st>>>(n, L, X.get());
+  X.zero(st);
+  k_tri_inverse_diag<<<ceil_div(n, kCholNb), 32, 0, st>>>(n, L, X.get());
   CHRONOS_CHECK_LAUNCH();
-  dim3 grid(ceil_div(n, 16), ceil_div(n, 16)), blk(16, 16);
-  k_gram<<<grid, blk, 0, st>>>(n, X.get(), W);
+  for (int s = kCholNb; s < n; s *= 2) {       // T in W, which is written last
+    const unsigned t = ceil_div(s, 64), pairs = ceil_div(n - s, 2 * s);
+    k_tri_inverse_merge<true><<<dim3(t, t, pairs), 256, 0, st>>>(n, s, L, X.get(), W);
+    CHRONOS_CHECK_LAUNCH();
+    k_tri_inverse_merge<false><<<dim3(t, t, pairs), 256, 0, st>>>(n, s, L, X.get(), W);
+    CHRONOS_CHECK_LAUNCH();
+  }
+  const unsigned t = ceil_div(n, 64);
+  k_gram<<<dim3(t, t), 256, 0, st>>>(n, X.get(), W);
   CHRONOS_CHECK_LAUNCH();
   CHRONOS_CUDA(cudaStreamSynchronize(st));
 }

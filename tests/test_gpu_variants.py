@@ -154,3 +154,35 @@ def test_galerkin_rows_of_every_table_size(lib, row_lens):
     assert np.array_equal(got.indptr, want.indptr)
     assert np.array_equal(got.indices, want.indices)
     assert np.array_equal(got.data, want.data)
+
+
+@pytest.mark.parametrize("n", [1, 2, 31, 32, 33, 63, 64, 65, 96, 97, 200, 257, 700])
+def test_dense_cholesky_edges(lib, n):
+    """Panels and tiles at their edges: |L L' - A| within 4 n eps |A| and the
+    strict upper triangle zero; a negative pivot is refused wherever it lies."""
+    rng = np.random.default_rng(n)
+    B = rng.standard_normal((n, n))
+    A = B @ B.T + n * np.eye(n)
+    L = cb.dense_chol(A)
+    assert not np.any(np.triu(L, 1))
+    assert np.abs(L @ L.T - A).max() <= 4 * n * 2.2e-16 * np.abs(A).max()
+    for k in {0, n // 2, n - 1}:
+        C = A.copy()
+        C[k, k] = -1.0
+        with pytest.raises(cb.ChronosError) as e:
+            cb.dense_chol(C)
+        assert e.value.code == -4
+
+
+@pytest.mark.parametrize("nx", [3, 4, 5, 7, 9])
+def test_single_level_vcycle_is_the_dense_solve(lib, nx):
+    """A problem no larger than the coarsest level: the V-cycle is A^-1 b, to
+    the condition of the operator (below 200 here) times n eps."""
+    from chronoslab_b200 import problems as PB
+    A = PB.poisson7(nx)
+    b = np.random.default_rng(nx).standard_normal(nx ** 3)
+    with cb.Hierarchy(A, np.ones(nx ** 3), cb.params(precision=cb.CHRONOS_FP64, ntv=1)) as h:
+        assert h.nlevels == 1
+        x = h.vcycle(b)
+    want = np.linalg.solve(A.toarray(), b)
+    assert np.linalg.norm(x - want) <= 200 * nx ** 3 * 2.2e-16 * np.linalg.norm(want)
