@@ -154,15 +154,15 @@ int chronos_batch_setup(const chronos_params *prm, int nprob, const int *n,
     std::vector<int> flag_of(nprob, 0);
     if (!jobs.empty()) {
       cudaStream_t bst;
-      CHRONOS_CUDA(cudaStreamCreateWithFlags(&bst, cudaStreamNonBlocking));
+      bst = stream_create();
       std::vector<int> fl;
       try {
         fl = fsai_numeric_batched(jobs, bst);
       } catch (...) {
-        cudaStreamDestroy(bst);
+        stream_destroy(bst);
         throw;
       }
-      cudaStreamDestroy(bst);
+      stream_destroy(bst);
       const double share = (now_seconds() - t1) / (double)jobs.size();
       for (size_t k = 0; k < batched.size(); ++k) {
         flag_of[batched[k]] = fl[k];
@@ -226,7 +226,7 @@ int chronos_batch_solve(chronos_batch *bt, const double *const *b_h, double *con
       CHRONOS_CUDA(cudaStreamSynchronize(h.st));
     }
     cudaStream_t fork;
-    CHRONOS_CUDA(cudaStreamCreateWithFlags(&fork, cudaStreamNonBlocking));
+    fork = stream_create();
     cudaEvent_t start;
     std::vector<cudaEvent_t> done(np);
     CHRONOS_CUDA(cudaEventCreate(&start));
@@ -260,7 +260,7 @@ int chronos_batch_solve(chronos_batch *bt, const double *const *b_h, double *con
     }
     cudaEventDestroy(start);
     for (auto &e : done) cudaEventDestroy(e);
-    cudaStreamDestroy(fork);
+    stream_destroy(fork);
     if (seconds) *seconds = ms * 1e-3;
   });
 }

@@ -617,6 +617,7 @@ static void block_solve(Hier &h, int m, const BlockIn &B, const double *X0_h, do
     // one iteration per graph launch from a host loop (profilers cannot see
     // the kernel nodes of a graph holding a conditional node); same kernels
     if (!s.exec) {
+      std::lock_guard<std::mutex> capturing(lib_streams().mu);
       CHRONOS_CUDA(cudaStreamBeginCapture(st, cudaStreamCaptureModeThreadLocal));
       try {
         capture_block_iteration<K>(h, s, 0, 0);
@@ -651,6 +652,7 @@ static void block_solve(Hier &h, int m, const BlockIn &B, const double *X0_h, do
       cudaGraphNode_t node;
       CHRONOS_CUDA(cudaGraphAddNode(&node, s.graph, nullptr, 0, &np));
       cudaGraph_t body = np.conditional.phGraph_out[0];
+      std::lock_guard<std::mutex> capturing(lib_streams().mu);
       CHRONOS_CUDA(cudaStreamBeginCaptureToGraph(st, body, nullptr, nullptr, 0,
                                                  cudaStreamCaptureModeThreadLocal));
       try {

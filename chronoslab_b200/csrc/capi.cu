@@ -122,8 +122,8 @@ static HostCSR from_csr0_any(int n, int ncols, const int *iat, const int *ja, co
 
 struct ScopedStream {
   cudaStream_t st = nullptr;
-  ScopedStream() { CHRONOS_CUDA(cudaStreamCreateWithFlags(&st, cudaStreamNonBlocking)); }
-  ~ScopedStream() { if (st) { cudaStreamSynchronize(st); cudaStreamDestroy(st); } }
+  ScopedStream() : st(stream_create()) {}
+  ~ScopedStream() { stream_destroy(st); }
 };
 
 // A caller's host CSR in device memory, as the setup kernels read it.
@@ -323,7 +323,7 @@ int chronos_coarsen_device(const chronos_params *prm, int n, const int *iat_h, c
     MT19937 rng((uint32_t)(prm->seed ? prm->seed : 5489));
     for (uint64_t k = 0; k < rng_skip; ++k) rng.next_res53();
     cudaStream_t st;
-    CHRONOS_CUDA(cudaStreamCreateWithFlags(&st, cudaStreamNonBlocking));
+    st = stream_create();
     try {
       DMat d;
       upload_csr(A, d, false, st);
@@ -337,10 +337,10 @@ int chronos_coarsen_device(const chronos_params *prm, int n, const int *iat_h, c
         *S = wrap_csr(std::move(Sm));
       }
     } catch (...) {
-      cudaStreamDestroy(st);
+      stream_destroy(st);
       throw;
     }
-    cudaStreamDestroy(st);
+    stream_destroy(st);
   });
 }
 

@@ -381,8 +381,7 @@ GroupSolve::~GroupSolve() {
   if (exec) cudaGraphExecDestroy(exec);
   if (graph) cudaGraphDestroy(graph);
   if (st) {
-    cudaStreamSynchronize(st);
-    cudaStreamDestroy(st);
+    stream_destroy(st);
   }
 }
 
@@ -390,7 +389,7 @@ std::unique_ptr<GroupSolve> group_build(const std::vector<std::unique_ptr<Hier>>
                                         const chronos_params &prm) {
   auto G = std::make_unique<GroupSolve>();
   GroupSolve &g = *G;
-  CHRONOS_CUDA(cudaStreamCreateWithFlags(&g.st, cudaStreamNonBlocking));
+  g.st = stream_create();
   cudaStream_t st = g.st;
   g.np = (int)hs.size();
   g.prm = prm;
@@ -678,6 +677,7 @@ void group_solve(GroupSolve &g, const std::vector<const double *> &b_h,
     // one iteration per graph launch from a host loop (profilers cannot see
     // the kernel nodes of a graph holding a conditional node); same kernels
     if (!g.exec) {
+      std::lock_guard<std::mutex> capturing(lib_streams().mu);
       CHRONOS_CUDA(cudaStreamBeginCapture(st, cudaStreamCaptureModeThreadLocal));
       try {
         group_capture_iteration(g, 0, 0, tol, itmax);
@@ -711,6 +711,7 @@ void group_solve(GroupSolve &g, const std::vector<const double *> &b_h,
       cudaGraphNode_t node;
       CHRONOS_CUDA(cudaGraphAddNode(&node, g.graph, nullptr, 0, &np_));
       cudaGraph_t body = np_.conditional.phGraph_out[0];
+      std::lock_guard<std::mutex> capturing(lib_streams().mu);
       CHRONOS_CUDA(cudaStreamBeginCaptureToGraph(st, body, nullptr, nullptr, 0,
                                                  cudaStreamCaptureModeThreadLocal));
       try {

@@ -69,7 +69,7 @@ Hier::~Hier() {
   if (pcg.graph) { cudaGraphDestroy(pcg.graph); pcg.graph = nullptr; }
   if (ev_in) cudaEventDestroy(ev_in);
   if (ev_out) cudaEventDestroy(ev_out);
-  if (st) cudaStreamDestroy(st);
+  stream_destroy(st);
 }
 
 CallerStream::CallerStream(Hier &h, void *stream)
@@ -1080,7 +1080,7 @@ HierBuilder::HierBuilder(const chronos_params &prm_in, HostCSR A0, int ntv0,
   h_->prm = prm;
   h_->precision = prm.precision;
   fp32_ = prm.precision == CHRONOS_FP32;
-  CHRONOS_CUDA(cudaStreamCreateWithFlags(&h_->st, cudaStreamNonBlocking));
+  h_->st = stream_create();
   nth_ = prm.nthread > 0 ? prm.nthread : 0;
   if (nth_ <= 0) {
 #ifdef _OPENMP
@@ -1554,7 +1554,7 @@ std::unique_ptr<Hier> load_hierarchy(const char *path) {
   h->prm = prm;
   h->precision = prm.precision;
   const bool fp32 = prm.precision == CHRONOS_FP32;
-  CHRONOS_CUDA(cudaStreamCreateWithFlags(&h->st, cudaStreamNonBlocking));
+  h->st = stream_create();
   cudaStream_t st = h->st;
   int nprev = -1;
   for (int l = 0; l < nlev; ++l) {
@@ -2236,6 +2236,7 @@ static void build_pcg_graph(Hier &h) {
     cudaGraphNode_t node;
     CHRONOS_CUDA(cudaGraphAddNode(&node, s.graph, nullptr, 0, &np));
     cudaGraph_t body = np.conditional.phGraph_out[0];
+    std::lock_guard<std::mutex> capturing(lib_streams().mu);
     CHRONOS_CUDA(cudaStreamBeginCaptureToGraph(st, body, nullptr, nullptr, 0,
                                                cudaStreamCaptureModeThreadLocal));
     try {
@@ -2249,6 +2250,7 @@ static void build_pcg_graph(Hier &h) {
     CHRONOS_CUDA(cudaGraphInstantiate(&s.exec, s.graph, 0));
     s.conditional = true;
   } else {
+    std::lock_guard<std::mutex> capturing(lib_streams().mu);
     CHRONOS_CUDA(cudaStreamBeginCapture(st, cudaStreamCaptureModeThreadLocal));
     try {
       capture_iteration(h, 0, 0);
