@@ -161,6 +161,20 @@ void upload_csr(const HostCSR &h, DMat &d, bool fp32, cudaStream_t st) {
   finish_csr(d, d.nnz >= kDeviceLayoutNnz ? nullptr : &h, fp32, st);
 }
 
+void adopt_csr(int nrows, int ncols, int64_t nnz, DBuf<int> &rp, DBuf<int> &ci, DBuf<double> &v,
+               DMat &d, bool fp32, cudaStream_t st) {
+  d.nrows = nrows;
+  d.ncols = ncols;
+  d.nnz = nnz;
+  d.rp = std::move(rp);
+  d.ci = std::move(ci);
+  d.v64 = std::move(v);
+  d.rp_h.resize((size_t)nrows + 1);
+  d.rp.download(d.rp_h.data(), (size_t)nrows + 1, st);
+  CHRONOS_CUDA(cudaStreamSynchronize(st));
+  finish_csr(d, nullptr, fp32, st);
+}
+
 static HostCSR download_csr(int nrows, int ncols, const DBuf<int> &rp, const DBuf<int> &ci,
                             const DBuf<double> &v, int64_t nnz, cudaStream_t st);
 
@@ -1392,15 +1406,25 @@ std::unique_ptr<Hier> build_hierarchy(const chronos_params &prm, HostCSR A0, int
 void tune_hierarchy(Hier &h) {
   const bool fp32 = h.precision == CHRONOS_FP32;
   const int fmt = h.prm.spmv_format;
-  // SpMV lane counts
-  for (auto &L : h.levels) {
-    autotune_lanes(L.A, fp32, h.st, fmt);
-    if (!L.coarsest) {
+  build_folds(h);
+  // SpMV lane counts of the operators that the cycle applies (level 1's also
+  // serve the outer product and other callers of its operators)
+  for (size_t l = 0; l < h.levels.size(); ++l) {
+    Level &L = h.levels[l];
+    Fold *F = L.fold.get();
+    if (F && F->form == FOLD_DENSE) continue;
+    if (l == 0 || !F || F->form != FOLD_ALL) autotune_lanes(L.A, fp32, h.st, fmt);
+    if (L.coarsest) continue;
+    if (l == 0 || !F) {
       autotune_lanes(L.G, fp32, h.st, fmt);
       autotune_lanes(L.Gt, fp32, h.st, fmt);
+    }
+    if (!F || F->form == FOLD_SMOOTH) {
       autotune_lanes(L.P, fp32, h.st, fmt);
       autotune_lanes(L.Pt, fp32, h.st, fmt);
     }
+    if (F && F->form != FOLD_ALL) autotune_lanes(F->Q, fp32, h.st, fmt);
+    if (F && F->form == FOLD_DOWN) autotune_lanes(F->R, fp32, h.st, fmt);
   }
   // the level-1 FP64 operator of the outer PCG
   if (fp32 && h.prm.exact_outer) autotune_lanes(h.levels[0].A, false, h.st);
@@ -1611,6 +1635,144 @@ __global__ void k_dot_store(int n, const double *a, const double *b, double *par
   grid_reduce<1>(v, part, ticket, StoreScalar{out});
 }
 
+// y = R b, a block per row: R's rows are the products of P' with two operators
+// and on the levels that end a hierarchy a few hundred of them hold thousands of
+// entries each (elasticity 24^3, FP64, 205 rows of 2270 entries: 77 us per PCG
+// iteration with a warp per row, 61 with a block).
+template <typename T, typename BT, bool I16>
+__global__ void __launch_bounds__(kApplyThreads)
+k_wide_rows(int n, const int *__restrict__ rp, const int *__restrict__ ci,
+            const int *__restrict__ cbase, const uint16_t *__restrict__ c16,
+            const T *__restrict__ v, const BT *__restrict__ b, T *__restrict__ y) {
+  pdl_begin();
+  __shared__ T red[kApplyThreads / 32];
+  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+  for (int row = blockIdx.x; row < n; row += gridDim.x) {
+    const int s = __ldg(rp + row), e = __ldg(rp + row + 1);
+    const T a = warp_sum(csr_row_dot<T, T, BT, kApplyThreads, I16>(
+        s + (int)threadIdx.x, e, I16 ? __ldg(cbase + row) : 0, ci, c16, v, b));
+    if (lane == 0) red[wid] = a;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+      T t = red[0];
+      for (int w = 1; w < kApplyThreads / 32; ++w) t += red[w];
+      y[row] = t;
+    }
+    __syncthreads();
+  }
+}
+
+// Restriction of a folded level: a block per row from an average row of a warp's
+// eight batches on, else the tuned row-group kernel.
+template <typename T, typename BT>
+static void restrict_apply(cudaStream_t st, const DMat &R, const BT *b, T *y) {
+  if (R.nnz < (int64_t)256 * R.nrows) {
+    mat_apply<T, BT, T, T, MODE_PLAIN, false>(st, R, vals<T>(R), b, nullptr, y, T(1));
+    return;
+  }
+  const int grid = std::min(R.nrows, num_sms() * 8);
+  launch_pdl(R.idx16 ? k_wide_rows<T, BT, true> : k_wide_rows<T, BT, false>, grid, kApplyThreads,
+             st, R.nrows, (const int *)R.rp.get(), (const int *)R.ci.get(),
+             (const int *)R.cbase.get(), (const uint16_t *)R.c16.get(), vals<T>(R), b, y);
+}
+
+// out = Q b + E e on a folded level, L lanes per row (and out . dw).
+template <typename T, typename BT, typename OT, int L, bool DOT, bool QI16, bool EI16>
+__global__ void __launch_bounds__(kApplyThreads)
+k_fold_apply(int n, const int *__restrict__ qrp, const int *__restrict__ qci,
+             const int *__restrict__ qbase, const uint16_t *__restrict__ q16,
+             const T *__restrict__ qv, const int *__restrict__ erp, const int *__restrict__ eci,
+             const int *__restrict__ ebase, const uint16_t *__restrict__ e16,
+             const T *__restrict__ ev, const BT *__restrict__ b, const T *__restrict__ e,
+             OT *__restrict__ out, const double *__restrict__ dw, double *part, unsigned *ticket,
+             double *dot_out) {
+  pdl_begin();
+  constexpr int R = 32 / L;
+  const int lane = threadIdx.x & 31, g = lane / L, gl = lane & (L - 1);
+  const int warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+  const int nwarps = (gridDim.x * blockDim.x) >> 5;
+  double dacc = 0.0;
+  for (int base = warp * R; base < n; base += nwarps * R) {     // warp-uniform trip count
+    const int row = base + g;
+    T a = T(0);
+    if (row < n) {
+      const int qs = __ldg(qrp + row), qe = __ldg(qrp + row + 1);
+      const int es = __ldg(erp + row), ee = __ldg(erp + row + 1);
+      const int qb = QI16 ? __ldg(qbase + row) : 0, eb = EI16 ? __ldg(ebase + row) : 0;
+      a = csr_row_dot<T, T, T, L, EI16>(es + gl, ee, eb, eci, e16, ev, e);
+      a += csr_row_dot<T, T, BT, L, QI16>(qs + gl, qe, qb, qci, q16, qv, b);
+    }
+    a = group_sum<L>(a);
+    if (row < n && gl == 0) {
+      const OT o = (OT)a;
+      out[row] = o;
+      if (DOT) dacc += (double)o * dw[row];
+    }
+  }
+  if (DOT) {
+    double vals[1] = {dacc};
+    grid_reduce<1>(vals, part, ticket, StoreScalar{dot_out});
+  }
+}
+
+template <typename T, typename BT, typename OT, bool DOT>
+static void fold_apply(cudaStream_t st, int lanes, const DMat &Q, const DMat &E, const BT *b,
+                       const T *e, OT *out, const double *dw, double *part, unsigned *tick,
+                       double *dot_out) {
+  const int n = Q.nrows;
+  const int grid = std::min<int>(ceil_div((int64_t)n * lanes, kApplyThreads), num_sms() * 8);
+  auto launch = [&](auto kern) {
+    launch_pdl(kern, grid, kApplyThreads, st, n, (const int *)Q.rp.get(), (const int *)Q.ci.get(),
+               (const int *)Q.cbase.get(), (const uint16_t *)Q.c16.get(), vals<T>(Q),
+               (const int *)E.rp.get(), (const int *)E.ci.get(), (const int *)E.cbase.get(),
+               (const uint16_t *)E.c16.get(), vals<T>(E), b, e, out, dw, part, tick, dot_out);
+  };
+#define CHRONOS_FOLD_CASE(LL)                                                              \
+  case LL:                                                                                 \
+    if (Q.idx16 && E.idx16) launch(k_fold_apply<T, BT, OT, LL, DOT, true, true>);          \
+    else if (E.idx16) launch(k_fold_apply<T, BT, OT, LL, DOT, false, true>);               \
+    else if (Q.idx16) launch(k_fold_apply<T, BT, OT, LL, DOT, true, false>);               \
+    else launch(k_fold_apply<T, BT, OT, LL, DOT, false, false>);                           \
+    break;
+  switch (lanes) {
+    CHRONOS_FOLD_CASE(1)
+    CHRONOS_FOLD_CASE(2)
+    CHRONOS_FOLD_CASE(4)
+    CHRONOS_FOLD_CASE(8)
+    CHRONOS_FOLD_CASE(16)
+    CHRONOS_FOLD_CASE(32)
+    default: throw Error(CHRONOS_EINVAL, "fold_apply: bad lane count");
+  }
+#undef CHRONOS_FOLD_CASE
+}
+
+// x = D b, D with rows of ld values (ld even): a warp per row, 16-byte loads.
+template <typename TI, typename TO>
+__global__ void __launch_bounds__(256)
+k_dense_tail_apply(int n, const double *__restrict__ D, int ld, const TI *__restrict__ b,
+                   TO *__restrict__ x) {
+  pdl_begin();
+  const int lane = threadIdx.x & 31;
+  const int row = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+  if (row >= n) return;
+  const double2 *d = reinterpret_cast<const double2 *>(D + (size_t)row * ld);
+  double s0 = 0.0, s1 = 0.0;
+#pragma unroll 4
+  for (int j = lane; 2 * j + 1 < n; j += 32) {
+    const double2 w = __ldg(d + j);
+    s0 = fma(w.x, (double)__ldg(b + 2 * j), s0);
+    s1 = fma(w.y, (double)__ldg(b + 2 * j + 1), s1);
+  }
+  if ((n & 1) && lane == 0) s0 = fma(D[(size_t)row * ld + n - 1], (double)__ldg(b + n - 1), s0);
+  const double s = warp_sum(s0 + s1);
+  if (lane == 0) x[row] = (TO)s;
+}
+
+template <typename TI, typename TO>
+static void dense_tail_apply(cudaStream_t st, int n, const double *D, int ld, const TI *b, TO *x) {
+  launch_pdl(k_dense_tail_apply<TI, TO>, ceil_div((int64_t)n * 32, 256), 256, st, n, D, ld, b, x);
+}
+
 template <typename T, typename BT, typename OT, bool TOP>
 static void vcycle_level(Hier &h, int l, const BT *b, OT *out, const double *dw, double *dot_out) {
   Level &L = h.levels[l];
@@ -1625,6 +1787,47 @@ static void vcycle_level(Hier &h, int l, const BT *b, OT *out, const double *dw,
                  (const double *)out, dw, part, tick, dot_out);
       CHRONOS_CHECK_LAUNCH();
     }
+    return;
+  }
+  if (L.fold) {
+    const Fold &F = *L.fold;
+    if constexpr (!TOP) {
+      if (F.form == FOLD_DENSE) {
+        dense_tail_apply<BT, OT>(st, n, F.D.get(), F.ld, b, out);
+        return;
+      }
+    }
+    Level &C = h.levels[l + 1];
+    T *x = L.x<T>(), *r = L.r<T>(), *bc = C.b<T>(), *e = C.x<T>();
+    // down: b_c = R b, or through the residual of x = S b
+    if (F.form == FOLD_SMOOTH) {
+      mat_apply<T, BT, T, T, MODE_PLAIN, false>(st, F.Q, vals<T>(F.Q), b, nullptr, x, T(1));
+      op_apply<T, T, BT, T, MODE_RESID, false>(st, L.A, x, b, r, T(1));
+      mat_apply<T, T, T, T, MODE_PLAIN, false>(st, L.Pt, vals<T>(L.Pt), r, nullptr, bc, T(1));
+    } else {
+      restrict_apply<T, BT>(st, F.R, b, bc);
+    }
+    vcycle_level<T, T, T, false>(h, l + 1, bc, e, nullptr, nullptr);
+    // up: out = Q b + E e, or x += P e (x = S b + P e), r = b - A x, out = x + S r
+    if (F.form == FOLD_ALL) {
+      if (TOP && dw)
+        fold_apply<T, BT, OT, TOP>(st, F.lanes, F.Q, F.E, b, e, out, dw, part, tick, dot_out);
+      else
+        fold_apply<T, BT, OT, false>(st, F.lanes, F.Q, F.E, b, e, out, nullptr, nullptr, nullptr,
+                                     nullptr);
+      return;
+    }
+    if (F.form == FOLD_SMOOTH)
+      mat_apply<T, T, T, T, MODE_AXPY, false>(st, L.P, vals<T>(L.P), e, x, x, T(1));
+    else
+      fold_apply<T, BT, T, false>(st, F.lanes, F.Q, L.P, b, e, x, nullptr, nullptr, nullptr,
+                                  nullptr);
+    op_apply<T, T, BT, T, MODE_RESID, false>(st, L.A, x, b, r, T(1));
+    if (TOP && dw)
+      mat_apply<T, T, T, OT, MODE_AXPY, TOP>(st, F.Q, vals<T>(F.Q), r, x, out, T(1), dw, part,
+                                             tick, dot_out);
+    else
+      mat_apply<T, T, T, OT, MODE_AXPY, false>(st, F.Q, vals<T>(F.Q), r, x, out, T(1));
     return;
   }
   T *x = L.x<T>(), *r = L.r<T>(), *t = L.t<T>();
@@ -2430,6 +2633,20 @@ static double vcycle_bytes_level(const Hier &h, int l, double s, double sb, doub
   const int n = L.n;
   if (L.coarsest) return (double)n * n * 8.0 + n * (sb + sout);
   double b = 0.0;
+  if (L.fold) {
+    const Fold &F = *L.fold;
+    if (F.form == FOLD_DENSE) return (double)n * F.ld * 8.0 + n * (sb + sout);
+    const double dot = top ? 8.0 : 0.0, coarse = vcycle_bytes_level(h, l + 1, s, s, s, false);
+    if (F.form == FOLD_ALL)
+      return apply_bytes(F.R, s, sb, s, 0.0) + coarse + apply_bytes(F.Q, s, sb, sout, dot) +
+             apply_bytes(F.E, s, s, 0.0, 0.0);
+    const double resid = apply_bytes(L.A, s, s, s, sb), up = apply_bytes(F.Q, s, s, sout, s + dot);
+    if (F.form == FOLD_DOWN)
+      return apply_bytes(F.R, s, sb, s, 0.0) + coarse + apply_bytes(F.Q, s, sb, s, 0.0) +
+             apply_bytes(L.P, s, s, 0.0, 0.0) + resid + up;
+    return apply_bytes(F.Q, s, sb, s, 0.0) + 2 * resid + apply_bytes(L.Pt, s, s, s, 0.0) + coarse +
+           apply_bytes(L.P, s, s, s, s) + up;
+  }
   b += apply_bytes(L.G, s, sb, s, 0.0);                     // t = G b
   b += apply_bytes(L.Gt, s, s, s, 0.0);                     // x = w G' t
   for (int k = 1; k < h.prm.nupre; ++k)
@@ -2451,7 +2668,11 @@ static double vcycle_bytes_level(const Hier &h, int l, double s, double sb, doub
 static int vcycle_kernels(const Hier &h) {
   int k = 0;
   for (const auto &L : h.levels) {
-    if (L.coarsest) { k += 1; break; }
+    if (L.coarsest || (L.fold && L.fold->form == FOLD_DENSE)) { k += 1; break; }
+    if (L.fold) {
+      k += L.fold->form == FOLD_ALL ? 2 : L.fold->form == FOLD_DOWN ? 4 : 6;
+      continue;
+    }
     k += 2 + 3 * (h.prm.nupre - 1) + 2 + 1 + 3 * h.prm.nupost + (h.prm.nupost == 0 ? 1 : 0);
   }
   if (h.levels[0].coarsest) k += 1;                         // the separate dot

@@ -45,12 +45,24 @@ void validate_csr(const HostCSR &A);
 // CHRONOS_GPU_COARSEN not set to 0.
 bool gpu_coarsening(const char *soc_type);
 
+// The folded form of a level (fold.cu).  FOLD_SMOOTH: Q = S; FOLD_DOWN: Q = S and
+// R; FOLD_ALL: R, Q, E; FOLD_DENSE: D, n rows of ld values (ld even).
+enum FoldForm { FOLD_SMOOTH, FOLD_DOWN, FOLD_ALL, FOLD_DENSE };
+struct Fold {
+  FoldForm form = FOLD_SMOOTH;
+  DMat R, Q, E;
+  int lanes = 8;                   // lanes per row of S b + P e or Q b + E e
+  DBuf<double> D;
+  int ld = 0;
+};
+
 struct Level {
   int n = 0, nc = 0;
   bool coarsest = false;
   DMat A, G, Gt, P, Pt;
   DBuf<double> W;                  // coarsest: A^{-1} from the Cholesky factor
   double omega = 1.0, lambda = 0.0;
+  std::unique_ptr<Fold> fold;      // used instead of A, G, G', P, P' when set
   // work vectors (one set per precision in use)
   DBuf<float> b32, x32, r32, t32;
   DBuf<double> b64, x64, r64, t64;
@@ -250,6 +262,9 @@ std::unique_ptr<Hier> build_hierarchy(const chronos_params &prm, HostCSR A,
                                       int ntv0, const double *TV0, bool tune = true,
                                       const ProlongFn *prolong = nullptr);
 void tune_hierarchy(Hier &h);
+// Folds the levels for which that is the faster form (fold.cu); part of
+// tune_hierarchy.
+void build_folds(Hier &h);
 
 // One hierarchy built level by level (what build_hierarchy runs): a level is
 // begun (its operator uploaded; the coarsest factored, begin_level then
@@ -299,6 +314,10 @@ void params_read(const char *fnames_path, chronos_params *p);
 
 // Upload a host CSR (FP64) to a device matrix, with FP32 values when fp32.
 void upload_csr(const HostCSR &h, DMat &d, bool fp32, cudaStream_t st);
+// A device CSR taken over into a device matrix (16-bit offsets, FP32 copy, lane
+// heuristic).
+void adopt_csr(int nrows, int ncols, int64_t nnz, DBuf<int> &rp, DBuf<int> &ci, DBuf<double> &v,
+               DMat &d, bool fp32, cudaStream_t st);
 // T = M' built on the device from M's device arrays (as upload_csr of the
 // host transpose would give); Mh: the same matrix on the host, if at hand.
 void upload_transpose(const DMat &M, DMat &T, bool fp32, cudaStream_t st,

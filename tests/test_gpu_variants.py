@@ -186,3 +186,45 @@ def test_single_level_vcycle_is_the_dense_solve(lib, nx):
         x = h.vcycle(b)
     want = np.linalg.solve(A.toarray(), b)
     assert np.linalg.norm(x - want) <= 200 * nx ** 3 * 2.2e-16 * np.linalg.norm(want)
+
+
+@pytest.mark.parametrize("prec,tol", [(cb.CHRONOS_FP64, 1e-12), (cb.CHRONOS_FP32, 2e-5)])
+@pytest.mark.parametrize("problem,nx,coarse", [
+    ("poisson", 11, 1000), ("poisson", 21, 50), ("poisson", 33, 1000), ("poisson", 50, 300),
+    ("elasticity", 7, 100), ("elasticity", 11, 1000), ("elasticity", 18, 40),
+    ("elasticity", 27, 300), ("fsai", 14, 200), ("fsai", 30, 1000)])
+def test_folded_levels_match_the_operator_form(lib, problem, nx, coarse, prec, tol):
+    """Every folded form (dense tails with even and odd rows, two, four and six
+    kernels, wide restriction rows, smoother factors with long rows that stay
+    unfolded) against the operator by operator cycle (spmv_format = 1), to the
+    tolerances that the storage formats are held to; vectors in both types."""
+    import torch
+    from chronoslab_b200 import problems as PB
+    if problem == "elasticity":
+        A, X = PB.elasticity_q1(nx, return_coords=True)
+        TV, more = PB.rbm_test_space(X), {}
+    else:
+        A = PB.poisson7(nx) if problem == "poisson" else PB.diffusion7(nx, seed=2)[0]
+        TV, more = np.ones((A.shape[0], 1)), {"ntv": 1}
+        if problem == "fsai":
+            more.update(fsai_fabs=1)
+    n = A.shape[0]
+    b = np.random.default_rng(nx).standard_normal(n)
+    with cb.Hierarchy(A, TV, cb.params(precision=prec, maxCoarseSZ=coarse, **more)) as hf, \
+            cb.Hierarchy(A, TV, cb.params(precision=prec, maxCoarseSZ=coarse, spmv_format=1,
+                                          **more)) as hp:
+        assert hf.nlevels == hp.nlevels >= 2
+        xf, xp = hf.vcycle(b), hp.vcycle(b)
+        assert np.linalg.norm(xf - xp) <= tol * np.linalg.norm(xp)
+        for t, code in ((torch.float32, cb.CHRONOS_FP32), (torch.float64, cb.CHRONOS_FP64)):
+            bd = torch.from_numpy(b).to("cuda", t)
+            out = torch.zeros_like(bd)
+            hf.vcycle_dev(bd.data_ptr(), out.data_ptr(), code)
+            torch.cuda.synchronize()
+            got = out.double().cpu().numpy()
+            assert np.linalg.norm(got - xp) <= max(tol, 2e-5 if t == torch.float32 else 0.0) \
+                * np.linalg.norm(xp)
+        x1, it1, _, f1, _ = hf.pcg(b, itmax=400, tol=1e-8)
+        x2, it2, _, f2, _ = hp.pcg(b, itmax=400, tol=1e-8)
+        assert f1 == 0 and f2 == 0 and abs(it1 - it2) <= 1
+        assert np.linalg.norm(b - A @ x1) <= 1e-8 * np.linalg.norm(b)
