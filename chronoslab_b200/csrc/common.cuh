@@ -338,6 +338,10 @@ __device__ __forceinline__ double block_sum(double v, double *smem32) {
   return r;
 }
 
+// Orders this thread's earlier accesses before its later ones for the whole
+// GPU (release before, acquire after a ticket).
+__device__ __forceinline__ void fence_gpu() { asm volatile("fence.acq_rel.gpu;" ::: "memory"); }
+
 // ---- programmatic dependent launch ------------------------------------------
 // Kernels of the solve loop begin with pdl_begin(): griddepcontrol.wait
 // returns once the preceding kernel of the stream has completed and its

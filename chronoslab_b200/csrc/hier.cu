@@ -56,17 +56,18 @@ class SetupPhase {
   double *acc_;
 };
 
+static void drop_pcg_graph(PcgState &s);
+
 PcgState::~PcgState() {
-  if (exec) cudaGraphExecDestroy(exec);
-  if (graph) cudaGraphDestroy(graph);
+  for (auto e : {exec, far_exec}) if (e) cudaGraphExecDestroy(e);
+  for (auto g : {graph, far_graph}) if (g) cudaGraphDestroy(g);
   if (sc_pinned) cudaFreeHost(sc_pinned);
 }
 
 Hier::~Hier() {
   if (st) cudaStreamSynchronize(st);
   levels.clear();
-  if (pcg.exec) { cudaGraphExecDestroy(pcg.exec); pcg.exec = nullptr; }
-  if (pcg.graph) { cudaGraphDestroy(pcg.graph); pcg.graph = nullptr; }
+  drop_pcg_graph(pcg);
   if (ev_in) cudaEventDestroy(ev_in);
   if (ev_out) cudaEventDestroy(ev_out);
   stream_destroy(st);
@@ -1928,6 +1929,7 @@ struct FinAlpha {
   double *sc;
   __device__ void operator()(const double *t) const {
     const double ptap = t[0], pres = t[1];
+    if (sc[SC_DONE] != 0.0) return;             // an iteration after the stop (far_exec)
     sc[SC_PTAP] = ptap;
     sc[SC_PRES] = pres;
     if (!(ptap > 0.0) || !isfinite(pres)) {     // breakdown: p'Ap <= 0 or NaN
@@ -2133,31 +2135,46 @@ static void launch_pcg_spmv(cudaStream_t st, const DMat &A, bool fp32vals, const
 // true residual (k_pcg_replace) when it has fallen below replace_ratio times
 // its largest value since the last replacement, when it passes the
 // tolerance, and at itmax; the stop is then decided on the true residual.
+// The scalars are read before the first store (and by the kernels before their
+// loop): in the order of use they were a chain of L2 round trips behind the
+// reduction.  far > 0 (the unrolled loop of far_exec): go on only while the
+// residual is above far times the tolerance.
 struct FinResidual {
   double *sc, *resvec;
   cudaGraphConditionalHandle handle;
   int use_cond, mixed;
+  double far;
+  double bnorm, it, breakdown, tol, itmax, rmax, ratio;
+  __device__ void load() {
+    bnorm = sc[SC_BNORM];
+    it = sc[SC_ITER];
+    breakdown = sc[SC_BREAKDOWN];
+    tol = sc[SC_TOL];
+    itmax = sc[SC_ITMAX];
+    rmax = sc[SC_RMAX];
+    ratio = sc[SC_RATIO];
+  }
   __device__ void operator()(const double *t) const {
     const double rn = sqrt(t[0]);
-    const double resiter = rn / sc[SC_BNORM];
-    const double it = sc[SC_ITER] + 1.0;
-    sc[SC_ITER] = it;
-    sc[SC_RR] = t[0];
-    sc[SC_RESITER] = resiter;
-    resvec[(int)it] = resiter;
-    const bool bad = sc[SC_BREAKDOWN] != 0.0 || !isfinite(resiter);
+    const double resiter = rn / bnorm;
+    const double now = it + 1.0;
+    const bool bad = breakdown != 0.0 || !isfinite(resiter);
     bool stop;
     if (mixed) {
-      const double rmax = fmax(sc[SC_RMAX], rn);
-      sc[SC_RMAX] = rmax;
-      const bool rep = !bad && (rn < sc[SC_RATIO] * rmax || resiter < sc[SC_TOL] ||
-                                it >= sc[SC_ITMAX]);
+      const double rm = fmax(rmax, rn);
+      const bool rep = !bad && (rn < ratio * rm || resiter < tol || now >= itmax);
+      sc[SC_RMAX] = rm;
       sc[SC_REPLACE] = rep ? 1.0 : 0.0;
       stop = bad;                      // otherwise k_pcg_replace decides when it runs
     } else {
-      stop = resiter < sc[SC_TOL] || it >= sc[SC_ITMAX] || bad;
+      stop = resiter < tol || now >= itmax || bad;
     }
-    if (use_cond) cudaGraphSetConditional(handle, stop ? 0u : 1u);
+    sc[SC_ITER] = now;
+    sc[SC_RR] = t[0];
+    sc[SC_RESITER] = resiter;
+    sc[SC_DONE] = stop ? 1.0 : 0.0;
+    resvec[(int)now] = resiter;
+    if (use_cond) cudaGraphSetConditional(handle, !stop && resiter > far * tol ? 1u : 0u);
   }
 };
 
@@ -2166,9 +2183,15 @@ __global__ void __launch_bounds__(256)
 k_pcg_xr_update(int n, double *__restrict__ x, double *__restrict__ res,
                 const double *__restrict__ p, const double *__restrict__ axp, double *part,
                 unsigned *ticket, double *sc, double *resvec, cudaGraphConditionalHandle handle,
-                int use_cond, int mixed) {
+                int use_cond, int mixed, double far) {
   pdl_begin();
+  FinResidual fin{sc, resvec, handle, use_cond, mixed, far};
+  fin.load();
   const double alpha = sc[SC_ALPHA];
+  if (sc[SC_DONE] != 0.0) {            // stopped in an earlier iteration of this pass
+    if (use_cond && blockIdx.x == 0 && threadIdx.x == 0) cudaGraphSetConditional(handle, 0u);
+    return;
+  }
   double rr = 0.0;
   for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
     x[i] += alpha * p[i];
@@ -2177,7 +2200,7 @@ k_pcg_xr_update(int n, double *__restrict__ x, double *__restrict__ res,
     rr += ri * ri;
   }
   double v[1] = {rr};
-  grid_reduce<1>(v, part, ticket, FinResidual{sc, resvec, handle, use_cond, mixed});
+  grid_reduce<1>(v, part, ticket, fin);
 }
 
 // Stop decision on the true residual after a replacement.
@@ -2185,16 +2208,18 @@ struct FinReplace {
   double *sc, *resvec;
   cudaGraphConditionalHandle handle;
   int use_cond;
+  double far;
   __device__ void operator()(const double *t) const {
+    const double bnorm = sc[SC_BNORM], it = sc[SC_ITER], tol = sc[SC_TOL], itmax = sc[SC_ITMAX];
     const double rn = sqrt(t[0]);
-    const double resiter = rn / sc[SC_BNORM];
-    const double it = sc[SC_ITER];
+    const double resiter = rn / bnorm;
+    const bool stop = resiter < tol || it >= itmax || !isfinite(resiter);
     sc[SC_RR] = t[0];
     sc[SC_RESITER] = resiter;
     sc[SC_RMAX] = rn;
+    sc[SC_DONE] = stop ? 1.0 : 0.0;
     resvec[(int)it] = resiter;
-    const bool stop = resiter < sc[SC_TOL] || it >= sc[SC_ITMAX] || !isfinite(resiter);
-    if (use_cond) cudaGraphSetConditional(handle, stop ? 0u : 1u);
+    if (use_cond) cudaGraphSetConditional(handle, !stop && resiter > far * tol ? 1u : 0u);
   }
 };
 
@@ -2209,9 +2234,9 @@ k_pcg_replace(int n, const int *__restrict__ rp, const int *__restrict__ ci,
               const double *__restrict__ b, double *__restrict__ res, int short_blocks,
               int lthresh, const int *__restrict__ longrows, int nlong, double *part,
               unsigned *ticket, double *sc, double *resvec, cudaGraphConditionalHandle handle,
-              int use_cond) {
+              int use_cond, double far) {
   pdl_begin();
-  if (sc[SC_REPLACE] == 0.0) return;
+  if (sc[SC_REPLACE] == 0.0 || sc[SC_DONE] != 0.0) return;
   const int lane = threadIdx.x & 31;
   double rr = 0.0;
   if ((int)blockIdx.x < short_blocks) {
@@ -2255,7 +2280,7 @@ k_pcg_replace(int n, const int *__restrict__ rp, const int *__restrict__ ci,
     }
   }
   double vals[1] = {rr};
-  grid_reduce<1>(vals, part, ticket, FinReplace{sc, resvec, handle, use_cond});
+  grid_reduce<1>(vals, part, ticket, FinReplace{sc, resvec, handle, use_cond, far});
 }
 
 template <int T>
@@ -2265,9 +2290,9 @@ k_pcg_replace_sell3(int nb, int nchunk, const int *__restrict__ choff,
                     const double *__restrict__ V, int64_t nslots, const double *__restrict__ x,
                     const double *__restrict__ b, double *__restrict__ res, double *part,
                     unsigned *ticket, double *sc, double *resvec,
-                    cudaGraphConditionalHandle handle, int use_cond) {
+                    cudaGraphConditionalHandle handle, int use_cond, double far) {
   pdl_begin();
-  if (sc[SC_REPLACE] == 0.0) return;
+  if (sc[SC_REPLACE] == 0.0 || sc[SC_DONE] != 0.0) return;
   constexpr int C = 32 / T;
   const int lane = threadIdx.x & 31;
   const int warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
@@ -2295,12 +2320,13 @@ k_pcg_replace_sell3(int nb, int nchunk, const int *__restrict__ choff,
     }
   }
   double vals[1] = {rr};
-  grid_reduce<1>(vals, part, ticket, FinReplace{sc, resvec, handle, use_cond});
+  grid_reduce<1>(vals, part, ticket, FinReplace{sc, resvec, handle, use_cond, far});
 }
 
 static void launch_pcg_replace(cudaStream_t st, const DMat &A, const double *x, const double *b,
                                double *res, double *part, unsigned *tick, double *sc,
-                               double *resvec, cudaGraphConditionalHandle handle, int use_cond) {
+                               double *resvec, cudaGraphConditionalHandle handle, int use_cond,
+                               double far) {
   int sb = 0;
   const int grid = pcg_grid(A, &sb);
   if (A.nb > 0) {
@@ -2308,7 +2334,7 @@ static void launch_pcg_replace(cudaStream_t st, const DMat &A, const double *x, 
   case TT:                                                                                     \
     launch_pdl(k_pcg_replace_sell3<TT>, grid, kApplyThreads, st, A.nb, A.nchunk,               \
                A.choff.get(), A.chw.get(), A.sci.get(), A.bv64.get(), A.nslots, x, b, res, part, \
-               tick, sc, resvec, handle, use_cond);                                            \
+               tick, sc, resvec, handle, use_cond, far);                                       \
     break;
     switch (A.sell_T) {
       CHRONOS_REP3_CASE(1)
@@ -2323,11 +2349,11 @@ static void launch_pcg_replace(cudaStream_t st, const DMat &A, const double *x, 
     if (A.idx16)                                                                               \
       launch_pdl(k_pcg_replace<LL, true>, grid, kApplyThreads, st, A.nrows, A.rp.get(),        \
                  A.ci.get(), A.cbase.get(), A.c16.get(), A.v64.get(), x, b, res, sb, A.lthresh,\
-                 A.longrows.get(), A.nlong, part, tick, sc, resvec, handle, use_cond);         \
+                 A.longrows.get(), A.nlong, part, tick, sc, resvec, handle, use_cond, far);    \
     else                                                                                       \
       launch_pdl(k_pcg_replace<LL, false>, grid, kApplyThreads, st, A.nrows, A.rp.get(),       \
                  A.ci.get(), A.cbase.get(), A.c16.get(), A.v64.get(), x, b, res, sb, A.lthresh,\
-                 A.longrows.get(), A.nlong, part, tick, sc, resvec, handle, use_cond);         \
+                 A.longrows.get(), A.nlong, part, tick, sc, resvec, handle, use_cond, far);    \
     break;
     switch (A.lanes) {
       CHRONOS_REP_CASE(1)
@@ -2354,8 +2380,14 @@ static bool mixed_outer(const Hier &h) {
 }
 
 static void drop_pcg_graph(PcgState &s) {
-  if (s.exec) { cudaGraphExecDestroy(s.exec); s.exec = nullptr; }
-  if (s.graph) { cudaGraphDestroy(s.graph); s.graph = nullptr; }
+  for (auto *e : {&s.exec, &s.far_exec}) {
+    if (*e) cudaGraphExecDestroy(*e);
+    *e = nullptr;
+  }
+  for (auto *g : {&s.graph, &s.far_graph}) {
+    if (*g) cudaGraphDestroy(*g);
+    *g = nullptr;
+  }
 }
 
 void Hier::set_outer_operator(const HostCSR *A) {
@@ -2377,7 +2409,8 @@ void Hier::set_outer_operator(const HostCSR *A) {
 }
 
 // Captures one PCG_CJ iteration (PCG_CJ.m:36-64) into the current stream capture.
-static void capture_iteration(Hier &h, cudaGraphConditionalHandle handle, int use_cond) {
+static void capture_iteration(Hier &h, cudaGraphConditionalHandle handle, int use_cond,
+                              double far = 0.0) {
   PcgState &s = h.pcg;
   cudaStream_t st = h.st;
   const int n = s.n;
@@ -2394,12 +2427,12 @@ static void capture_iteration(Hier &h, cudaGraphConditionalHandle handle, int us
                   s.part.get() + 4 * 3 * 2048, tk + 1, sc);
   launch_pdl(k_pcg_xr_update, nb, 256, st, n, s.x.get(), s.res.get(), (const double *)s.p.get(),
              (const double *)s.axp.get(), s.part.get() + 8 * 3 * 2048, tk + 2, sc,
-             s.resvec.get(), handle, use_cond, mixed ? 1 : 0);
+             s.resvec.get(), handle, use_cond, mixed ? 1 : 0, far);
   CHRONOS_CHECK_LAUNCH();
   if (mixed)
     launch_pcg_replace(st, h.levels[0].A, s.x.get(), s.b.get(), s.res.get(),
                        s.part.get() + 10 * 3 * 2048, tk + 4, sc, s.resvec.get(), handle,
-                       use_cond);
+                       use_cond, far);
 }
 
 static void ensure_pcg_state(Hier &h, int itmax) {
@@ -2423,34 +2456,53 @@ static void ensure_pcg_state(Hier &h, int itmax) {
   }
 }
 
+// A pass of a conditional while node costs about 5 us beyond its kernels
+// (bodies of 1 to 16 empty kernels: 5.7 us for one, 0.4 us for each further
+// one).  So a solve whose residual is more than kFarFactor times the tolerance
+// begins with passes of kFarUnroll iterations and goes on one by one below
+// that; a stop inside an unrolled pass turns the iterations after it into
+// no-ops (SC_DONE), so iteration counts, iterates and flags are those of the
+// plain loop.  us per iteration, one by one and so: Poisson 20^3 FP64 34.6 and
+// 32.6, Poisson 32^3 FP32 49.2 and 46.4, elasticity 24^3 FP64 66.5 and 64.0; a
+// handle's first solve takes 0.2 ms longer for the second graph.
+constexpr int kFarUnroll = 4;
+constexpr double kFarFactor = 30.0;
+
+// One while loop over `unroll` iterations per pass.
+static void build_while_graph(Hier &h, int unroll, double far, cudaGraph_t *graph,
+                              cudaGraphExec_t *exec) {
+  cudaStream_t st = h.st;
+  CHRONOS_CUDA(cudaGraphCreate(graph, 0));
+  cudaGraphConditionalHandle handle;
+  CHRONOS_CUDA(cudaGraphConditionalHandleCreate(&handle, *graph, 1, cudaGraphCondAssignDefault));
+  cudaGraphNodeParams np{};
+  np.type = cudaGraphNodeTypeConditional;
+  np.conditional.handle = handle;
+  np.conditional.type = cudaGraphCondTypeWhile;
+  np.conditional.size = 1;
+  cudaGraphNode_t node;
+  CHRONOS_CUDA(cudaGraphAddNode(&node, *graph, nullptr, 0, &np));
+  cudaGraph_t body = np.conditional.phGraph_out[0];
+  std::lock_guard<std::mutex> capturing(lib_streams().mu);
+  CHRONOS_CUDA(cudaStreamBeginCaptureToGraph(st, body, nullptr, nullptr, 0,
+                                             cudaStreamCaptureModeThreadLocal));
+  try {
+    for (int k = 0; k < unroll; ++k) capture_iteration(h, handle, k + 1 == unroll, far);
+  } catch (...) {
+    cudaGraph_t dummy;
+    cudaStreamEndCapture(st, &dummy);
+    throw;
+  }
+  CHRONOS_CUDA(cudaStreamEndCapture(st, &body));
+  CHRONOS_CUDA(cudaGraphInstantiate(exec, *graph, 0));
+}
+
 static void build_pcg_graph(Hier &h) {
   PcgState &s = h.pcg;
   cudaStream_t st = h.st;
   if (s.exec) return;
   if (h.prm.use_graph) {
-    CHRONOS_CUDA(cudaGraphCreate(&s.graph, 0));
-    cudaGraphConditionalHandle handle;
-    CHRONOS_CUDA(cudaGraphConditionalHandleCreate(&handle, s.graph, 1, cudaGraphCondAssignDefault));
-    cudaGraphNodeParams np{};
-    np.type = cudaGraphNodeTypeConditional;
-    np.conditional.handle = handle;
-    np.conditional.type = cudaGraphCondTypeWhile;
-    np.conditional.size = 1;
-    cudaGraphNode_t node;
-    CHRONOS_CUDA(cudaGraphAddNode(&node, s.graph, nullptr, 0, &np));
-    cudaGraph_t body = np.conditional.phGraph_out[0];
-    std::lock_guard<std::mutex> capturing(lib_streams().mu);
-    CHRONOS_CUDA(cudaStreamBeginCaptureToGraph(st, body, nullptr, nullptr, 0,
-                                               cudaStreamCaptureModeThreadLocal));
-    try {
-      capture_iteration(h, handle, 1);
-    } catch (...) {
-      cudaGraph_t dummy;
-      cudaStreamEndCapture(st, &dummy);
-      throw;
-    }
-    CHRONOS_CUDA(cudaStreamEndCapture(st, &body));
-    CHRONOS_CUDA(cudaGraphInstantiate(&s.exec, s.graph, 0));
+    build_while_graph(h, 1, 0.0, &s.graph, &s.exec);
     s.conditional = true;
   } else {
     std::lock_guard<std::mutex> capturing(lib_streams().mu);
@@ -2486,6 +2538,7 @@ __global__ void k_pcg_init(double *sc, double *resvec, double tol, double itmax,
   sc[SC_TOL] = tol;
   sc[SC_ITMAX] = itmax;
   sc[SC_BREAKDOWN] = 0.0;
+  sc[SC_DONE] = 0.0;
 }
 
 void Hier::pcg_solve(const double *b, double *x, int itmax, double tol, int *iters, int *flag,
@@ -2531,6 +2584,13 @@ void Hier::pcg_solve(const double *b, double *x, int itmax, double tol, int *ite
   if (itmax > 0) {
     build_pcg_graph(*this);
     if (s.conditional) {
+      // the unrolled loop leaves the last iterations (one at least, a no-op if
+      // it stopped the solve) to the plain one
+      if (itmax > kFarUnroll && sc_h[SC_RESITER] > kFarFactor * tol) {
+        if (!s.far_exec)
+          build_while_graph(*this, kFarUnroll, kFarFactor, &s.far_graph, &s.far_exec);
+        CHRONOS_CUDA(cudaGraphLaunch(s.far_exec, st));
+      }
       CHRONOS_CUDA(cudaGraphLaunch(s.exec, st));
     } else {
       double *pinned = nullptr;

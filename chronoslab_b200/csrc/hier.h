@@ -88,7 +88,7 @@ template <> inline const double *vals<double>(const DMat &m) { return m.v64.get(
 // Device scalars of the PCG recurrence.
 enum PcgScalar {
   SC_BNORM = 0, SC_PTAP, SC_ALPHA, SC_PRES_AXP, SC_RR, SC_RESITER, SC_ITER, SC_TOL, SC_ITMAX,
-  SC_BREAKDOWN, SC_PRES, SC_RMAX, SC_REPLACE, SC_RATIO, SC_COUNT = 16
+  SC_BREAKDOWN, SC_PRES, SC_RMAX, SC_REPLACE, SC_RATIO, SC_DONE, SC_COUNT = 16
 };
 
 struct PcgState {
@@ -100,6 +100,8 @@ struct PcgState {
   DBuf<unsigned> tickets;           // one ticket per reducing kernel
   cudaGraphExec_t exec = nullptr;   // the whole solve (device-side loop) or one iteration
   cudaGraph_t graph = nullptr;
+  cudaGraphExec_t far_exec = nullptr;   // kFarUnroll iterations per pass, far from the tolerance
+  cudaGraph_t far_graph = nullptr;
   bool conditional = false;
   int resvec_cap = 0;
   double *sc_pinned = nullptr;      // pinned copy of the scalars for queued solves

@@ -50,13 +50,13 @@ __device__ __forceinline__ void grid_reduce(double (&v)[K], double *part, unsign
       for (int w = 0; w < nw; ++w) s += red[j][w];
       part[(size_t)blockIdx.x * K + j] = s;
     }
-    __threadfence();
+    fence_gpu();
     unsigned t = atomicAdd(ticket, 1u);
     last = (t == gridDim.x - 1);
   }
   __syncthreads();
   if (!last) return;
-  __threadfence();
+  fence_gpu();
   double acc[K];
 #pragma unroll
   for (int j = 0; j < K; ++j) acc[j] = 0.0;

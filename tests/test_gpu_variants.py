@@ -228,3 +228,30 @@ def test_folded_levels_match_the_operator_form(lib, problem, nx, coarse, prec, t
         x2, it2, _, f2, _ = hp.pcg(b, itmax=400, tol=1e-8)
         assert f1 == 0 and f2 == 0 and abs(it1 - it2) <= 1
         assert np.linalg.norm(b - A @ x1) <= 1e-8 * np.linalg.norm(b)
+
+
+@pytest.mark.parametrize("more", [{"precision": cb.CHRONOS_FP64}, {"precision": cb.CHRONOS_FP32},
+                                  {"precision": cb.CHRONOS_FP32, "exact_outer": 1},
+                                  {"precision": cb.CHRONOS_FP32, "replace_ratio": 0.5}])
+def test_unrolled_loop_stops_as_the_host_loop(lib, more):
+    """The device-side loop, several iterations per pass far from the tolerance,
+    gives the one-iteration host loop's iterates bit for bit wherever a solve
+    stops: at every itmax of a pass, at tolerances met inside one, at once."""
+    from chronoslab_b200 import problems as PB
+    A = PB.poisson7(14)
+    n = A.shape[0]
+    b = PB.uniform_rhs(n, 3)
+    with cb.Hierarchy(A, np.ones(n), cb.params(ntv=1, maxCoarseSZ=100, **more)) as h1, \
+            cb.Hierarchy(A, np.ones(n), cb.params(ntv=1, maxCoarseSZ=100, use_graph=0,
+                                                  **more)) as h0:
+        runs = [(k, 1e-12) for k in range(0, 11)] + [(100, 10.0 ** -e) for e in range(0, 13)]
+        for itmax, tol in runs:
+            x1, it1, rv1, f1, _ = h1.pcg(b, itmax=itmax, tol=tol)
+            x0, it0, rv0, f0, _ = h0.pcg(b, itmax=itmax, tol=tol)
+            assert (it1, f1) == (it0, f0), (itmax, tol)
+            assert np.array_equal(x1, x0) and np.array_equal(rv1, rv0), (itmax, tol)
+        bad = b.copy()
+        bad[5] = np.nan
+        with pytest.raises(cb.ChronosError):
+            h1.pcg(bad)
+        assert h1.pcg(b, tol=1e-8)[1] == h0.pcg(b, tol=1e-8)[1]
