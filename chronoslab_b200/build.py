@@ -24,7 +24,7 @@ NVCC = os.path.join(CUDA_HOME, "bin", "nvcc")
 CXX = "/usr/bin/g++" if os.path.exists("/usr/bin/g++") else "g++"
 
 CU_SOURCES = ["setup_kernels.cu", "hier.cu", "block.cu", "batch.cu", "group.cu", "capi.cu",
-              "coarsen_gpu.cu", "gmres.cu", "bamg_gpu.cu", "emin_gpu.cu", "fold.cu"]
+              "coarsen_gpu.cu", "gmres.cu", "bamg_gpu.cu", "emin_gpu.cu", "fold.cu", "sqmr.cu"]
 # per-file flags: the GPU BAMG reproduces the host restatement (built with
 # -ffp-contract=off) bit for bit, so its products and sums are not fused
 CU_EXTRA = {"bamg_gpu.cu": ["-fmad=false"]}

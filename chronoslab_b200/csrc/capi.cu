@@ -1057,71 +1057,13 @@ int chronos_sqmr(chronos_hier *hh, const int *iat_h, const int *ja_h, const doub
     CallRange range_("chronos_sqmr");
     CHRONOS_REQUIRE(hh && b_h && x_h && iters && relres && info, CHRONOS_EINVAL, "null argument");
     Hier &h = *hh->h;
-    cudaStream_t st = h.st;
     const int n = h.levels[0].n;
     DMat op;
     if (iat_h) {
-      upload_csr(from_csr0(n, n, iat_h, ja_h, val_h), op, false, st);
-      autotune_lanes(op, false, st);
+      upload_csr(from_csr0(n, n, iat_h, ja_h, val_h), op, false, h.st);
+      autotune_lanes(op, false, h.st);
     }
-    auto apply_op = [&](const double *x, double *y) {
-      if (!iat_h) { h.apply_A(x, y); return; }
-      csr_apply<double, double, double, double, MODE_PLAIN, false>(st, op.lanes, n, op.rp, op.ci,
-                                                                  op.v64, x, nullptr, y, 1.0);
-    };
-    DBuf<double> rhs, pnew, r(n), q(n), d(n), vscr(n), u(n), tmp(n), scratch(256);
-    rhs.upload(b_h, n, st);
-    pnew.upload(x_h, n, st);
-    d.zero(st);
-    auto dot = [&](const double *a, const double *b) { return device_dot(n, a, b, scratch.get(), st); };
-    auto lprec = [&](const double *in, double *out) { h.vcycle(in, out, nullptr, nullptr); };
-    // SQMR.m:24-36
-    const double bnorm = std::sqrt(dot(rhs.get(), rhs.get()));
-    apply_op(pnew.get(), tmp.get());
-    device_scale_copy(n, 1.0, rhs.get(), r.get(), st);
-    device_axpby(n, -1.0, tmp.get(), 1.0, r.get(), st);
-    lprec(r.get(), vscr.get());
-    device_scale_copy(n, 1.0, vscr.get(), q.get(), st);
-    double tau = std::sqrt(dot(vscr.get(), vscr.get()));
-    double rho0 = dot(r.get(), q.get());
-    double theta0 = 0.0;
-    int niter = 0, inf = 0;
-    bool exit_test = false;
-    while (!exit_test && niter < itmax) {
-      ++niter;
-      apply_op(q.get(), vscr.get());
-      const double sigma = dot(q.get(), vscr.get());
-      if (std::fabs(sigma) < 1e-20 * rho0) { inf = 10; break; }
-      const double alpha = rho0 / sigma;
-      device_axpby(n, -alpha, vscr.get(), 1.0, r.get(), st);
-      lprec(r.get(), vscr.get());
-      const double theta1 = std::sqrt(dot(vscr.get(), vscr.get())) / tau;
-      const double gamma = 1.0 / std::sqrt(1.0 + theta1 * theta1);
-      tau = tau * theta1 * gamma;
-      // d = d*gamma^2*theta0^2 + gamma^2*alpha*q
-      device_axpby(n, gamma * gamma * alpha, q.get(), gamma * gamma * theta0 * theta0, d.get(), st);
-      theta0 = theta1;
-      device_axpby(n, 1.0, d.get(), 1.0, pnew.get(), st);
-      const double resnorm = std::sqrt(dot(r.get(), r.get())) / bnorm;
-      if (resnorm < tol) {
-        exit_test = true;
-      } else {
-        device_scale_copy(n, 1.0, vscr.get(), u.get(), st);
-        const double rho1 = dot(r.get(), u.get());
-        if (std::fabs(rho0) < 1e-20 * rho1) { inf = 20; break; }
-        const double beta = rho1 / rho0;
-        rho0 = rho1;
-        device_axpby(n, 1.0, u.get(), beta, q.get(), st);
-      }
-    }
-    if (niter >= itmax) inf = 1;
-    apply_op(pnew.get(), tmp.get());
-    device_axpby(n, 1.0, rhs.get(), -1.0, tmp.get(), st);
-    *relres = std::sqrt(dot(tmp.get(), tmp.get())) / bnorm;
-    *iters = niter;
-    *info = inf;
-    pnew.download(x_h, n, st);
-    CHRONOS_CUDA(cudaStreamSynchronize(st));
+    sqmr_solve(h, iat_h ? &op : nullptr, b_h, x_h, itmax, tol, iters, relres, info);
   });
 }
 

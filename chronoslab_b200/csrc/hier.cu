@@ -2497,6 +2497,8 @@ static void build_while_graph(Hier &h, int unroll, double far, cudaGraph_t *grap
   CHRONOS_CUDA(cudaGraphInstantiate(exec, *graph, 0));
 }
 
+void ensure_reduction_state(Hier &h) { ensure_pcg_state(h, std::max(h.pcg.resvec_cap - 1, 1)); }
+
 static void build_pcg_graph(Hier &h) {
   PcgState &s = h.pcg;
   cudaStream_t st = h.st;

@@ -109,6 +109,7 @@ struct PcgState {
 };
 
 struct BlockState;   // block-of-right-hand-sides solve state (block.cu)
+struct SqmrState;    // SQMR vectors and graph (sqmr.cu)
 
 // A host block of right-hand sides: column-major with n rows (ld = 0), or
 // row-major with rows ld elements apart.
@@ -163,8 +164,16 @@ struct Hier {
   void pcg_block(int nrhs, const BlockIn &B, const double *X0_h, double *X_h, int itmax,
                  double tol, int *iters, int *flags, double *seconds);
   std::shared_ptr<BlockState> block;
+  std::shared_ptr<SqmrState> sqmr;
   DBuf<double> stage_b, stage_x;    // host-buffer entry points' device staging
 };
+
+// SQMR (sqmr.cu) from host vectors b and x (x0 on entry, the solution on
+// return) with the FP64 operator op, null: the hierarchy's level-1 operator.
+void sqmr_solve(Hier &h, const DMat *op, const double *b_h, double *x_h, int itmax, double tol,
+                int *iters, double *relres, int *info);
+// The buffers that a V-cycle with a fused dot reduces in.
+void ensure_reduction_state(Hier &h);
 
 // BAMG prolongation with the GPU doing the per-row work (bamg_gpu.cu): the
 // result of bamg_prolongation bit for bit; rows whose neighbourhood outgrows

@@ -255,3 +255,35 @@ def test_unrolled_loop_stops_as_the_host_loop(lib, more):
         with pytest.raises(cb.ChronosError):
             h1.pcg(bad)
         assert h1.pcg(b, tol=1e-8)[1] == h0.pcg(b, tol=1e-8)[1]
+
+
+@pytest.mark.parametrize("prec", [cb.CHRONOS_FP64, cb.CHRONOS_FP32])
+@pytest.mark.parametrize("nx,coarse", [(4, 1000), (9, 1000), (13, 100)])
+def test_device_sqmr_loop(lib, nx, coarse, prec):
+    """The device-side SQMR loop against the oracle's SQMR with the same V-cycle
+    (iterations within one, solutions to the tolerance), the host loop bit for
+    bit, with the operator passed in, at every small itmax, from the solution."""
+    from chronoslab_b200 import problems as PB
+    from oracle import amg_oracle as O
+    A, X = PB.elasticity_q1(nx, return_coords=True)
+    n, TV = A.shape[0], PB.rbm_test_space(X)
+    b = np.random.default_rng(nx).standard_normal(n)
+    prm = dict(precision=prec, maxCoarseSZ=coarse)
+    with cb.Hierarchy(A, TV, cb.params(**prm)) as h, \
+            cb.Hierarchy(A, TV, cb.params(use_graph=0, **prm)) as h0:
+        x, info, relres, it = cb.SQMR(h, b, 1e-8, 200)
+        assert info == 0
+        assert relres == pytest.approx(np.linalg.norm(b - A @ x) / np.linalg.norm(b), rel=1e-6)
+        xo, io, ro, ito, _ = O.sqmr(lambda v: A @ v, b, 1e-8, 200, lambda r: h.vcycle(r))
+        assert io == 0 and abs(it - ito) <= 1
+        assert np.linalg.norm(b - A @ x) <= 1.1e-8 * np.linalg.norm(b)
+        xu, iu, _, itu = cb.SQMR(h, b, 1e-8, 200, A=A)
+        assert iu == 0 and abs(itu - it) <= 1
+        assert np.linalg.norm(xu - x) <= 1e-6 * np.linalg.norm(x)
+        for itmax in (0, 1, 2, 5, it, it + 1):
+            got, want = cb.SQMR(h, b, 1e-8, itmax), cb.SQMR(h0, b, 1e-8, itmax)
+            assert np.array_equal(got[0], want[0]) and got[1:] == want[1:], itmax
+            assert got[3] == min(itmax, it) and got[1] == (1 if itmax <= it else 0)
+        # from the solution the first residual meets the test after one step
+        x2, i2, _, it2 = cb.SQMR(h, b, 1e-6, 200, x0=x)
+        assert i2 == 0 and it2 == 1
