@@ -156,58 +156,53 @@ void adopt(Prod &p, DMat &d, bool fp32, cudaStream_t st) {
   adopt_csr(p.rows, p.cols, p.nnz, p.rp, p.ci, p.v, d, fp32, st);
 }
 
-// Level l's folded form, or none.
-std::unique_ptr<Fold> fold_level(Hier &h, int l) {
-  const bool fp32 = h.precision == CHRONOS_FP32;
-  cudaStream_t st = h.st;
-  Level &L = h.levels[l];
-  const Level &C = h.levels[l + 1];
-  const int n = L.n, nc = L.nc;
+}  // namespace
+
+std::unique_ptr<Fold> fold_operators(const DMat &A, const DMat &G, const DMat &Gt, const DMat &P,
+                                     const DMat &Pt, double omega, const double *B, int ldb,
+                                     bool fp32, cudaStream_t st) {
+  const int n = A.nrows, nc = P.ncols;
   auto f = std::make_unique<Fold>();
-  const double *B = C.coarsest ? C.W.get()
-                    : C.fold && C.fold->form == FOLD_DENSE ? C.fold->D.get() : nullptr;
-  // the top level's product stays with its fused dot and conversions
-  const bool dense = l > 0 && B && n <= kFoldDenseRows &&
-                     (int64_t)n * n <= kFoldDenseRatio * L.A.nnz;
+  const bool dense = B && n <= kFoldDenseRows && (int64_t)n * n <= kFoldDenseRatio * A.nnz;
   // S replaces G and G' in both smoothing steps and spares a vector between
   // them; a factor with long rows fills up when it is squared
-  const int64_t worth = 2 * L.G.nnz + 2 * (int64_t)n + kFoldEntries / 2;
-  if (!dense && smoother_bound(L.G) > 4 * worth) return nullptr;
-  Prod S = multiply(n, n, View(L.Gt), View(L.G), st);
+  const int64_t worth = 2 * G.nnz + 2 * (int64_t)n + kFoldEntries / 2;
+  if (!dense && smoother_bound(G) > 4 * worth) return nullptr;
+  Prod S = multiply(n, n, View(Gt), View(G), st);
   if (!dense && S.nnz > worth) return nullptr;
   k_scale_values<<<std::max<int>(1, std::min<int64_t>(ceil_div(S.nnz, 256), num_sms() * 8)), 256,
-                   0, st>>>(S.nnz, L.omega, S.v.get());
+                   0, st>>>(S.nnz, omega, S.v.get());
   CHRONOS_CHECK_LAUNCH();
   auto smooth_only = [&] {
-    adopt(S, f->Q, fp32, st);
+    adopt(S, f->S, fp32, st);
     f->form = FOLD_SMOOTH;
     return std::move(f);
   };
   // R and Q have at least about as many entries as A and several times as many
-  if (!dense && L.A.nnz > kFoldEntries) return smooth_only();
-  Prod U = multiply(n, n, View(L.A), S, st);
+  if (!dense && A.nnz > kFoldEntries) return smooth_only();
+  Prod U = multiply(n, n, View(A), S, st);
   if (!add_identity(U, -1.0, 1.0, st)) return smooth_only();        // U = I - A S
-  Prod R = multiply(nc, n, View(L.Pt), U, st);
+  Prod R = multiply(nc, n, View(Pt), U, st);
   if (!dense && R.nnz > kFoldEntries) return smooth_only();
   Prod Q, E;
-  bool all = dense || 3 * L.A.nnz <= kFoldEntries;
+  bool all = dense || 3 * A.nnz <= kFoldEntries;
   if (all && add_identity(U, 1.0, 1.0, st)) {                       // I + U
     Q = multiply(n, n, S, U, st);
     U = Prod();
     all = dense || Q.nnz <= kFoldEntries;
     if (all) {
-      Prod X = multiply(n, n, S, View(L.A), st);
+      Prod X = multiply(n, n, S, View(A), st);
       all = add_identity(X, -1.0, 1.0, st);                         // I - S A
-      if (all) E = multiply(n, nc, X, View(L.P), st);
+      if (all) E = multiply(n, nc, X, View(P), st);
       all = all && (dense || Q.nnz + E.nnz <= kFoldEntries);
     }
   } else {
     all = false;
   }
   if (!all) {
-    adopt(S, f->Q, fp32, st);
+    adopt(S, f->S, fp32, st);
     adopt(R, f->R, fp32, st);
-    f->lanes = fold_lanes(f->Q.nnz + L.P.nnz, n);
+    f->lanes = fold_lanes(f->S.nnz + P.nnz, n);
     f->form = FOLD_DOWN;
     return f;
   }
@@ -218,7 +213,7 @@ std::unique_ptr<Fold> fold_level(Hier &h, int l) {
     DBuf<int> trp, tci;
     csr_transpose_device(nc, n, R.nnz, R.rp, R.ci, R.v, trp, tci, tv, st);
     k_sparse_dense<<<n, 256, 0, st>>>(nc, E.rp.get(), E.ci.get(), E.v.get(), B,
-                                      C.coarsest ? nc : C.fold->ld, Y.get());
+                                      ldb, Y.get());
     CHRONOS_CHECK_LAUNCH();
     k_dense_tail<<<n, 256, sizeof(double) * nc, st>>>(n, nc, Y.get(), trp.get(), tci.get(),
                                                       tv.get(), Q.rp.get(), Q.ci.get(),
@@ -228,6 +223,7 @@ std::unique_ptr<Fold> fold_level(Hier &h, int l) {
     f->form = FOLD_DENSE;
     return f;
   }
+  adopt(S, f->S, fp32, st);
   adopt(Q, f->Q, fp32, st);
   adopt(E, f->E, fp32, st);
   adopt(R, f->R, fp32, st);
@@ -236,14 +232,27 @@ std::unique_ptr<Fold> fold_level(Hier &h, int l) {
   return f;
 }
 
-}  // namespace
+void tune_fold(Fold &F, bool fp32, cudaStream_t st) {
+  if (F.form == FOLD_SMOOTH || F.form == FOLD_DOWN) autotune_lanes(F.S, fp32, st);
+  if (F.form == FOLD_DOWN) autotune_lanes(F.R, fp32, st);
+}
 
 void build_folds(Hier &h) {
   for (auto &L : h.levels) L.fold.reset();
   // the algebra above is one pre- and one postsmoothing step; a caller who
   // chose the storage of the operators (spmv_format) gets them applied so
   if (h.prm.nupre > 1 || h.prm.nupost != 1 || h.prm.spmv_format != 0) return;
-  for (int l = (int)h.levels.size() - 2; l >= 0; --l) h.levels[l].fold = fold_level(h, l);
+  for (int l = (int)h.levels.size() - 2; l >= 0; --l) {
+    Level &L = h.levels[l];
+    const Level &C = h.levels[l + 1];
+    // level 1 keeps its fused dot and conversions: no dense form
+    const double *B = nullptr;
+    int ldb = 0;
+    if (l > 0 && C.coarsest) { B = C.W.get(); ldb = C.n; }
+    else if (l > 0 && C.fold && C.fold->form == FOLD_DENSE) { B = C.fold->D.get(); ldb = C.fold->ld; }
+    L.fold = fold_operators(L.A, L.G, L.Gt, L.P, L.Pt, L.omega, B, ldb,
+                            h.precision == CHRONOS_FP32, h.st);
+  }
 }
 
 }  // namespace chronos

@@ -24,6 +24,7 @@
 #include <vector>
 
 #include "group.h"
+#include "fold.cuh"
 #include "spmv.cuh"
 
 namespace chronos {
@@ -441,7 +442,17 @@ std::unique_ptr<GroupSolve> group_build(const std::vector<std::unique_ptr<Hier>>
     upload_csr(stack_blocks(ppt, L.nS, st), L.Pt, fp32, st);
     CHRONOS_CUDA(cudaStreamSynchronize(st));
     const auto tl1 = std::chrono::steady_clock::now();
-    for (DMat *m : {&L.A, &L.G, &L.Gt, &L.P, &L.Pt}) autotune_lanes(*m, fp32, st, prm.spmv_format);
+    // one pre- and one postsmoothing step in the autotuner's storage: folded as a
+    // single hierarchy's level is (the stack is block diagonal, G' scaled)
+    if (prm.nupre <= 1 && prm.nupost == 1 && prm.spmv_format == 0)
+      L.fold = fold_operators(L.A, L.G, L.Gt, L.P, L.Pt, 1.0, nullptr, 0, fp32, st);
+    const Fold *F = L.fold.get();
+    if (F) tune_fold(*L.fold, fp32, st);
+    if (!F || F->form != FOLD_ALL) autotune_lanes(L.A, fp32, st, prm.spmv_format);
+    if (!F)
+      for (DMat *m : {&L.G, &L.Gt}) autotune_lanes(*m, fp32, st, prm.spmv_format);
+    if (!F || F->form == FOLD_SMOOTH)
+      for (DMat *m : {&L.P, &L.Pt}) autotune_lanes(*m, fp32, st, prm.spmv_format);
     CHRONOS_CUDA(cudaStreamSynchronize(st));
     if (verbose)
       std::fprintf(stderr, "chronos group: level %d stacked in %.3f s, tuned in %.3f s\n", l,
@@ -495,7 +506,9 @@ std::unique_ptr<GroupSolve> group_build(const std::vector<std::unique_ptr<Hier>>
   for (int p = 0; p < np; ++p) {
     const int n = hs[p]->levels[0].n;
     rs[p + 1] = rs[p] + n;
-    bs[p + 1] = bs[p] + std::max(1, std::min(256, (int)ceil_div(n, 2048)));
+    // a block per 512 rows: two a thread, enough blocks to fill the GPU from a
+    // batch of 76k rows on (at 2048 a batch of 223k rows ran 109 blocks)
+    bs[p + 1] = bs[p] + std::max(1, std::min(256, (int)ceil_div(n, 512)));
   }
   g.nblocks = bs[np];
   g.rstart.upload(rs, st);
@@ -512,6 +525,39 @@ std::unique_ptr<GroupSolve> group_build(const std::vector<std::unique_ptr<Hier>>
   return G;
 }
 
+// The two halves of a folded level, as vcycle_level runs them.
+template <typename T, typename BT>
+static void group_fold_down(GroupSolve &g, GroupLevel &L, const BT *b, T *bc) {
+  cudaStream_t st = g.st;
+  const Fold &F = *L.fold;
+  T *x = gvec<T>(L.x32, L.x64), *r = gvec<T>(L.r32, L.r64);
+  if (F.form != FOLD_SMOOTH) {
+    restrict_apply<T, BT>(st, F.R, b, bc);
+    return;
+  }
+  mat_apply<T, BT, T, T, MODE_PLAIN, false>(st, F.S, vals<T>(F.S), b, nullptr, x, T(1));
+  mat_apply<T, T, BT, T, MODE_RESID, false>(st, L.A, vals<T>(L.A), x, b, r, T(1));
+  mat_apply<T, T, T, T, MODE_PLAIN, false>(st, L.Pt, vals<T>(L.Pt), r, nullptr, bc, T(1));
+}
+
+template <typename T, typename BT, typename OT>
+static void group_fold_up(GroupSolve &g, GroupLevel &L, const BT *b, const T *e, OT *out) {
+  cudaStream_t st = g.st;
+  const Fold &F = *L.fold;
+  T *x = gvec<T>(L.x32, L.x64), *r = gvec<T>(L.r32, L.r64);
+  if (F.form == FOLD_ALL) {
+    fold_apply<T, BT, OT, false>(st, F.lanes, F.Q, F.E, b, e, out, nullptr, nullptr, nullptr,
+                                 nullptr);
+    return;
+  }
+  if (F.form == FOLD_SMOOTH)
+    mat_apply<T, T, T, T, MODE_AXPY, false>(st, L.P, vals<T>(L.P), e, x, x, T(1));
+  else
+    fold_apply<T, BT, T, false>(st, F.lanes, F.S, L.P, b, e, x, nullptr, nullptr, nullptr, nullptr);
+  mat_apply<T, T, BT, T, MODE_RESID, false>(st, L.A, vals<T>(L.A), x, b, r, T(1));
+  mat_apply<T, T, T, OT, MODE_AXPY, false>(st, F.S, vals<T>(F.S), r, x, out, T(1));
+}
+
 // The level-synchronous V-cycle: res (FP64) -> pres (FP64) for every problem.
 template <typename T>
 static void group_vcycle(GroupSolve &g) {
@@ -525,6 +571,11 @@ static void group_vcycle(GroupSolve &g) {
     T *x = gvec<T>(L.x32, L.x64), *r = gvec<T>(L.r32, L.r64), *t = gvec<T>(L.t32, L.t64);
     GroupLevel &N = g.lev[l + 1];
     T *bc = gvec<T>(N.b32, N.b64);
+    if (L.fold) {
+      if (l == 0) group_fold_down<T, double>(g, L, g.res.get(), bc);
+      else group_fold_down<T, T>(g, L, gvec<T>(L.b32, L.b64), bc);
+      continue;
+    }
     if (l == 0) {
       const double *b = g.res.get();
       mat_apply<T, double, T, T, MODE_PLAIN, false>(st, L.G, vals<T>(L.G), b, nullptr, t, T(1));
@@ -562,6 +613,11 @@ static void group_vcycle(GroupSolve &g) {
     T *x = gvec<T>(L.x32, L.x64), *r = gvec<T>(L.r32, L.r64), *t = gvec<T>(L.t32, L.t64);
     GroupLevel &N = g.lev[l + 1];
     const T *xc = gvec<T>(N.x32, N.x64);
+    if (L.fold) {
+      if (l == 0) group_fold_up<T, double, double>(g, L, g.res.get(), xc, g.pres.get());
+      else group_fold_up<T, T, T>(g, L, gvec<T>(L.b32, L.b64), xc, x);
+      continue;
+    }
     mat_apply<T, T, T, T, MODE_AXPY, false>(st, L.P, vals<T>(L.P), xc, x, x, T(1));
     for (int k = 0; k < npost; ++k) {
       const bool lastk = k + 1 == npost;

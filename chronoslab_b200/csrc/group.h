@@ -18,6 +18,7 @@ struct GroupLevel {
   // A, G, G' (scaled by each problem's omega) over the nS rows; P: nS rows x
   // the next level's nV columns; P': the next level's nV rows x nS columns
   DMat A, G, Gt, P, Pt;
+  std::unique_ptr<Fold> fold;   // the stacked operators folded (fold.cu), else null
   DBuf<float> b32, x32, r32, t32;
   DBuf<double> b64, x64, r64, t64;
 };

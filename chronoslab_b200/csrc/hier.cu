@@ -27,6 +27,7 @@
 
 #include <nvtx3/nvToolsExt.h>
 
+#include "fold.cuh"
 #include "hier.h"
 #include "spmv.cuh"
 
@@ -1424,8 +1425,7 @@ void tune_hierarchy(Hier &h) {
       autotune_lanes(L.P, fp32, h.st, fmt);
       autotune_lanes(L.Pt, fp32, h.st, fmt);
     }
-    if (F && F->form != FOLD_ALL) autotune_lanes(F->Q, fp32, h.st, fmt);
-    if (F && F->form == FOLD_DOWN) autotune_lanes(F->R, fp32, h.st, fmt);
+    if (F) tune_fold(*F, fp32, h.st);
   }
   // the level-1 FP64 operator of the outer PCG
   if (fp32 && h.prm.exact_outer) autotune_lanes(h.levels[0].A, false, h.st);
@@ -1636,117 +1636,6 @@ __global__ void k_dot_store(int n, const double *a, const double *b, double *par
   grid_reduce<1>(v, part, ticket, StoreScalar{out});
 }
 
-// y = R b, a block per row: R's rows are the products of P' with two operators
-// and on the levels that end a hierarchy a few hundred of them hold thousands of
-// entries each (elasticity 24^3, FP64, 205 rows of 2270 entries: 77 us per PCG
-// iteration with a warp per row, 61 with a block).
-template <typename T, typename BT, bool I16>
-__global__ void __launch_bounds__(kApplyThreads)
-k_wide_rows(int n, const int *__restrict__ rp, const int *__restrict__ ci,
-            const int *__restrict__ cbase, const uint16_t *__restrict__ c16,
-            const T *__restrict__ v, const BT *__restrict__ b, T *__restrict__ y) {
-  pdl_begin();
-  __shared__ T red[kApplyThreads / 32];
-  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-  for (int row = blockIdx.x; row < n; row += gridDim.x) {
-    const int s = __ldg(rp + row), e = __ldg(rp + row + 1);
-    const T a = warp_sum(csr_row_dot<T, T, BT, kApplyThreads, I16>(
-        s + (int)threadIdx.x, e, I16 ? __ldg(cbase + row) : 0, ci, c16, v, b));
-    if (lane == 0) red[wid] = a;
-    __syncthreads();
-    if (threadIdx.x == 0) {
-      T t = red[0];
-      for (int w = 1; w < kApplyThreads / 32; ++w) t += red[w];
-      y[row] = t;
-    }
-    __syncthreads();
-  }
-}
-
-// Restriction of a folded level: a block per row from an average row of a warp's
-// eight batches on, else the tuned row-group kernel.
-template <typename T, typename BT>
-static void restrict_apply(cudaStream_t st, const DMat &R, const BT *b, T *y) {
-  if (R.nnz < (int64_t)256 * R.nrows) {
-    mat_apply<T, BT, T, T, MODE_PLAIN, false>(st, R, vals<T>(R), b, nullptr, y, T(1));
-    return;
-  }
-  const int grid = std::min(R.nrows, num_sms() * 8);
-  launch_pdl(R.idx16 ? k_wide_rows<T, BT, true> : k_wide_rows<T, BT, false>, grid, kApplyThreads,
-             st, R.nrows, (const int *)R.rp.get(), (const int *)R.ci.get(),
-             (const int *)R.cbase.get(), (const uint16_t *)R.c16.get(), vals<T>(R), b, y);
-}
-
-// out = Q b + E e on a folded level, L lanes per row (and out . dw).
-template <typename T, typename BT, typename OT, int L, bool DOT, bool QI16, bool EI16>
-__global__ void __launch_bounds__(kApplyThreads)
-k_fold_apply(int n, const int *__restrict__ qrp, const int *__restrict__ qci,
-             const int *__restrict__ qbase, const uint16_t *__restrict__ q16,
-             const T *__restrict__ qv, const int *__restrict__ erp, const int *__restrict__ eci,
-             const int *__restrict__ ebase, const uint16_t *__restrict__ e16,
-             const T *__restrict__ ev, const BT *__restrict__ b, const T *__restrict__ e,
-             OT *__restrict__ out, const double *__restrict__ dw, double *part, unsigned *ticket,
-             double *dot_out) {
-  pdl_begin();
-  constexpr int R = 32 / L;
-  const int lane = threadIdx.x & 31, g = lane / L, gl = lane & (L - 1);
-  const int warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-  const int nwarps = (gridDim.x * blockDim.x) >> 5;
-  double dacc = 0.0;
-  for (int base = warp * R; base < n; base += nwarps * R) {     // warp-uniform trip count
-    const int row = base + g;
-    T a = T(0);
-    if (row < n) {
-      const int qs = __ldg(qrp + row), qe = __ldg(qrp + row + 1);
-      const int es = __ldg(erp + row), ee = __ldg(erp + row + 1);
-      const int qb = QI16 ? __ldg(qbase + row) : 0, eb = EI16 ? __ldg(ebase + row) : 0;
-      a = csr_row_dot<T, T, T, L, EI16>(es + gl, ee, eb, eci, e16, ev, e);
-      a += csr_row_dot<T, T, BT, L, QI16>(qs + gl, qe, qb, qci, q16, qv, b);
-    }
-    a = group_sum<L>(a);
-    if (row < n && gl == 0) {
-      const OT o = (OT)a;
-      out[row] = o;
-      if (DOT) dacc += (double)o * dw[row];
-    }
-  }
-  if (DOT) {
-    double vals[1] = {dacc};
-    grid_reduce<1>(vals, part, ticket, StoreScalar{dot_out});
-  }
-}
-
-template <typename T, typename BT, typename OT, bool DOT>
-static void fold_apply(cudaStream_t st, int lanes, const DMat &Q, const DMat &E, const BT *b,
-                       const T *e, OT *out, const double *dw, double *part, unsigned *tick,
-                       double *dot_out) {
-  const int n = Q.nrows;
-  const int grid = std::min<int>(ceil_div((int64_t)n * lanes, kApplyThreads), num_sms() * 8);
-  auto launch = [&](auto kern) {
-    launch_pdl(kern, grid, kApplyThreads, st, n, (const int *)Q.rp.get(), (const int *)Q.ci.get(),
-               (const int *)Q.cbase.get(), (const uint16_t *)Q.c16.get(), vals<T>(Q),
-               (const int *)E.rp.get(), (const int *)E.ci.get(), (const int *)E.cbase.get(),
-               (const uint16_t *)E.c16.get(), vals<T>(E), b, e, out, dw, part, tick, dot_out);
-  };
-#define CHRONOS_FOLD_CASE(LL)                                                              \
-  case LL:                                                                                 \
-    if (Q.idx16 && E.idx16) launch(k_fold_apply<T, BT, OT, LL, DOT, true, true>);          \
-    else if (E.idx16) launch(k_fold_apply<T, BT, OT, LL, DOT, false, true>);               \
-    else if (Q.idx16) launch(k_fold_apply<T, BT, OT, LL, DOT, true, false>);               \
-    else launch(k_fold_apply<T, BT, OT, LL, DOT, false, false>);                           \
-    break;
-  switch (lanes) {
-    CHRONOS_FOLD_CASE(1)
-    CHRONOS_FOLD_CASE(2)
-    CHRONOS_FOLD_CASE(4)
-    CHRONOS_FOLD_CASE(8)
-    CHRONOS_FOLD_CASE(16)
-    CHRONOS_FOLD_CASE(32)
-    default: throw Error(CHRONOS_EINVAL, "fold_apply: bad lane count");
-  }
-#undef CHRONOS_FOLD_CASE
-}
-
 // x = D b, D with rows of ld values (ld even): a warp per row, 16-byte loads.
 template <typename TI, typename TO>
 __global__ void __launch_bounds__(256)
@@ -1802,7 +1691,7 @@ static void vcycle_level(Hier &h, int l, const BT *b, OT *out, const double *dw,
     T *x = L.x<T>(), *r = L.r<T>(), *bc = C.b<T>(), *e = C.x<T>();
     // down: b_c = R b, or through the residual of x = S b
     if (F.form == FOLD_SMOOTH) {
-      mat_apply<T, BT, T, T, MODE_PLAIN, false>(st, F.Q, vals<T>(F.Q), b, nullptr, x, T(1));
+      mat_apply<T, BT, T, T, MODE_PLAIN, false>(st, F.S, vals<T>(F.S), b, nullptr, x, T(1));
       op_apply<T, T, BT, T, MODE_RESID, false>(st, L.A, x, b, r, T(1));
       mat_apply<T, T, T, T, MODE_PLAIN, false>(st, L.Pt, vals<T>(L.Pt), r, nullptr, bc, T(1));
     } else {
@@ -1821,14 +1710,14 @@ static void vcycle_level(Hier &h, int l, const BT *b, OT *out, const double *dw,
     if (F.form == FOLD_SMOOTH)
       mat_apply<T, T, T, T, MODE_AXPY, false>(st, L.P, vals<T>(L.P), e, x, x, T(1));
     else
-      fold_apply<T, BT, T, false>(st, F.lanes, F.Q, L.P, b, e, x, nullptr, nullptr, nullptr,
+      fold_apply<T, BT, T, false>(st, F.lanes, F.S, L.P, b, e, x, nullptr, nullptr, nullptr,
                                   nullptr);
     op_apply<T, T, BT, T, MODE_RESID, false>(st, L.A, x, b, r, T(1));
     if (TOP && dw)
-      mat_apply<T, T, T, OT, MODE_AXPY, TOP>(st, F.Q, vals<T>(F.Q), r, x, out, T(1), dw, part,
+      mat_apply<T, T, T, OT, MODE_AXPY, TOP>(st, F.S, vals<T>(F.S), r, x, out, T(1), dw, part,
                                              tick, dot_out);
     else
-      mat_apply<T, T, T, OT, MODE_AXPY, false>(st, F.Q, vals<T>(F.Q), r, x, out, T(1));
+      mat_apply<T, T, T, OT, MODE_AXPY, false>(st, F.S, vals<T>(F.S), r, x, out, T(1));
     return;
   }
   T *x = L.x<T>(), *r = L.r<T>(), *t = L.t<T>();
@@ -2702,11 +2591,11 @@ static double vcycle_bytes_level(const Hier &h, int l, double s, double sb, doub
     if (F.form == FOLD_ALL)
       return apply_bytes(F.R, s, sb, s, 0.0) + coarse + apply_bytes(F.Q, s, sb, sout, dot) +
              apply_bytes(F.E, s, s, 0.0, 0.0);
-    const double resid = apply_bytes(L.A, s, s, s, sb), up = apply_bytes(F.Q, s, s, sout, s + dot);
+    const double resid = apply_bytes(L.A, s, s, s, sb), up = apply_bytes(F.S, s, s, sout, s + dot);
     if (F.form == FOLD_DOWN)
-      return apply_bytes(F.R, s, sb, s, 0.0) + coarse + apply_bytes(F.Q, s, sb, s, 0.0) +
+      return apply_bytes(F.R, s, sb, s, 0.0) + coarse + apply_bytes(F.S, s, sb, s, 0.0) +
              apply_bytes(L.P, s, s, 0.0, 0.0) + resid + up;
-    return apply_bytes(F.Q, s, sb, s, 0.0) + 2 * resid + apply_bytes(L.Pt, s, s, s, 0.0) + coarse +
+    return apply_bytes(F.S, s, sb, s, 0.0) + 2 * resid + apply_bytes(L.Pt, s, s, s, 0.0) + coarse +
            apply_bytes(L.P, s, s, s, s) + up;
   }
   b += apply_bytes(L.G, s, sb, s, 0.0);                     // t = G b

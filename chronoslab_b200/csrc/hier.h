@@ -45,12 +45,13 @@ void validate_csr(const HostCSR &A);
 // CHRONOS_GPU_COARSEN not set to 0.
 bool gpu_coarsening(const char *soc_type);
 
-// The folded form of a level (fold.cu).  FOLD_SMOOTH: Q = S; FOLD_DOWN: Q = S and
-// R; FOLD_ALL: R, Q, E; FOLD_DENSE: D, n rows of ld values (ld even).
+// The folded form of a level (fold.cu).  FOLD_SMOOTH: S; FOLD_DOWN: S and R;
+// FOLD_ALL: R, Q, E (and S, for block solves); FOLD_DENSE: D, n rows of ld
+// values (ld even).
 enum FoldForm { FOLD_SMOOTH, FOLD_DOWN, FOLD_ALL, FOLD_DENSE };
 struct Fold {
   FoldForm form = FOLD_SMOOTH;
-  DMat R, Q, E;
+  DMat S, R, Q, E;
   int lanes = 8;                   // lanes per row of S b + P e or Q b + E e
   DBuf<double> D;
   int ld = 0;
@@ -276,6 +277,14 @@ void tune_hierarchy(Hier &h);
 // Folds the levels for which that is the faster form (fold.cu); part of
 // tune_hierarchy.
 void build_folds(Hier &h);
+// The folded form of one level's operators, or null where none pays: A, G, G',
+// P, P' as the cycle applies them, the smoother scaled by omega; B: the dense
+// operator (rows of ldb values) of everything below, null if there is none.
+std::unique_ptr<Fold> fold_operators(const DMat &A, const DMat &G, const DMat &Gt, const DMat &P,
+                                     const DMat &Pt, double omega, const double *B, int ldb,
+                                     bool fp32, cudaStream_t st);
+// Tunes the operators of a folded form that go through mat_apply.
+void tune_fold(Fold &F, bool fp32, cudaStream_t st);
 
 // One hierarchy built level by level (what build_hierarchy runs): a level is
 // begun (its operator uploaded; the coarsest factored, begin_level then
