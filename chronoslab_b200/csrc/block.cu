@@ -195,14 +195,15 @@ static void spmm(cudaStream_t st, const DMat &M, const VT *vals, const XT *X, co
 }
 
 // Y = W B on the coarsest level (W FP64 n x n row-major, B n x K row-major).
+// (rows of W ld values apart)
 template <typename TI, typename TO, int K>
-__global__ void k_dense_matmat(int n, const double *__restrict__ W, const TI *__restrict__ B,
-                               TO *__restrict__ Y) {
+__global__ void k_dense_matmat(int n, int ld, const double *__restrict__ W,
+                               const TI *__restrict__ B, TO *__restrict__ Y) {
   pdl_begin();
   const int row = blockIdx.x, j = threadIdx.x % K, g = threadIdx.x / K, G = blockDim.x / K;
   __shared__ double red[256];
   double s = 0.0;
-  for (int c = g; c < n; c += G) s += W[(size_t)row * n + c] * (double)B[(size_t)c * K + j];
+  for (int c = g; c < n; c += G) s += W[(size_t)row * ld + c] * (double)B[(size_t)c * K + j];
   red[threadIdx.x] = s;
   __syncthreads();
   if (g == 0) {
@@ -255,12 +256,47 @@ static void vcycle_block(Hier &h, BlockState &s, int l, const BT *b, OT *out, co
   double *part = s.part.get();
   unsigned *tick = s.tickets.get();
   if (L.coarsest) {
-    launch_pdl(k_dense_matmat<BT, OT, K>, n, 256, st, n, (const double *)L.W.get(), b, out);
+    launch_pdl(k_dense_matmat<BT, OT, K>, n, 256, st, n, n, (const double *)L.W.get(), b, out);
     CHRONOS_CHECK_LAUNCH();
     return;
   }
   T *x = blk<T>(s.x32, s.x64, l), *r = blk<T>(s.r32, s.r64, l), *t = blk<T>(s.t32, s.t64, l);
   const T w = (T)L.omega;
+  if (L.fold && L.fold->form == FOLD_DENSE) {
+    launch_pdl(k_dense_matmat<BT, OT, K>, n, 256, st, n, L.fold->ld,
+               (const double *)L.fold->D.get(), b, out);
+    CHRONOS_CHECK_LAUNCH();
+    return;
+  }
+  if (L.fold) {
+    // the smoother folded, and the restriction (fold.cu) where its longer rows
+    // gather at most 16 MB (some 4 us, two launches) more over the K columns; Q
+    // and E would gather several times as much.  Diffusion 64^3 x 16 FP32: 366 us
+    // per iteration unfolded, 349 with R on every folded level, 342 so; 45^3 x 5
+    // FP64: 187, 191 and 172.
+    const Fold &F = *L.fold;
+    const bool down = F.form != FOLD_SMOOTH &&
+                      (double)(F.R.nnz - L.A.nnz - L.Pt.nnz) * K * sizeof(T) <= 16e6;
+    T *bc = blk<T>(s.b32, s.b64, l + 1), *xc = blk<T>(s.x32, s.x64, l + 1);
+    spmm<T, BT, T, T, K, MODE_PLAIN, false>(st, F.S, vals<T>(F.S), b, (const T *)nullptr, x, T(1));
+    if (!down) {
+      spmm<T, T, BT, T, K, MODE_RESID, false>(st, L.A, vals<T>(L.A), x, b, r, T(1));
+      spmm<T, T, T, T, K, MODE_PLAIN, false>(st, L.Pt, vals<T>(L.Pt), r, (const T *)nullptr, bc,
+                                             T(1));
+    } else {
+      spmm<T, BT, T, T, K, MODE_PLAIN, false>(st, F.R, vals<T>(F.R), b, (const T *)nullptr, bc,
+                                              T(1));
+    }
+    vcycle_block<T, T, T, K>(h, s, l + 1, bc, xc, nullptr, nullptr);
+    spmm<T, T, T, T, K, MODE_AXPY, false>(st, L.P, vals<T>(L.P), xc, x, x, T(1));
+    spmm<T, T, BT, T, K, MODE_RESID, false>(st, L.A, vals<T>(L.A), x, b, r, T(1));
+    if (dw)
+      spmm<T, T, T, OT, K, MODE_AXPY, true>(st, F.S, vals<T>(F.S), r, x, out, T(1), dw, part, tick,
+                                            dot_out);
+    else
+      spmm<T, T, T, OT, K, MODE_AXPY, false>(st, F.S, vals<T>(F.S), r, x, out, T(1));
+    return;
+  }
   spmm<T, BT, T, T, K, MODE_PLAIN, false>(st, L.G, vals<T>(L.G), b, (const T *)nullptr, t, T(1));
   spmm<T, T, T, T, K, MODE_SCALE, false>(st, L.Gt, vals<T>(L.Gt), t, (const T *)nullptr, x, w);
   for (int k = 1; k < h.prm.nupre; ++k) {
@@ -585,8 +621,12 @@ static void block_solve(Hier &h, int m, const BlockIn &B, const double *X0_h, do
   auto pack = [&](const BlockIn &src, double *dst) {
     if (src.ld > 0) {                              // row-major, rows ld apart
       double *to = m == K ? dst : s.stage.get();
-      CHRONOS_CUDA(cudaMemcpy2DAsync(to, sizeof(double) * m, src.p, sizeof(double) * src.ld,
-                                     sizeof(double) * m, n, cudaMemcpyHostToDevice, st));
+      if (src.ld == m)                             // one copy: row by row is far slower
+        CHRONOS_CUDA(cudaMemcpyAsync(to, src.p, sizeof(double) * n * m, cudaMemcpyHostToDevice,
+                                     st));
+      else
+        CHRONOS_CUDA(cudaMemcpy2DAsync(to, sizeof(double) * m, src.p, sizeof(double) * src.ld,
+                                       sizeof(double) * m, n, cudaMemcpyHostToDevice, st));
       if (m == K) return;
       k_block_layout<K, true><<<lb, 256, 0, st>>>(n, m, m, 1, s.stage.get(), dst);
     } else {

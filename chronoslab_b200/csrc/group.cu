@@ -68,12 +68,12 @@ __device__ __forceinline__ void group_reduce(double (&v)[K], int p, int b0, int 
       for (int w = 0; w < nw; ++w) s += red[j][w];
       part[(size_t)blockIdx.x * K + j] = s;
     }
-    __threadfence();
+    fence_gpu();
     last = atomicAdd(tickets + p, 1u) == (unsigned)(nbp - 1);
   }
   __syncthreads();
   if (!last) return;
-  __threadfence();
+  fence_gpu();
   double acc[K];
 #pragma unroll
   for (int j = 0; j < K; ++j) acc[j] = 0.0;
@@ -250,6 +250,8 @@ k_group_spmv(int np, const int *__restrict__ bstart, const int *__restrict__ rst
 
 // x += alpha p; res -= alpha axp; ||res||^2; stop test per problem, and the
 // loop condition once every active problem is done.
+// (scalars read before the first store: between stores they were a chain of
+// L2 round trips)
 struct FinResidualGroup {
   GroupCtl c;
   cudaGraphConditionalHandle handle;
@@ -259,19 +261,19 @@ struct FinResidualGroup {
     // problems active when this update began; only the last of their
     // finalisers changes it, after every one of them has taken a ticket
     const unsigned nact = *(volatile unsigned *)c.g;
-    const double resiter = sqrt(t[0]) / s[GS_BNORM];
-    const double it = s[GS_ITER] + 1.0;
+    const double bnorm = s[GS_BNORM], it0 = s[GS_ITER], broke = s[GS_BREAKDOWN];
+    const double resiter = sqrt(t[0]) / bnorm;
+    const double it = it0 + 1.0;
+    const bool stop = resiter < c.tol || it >= c.itmax || broke != 0.0 || !isfinite(resiter);
     s[GS_ITER] = it;
     s[GS_RESITER] = resiter;
-    const bool stop = resiter < c.tol || it >= c.itmax || s[GS_BREAKDOWN] != 0.0 ||
-                      !isfinite(resiter);
     if (stop) {
       s[GS_ACTIVE] = 0.0;
       atomicSub(c.g + 2, 1u);
     }
-    __threadfence();
+    fence_gpu();
     if (atomicAdd(c.g + 1, 1u) == nact - 1) {     // the last active problem's finaliser
-      __threadfence();
+      fence_gpu();
       const unsigned left = atomicAdd(c.g + 2, 0u);
       c.g[0] = left;
       c.g[1] = 0u;
@@ -302,23 +304,31 @@ k_group_xr_update(int np, const int *__restrict__ bstart, const int *__restrict_
 }
 
 // Batched coarsest solves x = W b: a warp per row of every problem whose
-// coarsest level this is (rows of all such problems listed back to back).
-template <typename T>
+// coarsest level this is.  Each row's addresses lie in one record: looked up
+// through the row's problem they were two more dependent loads before the
+// first of W (6928 rows of 577 on average: 15.2 us; 11.9 us so, eight loads in
+// flight).
 __global__ void __launch_bounds__(256)
-k_group_dense(int nrows, const int *__restrict__ row_prob, const int *__restrict__ row_local,
-              const double *const *__restrict__ W, const int *__restrict__ n,
-              const T *const *__restrict__ b, T *const *__restrict__ x) {
+k_group_dense(int nrows, const GroupDenseRow *__restrict__ rows, int fp32) {
   pdl_begin();
   const int lane = threadIdx.x & 31;
   const int r = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   if (r >= nrows) return;
-  const int q = __ldg(row_prob + r), i = __ldg(row_local + r), m = __ldg(n + q);
-  const double *w = W[q] + (size_t)i * m;
-  const T *bq = b[q];
+  const GroupDenseRow q = rows[r];
   double s = 0.0;
-  for (int j = lane; j < m; j += 32) s += w[j] * (double)bq[j];
-  s = warp_sum(s);
-  if (lane == 0) x[q][i] = (T)s;
+  if (fp32) {
+    const float *b = static_cast<const float *>(q.b);
+#pragma unroll 8
+    for (int j = lane; j < q.m; j += 32) s += __ldg(q.w + j) * (double)b[j];
+    s = warp_sum(s);
+    if (lane == 0) *static_cast<float *>(q.x) = (float)s;
+  } else {
+    const double *b = static_cast<const double *>(q.b);
+#pragma unroll 8
+    for (int j = lane; j < q.m; j += 32) s += __ldg(q.w + j) * b[j];
+    s = warp_sum(s);
+    if (lane == 0) *static_cast<double *>(q.x) = s;
+  }
 }
 
 // ---------------------------------------------------------------------------
@@ -466,32 +476,29 @@ std::unique_ptr<GroupSolve> group_build(const std::vector<std::unique_ptr<Hier>>
   }
   // coarsest solves of every level, listed row by row
   {
-    std::vector<int> rprob, rloc, nq;
-    std::vector<const double *> W;
-    std::vector<void *> bq, xq;
+    std::vector<GroupDenseRow> rows;
     for (int l = 1; l <= lmax; ++l)
       for (int p : g.lev[l].C) {
         const Level &lv = hs[p]->levels[l];
-        const int q = (int)W.size();
-        W.push_back(lv.W.get());
-        nq.push_back(lv.n);
-        const size_t off = g.lev[l].off[p];
-        if (fp32) {
-          bq.push_back(g.lev[l].b32.get() + off);
-          xq.push_back(g.lev[l].x32.get() + off);
-        } else {
-          bq.push_back(g.lev[l].b64.get() + off);
-          xq.push_back(g.lev[l].x64.get() + off);
+        GroupLevel &G2 = g.lev[l];
+        const size_t off = G2.off[p];
+        for (int i = 0; i < lv.n; ++i) {
+          GroupDenseRow r;
+          r.w = lv.W.get() + (size_t)i * lv.n;
+          r.m = lv.n;
+          if (fp32) {
+            r.b = G2.b32.get() + off;
+            r.x = G2.x32.get() + off + i;
+          } else {
+            r.b = G2.b64.get() + off;
+            r.x = G2.x64.get() + off + i;
+          }
+          rows.push_back(r);
         }
-        for (int i = 0; i < lv.n; ++i) { rprob.push_back(q); rloc.push_back(i); }
       }
-    g.ncoarse_rows = (int)rprob.size();
-    g.c_prob.upload(rprob, st);
-    g.c_row.upload(rloc, st);
-    g.c_n.upload(nq, st);
-    g.c_W.upload(reinterpret_cast<const uintptr_t *>(W.data()), W.size(), st);
-    g.c_b.upload(reinterpret_cast<const uintptr_t *>(bq.data()), bq.size(), st);
-    g.c_x.upload(reinterpret_cast<const uintptr_t *>(xq.data()), xq.size(), st);
+    g.ncoarse_rows = (int)rows.size();
+    g.c_rows.upload(rows, st);
+    CHRONOS_CUDA(cudaStreamSynchronize(st));
   }
   // finest operators of all problems for the outer product (FP64)
   {
@@ -601,11 +608,9 @@ static void group_vcycle(GroupSolve &g) {
   }
   // coarsest solves of every problem
   if (g.ncoarse_rows > 0)
-    launch_pdl(k_group_dense<T>, ceil_div((int64_t)g.ncoarse_rows * 32, 256), 256, st,
-               g.ncoarse_rows, (const int *)g.c_prob.get(), (const int *)g.c_row.get(),
-               reinterpret_cast<const double *const *>(g.c_W.get()), (const int *)g.c_n.get(),
-               reinterpret_cast<const T *const *>(g.c_b.get()),
-               reinterpret_cast<T *const *>(g.c_x.get()));
+    launch_pdl(k_group_dense, ceil_div((int64_t)g.ncoarse_rows * 32, 256), 256, st,
+               g.ncoarse_rows, (const GroupDenseRow *)g.c_rows.get(),
+               g.precision == CHRONOS_FP32 ? 1 : 0);
   // up
   for (int l = lmax - 1; l >= 0; --l) {
     GroupLevel &L = g.lev[l];

@@ -23,6 +23,15 @@ struct GroupLevel {
   DBuf<double> b64, x64, r64, t64;
 };
 
+// One row of a coarsest solve: x = w' b over m entries (b, x in the hierarchy's
+// precision).
+struct GroupDenseRow {
+  const double *w = nullptr;
+  const void *b = nullptr;
+  void *x = nullptr;
+  int m = 0;
+};
+
 struct GroupSolve {
   int np = 0, nrows = 0, precision = CHRONOS_FP32;
   chronos_params prm{};
@@ -31,8 +40,7 @@ struct GroupSolve {
   DBuf<int> rstart, bstart;                  // per problem: rows and blocks of the vector kernels
   int nblocks = 0;
   int ncoarse_rows = 0;                      // batched coarsest solves
-  DBuf<int> c_prob, c_row, c_n;
-  DBuf<uintptr_t> c_W, c_b, c_x;
+  DBuf<GroupDenseRow> c_rows;
   DBuf<double> x, res, p, axp, pres, b, sc, part;
   DBuf<unsigned> tickets, ctl;
   cudaStream_t st = nullptr;
