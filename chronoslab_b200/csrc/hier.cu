@@ -590,7 +590,9 @@ static void launch_pcg_spmv(cudaStream_t st, const DMat &A, bool fp32vals, const
 static void attach_sell3(const HostCSR &A, DMat &d, bool fp32, cudaStream_t st) {
   const std::vector<int> blen = block_row_lengths(A);
   if (blen.empty()) return;
-  const TuneKey key('B', (int)blen.size(), A.nnz(), A.ncols, fp32,
+  // 'b': decisions timed before the kernels read their block columns ahead ('B')
+  // are not theirs
+  const TuneKey key('b', (int)blen.size(), A.nnz(), A.ncols, fp32,
                     *std::max_element(blen.begin(), blen.end()));
   int T = -1;
   {
@@ -1889,26 +1891,6 @@ k_pcg_spmv(int n, const int *__restrict__ rp, const int *__restrict__ ci,
   }
   double vals2[2] = {d0, d1};
   grid_reduce<2>(vals2, part, ticket, FinAlpha{sc});
-}
-
-// The three row sums of one block row of the sliced 3x3 block form (lane's
-// slots; the T partial sums are combined by the caller), accumulated in AT.
-template <typename AT, typename VT, typename XT>
-__device__ __forceinline__ void sell3_rows(int off, int w, const int *__restrict__ sci,
-                                           const VT *__restrict__ V, int64_t nslots,
-                                           const XT *__restrict__ x, AT &s0, AT &s1, AT &s2) {
-#pragma unroll 2
-  for (int j = 0; j < w; ++j) {
-    const int k = off + 32 * j;
-    const int col = 3 * __ldg(sci + k);
-    const AT xa = (AT)__ldg(x + col), xb = (AT)__ldg(x + col + 1), xc = (AT)__ldg(x + col + 2);
-    s0 += (AT)__ldg(V + k) * xa + (AT)__ldg(V + nslots + k) * xb +
-          (AT)__ldg(V + 2 * nslots + k) * xc;
-    s1 += (AT)__ldg(V + 3 * nslots + k) * xa + (AT)__ldg(V + 4 * nslots + k) * xb +
-          (AT)__ldg(V + 5 * nslots + k) * xc;
-    s2 += (AT)__ldg(V + 6 * nslots + k) * xa + (AT)__ldg(V + 7 * nslots + k) * xb +
-          (AT)__ldg(V + 8 * nslots + k) * xc;
-  }
 }
 
 // The same on the sliced 3x3 block form (see k_sell3_apply).

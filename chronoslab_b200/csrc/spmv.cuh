@@ -258,6 +258,49 @@ __device__ __forceinline__ VT slot_sum(VT v) {
   return v;
 }
 
+// The three row sums of one block row (lane's slots; the T partial sums are
+// combined by the caller), accumulated in AT.  Bound by the memory latency of a
+// warp's chain: two slots at a time, the block columns of the next two already
+// loaded, so that the gathers of x issue together with the values instead of a
+// latency behind their columns.  Elasticity 64^3 (63.7M entries): FP32 residual
+// 58.5 -> 53.9 us, outer product 83 -> 67 us; 45^3 FP64 40.1 -> 36.9 and 48.8 ->
+// 39.5 us.  One slot at a time 71 and 108 us at 64^3, three 68 and 93, four 84
+// and 113: fewer bytes in flight, or registers that cost resident warps.
+template <typename AT, typename VT, typename XT>
+__device__ __forceinline__ void sell3_rows(int off, int w, const int *__restrict__ sci,
+                                           const VT *__restrict__ V, int64_t nslots,
+                                           const XT *__restrict__ x, AT &s0, AT &s1, AT &s2) {
+  int c[2];
+#pragma unroll
+  for (int u = 0; u < 2; ++u) c[u] = u < w ? __ldg(sci + off + 32 * u) : 0;
+  for (int j = 0; j < w; j += 2) {
+    const int k = off + 32 * j;
+    const bool two = j + 1 < w;
+    VT v[2][9];
+    XT xv[2][3];
+#pragma unroll
+    for (int u = 0; u < 2; ++u) {
+      if (u == 0 || two) {
+#pragma unroll
+        for (int e = 0; e < 9; ++e) v[u][e] = __ldg(V + (int64_t)e * nslots + k + 32 * u);
+#pragma unroll
+        for (int e = 0; e < 3; ++e) xv[u][e] = __ldg(x + 3 * c[u] + e);
+      }
+    }
+#pragma unroll
+    for (int u = 0; u < 2; ++u) c[u] = j + 2 + u < w ? __ldg(sci + k + 64 + 32 * u) : 0;
+#pragma unroll
+    for (int u = 0; u < 2; ++u) {
+      if (u == 0 || two) {
+        const AT xa = (AT)xv[u][0], xb = (AT)xv[u][1], xc = (AT)xv[u][2];
+        s0 += (AT)v[u][0] * xa + (AT)v[u][1] * xb + (AT)v[u][2] * xc;
+        s1 += (AT)v[u][3] * xa + (AT)v[u][4] * xb + (AT)v[u][5] * xc;
+        s2 += (AT)v[u][6] * xa + (AT)v[u][7] * xb + (AT)v[u][8] * xc;
+      }
+    }
+  }
+}
+
 template <typename VT, typename XT, typename ZT, typename YT, int T, int MODE, bool DOT>
 __global__ void __launch_bounds__(kApplyThreads)
 k_sell3_apply(int nb, int nchunk, const int *__restrict__ choff, const int *__restrict__ chw,
@@ -271,19 +314,8 @@ k_sell3_apply(int nb, int nchunk, const int *__restrict__ choff, const int *__re
   const int nwarps = (gridDim.x * blockDim.x) >> 5;
   double dacc = 0.0;
   for (int c = warp; c < nchunk; c += nwarps) {
-    const int off = __ldg(choff + c) + lane, w = __ldg(chw + c);
     VT s0 = VT(0), s1 = VT(0), s2 = VT(0);
-#pragma unroll 2
-    for (int j = 0; j < w; ++j) {
-      const int k = off + 32 * j;
-      const int col = 3 * __ldg(sci + k);
-      const VT xa = (VT)__ldg(x + col), xb = (VT)__ldg(x + col + 1), xc = (VT)__ldg(x + col + 2);
-      s0 += __ldg(V + k) * xa + __ldg(V + nslots + k) * xb + __ldg(V + 2 * nslots + k) * xc;
-      s1 += __ldg(V + 3 * nslots + k) * xa + __ldg(V + 4 * nslots + k) * xb +
-            __ldg(V + 5 * nslots + k) * xc;
-      s2 += __ldg(V + 6 * nslots + k) * xa + __ldg(V + 7 * nslots + k) * xb +
-            __ldg(V + 8 * nslots + k) * xc;
-    }
+    sell3_rows<VT, VT, XT>(__ldg(choff + c) + lane, __ldg(chw + c), sci, V, nslots, x, s0, s1, s2);
     if (T > 1) {
       s0 = slot_sum<T>(s0);
       s1 = slot_sum<T>(s1);

@@ -287,3 +287,35 @@ def test_device_sqmr_loop(lib, nx, coarse, prec):
         # from the solution the first residual meets the test after one step
         x2, i2, _, it2 = cb.SQMR(h, b, 1e-6, 200, x0=x)
         assert i2 == 0 and it2 == 1
+
+
+@pytest.mark.parametrize("prec", [cb.CHRONOS_FP64, cb.CHRONOS_FP32])
+@pytest.mark.parametrize("lens", [[1], [2], [3], [1, 2, 4, 5], [7, 8, 9], [27], [1, 30, 64]])
+def test_block_rows_of_every_length(lib, lens, prec):
+    """The sliced 3x3 block form with odd, even, single and very uneven block
+    rows that do not fill a chunk, against numpy: the first residual of a PCG
+    from a random start (FP64 rows of at most 400 terms), and the solve, which a
+    single-level hierarchy's exact preconditioner ends in two steps only if the
+    outer product is A p."""
+    rng = np.random.default_rng(sum(lens))
+    nb = 301
+    want = rng.choice(lens, nb)
+    pat = sp.lil_matrix((nb, nb))
+    for i in range(nb):
+        pat[i, (i + rng.choice(nb, want[i] // 2, replace=False)) % nb] = 1.0
+    pat = sp.csr_matrix(((pat + pat.T) > 0).astype(float))
+    pat.setdiag(1.0)
+    U = sp.csr_matrix(sp.kron(pat, np.ones((3, 3))))
+    U.data = rng.uniform(-1.0, 1.0, U.nnz)
+    A = sp.csr_matrix(U + U.T)                     # every block whole: nothing cancels
+    A = sp.csr_matrix(A + sp.diags(np.asarray(abs(A).sum(1)).ravel() + 1.0))
+    A.sort_indices()
+    n = A.shape[0]
+    b, x0 = rng.standard_normal(n), rng.standard_normal(n)
+    with cb.Hierarchy(A, np.ones((n, 1)), cb.params(precision=prec, ntv=1, nLevMax=1)) as h:
+        assert h.nlevels == 1 and h.level_info(0)["block_rows"] == nb
+        x, it, rv, flag, _ = h.pcg(b, x0=x0, tol=1e-10, itmax=20)
+        first = np.linalg.norm(b - A @ x0) / np.linalg.norm(b)
+        assert rv[0] == pytest.approx(first, rel=1e-12)
+        assert flag == 0 and it <= (2 if prec == cb.CHRONOS_FP64 else 3)
+        assert np.linalg.norm(b - A @ x) <= 1e-10 * np.linalg.norm(b)
