@@ -913,9 +913,10 @@ int chronos_diag_fix(int n, const int *iat_h, const int *ja_h, double *val_h) {
     ScopedStream s;
     DMat d;
     upload_csr(A, d, false, s.st);
-    auto mv = [&](const double *x, double *y) {
+    auto mv = [&](const double *x, double *y, double *, unsigned *, double *) {
       csr_apply<double, double, double, double, MODE_PLAIN, false>(s.st, 8, n, d.rp, d.ci, d.v64, x,
                                                                   nullptr, y, 1.0);
+      return false;
     };
     // |lambda|_max of A (eigs(A,1,'lm'), A SPD: the largest eigenvalue)
     const double lmax = lanczos_lmax(n, mv, 1e-3, 300, s.st);

@@ -144,11 +144,13 @@ int64_t smoother_bound(const DMat &G) {
 }
 
 // Lanes per row of a two-matrix apply: one batch of four entries a lane covers
-// an average row.
+// an average row, and as many more lanes, up to one an entry, as the GPU has
+// threads idle (the longest rows' batches are then shorter chains).
 int fold_lanes(int64_t entries, int rows) {
   const double avg = (double)entries / std::max(rows, 1);
+  const int64_t resident = (int64_t)num_sms() * 2048;
   int L = 1;
-  while (L < 32 && 4 * L < avg) L *= 2;
+  while (L < 32 && (4 * L < avg || (L < avg && (int64_t)rows * 2 * L <= resident / 4))) L *= 2;
   return L;
 }
 
@@ -178,14 +180,15 @@ std::unique_ptr<Fold> fold_operators(const DMat &A, const DMat &G, const DMat &G
     f->form = FOLD_SMOOTH;
     return std::move(f);
   };
-  // R and Q have at least about as many entries as A and several times as many
-  if (!dense && A.nnz > kFoldEntries) return smooth_only();
+  // R has at least about as many entries as A, Q and E four times R's
+  // (twice and more where its rows are short): no product that would be dropped
+  if (!dense && (A.nnz < (int64_t)16 * n ? 2 : 1) * A.nnz > kFoldEntries) return smooth_only();
   Prod U = multiply(n, n, View(A), S, st);
   if (!add_identity(U, -1.0, 1.0, st)) return smooth_only();        // U = I - A S
   Prod R = multiply(nc, n, View(Pt), U, st);
   if (!dense && R.nnz > kFoldEntries) return smooth_only();
   Prod Q, E;
-  bool all = dense || 3 * A.nnz <= kFoldEntries;
+  bool all = dense || (3 * A.nnz <= kFoldEntries && 4 * R.nnz <= kFoldEntries);
   if (all && add_identity(U, 1.0, 1.0, st)) {                       // I + U
     Q = multiply(n, n, S, U, st);
     U = Prod();
@@ -228,6 +231,7 @@ std::unique_ptr<Fold> fold_operators(const DMat &A, const DMat &G, const DMat &G
   adopt(E, f->E, fp32, st);
   adopt(R, f->R, fp32, st);
   f->lanes = fold_lanes(f->Q.nnz, n);
+  f->R.wide = wide_rows(f->R, kWideTake);
   f->form = FOLD_ALL;
   return f;
 }

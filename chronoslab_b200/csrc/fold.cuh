@@ -1,52 +1,10 @@
-// Apply kernels of folded levels (fold.cu): the restriction R b and the
-// two-matrix row products.
+// Apply kernel of folded levels (fold.cu): the two-matrix row product.
 #pragma once
 
 #include "hier.h"
 #include "spmv.cuh"
 
 namespace chronos {
-
-// y = R b, a block per row: R's rows are the products of P' with two operators
-// and on the levels that end a hierarchy a few hundred of them hold thousands of
-// entries each (elasticity 24^3, FP64, 205 rows of 2270 entries: 77 us per PCG
-// iteration with a warp per row, 61 with a block).
-template <typename T, typename BT, bool I16>
-__global__ void __launch_bounds__(kApplyThreads)
-k_wide_rows(int n, const int *__restrict__ rp, const int *__restrict__ ci,
-            const int *__restrict__ cbase, const uint16_t *__restrict__ c16,
-            const T *__restrict__ v, const BT *__restrict__ b, T *__restrict__ y) {
-  pdl_begin();
-  __shared__ T red[kApplyThreads / 32];
-  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-  for (int row = blockIdx.x; row < n; row += gridDim.x) {
-    const int s = __ldg(rp + row), e = __ldg(rp + row + 1);
-    const T a = warp_sum(csr_row_dot<T, T, BT, kApplyThreads, I16>(
-        s + (int)threadIdx.x, e, I16 ? __ldg(cbase + row) : 0, ci, c16, v, b));
-    if (lane == 0) red[wid] = a;
-    __syncthreads();
-    if (threadIdx.x == 0) {
-      T t = red[0];
-      for (int w = 1; w < kApplyThreads / 32; ++w) t += red[w];
-      y[row] = t;
-    }
-    __syncthreads();
-  }
-}
-
-// Restriction of a folded level: a block per row from an average row of a warp's
-// eight batches on, else the tuned row-group kernel.
-template <typename T, typename BT>
-void restrict_apply(cudaStream_t st, const DMat &R, const BT *b, T *y) {
-  if (R.nnz < (int64_t)256 * R.nrows) {
-    mat_apply<T, BT, T, T, MODE_PLAIN, false>(st, R, vals<T>(R), b, nullptr, y, T(1));
-    return;
-  }
-  const int grid = std::min(R.nrows, num_sms() * 8);
-  launch_pdl(R.idx16 ? k_wide_rows<T, BT, true> : k_wide_rows<T, BT, false>, grid, kApplyThreads,
-             st, R.nrows, (const int *)R.rp.get(), (const int *)R.ci.get(),
-             (const int *)R.cbase.get(), (const uint16_t *)R.c16.get(), vals<T>(R), b, y);
-}
 
 // out = Q b + E e on a folded level, L lanes per row (and out . dw).
 template <typename T, typename BT, typename OT, int L, bool DOT, bool QI16, bool EI16>

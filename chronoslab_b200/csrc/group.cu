@@ -539,7 +539,7 @@ static void group_fold_down(GroupSolve &g, GroupLevel &L, const BT *b, T *bc) {
   const Fold &F = *L.fold;
   T *x = gvec<T>(L.x32, L.x64), *r = gvec<T>(L.r32, L.r64);
   if (F.form != FOLD_SMOOTH) {
-    restrict_apply<T, BT>(st, F.R, b, bc);
+    mat_apply<T, BT, T, T, MODE_PLAIN, false>(st, F.R, vals<T>(F.R), b, nullptr, bc, T(1));
     return;
   }
   mat_apply<T, BT, T, T, MODE_PLAIN, false>(st, F.S, vals<T>(F.S), b, nullptr, x, T(1));

@@ -382,7 +382,10 @@ void autotune_lanes(DMat &m, bool fp32, cudaStream_t st, int format) {
   // shape.  A cached value is lanes + 100 * form (decoded at the end).
   int maxrow = 0;
   for (int i = 0; i < m.nrows; ++i) maxrow = std::max(maxrow, m.rp_h[i + 1] - m.rp_h[i]);
-  const TuneKey key(m.idx16 ? 'h' : 'H', m.nrows, m.nnz, m.ncols, fp32, maxrow);
+  // 'w', 'W': operators for which the wide form is tried as well
+  const bool try_wide = format == 0 && wide_rows(m, kWideTry);
+  const TuneKey key(try_wide ? (m.idx16 ? 'w' : 'W') : (m.idx16 ? 'h' : 'H'), m.nrows, m.nnz,
+                    m.ncols, fp32, maxrow);
   int L = -1;
   {
     std::lock_guard<std::mutex> lk(g_tune_mu);
@@ -444,8 +447,17 @@ void autotune_lanes(DMat &m, bool fp32, cudaStream_t st, int format) {
         if (verbose)
           std::fprintf(stderr, "chronos tune: csr %d x %d (%lld) sliced ELL  %.4f ms\n",
                        m.nrows, m.ncols, (long long)m.nnz, t / 4);
-        if (t < best) L += 100;
+        if (t < best) { best = t; L += 100; }
         drop_sell(m);
+      }
+      if (try_wide) {
+        m.wide = true;
+        const float t = time_it();
+        if (verbose)
+          std::fprintf(stderr, "chronos tune: csr %d x %d (%lld) wide  %.4f ms\n", m.nrows, m.ncols,
+                       (long long)m.nnz, t / 4);
+        if (t < best) L = L % 100 + 200;
+        m.wide = false;
       }
       cudaEventDestroy(e0);
       cudaEventDestroy(e1);
@@ -453,7 +465,7 @@ void autotune_lanes(DMat &m, bool fp32, cudaStream_t st, int format) {
     std::lock_guard<std::mutex> lk(g_tune_mu);
     tune_store_locked(key, L);
   }
-  // L = lanes + 100 * form: 0 row-grouped CSR, 1 sliced ELL
+  // L = lanes + 100 * form: 0 row-grouped CSR, 1 sliced ELL, 2 wide
   int form = L / 100;
   const int lanes = L % 100;
   if (format == 1) form = 0;
@@ -464,6 +476,7 @@ void autotune_lanes(DMat &m, bool fp32, cudaStream_t st, int format) {
     set_long_rows(m, kSellLongRow, st);
   } else {
     set_lanes(m, lanes, st);
+    m.wide = form == 2;
   }
 }
 
@@ -804,7 +817,7 @@ static double tridiag_last_component(const std::vector<double> &a, const std::ve
 namespace {
 constexpr int kLanczosBatch = 8;
 
-// alpha = v'w into a[j]
+// alpha = v'w into a[j], for operators that do not reduce it themselves
 __global__ void __launch_bounds__(256)
 k_lanczos_alpha(int n, const double *__restrict__ v, const double *__restrict__ w, double *part,
                 unsigned *ticket, double *alpha) {
@@ -845,11 +858,10 @@ k_lanczos_next(int n, const double *__restrict__ w, const double *__restrict__ b
 }
 }  // namespace
 
-double lanczos_lmax(int n, const std::function<void(const double *, double *)> &mv, double tol,
-                    int maxit, cudaStream_t st) {
+double lanczos_lmax(int n, const LanczosOp &mv, double tol, int maxit, cudaStream_t st) {
   const int grid = std::max(1, std::min(num_sms() * 4, (int)ceil_div(n, 256)));
   // three vectors, alpha and beta^2 of every step, block partials
-  DBuf<double> work(3 * (size_t)n + 2 * (size_t)maxit + grid);
+  DBuf<double> work(3 * (size_t)n + 2 * (size_t)maxit + std::max(grid, num_sms() * 8));
   DBuf<unsigned> ticket(1);
   ticket.zero(st);
   double *v = work.get(), *vp = v + n, *w = vp + n, *a_d = w + n, *b2_d = a_d + maxit,
@@ -872,9 +884,9 @@ double lanczos_lmax(int n, const std::function<void(const double *, double *)> &
   for (int j0 = 0; j0 < maxit; j0 += kLanczosBatch) {
     const int j1 = std::min(maxit, j0 + kLanczosBatch);
     for (int j = j0; j < j1; ++j) {
-      mv(v, w);
-      launch_pdl(k_lanczos_alpha, grid, 256, st, n, (const double *)v, (const double *)w, part,
-                 ticket.get(), a_d + j);
+      if (!mv(v, w, part, ticket.get(), a_d + j))
+        launch_pdl(k_lanczos_alpha, grid, 256, st, n, (const double *)v, (const double *)w, part,
+                   ticket.get(), a_d + j);
       launch_pdl(k_lanczos_update, grid, 256, st, n, (const double *)v, (const double *)vp, w,
                  (const double *)(a_d + j), j > 0 ? (const double *)(b2_d + j - 1) : nullptr, part,
                  ticket.get(), b2_d + j);
@@ -973,11 +985,12 @@ static HostCSR smooth_prolongation(const HostCSR &A, const DMat &dA, const HostC
   }
   DBuf<double> ddm, t1(n), t2(n);
   ddm.upload(dm, st);
-  auto mv = [&](const double *v, double *w) {
+  auto mv = [&](const double *v, double *w, double *, unsigned *, double *) {
     device_diag_mul(n, ddm.get(), v, t1.get(), st);
     csr_apply<double, double, double, double, MODE_PLAIN, false>(
         st, 8, n, dA.rp, dA.ci, dA.v64, t1.get(), (const double *)nullptr, t2.get(), 1.0);
     device_diag_mul(n, ddm.get(), t2.get(), w, st);
+    return false;
   };
   const double lam = lanczos_lmax(n, mv, 1e-3, 300, st);
   const double omega = 1.9 / lam;
@@ -1254,13 +1267,15 @@ void HierBuilder::end_level(int fl) {
   {
     DBuf<double> t1(n), t2(n);
     Level *Lp = &L;
-    auto mv = [&](const double *v, double *w) {
+    auto mv = [&](const double *v, double *w, double *part, unsigned *ticket, double *dot) {
       mat_apply<double, double, double, double, MODE_PLAIN, false>(
           st, Lp->Gt, Lp->Gt.v64.get(), v, (const double *)nullptr, t1.get(), 1.0);
       op_apply<double, double, double, double, MODE_PLAIN, false>(
           st, Lp->A, t1.get(), (const double *)nullptr, t2.get(), 1.0);
-      mat_apply<double, double, double, double, MODE_PLAIN, false>(
-          st, Lp->G, Lp->G.v64.get(), t2.get(), (const double *)nullptr, w, 1.0);
+      mat_apply<double, double, double, double, MODE_PLAIN, true>(
+          st, Lp->G, Lp->G.v64.get(), t2.get(), (const double *)nullptr, w, 1.0, v, part, ticket,
+          dot);
+      return true;
     };
     L.lambda = lanczos_lmax(n, mv, 5e-4, 200, st);
     L.omega = std::min(1.0, 1.9 / L.lambda);
@@ -1697,7 +1712,7 @@ static void vcycle_level(Hier &h, int l, const BT *b, OT *out, const double *dw,
       op_apply<T, T, BT, T, MODE_RESID, false>(st, L.A, x, b, r, T(1));
       mat_apply<T, T, T, T, MODE_PLAIN, false>(st, L.Pt, vals<T>(L.Pt), r, nullptr, bc, T(1));
     } else {
-      restrict_apply<T, BT>(st, F.R, b, bc);
+      mat_apply<T, BT, T, T, MODE_PLAIN, false>(st, F.R, vals<T>(F.R), b, nullptr, bc, T(1));
     }
     vcycle_level<T, T, T, false>(h, l + 1, bc, e, nullptr, nullptr);
     // up: out = Q b + E e, or x += P e (x = S b + P e), r = b - A x, out = x + S r

@@ -352,7 +352,9 @@ int heuristic_lanes(const DMat &m);
 void set_lanes(DMat &m, int L, cudaStream_t st);
 // Largest eigenvalue of the symmetric operator given as a device FP64 matvec,
 // by Lanczos with a unit start vector; relative tolerance tol.
-double lanczos_lmax(int n, const std::function<void(const double *, double *)> &mv, double tol,
-                    int maxit, cudaStream_t st);
+// mv(v, w, part, ticket, dot): w = Op v queued, and v'w into *dot (reduced in part,
+// num_sms()*8 doubles) if it returns true.
+using LanczosOp = std::function<bool(const double *, double *, double *, unsigned *, double *)>;
+double lanczos_lmax(int n, const LanczosOp &mv, double tol, int maxit, cudaStream_t st);
 
 }  // namespace chronos

@@ -45,6 +45,9 @@ struct DMat {
   DBuf<uint16_t> s_c16;
   DBuf<double> s_v64;
   DBuf<float> s_v32;
+  // Rows applied by a block of 128 or 256 threads each (long rows of small
+  // levels; chosen by the autotuner or by wide_rows).
+  bool wide = false;
   // Optional sliced 3x3 block form of the same matrix (chunks of 32 block
   // rows, slot-major, plane-major values), used when every row triple shares
   // a pattern of whole aligned 3x3 blocks.

@@ -473,6 +473,49 @@ k_csrh_apply(int n, const int *__restrict__ rp, const int *__restrict__ ci,
   }
 }
 
+// A block of W threads per row (DMat::wide): the levels that end a hierarchy, and
+// their folded restrictions, have a few thousand rows or less of hundreds to
+// thousands of entries; with a warp per row a level's time is one row's chain of
+// batches.  The partial sums meet in warp order.
+template <typename VT, typename XT, typename ZT, typename YT, int W, int MODE, bool DOT, bool I16>
+__global__ void __launch_bounds__(W)
+k_csr_wide(int n, const int *__restrict__ rp, const int *__restrict__ ci,
+           const int *__restrict__ cbase, const uint16_t *__restrict__ c16,
+           const VT *__restrict__ v, const XT *__restrict__ x, const ZT *z, YT *y, VT alpha,
+           const double *__restrict__ dw, double *part, unsigned *ticket, double *dot_out) {
+  pdl_begin();
+  __shared__ VT red[W / 32];
+  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+  double dacc = 0.0;
+  for (int row = blockIdx.x; row < n; row += gridDim.x) {
+    const int s = __ldg(rp + row), e = __ldg(rp + row + 1);
+    const VT a = warp_sum(csr_row_dot<VT, VT, XT, W, I16>(
+        s + (int)threadIdx.x, e, I16 ? __ldg(cbase + row) : 0, ci, c16, v, x));
+    if (lane == 0) red[wid] = a;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+      VT t = red[0];
+#pragma unroll
+      for (int w = 1; w < W / 32; ++w) t += red[w];
+      const YT out = (YT)apply_epilogue<VT, MODE>(t, alpha, z, row);
+      y[row] = out;
+      if (DOT) dacc += (double)out * dw[row];
+    }
+    __syncthreads();
+  }
+  if (DOT) {
+    double vals[1] = {dacc};
+    grid_reduce<1>(vals, part, ticket, StoreScalar{dot_out});
+  }
+}
+
+// Average rows from which the autotuner tries, and an untuned operator takes,
+// the wide form; from kWideLong on 256 threads a row instead of 128.
+constexpr int kWideTry = 64, kWideTake = 256, kWideLong = 768;
+inline bool wide_rows(const DMat &M, int average) {
+  return M.nnz >= (int64_t)average * M.nrows && M.nrows <= 16 * num_sms() * 8;
+}
+
 // Sliced ELL apply (see DMat::use_sell): a warp per chunk of 32 rows, lane l
 // owns chunk row l and walks its slots with coalesced 128-byte (values) and
 // 64-byte (16-bit offsets) warp loads, four slots' loads in flight before
@@ -594,6 +637,21 @@ void mat_apply(cudaStream_t st, const DMat &M, const VT *v, const XT *x, const Z
   const int cap = num_sms() * 8;
   const int wpb = kApplyThreads / 32;
   const int lb = long_blocks(M, cap);
+  if (M.wide) {
+    const int grid = std::min(n, cap);
+#define CHRONOS_WIDE(WW, I16)                                                                 \
+  launch_pdl(k_csr_wide<VT, XT, ZT, YT, WW, MODE, DOT, I16>, grid, WW, st, n, M.rp.get(),      \
+             M.ci.get(), M.cbase.get(), M.c16.get(), v, x, z, y, alpha, dw, part, ticket, dot_out)
+    if (M.nnz >= (int64_t)kWideLong * n) {
+      if (M.idx16) CHRONOS_WIDE(256, true);
+      else CHRONOS_WIDE(256, false);
+    } else {
+      if (M.idx16) CHRONOS_WIDE(128, true);
+      else CHRONOS_WIDE(128, false);
+    }
+#undef CHRONOS_WIDE
+    return;
+  }
   if (M.use_sell) {
     const int sb = (int)std::min<int64_t>(ceil_div(M.s_nchunk, wpb), cap - lb);
     const VT *sv = sell_vals<VT>(M), *cv = csr_vals<VT>(M);
