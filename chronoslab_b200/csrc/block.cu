@@ -220,7 +220,6 @@ struct BlockState {
   std::vector<DBuf<float>> b32, x32, r32, t32;
   std::vector<DBuf<double>> b64, x64, r64, t64;
   DBuf<double> x, res, p, axp, pres, b;
-  DBuf<double> stage;           // n x K: the host blocks as they come and go
   DBuf<double> norms;           // ||b||^2 and ||r0||^2 per column
   DBuf<double> sc;              // per-column scalars, see BS_* below
   DBuf<double> part;
@@ -604,7 +603,7 @@ static void block_solve(Hier &h, int m, const BlockIn &B, const double *X0_h, do
     }
     const size_t m0 = (size_t)s.n * K;
     s.x.alloc(m0); s.res.alloc(m0); s.p.alloc(m0); s.axp.alloc(m0); s.pres.alloc(m0);
-    s.b.alloc(m0); s.stage.alloc(m0); s.norms.alloc(2 * K);
+    s.b.alloc(m0); s.norms.alloc(2 * K);
     s.p.zero(st);
     s.axp.zero(st);
     s.sc.alloc((size_t)BS_COUNT * K + 8);
@@ -614,13 +613,14 @@ static void block_solve(Hier &h, int m, const BlockIn &B, const double *X0_h, do
   }
   BlockState &s = *sp;
   const int n = s.n;
-  double *b = s.b.get(), *b2 = s.norms.get(), *r2 = s.norms.get() + K;
+  // (A p is not formed yet when the host blocks come in, nor needed when x goes out)
+  double *staged = s.axp.get(), *b = s.b.get(), *b2 = s.norms.get(), *r2 = s.norms.get() + K;
   // host blocks -> row-major device blocks; a row-major host block of exactly
   // K columns is already in the solve's layout
   const int lb = std::max(1, std::min(num_sms() * 8, (int)ceil_div(n, 32)));
   auto pack = [&](const BlockIn &src, double *dst) {
     if (src.ld > 0) {                              // row-major, rows ld apart
-      double *to = m == K ? dst : s.stage.get();
+      double *to = m == K ? dst : staged;
       if (src.ld == m)                             // one copy: row by row is far slower
         CHRONOS_CUDA(cudaMemcpyAsync(to, src.p, sizeof(double) * n * m, cudaMemcpyHostToDevice,
                                      st));
@@ -628,11 +628,11 @@ static void block_solve(Hier &h, int m, const BlockIn &B, const double *X0_h, do
         CHRONOS_CUDA(cudaMemcpy2DAsync(to, sizeof(double) * m, src.p, sizeof(double) * src.ld,
                                        sizeof(double) * m, n, cudaMemcpyHostToDevice, st));
       if (m == K) return;
-      k_block_layout<K, true><<<lb, 256, 0, st>>>(n, m, m, 1, s.stage.get(), dst);
+      k_block_layout<K, true><<<lb, 256, 0, st>>>(n, m, m, 1, staged, dst);
     } else {
-      CHRONOS_CUDA(cudaMemcpyAsync(s.stage.get(), src.p, sizeof(double) * n * m,
+      CHRONOS_CUDA(cudaMemcpyAsync(staged, src.p, sizeof(double) * n * m,
                                    cudaMemcpyHostToDevice, st));
-      k_block_layout<K, true><<<lb, 256, 0, st>>>(n, m, 1, n, s.stage.get(), dst);
+      k_block_layout<K, true><<<lb, 256, 0, st>>>(n, m, 1, n, staged, dst);
     }
     CHRONOS_CHECK_LAUNCH();
   };
@@ -718,11 +718,11 @@ static void block_solve(Hier &h, int m, const BlockIn &B, const double *X0_h, do
   k_zero_null_columns<K><<<nb, 256, 0, st>>>(n, s.x.get(), s.sc.get());
   CHRONOS_CHECK_LAUNCH();
   CHRONOS_CUDA(cudaEventRecord(e1, st));
-  k_block_layout<K, false><<<lb, 256, 0, st>>>(n, m, 1, n, s.stage.get(), s.x.get());
+  k_block_layout<K, false><<<lb, 256, 0, st>>>(n, m, 1, n, staged, s.x.get());
   CHRONOS_CHECK_LAUNCH();
   std::vector<double> sc_h((size_t)BS_COUNT * K + 8);
   s.sc.download(sc_h.data(), sc_h.size(), st);
-  s.stage.download(X_h, (size_t)n * m, st);
+  s.axp.download(X_h, (size_t)n * m, st);
   CHRONOS_CUDA(cudaStreamSynchronize(st));
   float ms = 0.f;
   CHRONOS_CUDA(cudaEventElapsedTime(&ms, e0, e1));

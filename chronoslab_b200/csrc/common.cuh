@@ -49,8 +49,8 @@ inline int64_t device_alloc_cap() {
 // The streams that the library's work runs on (entry points that take a
 // caller's stream join it by events).  A buffer is freed after waiting for
 // them, and a stream is waited for before it is destroyed.  The lock also
-// covers the library's stream captures: a stream that another thread is
-// capturing must not be synchronised.
+// covers the library's stream captures, and the joining of a handle's stream to
+// a caller's capture: a stream that is being captured must not be synchronised.
 struct LibStreams {
   std::mutex mu;
   std::vector<std::pair<int, cudaStream_t>> list;       // device, stream
@@ -83,11 +83,21 @@ inline void stream_destroy(cudaStream_t st) {
   }
   cudaStreamDestroy(st);
 }
-inline void wait_lib_streams(int device) {
+// Waits for the device's library streams; false where a caller's capture holds
+// one of them (its earlier work may still be running).
+inline bool wait_lib_streams(int device) {
   LibStreams &l = lib_streams();
   std::lock_guard<std::mutex> lk(l.mu);
-  for (auto &e : l.list)
-    if (e.first == device) cudaStreamSynchronize(e.second);
+  bool all = true;
+  for (auto &e : l.list) {
+    if (e.first != device) continue;
+    cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+    if (cudaStreamIsCapturing(e.second, &cap) == cudaSuccess && cap == cudaStreamCaptureStatusNone)
+      cudaStreamSynchronize(e.second);
+    else
+      all = false;
+  }
+  return all;
 }
 
 // Device memory comes from one memory pool per device, owned by the library
@@ -111,6 +121,7 @@ struct DevicePool {
     cudaError_t e = cudaMallocFromPoolAsync(p, bytes, pool, st);
     if (e == cudaErrorMemoryAllocation) {
       cudaGetLastError();
+      cudaStreamSynchronize(st);                        // frees still in its queue
       cudaMemPoolTrimTo(pool, 0);
       e = cudaMallocFromPoolAsync(p, bytes, pool, st);
     }
@@ -126,8 +137,10 @@ struct DevicePool {
     uint64_t held = 0, used = 0;
     if (cudaMemPoolGetAttribute(pool, cudaMemPoolAttrReservedMemCurrent, &held) == cudaSuccess &&
         cudaMemPoolGetAttribute(pool, cudaMemPoolAttrUsedMemCurrent, &used) == cudaSuccess &&
-        held > used + (uint64_t)kPoolKeepBytes)
+        held > used + (uint64_t)kPoolKeepBytes) {
+      cudaStreamSynchronize(st);
       cudaMemPoolTrimTo(pool, used + (uint64_t)kPoolKeepBytes);
+    }
   }
 };
 // The current device's pool.
@@ -176,9 +189,11 @@ class OnDevice {
 // Deferred frees.  A free waits for all work queued on the device, so
 // while a batch setup builds hierarchies on several host threads, one
 // thread's free of a setup temporary would wait for every other thread's
-// queued kernels.  Inside a DeferFrees scope (any thread) the buffers a DBuf
+// queued kernels; and nothing can be waited for while a caller's capture holds a
+// handle's stream: such a buffer is kept until a later free.
+// Inside a DeferFrees scope (any thread) the buffers a DBuf
 // lets go of are kept -- never reused -- and freed when the outermost scope
-// ends, after one device synchronisation.  They stay counted in
+// ends, after one wait for the streams.  They stay counted in
 // device_bytes_live() until then.
 struct DeferredFrees {
   struct Entry { void *p; int64_t bytes; DevicePool *pool; };
@@ -201,7 +216,11 @@ inline void flush_deferred_frees() {
   for (auto &e : list) {
     OnDevice on(e.pool->device);
     if (e.pool != synced) {
-      wait_lib_streams(e.pool->device);
+      if (!wait_lib_streams(e.pool->device)) {
+        std::lock_guard<std::mutex> lk(d.mu);
+        d.list.push_back(e);
+        continue;
+      }
       synced = e.pool;
     }
     e.pool->free_idle(e.p);
@@ -263,16 +282,13 @@ class DBuf {
   void release() {
     if (p_) {
       DeferredFrees &d = deferred_frees();
-      if (d.depth.load() > 0) {
+      bool kept = false;
+      {
         std::lock_guard<std::mutex> lk(d.mu);
         d.list.push_back({p_, (int64_t)(n_ * sizeof(T)), pool_});
-      } else {
-        OnDevice on(pool_->device);
-        wait_lib_streams(pool_->device);
-        pool_->free_idle(p_);
-        pool_->trim();
-        device_bytes_live() -= (int64_t)(n_ * sizeof(T));
+        kept = d.depth.load() > 0;
       }
+      if (!kept) flush_deferred_frees();
     }
     p_ = nullptr;
     n_ = 0;

@@ -396,8 +396,8 @@ GroupSolve::~GroupSolve() {
   }
 }
 
-std::unique_ptr<GroupSolve> group_build(const std::vector<std::unique_ptr<Hier>> &hs,
-                                        const chronos_params &prm) {
+static std::unique_ptr<GroupSolve> build_stack(const std::vector<std::unique_ptr<Hier>> &hs,
+                                               const chronos_params &prm, bool fold) {
   auto G = std::make_unique<GroupSolve>();
   GroupSolve &g = *G;
   g.st = stream_create();
@@ -454,7 +454,7 @@ std::unique_ptr<GroupSolve> group_build(const std::vector<std::unique_ptr<Hier>>
     const auto tl1 = std::chrono::steady_clock::now();
     // one pre- and one postsmoothing step in the autotuner's storage: folded as a
     // single hierarchy's level is (the stack is block diagonal, G' scaled)
-    if (prm.nupre <= 1 && prm.nupost == 1 && prm.spmv_format == 0)
+    if (fold && prm.nupre <= 1 && prm.nupost == 1 && prm.spmv_format == 0)
       L.fold = fold_operators(L.A, L.G, L.Gt, L.P, L.Pt, 1.0, nullptr, 0, fp32, st);
     const Fold *F = L.fold.get();
     if (F) tune_fold(*L.fold, fp32, st);
@@ -530,6 +530,17 @@ std::unique_ptr<GroupSolve> group_build(const std::vector<std::unique_ptr<Hier>>
   g.ctl.zero(st);
   CHRONOS_CUDA(cudaStreamSynchronize(st));
   return G;
+}
+
+std::unique_ptr<GroupSolve> group_build(const std::vector<std::unique_ptr<Hier>> &hs,
+                                        const chronos_params &prm) {
+  // folded where the memory for it is there
+  try {
+    return build_stack(hs, prm, true);
+  } catch (const Error &e) {
+    if (e.code != CHRONOS_ENOMEM) throw;
+  }
+  return build_stack(hs, prm, false);
 }
 
 // The two halves of a folded level, as vcycle_level runs them.

@@ -79,6 +79,12 @@ CallerStream::CallerStream(Hier &h, void *stream)
   if (!h_.ev_in) CHRONOS_CUDA(cudaEventCreateWithFlags(&h_.ev_in, cudaEventDisableTiming));
   if (!h_.ev_out) CHRONOS_CUDA(cudaEventCreateWithFlags(&h_.ev_out, cudaEventDisableTiming));
   CHRONOS_CUDA(cudaEventRecord(h_.ev_in, caller_));
+  // a capture that the caller runs takes the handle's stream in here: not while
+  // another thread's free waits for that stream
+  std::unique_lock<std::mutex> lk(lib_streams().mu, std::defer_lock);
+  cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+  if (cudaStreamIsCapturing(caller_, &cap) != cudaSuccess) cudaGetLastError();
+  if (cap != cudaStreamCaptureStatusNone) lk.lock();
   CHRONOS_CUDA(cudaStreamWaitEvent(h_.st, h_.ev_in, 0));
 }
 
@@ -1422,10 +1428,25 @@ std::unique_ptr<Hier> build_hierarchy(const chronos_params &prm, HostCSR A0, int
   return b.finish(tune);
 }
 
+static void tune_operators(Hier &h);
+
 void tune_hierarchy(Hier &h) {
+  // folded where the memory for it is there
+  try {
+    build_folds(h);
+    tune_operators(h);
+    return;
+  } catch (const Error &e) {
+    if (e.code != CHRONOS_ENOMEM) throw;
+  }
+  CHRONOS_CUDA(cudaStreamSynchronize(h.st));
+  for (auto &L : h.levels) L.fold.reset();
+  tune_operators(h);
+}
+
+static void tune_operators(Hier &h) {
   const bool fp32 = h.precision == CHRONOS_FP32;
   const int fmt = h.prm.spmv_format;
-  build_folds(h);
   // SpMV lane counts of the operators that the cycle applies (level 1's also
   // serve the outer product and other callers of its operators)
   for (size_t l = 0; l < h.levels.size(); ++l) {
@@ -1680,6 +1701,13 @@ static void dense_tail_apply(cudaStream_t st, int n, const double *D, int ld, co
   launch_pdl(k_dense_tail_apply<TI, TO>, ceil_div((int64_t)n * 32, 256), 256, st, n, D, ld, b, x);
 }
 
+// Whether n values at a and at b share memory.
+template <typename TA, typename TB>
+static bool overlap(const TA *a, const TB *b, int n) {
+  const uintptr_t pa = reinterpret_cast<uintptr_t>(a), pb = reinterpret_cast<uintptr_t>(b);
+  return pa < pb + (size_t)n * sizeof(TB) && pb < pa + (size_t)n * sizeof(TA);
+}
+
 template <typename T, typename BT, typename OT, bool TOP>
 static void vcycle_level(Hier &h, int l, const BT *b, OT *out, const double *dw, double *dot_out) {
   Level &L = h.levels[l];
@@ -1706,8 +1734,13 @@ static void vcycle_level(Hier &h, int l, const BT *b, OT *out, const double *dw,
     }
     Level &C = h.levels[l + 1];
     T *x = L.x<T>(), *r = L.r<T>(), *bc = C.b<T>(), *e = C.x<T>();
+    // Q b + E e gathers b while out is written: a caller's cycle in place (b and
+    // out the same vector) goes through the residual, which is done with b before
+    bool in_place = false;
+    if constexpr (TOP) in_place = overlap(b, out, n);
+    const FoldForm form = F.form == FOLD_ALL && in_place ? FOLD_SMOOTH : F.form;
     // down: b_c = R b, or through the residual of x = S b
-    if (F.form == FOLD_SMOOTH) {
+    if (form == FOLD_SMOOTH) {
       mat_apply<T, BT, T, T, MODE_PLAIN, false>(st, F.S, vals<T>(F.S), b, nullptr, x, T(1));
       op_apply<T, T, BT, T, MODE_RESID, false>(st, L.A, x, b, r, T(1));
       mat_apply<T, T, T, T, MODE_PLAIN, false>(st, L.Pt, vals<T>(L.Pt), r, nullptr, bc, T(1));
@@ -1716,7 +1749,7 @@ static void vcycle_level(Hier &h, int l, const BT *b, OT *out, const double *dw,
     }
     vcycle_level<T, T, T, false>(h, l + 1, bc, e, nullptr, nullptr);
     // up: out = Q b + E e, or x += P e (x = S b + P e), r = b - A x, out = x + S r
-    if (F.form == FOLD_ALL) {
+    if (form == FOLD_ALL) {
       if (TOP && dw)
         fold_apply<T, BT, OT, TOP>(st, F.lanes, F.Q, F.E, b, e, out, dw, part, tick, dot_out);
       else
@@ -1724,7 +1757,7 @@ static void vcycle_level(Hier &h, int l, const BT *b, OT *out, const double *dw,
                                      nullptr);
       return;
     }
-    if (F.form == FOLD_SMOOTH)
+    if (form == FOLD_SMOOTH)
       mat_apply<T, T, T, T, MODE_AXPY, false>(st, L.P, vals<T>(L.P), e, x, x, T(1));
     else
       fold_apply<T, BT, T, false>(st, F.lanes, F.S, L.P, b, e, x, nullptr, nullptr, nullptr,

@@ -319,3 +319,108 @@ def test_block_rows_of_every_length(lib, lens, prec):
         assert rv[0] == pytest.approx(first, rel=1e-12)
         assert flag == 0 and it <= (2 if prec == cb.CHRONOS_FP64 else 3)
         assert np.linalg.norm(b - A @ x) <= 1e-10 * np.linalg.norm(b)
+
+
+@pytest.mark.parametrize("prec,io,tol", [(cb.CHRONOS_FP64, "float64", 1e-12),
+                                         (cb.CHRONOS_FP32, "float64", 2e-5),
+                                         (cb.CHRONOS_FP32, "float32", 2e-5)])
+@pytest.mark.parametrize("shift", [0, 16])
+def test_vcycle_in_place(lib, prec, io, tol, shift):
+    """b and x the same device vector, or overlapping: the cycle of separate
+    vectors up to the rounding of its forms."""
+    import torch
+    from chronoslab_b200 import problems as PB
+    A = PB.poisson7(20)
+    n = A.shape[0]
+    ip = cb.CHRONOS_FP64 if io == "float64" else cb.CHRONOS_FP32
+    with cb.Hierarchy(A, np.ones((n, 1)), cb.params(precision=prec, ntv=1)) as h:
+        b = torch.from_numpy(np.random.default_rng(3).standard_normal(n)).to("cuda", getattr(torch, io))
+        x = torch.empty_like(b)
+        h.vcycle_dev(b.data_ptr(), x.data_ptr(), ip)
+        both = torch.zeros(n + shift, dtype=b.dtype, device="cuda")
+        both[:n] = b
+        torch.cuda.synchronize()
+        h.vcycle_dev(both.data_ptr(), both.data_ptr() + shift * both.element_size(), ip)
+        torch.cuda.synchronize()
+        err = (both[shift:].double() - x.double()).norm() / x.double().norm()
+        assert float(err) <= tol
+
+
+def test_free_while_a_caller_captures(lib):
+    """A V-cycle in a caller's relaxed capture, during which another handle is
+    destroyed: the capture survives and replays, and that handle's memory is
+    given back by a later free."""
+    import torch
+    from chronoslab_b200 import problems as PB
+    A = PB.poisson7(12)
+    n = A.shape[0]
+    prm = cb.params(precision=cb.CHRONOS_FP64, ntv=1)
+    before = cb.device_bytes()
+    with cb.Hierarchy(A, np.ones((n, 1)), prm) as h:
+        other = cb.Hierarchy(A, np.ones((n, 1)), prm)
+        b = torch.from_numpy(np.random.default_rng(3).standard_normal(n)).cuda()
+        x = torch.zeros_like(b)
+        h.vcycle_dev(b.data_ptr(), x.data_ptr())
+        torch.cuda.synchronize()
+        want = x.clone()
+        g = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(g, capture_error_mode="relaxed"):
+            h.vcycle_dev(b.data_ptr(), x.data_ptr(),
+                         stream=torch.cuda.current_stream().cuda_stream)
+            other.close()
+        x.zero_()
+        g.replay()
+        torch.cuda.synchronize()
+        assert torch.equal(x, want)
+        del g
+        cb.Hierarchy(A, np.ones((n, 1)), prm).close()   # allocations and frees as before
+    assert cb.device_bytes() == before
+
+
+def test_folding_gives_way_to_the_memory_cap(lib, tmp_path):
+    """Under the smallest CHRONOS_DEVICE_ALLOC_CAP (to 4 MB) at which a saved
+    hierarchy of the same operators that is never folded (two presmoothing
+    steps) loads with a cold autotuner, the foldable one loads and solves too."""
+    import os
+    import subprocess
+    import sys
+    root = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+    head = (f"import sys; sys.path.insert(0, {root!r})\n"
+            "import numpy as np\nimport chronoslab_b200 as cb\n"
+            "from chronoslab_b200 import problems as PB\nA = PB.poisson7(60)\nn = A.shape[0]\n")
+    files = [str(tmp_path / f"pre{k}.chh") for k in (2, 1)]
+
+    def child(code, cap=0):
+        env = dict(os.environ, CHRONOS_TUNE_CACHE=str(tmp_path / f"tune{cap}.txt"))
+        (tmp_path / f"tune{cap}.txt").unlink(missing_ok=True)
+        if cap:
+            env["CHRONOS_DEVICE_ALLOC_CAP"] = str(cap)
+        r = subprocess.run([sys.executable, "-c", head + code], env=env, timeout=900,
+                           capture_output=True, text=True)
+        if r.returncode:
+            assert cap and "ENOMEM" in r.stderr, r.stderr
+            return None
+        return [float(v) for v in r.stdout.split()[-2:]]
+
+    lean, full = child(
+        "out = []\n"
+        f"for k, f in zip((2, 1), {files!r}):\n"
+        "    with cb.Hierarchy(A, np.ones((n, 1)), cb.params(ntv=1, nupre=k,"
+        " precision=cb.CHRONOS_FP64)) as h: h.save(f)\n"
+        "    with cb.Hierarchy.load(f) as h: out.append(cb.device_bytes())\n"
+        "print(*out)\n")
+    assert full > lean
+    solve = ("with cb.Hierarchy.load(%r) as h:\n"
+             "    held = cb.device_bytes()\n    b = np.ones(n)\n"
+             "    x, it, _, flag, _ = h.pcg(b, tol=1e-8, itmax=200)\n"
+             "print(held, np.linalg.norm(b - A @ x) / np.linalg.norm(b))\n")
+    low, high = int(lean), int(lean) + (512 << 20)
+    assert child(solve % files[0], high)
+    while high - low > 4 << 20:
+        mid = (low + high) // 2
+        if child(solve % files[0], mid):
+            high = mid
+        else:
+            low = mid
+    held, rel = child(solve % files[1], high)
+    assert held < full and rel <= 1e-8
