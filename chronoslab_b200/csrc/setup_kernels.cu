@@ -136,39 +136,31 @@ __device__ __forceinline__ void fsai_row(int i, const int *__restrict__ arp,
 }
 
 // Positions of the columns col[u] in the sorted rows [lo[u], hi[u]) of aci, or
-// -1: U binary searches step together, so their dependent loads overlap.
+// -1: U binary searches step together, so their dependent loads overlap.  A
+// step's interval shrinks by the same amount whichever side is taken: one
+// compare and one add a search.
 template <int U>
 __device__ __forceinline__ void find_cols(const int *__restrict__ aci, int (&lo)[U],
                                           const int (&hi)[U], const int (&col)[U]) {
-  int n[U];
-  bool any = false;
+  int n[U], longest = 0;
 #pragma unroll
   for (int u = 0; u < U; ++u) {
     n[u] = hi[u] - lo[u];
-    any |= n[u] > 0;
+    longest = max(longest, n[u]);
   }
-  while (any) {
+  for (; longest > 1; longest -= longest >> 1) {
     int c[U];
 #pragma unroll
-    for (int u = 0; u < U; ++u) c[u] = n[u] > 0 ? __ldg(aci + lo[u] + (n[u] >> 1)) : 0;
-    any = false;
+    for (int u = 0; u < U; ++u) c[u] = n[u] > 1 ? __ldg(aci + lo[u] + (n[u] >> 1) - 1) : 0x7fffffff;
 #pragma unroll
     for (int u = 0; u < U; ++u) {
-      const int half = n[u] >> 1;
-      if (n[u] > 0) {
-        if (c[u] < col[u]) {
-          lo[u] += half + 1;
-          n[u] -= half + 1;
-        } else {
-          n[u] = half;
-        }
-      }
-      any |= n[u] > 0;
+      if (c[u] < col[u]) lo[u] += n[u] >> 1;
+      n[u] -= n[u] >> 1;
     }
   }
 #pragma unroll
   for (int u = 0; u < U; ++u)
-    if (lo[u] >= hi[u] || __ldg(aci + lo[u]) != col[u]) lo[u] = -1;
+    if (n[u] <= 0 || __ldg(aci + lo[u]) != col[u]) lo[u] = -1;
 }
 
 // Row i of G by T lanes (32/T rows per warp; i < 0: an idle group), local
@@ -185,9 +177,12 @@ __device__ __forceinline__ void find_cols(const int *__restrict__ aci, int (&lo)
 // row, the factor in shared memory and a lane per column walking A's rows
 // this took 1419 us for 227k rows of mostly 15 unknowns (61^3 diffusion),
 // bound by those and by the serial walk; with the column sent round by
-// shuffles 351 us, bound by issue (71 % of the slots); now 297 us.  The
-// entries A[P,P] are found by T lanes taking the pairs (c, c+s mod m) of each
-// distance s, four searches in flight.
+// shuffles 351 us, with the column from shared memory 297 us, with the shorter
+// search and blocks of four warps for eight 266 us, still bound by issue (71 %
+// of the slots).  Two unknowns a lane, which halves a row's shuffles, reciprocals
+// and column reads, took as long: its 96 registers leave 20 warps an SM for 32.
+// The entries A[P,P] are found by T lanes taking the pairs (c, c+s mod m) of
+// each distance s, four searches in flight.
 template <int T, int MMAX>
 __device__ __forceinline__ void fsai_row_reg(int i, const int *__restrict__ arp,
                                              const int *__restrict__ aci,
@@ -308,7 +303,7 @@ __device__ __forceinline__ void fsai_row_reg(int i, const int *__restrict__ arp,
 __host__ __device__ constexpr int fsai_lanes(int mmax) {
   return mmax <= 4 ? 4 : mmax <= 8 ? 8 : mmax <= 16 ? 16 : mmax <= 32 ? 32 : 0;
 }
-__host__ __device__ constexpr int fsai_warps(int mmax) { return mmax <= 16 ? 8 : mmax <= 32 ? 4 : 2; }
+__host__ __device__ constexpr int fsai_warps(int mmax) { return mmax <= 32 ? 4 : 2; }
 __host__ __device__ constexpr int fsai_group_doubles(int mmax) {
   return mmax <= 32 ? mmax * (mmax + 2) : mmax * mmax + 3 * mmax;
 }
