@@ -195,15 +195,14 @@ static void spmm(cudaStream_t st, const DMat &M, const VT *vals, const XT *X, co
 }
 
 // Y = W B on the coarsest level (W FP64 n x n row-major, B n x K row-major).
-// (rows of W ld values apart)
 template <typename TI, typename TO, int K>
-__global__ void k_dense_matmat(int n, int ld, const double *__restrict__ W,
+__global__ void k_dense_matmat(int n, const double *__restrict__ W,
                                const TI *__restrict__ B, TO *__restrict__ Y) {
   pdl_begin();
   const int row = blockIdx.x, j = threadIdx.x % K, g = threadIdx.x / K, G = blockDim.x / K;
   __shared__ double red[256];
   double s = 0.0;
-  for (int c = g; c < n; c += G) s += W[(size_t)row * ld + c] * (double)B[(size_t)c * K + j];
+  for (int c = g; c < n; c += G) s += W[(size_t)row * n + c] * (double)B[(size_t)c * K + j];
   red[threadIdx.x] = s;
   __syncthreads();
   if (g == 0) {
@@ -255,14 +254,14 @@ static void vcycle_block(Hier &h, BlockState &s, int l, const BT *b, OT *out, co
   double *part = s.part.get();
   unsigned *tick = s.tickets.get();
   if (L.coarsest) {
-    launch_pdl(k_dense_matmat<BT, OT, K>, n, 256, st, n, n, (const double *)L.W.get(), b, out);
+    launch_pdl(k_dense_matmat<BT, OT, K>, n, 256, st, n, (const double *)L.W.get(), b, out);
     CHRONOS_CHECK_LAUNCH();
     return;
   }
   T *x = blk<T>(s.x32, s.x64, l), *r = blk<T>(s.r32, s.r64, l), *t = blk<T>(s.t32, s.t64, l);
   const T w = (T)L.omega;
   if (L.fold && L.fold->form == FOLD_DENSE) {
-    launch_pdl(k_dense_matmat<BT, OT, K>, n, 256, st, n, L.fold->ld,
+    launch_pdl(k_dense_matmat<BT, OT, K>, n, 256, st, n,
                (const double *)L.fold->D.get(), b, out);
     CHRONOS_CHECK_LAUNCH();
     return;
@@ -487,7 +486,6 @@ template <int K>
 __global__ void __launch_bounds__(256)
 k_bnorm2(int n, const double *__restrict__ B, double *part, unsigned *ticket, double *dst) {
   pdl_begin();
-  const int j = threadIdx.x % K;
   double s = 0.0;
   const size_t total = (size_t)n * K;
   for (size_t o = blockIdx.x * (size_t)blockDim.x + threadIdx.x; o < total;

@@ -52,36 +52,35 @@ k_add_identity(int n, const int *__restrict__ rp, const int *__restrict__ ci,
 // Y = E B: row r of Y (m wide) from E's row and the dense rows of B.
 __global__ void __launch_bounds__(256)
 k_sparse_dense(int m, const int *__restrict__ rp, const int *__restrict__ ci,
-               const double *__restrict__ v, const double *__restrict__ B, int ldb,
+               const double *__restrict__ v, const double *__restrict__ B,
                double *__restrict__ Y) {
   const int r = blockIdx.x, s = rp[r], e = rp[r + 1];
   for (int j = threadIdx.x; j < m; j += blockDim.x) {
     double t = 0.0;
-    for (int k = s; k < e; ++k) t = fma(v[k], B[(size_t)ci[k] * ldb + j], t);
+    for (int k = s; k < e; ++k) t = fma(v[k], B[(size_t)ci[k] * m + j], t);
     Y[(size_t)r * m + j] = t;
   }
 }
 
 // D = Y R + Q, row r: Y's row in shared memory against the columns of R (the
-// rows of R'), then Q's entries on top; the padding columns are zero.
+// rows of R'), then Q's entries on top.
 __global__ void __launch_bounds__(256)
 k_dense_tail(int n, int m, const double *__restrict__ Y, const int *__restrict__ trp,
              const int *__restrict__ tci, const double *__restrict__ tv,
              const int *__restrict__ qrp, const int *__restrict__ qci,
-             const double *__restrict__ qv, double *__restrict__ D, int ld) {
+             const double *__restrict__ qv, double *__restrict__ D) {
   extern __shared__ double y[];
   const int r = blockIdx.x;
   for (int c = threadIdx.x; c < m; c += blockDim.x) y[c] = Y[(size_t)r * m + c];
   __syncthreads();
-  for (int j = threadIdx.x; j < ld; j += blockDim.x) {
+  for (int j = threadIdx.x; j < n; j += blockDim.x) {
     double t = 0.0;
-    if (j < n)
-      for (int k = trp[j]; k < trp[j + 1]; ++k) t = fma(y[tci[k]], tv[k], t);
-    D[(size_t)r * ld + j] = t;
+    for (int k = trp[j]; k < trp[j + 1]; ++k) t = fma(y[tci[k]], tv[k], t);
+    D[(size_t)r * n + j] = t;
   }
   __syncthreads();
   for (int k = qrp[r] + threadIdx.x; k < qrp[r + 1]; k += blockDim.x)
-    D[(size_t)r * ld + qci[k]] += qv[k];
+    D[(size_t)r * n + qci[k]] += qv[k];
 }
 
 // A sparse product on the device.
@@ -161,8 +160,8 @@ void adopt(Prod &p, DMat &d, bool fp32, cudaStream_t st) {
 }  // namespace
 
 std::unique_ptr<Fold> fold_operators(const DMat &A, const DMat &G, const DMat &Gt, const DMat &P,
-                                     const DMat &Pt, double omega, const double *B, int ldb,
-                                     bool fp32, cudaStream_t st) {
+                                     const DMat &Pt, double omega, const double *B, bool fp32,
+                                     cudaStream_t st) {
   const int n = A.nrows, nc = P.ncols;
   auto f = std::make_unique<Fold>();
   const bool dense = B && n <= kFoldDenseRows && (int64_t)n * n <= kFoldDenseRatio * A.nnz;
@@ -210,17 +209,16 @@ std::unique_ptr<Fold> fold_operators(const DMat &A, const DMat &G, const DMat &G
     return f;
   }
   if (dense) {
-    f->ld = (n + 1) & ~1;
-    f->D.alloc((size_t)n * f->ld);
+    f->D.alloc((size_t)n * n);
     DBuf<double> Y((size_t)n * nc), tv;
     DBuf<int> trp, tci;
     csr_transpose_device(nc, n, R.nnz, R.rp, R.ci, R.v, trp, tci, tv, st);
     k_sparse_dense<<<n, 256, 0, st>>>(nc, E.rp.get(), E.ci.get(), E.v.get(), B,
-                                      ldb, Y.get());
+                                      Y.get());
     CHRONOS_CHECK_LAUNCH();
     k_dense_tail<<<n, 256, sizeof(double) * nc, st>>>(n, nc, Y.get(), trp.get(), tci.get(),
                                                       tv.get(), Q.rp.get(), Q.ci.get(),
-                                                      Q.v.get(), f->D.get(), f->ld);
+                                                      Q.v.get(), f->D.get());
     CHRONOS_CHECK_LAUNCH();
     CHRONOS_CUDA(cudaStreamSynchronize(st));
     f->form = FOLD_DENSE;
@@ -251,11 +249,10 @@ void build_folds(Hier &h) {
     const Level &C = h.levels[l + 1];
     // level 1 keeps its fused dot and conversions: no dense form
     const double *B = nullptr;
-    int ldb = 0;
-    if (l > 0 && C.coarsest) { B = C.W.get(); ldb = C.n; }
-    else if (l > 0 && C.fold && C.fold->form == FOLD_DENSE) { B = C.fold->D.get(); ldb = C.fold->ld; }
-    L.fold = fold_operators(L.A, L.G, L.Gt, L.P, L.Pt, L.omega, B, ldb,
-                            h.precision == CHRONOS_FP32, h.st);
+    if (l > 0 && C.coarsest) B = C.W.get();
+    else if (l > 0 && C.fold && C.fold->form == FOLD_DENSE) B = C.fold->D.get();
+    L.fold = fold_operators(L.A, L.G, L.Gt, L.P, L.Pt, L.omega, B, h.precision == CHRONOS_FP32,
+                            h.st);
   }
 }
 

@@ -455,7 +455,7 @@ static std::unique_ptr<GroupSolve> build_stack(const std::vector<std::unique_ptr
     // one pre- and one postsmoothing step in the autotuner's storage: folded as a
     // single hierarchy's level is (the stack is block diagonal, G' scaled)
     if (fold && prm.nupre <= 1 && prm.nupost == 1 && prm.spmv_format == 0)
-      L.fold = fold_operators(L.A, L.G, L.Gt, L.P, L.Pt, 1.0, nullptr, 0, fp32, st);
+      L.fold = fold_operators(L.A, L.G, L.Gt, L.P, L.Pt, 1.0, nullptr, fp32, st);
     const Fold *F = L.fold.get();
     if (F) tune_fold(*L.fold, fp32, st);
     if (!F || F->form != FOLD_ALL) autotune_lanes(L.A, fp32, st, prm.spmv_format);

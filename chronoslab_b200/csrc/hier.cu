@@ -1674,33 +1674,6 @@ __global__ void k_dot_store(int n, const double *a, const double *b, double *par
   grid_reduce<1>(v, part, ticket, StoreScalar{out});
 }
 
-// x = D b, D with rows of ld values (ld even): a warp per row, 16-byte loads.
-template <typename TI, typename TO>
-__global__ void __launch_bounds__(256)
-k_dense_tail_apply(int n, const double *__restrict__ D, int ld, const TI *__restrict__ b,
-                   TO *__restrict__ x) {
-  pdl_begin();
-  const int lane = threadIdx.x & 31;
-  const int row = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-  if (row >= n) return;
-  const double2 *d = reinterpret_cast<const double2 *>(D + (size_t)row * ld);
-  double s0 = 0.0, s1 = 0.0;
-#pragma unroll 4
-  for (int j = lane; 2 * j + 1 < n; j += 32) {
-    const double2 w = __ldg(d + j);
-    s0 = fma(w.x, (double)__ldg(b + 2 * j), s0);
-    s1 = fma(w.y, (double)__ldg(b + 2 * j + 1), s1);
-  }
-  if ((n & 1) && lane == 0) s0 = fma(D[(size_t)row * ld + n - 1], (double)__ldg(b + n - 1), s0);
-  const double s = warp_sum(s0 + s1);
-  if (lane == 0) x[row] = (TO)s;
-}
-
-template <typename TI, typename TO>
-static void dense_tail_apply(cudaStream_t st, int n, const double *D, int ld, const TI *b, TO *x) {
-  launch_pdl(k_dense_tail_apply<TI, TO>, ceil_div((int64_t)n * 32, 256), 256, st, n, D, ld, b, x);
-}
-
 // Whether n values at a and at b share memory.
 template <typename TA, typename TB>
 static bool overlap(const TA *a, const TB *b, int n) {
@@ -1728,7 +1701,7 @@ static void vcycle_level(Hier &h, int l, const BT *b, OT *out, const double *dw,
     const Fold &F = *L.fold;
     if constexpr (!TOP) {
       if (F.form == FOLD_DENSE) {
-        dense_tail_apply<BT, OT>(st, n, F.D.get(), F.ld, b, out);
+        dense_matvec<BT, OT>(n, F.D.get(), b, out, st);
         return;
       }
     }
@@ -2616,7 +2589,7 @@ static double vcycle_bytes_level(const Hier &h, int l, double s, double sb, doub
   double b = 0.0;
   if (L.fold) {
     const Fold &F = *L.fold;
-    if (F.form == FOLD_DENSE) return (double)n * F.ld * 8.0 + n * (sb + sout);
+    if (F.form == FOLD_DENSE) return (double)n * n * 8.0 + n * (sb + sout);
     const double dot = top ? 8.0 : 0.0, coarse = vcycle_bytes_level(h, l + 1, s, s, s, false);
     if (F.form == FOLD_ALL)
       return apply_bytes(F.R, s, sb, s, 0.0) + coarse + apply_bytes(F.Q, s, sb, sout, dot) +

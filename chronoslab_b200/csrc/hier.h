@@ -46,15 +46,13 @@ void validate_csr(const HostCSR &A);
 bool gpu_coarsening(const char *soc_type);
 
 // The folded form of a level (fold.cu).  FOLD_SMOOTH: S; FOLD_DOWN: S and R;
-// FOLD_ALL: R, Q, E (and S, for block solves); FOLD_DENSE: D, n rows of ld
-// values (ld even).
+// FOLD_ALL: R, Q, E (and S, for block solves); FOLD_DENSE: D, n x n.
 enum FoldForm { FOLD_SMOOTH, FOLD_DOWN, FOLD_ALL, FOLD_DENSE };
 struct Fold {
   FoldForm form = FOLD_SMOOTH;
   DMat S, R, Q, E;
   int lanes = 8;                   // lanes per row of S b + P e or Q b + E e
   DBuf<double> D;
-  int ld = 0;
 };
 
 struct Level {
@@ -279,10 +277,10 @@ void tune_hierarchy(Hier &h);
 void build_folds(Hier &h);
 // The folded form of one level's operators, or null where none pays: A, G, G',
 // P, P' as the cycle applies them, the smoother scaled by omega; B: the dense
-// operator (rows of ldb values) of everything below, null if there is none.
+// operator (n x n) of everything below, null if there is none.
 std::unique_ptr<Fold> fold_operators(const DMat &A, const DMat &G, const DMat &Gt, const DMat &P,
-                                     const DMat &Pt, double omega, const double *B, int ldb,
-                                     bool fp32, cudaStream_t st);
+                                     const DMat &Pt, double omega, const double *B, bool fp32,
+                                     cudaStream_t st);
 // Tunes the operators of a folded form that go through mat_apply.
 void tune_fold(Fold &F, bool fp32, cudaStream_t st);
 
