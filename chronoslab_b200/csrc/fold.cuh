@@ -40,8 +40,7 @@ k_fold_apply(int n, const int *__restrict__ qrp, const int *__restrict__ qci,
     }
   }
   if (DOT) {
-    double vals[1] = {dacc};
-    grid_reduce<1>(vals, part, ticket, StoreScalar{dot_out});
+    grid_dot(dacc, part, ticket, dot_out);
   }
 }
 

@@ -598,8 +598,7 @@ static void upload_sell3(const DMat &src, const std::vector<int> &blen, int T, D
 }
 
 static void launch_pcg_spmv(cudaStream_t st, const DMat &A, bool fp32vals, const double *p,
-                            const double *res, double *axp, double *part, unsigned *tick,
-                            double *sc);
+                            const double *res, double *axp, double *part);
 
 // Attaches the sliced block form with the fastest threads-per-block-row.
 // The layout serves the V-cycle's residuals (two per cycle, hierarchy
@@ -621,15 +620,12 @@ static void attach_sell3(const HostCSR &A, DMat &d, bool fp32, cudaStream_t st) 
     if (it != g_tune.end()) T = it->second;
   }
   if (T < 0) {
-    DBuf<double> x64(A.ncols), y64(A.nrows), p64(A.ncols), q64(A.nrows), part(3 * 2048),
-        sc(SC_COUNT);
+    DBuf<double> x64(A.ncols), y64(A.nrows), p64(A.ncols), q64(A.nrows), part(3 * 2048);
     DBuf<float> x32(A.ncols), y32(A.nrows);
-    DBuf<unsigned> tick(1);
     DBuf<char> flush(kL2FlushBytes);
     x64.zero(st);
     x32.zero(st);
     p64.zero(st);
-    tick.zero(st);
     float best = 1e30f;
     cudaEvent_t e0, e1;
     CHRONOS_CUDA(cudaEventCreate(&e0));
@@ -651,8 +647,7 @@ static void attach_sell3(const HostCSR &A, DMat &d, bool fp32, cudaStream_t st) 
                 probe.bv64.get(), probe.nslots, x64.get(), (const double *)nullptr, y64.get(),
                 1.0);
         }
-        launch_pcg_spmv(st, probe, fp32, p64.get(), p64.get(), q64.get(), part.get(),
-                        tick.get(), sc.get());
+        launch_pcg_spmv(st, probe, fp32, p64.get(), p64.get(), q64.get(), part.get());
       };
       launch();
       float tmin = 1e30f;
@@ -674,8 +669,7 @@ static void attach_sell3(const HostCSR &A, DMat &d, bool fp32, cudaStream_t st) 
             CHRONOS_CUDA(cudaMemsetAsync(flush.get(), r, kL2FlushBytes, st));
             CHRONOS_CUDA(cudaEventRecord(e0, st));
             if (outer)
-              launch_pcg_spmv(st, probe, fp32, p64.get(), p64.get(), q64.get(), part.get(),
-                              tick.get(), sc.get());
+              launch_pcg_spmv(st, probe, fp32, p64.get(), p64.get(), q64.get(), part.get());
             else if (fp32)
               sell3_apply<float, float, float, float, MODE_PLAIN, false>(
                   st, t, probe.nb, probe.nchunk, probe.choff, probe.chw, probe.sci,
@@ -1440,7 +1434,13 @@ void tune_hierarchy(Hier &h) {
     if (e.code != CHRONOS_ENOMEM) throw;
   }
   CHRONOS_CUDA(cudaStreamSynchronize(h.st));
-  for (auto &L : h.levels) L.fold.reset();
+  for (auto &L : h.levels) {
+    L.fold.reset();
+    for (DMat *m : {&L.A, &L.G, &L.Gt, &L.P, &L.Pt}) {   // what the attempt left half tuned
+      drop_sell(*m);
+      m->wide = false;
+    }
+  }
   tune_operators(h);
 }
 
@@ -1670,8 +1670,7 @@ __global__ void k_dot_store(int n, const double *a, const double *b, double *par
   double s = 0.0;
   for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x)
     s += a[i] * b[i];
-  double v[1] = {s};
-  grid_reduce<1>(v, part, ticket, StoreScalar{out});
+  grid_dot(s, part, ticket, out);
 }
 
 // Whether n values at a and at b share memory.
@@ -1681,12 +1680,18 @@ static bool overlap(const TA *a, const TB *b, int n) {
   return pa < pb + (size_t)n * sizeof(TB) && pb < pa + (size_t)n * sizeof(TA);
 }
 
+// Where PcgState::part keeps the partials that a consumer kernel adds: the outer
+// product's two sums, and the V-cycle's dot.
+constexpr size_t kSpmvPartials = 4 * 3 * 2048, kDotPartials = kSpmvPartials + 2 * 2048;
+
 template <typename T, typename BT, typename OT, bool TOP>
 static void vcycle_level(Hier &h, int l, const BT *b, OT *out, const double *dw, double *dot_out) {
   Level &L = h.levels[l];
   cudaStream_t st = h.st;
   const int n = L.n;
+  // a dot without a place for its result: the partials, for the PCG's p update
   double *part = h.pcg.part.get();
+  if (dw && !dot_out) part += kDotPartials;
   unsigned *tick = h.pcg.tickets.get();
   if (L.coarsest) {
     dense_matvec<BT, OT>(n, L.W.get(), b, out, st);
@@ -1827,31 +1832,20 @@ void Hier::apply_A(const double *x, double *y) {
 // PCG_CJ
 // ---------------------------------------------------------------------------
 
-// p = pres (first iteration) or p = pres + beta p, beta = -(pres'axp)/ptap.
-__global__ void k_pcg_p_update(int n, const double *__restrict__ pres, double *__restrict__ p,
-                               const double *__restrict__ sc) {
+// p = pres (first iteration) or p = pres + beta p, beta = -(pres'axp)/ptap with
+// pres'axp from the V-cycle's partials.
+__global__ void __launch_bounds__(256)
+k_pcg_p_update(int n, const double *__restrict__ pres, double *__restrict__ p,
+               const double *__restrict__ part, int slots, const double *__restrict__ sc) {
   pdl_begin();
   const bool first = sc[SC_ITER] < 0.5;
-  const double beta = first ? 0.0 : -sc[SC_PRES_AXP] / sc[SC_PTAP];
+  const double ptap = sc[SC_PTAP];
+  double t[1];
+  sum_partials<1>(part, slots, t);
+  const double beta = first ? 0.0 : -t[0] / ptap;
   for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x)
     p[i] = first ? pres[i] : pres[i] + beta * p[i];
 }
-
-struct FinAlpha {
-  double *sc;
-  __device__ void operator()(const double *t) const {
-    const double ptap = t[0], pres = t[1];
-    if (sc[SC_DONE] != 0.0) return;             // an iteration after the stop (far_exec)
-    sc[SC_PTAP] = ptap;
-    sc[SC_PRES] = pres;
-    if (!(ptap > 0.0) || !isfinite(pres)) {     // breakdown: p'Ap <= 0 or NaN
-      sc[SC_BREAKDOWN] = 1.0;
-      sc[SC_ALPHA] = 0.0;
-    } else {
-      sc[SC_ALPHA] = pres / ptap;
-    }
-  }
-};
 
 // axp = A p with ptap = p'axp and p'res, accumulated in FP64; the stored
 // values VT are the FP64 operator (exact PCG_CJ arithmetic) or the FP32 copy
@@ -1863,8 +1857,7 @@ k_pcg_spmv(int n, const int *__restrict__ rp, const int *__restrict__ ci,
            const int *__restrict__ cbase, const uint16_t *__restrict__ c16,
            const VT *__restrict__ v, const double *__restrict__ p,
            const double *__restrict__ res, double *__restrict__ axp, int short_blocks,
-           int lthresh, const int *__restrict__ longrows, int nlong, double *part,
-           unsigned *ticket, double *sc) {
+           int lthresh, const int *__restrict__ longrows, int nlong, double *part) {
   pdl_begin();
   const int lane = threadIdx.x & 31;
   double d0 = 0.0, d1 = 0.0;
@@ -1911,7 +1904,7 @@ k_pcg_spmv(int n, const int *__restrict__ rp, const int *__restrict__ ci,
     }
   }
   double vals2[2] = {d0, d1};
-  grid_reduce<2>(vals2, part, ticket, FinAlpha{sc});
+  block_partials<2>(vals2, part);
 }
 
 // The same on the sliced 3x3 block form (see k_sell3_apply).
@@ -1920,7 +1913,7 @@ __global__ void __launch_bounds__(kApplyThreads)
 k_pcg_spmv_sell3(int nb, int nchunk, const int *__restrict__ choff, const int *__restrict__ chw,
                  const int *__restrict__ sci, const VT *__restrict__ V, int64_t nslots,
                  const double *__restrict__ p, const double *__restrict__ res,
-                 double *__restrict__ axp, double *part, unsigned *ticket, double *sc) {
+                 double *__restrict__ axp, double *part) {
   pdl_begin();
   constexpr int C = 32 / T;
   const int lane = threadIdx.x & 31;
@@ -1950,7 +1943,7 @@ k_pcg_spmv_sell3(int nb, int nchunk, const int *__restrict__ choff, const int *_
     }
   }
   double vals2[2] = {d0, d1};
-  grid_reduce<2>(vals2, part, ticket, FinAlpha{sc});
+  block_partials<2>(vals2, part);
 }
 
 static int pcg_grid(const DMat &A, int *short_blocks) {
@@ -1968,8 +1961,7 @@ static int pcg_grid(const DMat &A, int *short_blocks) {
 // axp = A p with ptap and p'res, through the block form when A has one; FP32
 // stored values when fp32vals (the FP32 hierarchy's copy), FP64 otherwise.
 static void launch_pcg_spmv(cudaStream_t st, const DMat &A, bool fp32vals, const double *p,
-                            const double *res, double *axp, double *part, unsigned *tick,
-                            double *sc) {
+                            const double *res, double *axp, double *part) {
   int sb = 0;
   const int grid = pcg_grid(A, &sb);
   if (A.nb > 0) {
@@ -1978,11 +1970,11 @@ static void launch_pcg_spmv(cudaStream_t st, const DMat &A, bool fp32vals, const
     if (fp32vals)                                                                              \
       launch_pdl(k_pcg_spmv_sell3<float, TT>, grid, kApplyThreads, st, A.nb, A.nchunk,         \
                  A.choff.get(), A.chw.get(), A.sci.get(), A.bv32.get(), A.nslots, p, res, axp, \
-                 part, tick, sc);                                                              \
+                 part);                                                                        \
     else                                                                                       \
       launch_pdl(k_pcg_spmv_sell3<double, TT>, grid, kApplyThreads, st, A.nb, A.nchunk,        \
                  A.choff.get(), A.chw.get(), A.sci.get(), A.bv64.get(), A.nslots, p, res, axp, \
-                 part, tick, sc);                                                              \
+                 part);                                                                        \
     break;
     switch (A.sell_T) {
       CHRONOS_PCGS_CASE(1)
@@ -1995,7 +1987,7 @@ static void launch_pcg_spmv(cudaStream_t st, const DMat &A, bool fp32vals, const
 #define CHRONOS_PCG_LAUNCH(VT, VALS, LL, I16)                                                  \
   launch_pdl(k_pcg_spmv<VT, LL, I16>, grid, kApplyThreads, st, A.nrows, A.rp.get(), A.ci.get(),  \
              A.cbase.get(), A.c16.get(), VALS, p, res, axp, sb, A.lthresh, A.longrows.get(),    \
-             A.nlong, part, tick, sc)
+             A.nlong, part)
 #define CHRONOS_PCG_CASE(LL)                                                                   \
   case LL:                                                                                     \
     if (fp32vals) {                                                                            \
@@ -2073,16 +2065,26 @@ struct FinResidual {
 // x += alpha p; res -= alpha axp; ||res||^2; stopping test of PCG_CJ.m:58-64.
 __global__ void __launch_bounds__(256)
 k_pcg_xr_update(int n, double *__restrict__ x, double *__restrict__ res,
-                const double *__restrict__ p, const double *__restrict__ axp, double *part,
-                unsigned *ticket, double *sc, double *resvec, cudaGraphConditionalHandle handle,
-                int use_cond, int mixed, double far) {
+                const double *__restrict__ p, const double *__restrict__ axp,
+                const double *__restrict__ spmv_part, int slots, double *part, unsigned *ticket,
+                double *sc, double *resvec, cudaGraphConditionalHandle handle, int use_cond,
+                int mixed, double far) {
   pdl_begin();
   FinResidual fin{sc, resvec, handle, use_cond, mixed, far};
   fin.load();
-  const double alpha = sc[SC_ALPHA];
-  if (sc[SC_DONE] != 0.0) {            // stopped in an earlier iteration of this pass
+  const bool done = sc[SC_DONE] != 0.0;
+  double t[2];
+  sum_partials<2>(spmv_part, slots, t);
+  if (done) {                          // stopped in an earlier iteration of this pass
     if (use_cond && blockIdx.x == 0 && threadIdx.x == 0) cudaGraphSetConditional(handle, 0u);
     return;
+  }
+  const bool broke = !(t[0] > 0.0) || !isfinite(t[1]);     // p'Ap <= 0 or NaN
+  const double alpha = broke ? 0.0 : t[1] / t[0];
+  if (broke) fin.breakdown = 1.0;
+  if (blockIdx.x == 0 && threadIdx.x == 0) {
+    sc[SC_PTAP] = t[0];
+    if (broke) sc[SC_BREAKDOWN] = 1.0;
   }
   double rr = 0.0;
   for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
@@ -2309,17 +2311,19 @@ static void capture_iteration(Hier &h, cudaGraphConditionalHandle handle, int us
   const int nb = reduce_blocks(n);
   const bool mixed = mixed_outer(h);
   double *sc = s.sc.get();
-  // pres = M^{-1} res  (with pres'axp for beta)
-  h.vcycle(s.res.get(), s.pres.get(), s.axp.get(), sc + SC_PRES_AXP);
+  double *spmv_part = s.part.get() + kSpmvPartials;
+  const int slots = num_sms() * 8;             // no producer's grid is larger
+  // pres = M^{-1} res  (with the partials of pres'axp for beta)
+  h.vcycle(s.res.get(), s.pres.get(), s.axp.get(), nullptr);
   launch_pdl(k_pcg_p_update, nb, 256, st, n, (const double *)s.pres.get(), s.p.get(),
-             (const double *)sc);
+             (const double *)(s.part.get() + kDotPartials), slots, (const double *)sc);
   CHRONOS_CHECK_LAUNCH();
   unsigned *tk = s.tickets.get();
-  launch_pcg_spmv(st, h.outer_A(), mixed, s.p.get(), s.res.get(), s.axp.get(),
-                  s.part.get() + 4 * 3 * 2048, tk + 1, sc);
+  launch_pcg_spmv(st, h.outer_A(), mixed, s.p.get(), s.res.get(), s.axp.get(), spmv_part);
   launch_pdl(k_pcg_xr_update, nb, 256, st, n, s.x.get(), s.res.get(), (const double *)s.p.get(),
-             (const double *)s.axp.get(), s.part.get() + 8 * 3 * 2048, tk + 2, sc,
-             s.resvec.get(), handle, use_cond, mixed ? 1 : 0, far);
+             (const double *)s.axp.get(), (const double *)spmv_part, slots,
+             s.part.get() + 8 * 3 * 2048, tk + 2, sc, s.resvec.get(), handle, use_cond,
+             mixed ? 1 : 0, far);
   CHRONOS_CHECK_LAUNCH();
   if (mixed)
     launch_pcg_replace(st, h.levels[0].A, s.x.get(), s.b.get(), s.res.get(),
@@ -2457,6 +2461,8 @@ void Hier::pcg_solve(const double *b, double *x, int itmax, double tol, int *ite
   k_dot_store<<<nb, 256, 0, st>>>(n, s.res.get(), s.res.get(), part, s.tickets.get() + 3,
                                    s.sc.get() + SC_RR);
   CHRONOS_CHECK_LAUNCH();
+  // partials past the producers' grids (which may have changed) are zero
+  CHRONOS_CUDA(cudaMemsetAsync(s.part.get() + kSpmvPartials, 0, sizeof(double) * 3 * 2048, st));
   k_pcg_init<<<1, 1, 0, st>>>(s.sc.get(), s.resvec.get(), tol, (double)itmax,
                               replace_ratio(*this));
   CHRONOS_CHECK_LAUNCH();
@@ -2549,6 +2555,8 @@ void Hier::pcg_enqueue(const double *b, double *x, int itmax, double tol) {
   k_dot_store<<<nb, 256, 0, st>>>(n, s.res.get(), s.res.get(), s.part.get(), s.tickets.get() + 3,
                                    s.sc.get() + SC_RR);
   CHRONOS_CHECK_LAUNCH();
+  // partials past the producers' grids (which may have changed) are zero
+  CHRONOS_CUDA(cudaMemsetAsync(s.part.get() + kSpmvPartials, 0, sizeof(double) * 3 * 2048, st));
   k_pcg_init<<<1, 1, 0, st>>>(s.sc.get(), s.resvec.get(), tol, (double)itmax,
                               replace_ratio(*this));
   CHRONOS_CHECK_LAUNCH();
@@ -2678,12 +2686,11 @@ void Hier::profile(int reps, chronos_profile *out) {
   }
   // outer SpMV with its two dots, as captured in the PCG iteration (stored
   // FP32 values with FP64 accumulation, or FP64 values)
-  double *part = ps.part.get() + 4 * 3 * 2048;
+  double *part = ps.part.get() + kSpmvPartials;
   CHRONOS_CUDA(cudaMemcpyAsync(ps.p.get(), b.get(), sizeof(double) * n, cudaMemcpyDeviceToDevice, st));
   CHRONOS_CUDA(cudaMemcpyAsync(ps.res.get(), b.get(), sizeof(double) * n, cudaMemcpyDeviceToDevice, st));
   out->outer_spmv_ms = time_it([&] {
-    launch_pcg_spmv(st, A, mixed_outer(*this), ps.p.get(), ps.res.get(), ps.axp.get(), part,
-                    ps.tickets.get() + 1, ps.sc.get());
+    launch_pcg_spmv(st, A, mixed_outer(*this), ps.p.get(), ps.res.get(), ps.axp.get(), part);
   });
   out->outer_spmv_bytes = apply_bytes(A, mixed_outer(*this) ? 4.0 : 8.0, 8.0, 8.0, 16.0);
   out->iteration_bytes = out->vcycle_bytes + out->outer_spmv_bytes + 3.0 * n * 8 + 6.0 * n * 8;

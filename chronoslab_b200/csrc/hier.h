@@ -86,8 +86,8 @@ template <> inline const double *vals<double>(const DMat &m) { return m.v64.get(
 
 // Device scalars of the PCG recurrence.
 enum PcgScalar {
-  SC_BNORM = 0, SC_PTAP, SC_ALPHA, SC_PRES_AXP, SC_RR, SC_RESITER, SC_ITER, SC_TOL, SC_ITMAX,
-  SC_BREAKDOWN, SC_PRES, SC_RMAX, SC_REPLACE, SC_RATIO, SC_DONE, SC_COUNT = 16
+  SC_BNORM = 0, SC_PTAP, SC_PRES_AXP, SC_RR, SC_RESITER, SC_ITER, SC_TOL, SC_ITMAX,
+  SC_BREAKDOWN, SC_RMAX, SC_REPLACE, SC_RATIO, SC_DONE, SC_COUNT = 16
 };
 
 struct PcgState {

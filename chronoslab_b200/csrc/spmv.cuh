@@ -82,6 +82,64 @@ __device__ __forceinline__ void grid_reduce(double (&v)[K], double *part, unsign
   }
 }
 
+// The first half of grid_reduce: this block's sums into part[blockIdx.x*K + j], for
+// a consumer kernel that adds them itself (sum_partials).  The second half, done
+// by the last block to arrive, is a chain of a fence, an atomic, a round of loads
+// and the block's sum behind every other block: about 2 us at the end of a kernel
+// that takes 3-7 us on small levels, where the consumer's 10 or 19 KB of partials
+// cost each of its blocks less than 1.  PCG_CJ, us per iteration with its three
+// dots finished by the producers and with two of them left as partials: Poisson
+// 20^3 FP64 30.4 and 28.2, Poisson 32^3 FP32 42.6 and 39.9, elasticity 12^3 FP64
+// 27.7 and 24.9, 64^3 FP32 355 and 348.
+template <int K>
+__device__ __forceinline__ void block_partials(double (&v)[K], double *part) {
+  __shared__ double red[K][32];
+  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, nw = blockDim.x >> 5;
+#pragma unroll
+  for (int j = 0; j < K; ++j) {
+    const double s = warp_sum(v[j]);
+    if (lane == 0) red[j][wid] = s;
+  }
+  __syncthreads();
+  if ((int)threadIdx.x < K) {
+    double s = 0.0;
+    for (int w = 0; w < nw; ++w) s += red[threadIdx.x][w];
+    part[(size_t)blockIdx.x * K + threadIdx.x] = s;
+  }
+}
+
+// The K sums of `slots` blocks' partials, in every thread of a block of 256
+// (slots past the producer's grid hold zero; the same fixed order everywhere).
+template <int K>
+__device__ __forceinline__ void sum_partials(const double *__restrict__ part, int slots,
+                                             double (&t)[K]) {
+  __shared__ double red[K][8];
+  double acc[K];
+#pragma unroll
+  for (int j = 0; j < K; ++j) acc[j] = 0.0;
+#pragma unroll 5
+  for (int b = threadIdx.x; b < slots; b += 256) {
+#pragma unroll
+    for (int j = 0; j < K; ++j) acc[j] += __ldg(part + (size_t)b * K + j);
+  }
+#pragma unroll
+  for (int j = 0; j < K; ++j) {
+    const double s = warp_sum(acc[j]);
+    if ((threadIdx.x & 31) == 0) red[j][threadIdx.x >> 5] = s;
+  }
+  __syncthreads();
+#pragma unroll
+  for (int j = 0; j < K; ++j) {
+    t[j] = red[j][0];
+#pragma unroll
+    for (int w = 1; w < 8; ++w) t[j] += red[j][w];
+  }
+}
+
+// An apply kernel's fused dot: finished into *out, or, out null, left as the
+// blocks' partials.
+__device__ __forceinline__ void grid_dot(double v, double *part, unsigned *ticket, double *out);
+
 // Deterministic grid reduction of NQ quantities of K columns (block
 // right-hand sides).  Lane l owns columns (l % (K/VEC))*VEC .. +VEC-1 and
 // v[q][e] is its partial of quantity q for the e-th of them; lanes owning the
@@ -183,6 +241,12 @@ struct StoreScalar {
   __device__ void operator()(const double *t) const { *dst = t[0]; }
 };
 
+__device__ __forceinline__ void grid_dot(double v, double *part, unsigned *ticket, double *out) {
+  double vals[1] = {v};
+  if (out) grid_reduce<1>(vals, part, ticket, StoreScalar{out});
+  else block_partials<1>(vals, part);
+}
+
 template <typename VT, int MODE, typename ZT>
 __device__ __forceinline__ VT apply_epilogue(VT sum, VT alpha, const ZT *z, int row) {
   if (MODE == MODE_PLAIN) return sum;
@@ -231,8 +295,7 @@ k_csr_apply(int n, const int *__restrict__ rp, const int *__restrict__ ci,
     }
   }
   if (DOT) {
-    double vals[1] = {dacc};
-    grid_reduce<1>(vals, part, ticket, StoreScalar{dot_out});
+    grid_dot(dacc, part, ticket, dot_out);
   }
 }
 
@@ -334,8 +397,7 @@ k_sell3_apply(int nb, int nchunk, const int *__restrict__ choff, const int *__re
     }
   }
   if (DOT) {
-    double vals[1] = {dacc};
-    grid_reduce<1>(vals, part, ticket, StoreScalar{dot_out});
+    grid_dot(dacc, part, ticket, dot_out);
   }
 }
 
@@ -468,8 +530,7 @@ k_csrh_apply(int n, const int *__restrict__ rp, const int *__restrict__ ci,
     }
   }
   if (DOT) {
-    double vals[1] = {dacc};
-    grid_reduce<1>(vals, part, ticket, StoreScalar{dot_out});
+    grid_dot(dacc, part, ticket, dot_out);
   }
 }
 
@@ -504,8 +565,7 @@ k_csr_wide(int n, const int *__restrict__ rp, const int *__restrict__ ci,
     __syncthreads();
   }
   if (DOT) {
-    double vals[1] = {dacc};
-    grid_reduce<1>(vals, part, ticket, StoreScalar{dot_out});
+    grid_dot(dacc, part, ticket, dot_out);
   }
 }
 
@@ -594,8 +654,7 @@ k_sell_apply(int nchunk, const int *__restrict__ choff, const int *__restrict__ 
     }
   }
   if (DOT) {
-    double vals[1] = {dacc};
-    grid_reduce<1>(vals, part, ticket, StoreScalar{dot_out});
+    grid_dot(dacc, part, ticket, dot_out);
   }
 }
 

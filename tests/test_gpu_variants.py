@@ -380,7 +380,8 @@ def test_free_while_a_caller_captures(lib):
 def test_folding_gives_way_to_the_memory_cap(lib, tmp_path):
     """Under the smallest CHRONOS_DEVICE_ALLOC_CAP (to 4 MB) at which a saved
     hierarchy of the same operators that is never folded (two presmoothing
-    steps) loads with a cold autotuner, the foldable one loads and solves too."""
+    steps) loads, the foldable one loads and solves too (both from one warm
+    autotuner cache: the same storage of the operators)."""
     import os
     import subprocess
     import sys
@@ -391,8 +392,7 @@ def test_folding_gives_way_to_the_memory_cap(lib, tmp_path):
     files = [str(tmp_path / f"pre{k}.chh") for k in (2, 1)]
 
     def child(code, cap=0):
-        env = dict(os.environ, CHRONOS_TUNE_CACHE=str(tmp_path / f"tune{cap}.txt"))
-        (tmp_path / f"tune{cap}.txt").unlink(missing_ok=True)
+        env = dict(os.environ, CHRONOS_TUNE_CACHE=str(tmp_path / "tune.txt"))
         if cap:
             env["CHRONOS_DEVICE_ALLOC_CAP"] = str(cap)
         r = subprocess.run([sys.executable, "-c", head + code], env=env, timeout=900,
