@@ -2316,7 +2316,7 @@ static void capture_iteration(Hier &h, cudaGraphConditionalHandle handle, int us
   // pres = M^{-1} res  (with the partials of pres'axp for beta)
   h.vcycle(s.res.get(), s.pres.get(), s.axp.get(), nullptr);
   launch_pdl(k_pcg_p_update, nb, 256, st, n, (const double *)s.pres.get(), s.p.get(),
-             (const double *)(s.part.get() + kDotPartials), slots, (const double *)sc);
+             vcycle_dot_partials(h), slots, (const double *)sc);
   CHRONOS_CHECK_LAUNCH();
   unsigned *tk = s.tickets.get();
   launch_pcg_spmv(st, h.outer_A(), mixed, s.p.get(), s.res.get(), s.axp.get(), spmv_part);
@@ -2393,6 +2393,13 @@ static void build_while_graph(Hier &h, int unroll, double far, cudaGraph_t *grap
   CHRONOS_CUDA(cudaGraphInstantiate(exec, *graph, 0));
 }
 
+const double *vcycle_dot_partials(Hier &h) { return h.pcg.part.get() + kDotPartials; }
+
+void zero_vcycle_partials(Hier &h) {
+  CHRONOS_CUDA(cudaMemsetAsync(h.pcg.part.get() + kSpmvPartials, 0, sizeof(double) * 3 * 2048,
+                               h.st));
+}
+
 void ensure_reduction_state(Hier &h) { ensure_pcg_state(h, std::max(h.pcg.resvec_cap - 1, 1)); }
 
 static void build_pcg_graph(Hier &h) {
@@ -2462,7 +2469,7 @@ void Hier::pcg_solve(const double *b, double *x, int itmax, double tol, int *ite
                                    s.sc.get() + SC_RR);
   CHRONOS_CHECK_LAUNCH();
   // partials past the producers' grids (which may have changed) are zero
-  CHRONOS_CUDA(cudaMemsetAsync(s.part.get() + kSpmvPartials, 0, sizeof(double) * 3 * 2048, st));
+  zero_vcycle_partials(*this);
   k_pcg_init<<<1, 1, 0, st>>>(s.sc.get(), s.resvec.get(), tol, (double)itmax,
                               replace_ratio(*this));
   CHRONOS_CHECK_LAUNCH();
@@ -2556,7 +2563,7 @@ void Hier::pcg_enqueue(const double *b, double *x, int itmax, double tol) {
                                    s.sc.get() + SC_RR);
   CHRONOS_CHECK_LAUNCH();
   // partials past the producers' grids (which may have changed) are zero
-  CHRONOS_CUDA(cudaMemsetAsync(s.part.get() + kSpmvPartials, 0, sizeof(double) * 3 * 2048, st));
+  zero_vcycle_partials(*this);
   k_pcg_init<<<1, 1, 0, st>>>(s.sc.get(), s.resvec.get(), tol, (double)itmax,
                               replace_ratio(*this));
   CHRONOS_CHECK_LAUNCH();

@@ -173,6 +173,10 @@ void sqmr_solve(Hier &h, const DMat *op, const double *b_h, double *x_h, int itm
                 int *iters, double *relres, int *info);
 // The buffers that a V-cycle with a fused dot reduces in.
 void ensure_reduction_state(Hier &h);
+// The partials that a V-cycle with a dot and no place for it leaves (num_sms()*8
+// slots, those past its grid as zeroed before).
+const double *vcycle_dot_partials(Hier &h);
+void zero_vcycle_partials(Hier &h);
 
 // BAMG prolongation with the GPU doing the per-row work (bamg_gpu.cu): the
 // result of bamg_prolongation bit for bit; rows whose neighbourhood outgrows

@@ -6,7 +6,8 @@
 // scalars, and the update of d, x and q.  Six vector kernels and five host
 // synchronisations an iteration took 6.6 ms for 37 iterations on elasticity
 // 17^3 (16,524 rows, FP64 hierarchy), 5.2 ms of them with the folded V-cycle;
-// now 1.95 ms.
+// 1.54 ms with the loop on the device, 1.42 ms with three of its four dots added
+// by the kernels that use them (sum_partials) instead of finished where they form.
 #include <algorithm>
 #include <cmath>
 
@@ -19,7 +20,7 @@ namespace {
 
 // Device scalars of the recurrence.
 enum SqmrScalar {
-  SQ_BB = 0, SQ_SIGMA, SQ_RHO0, SQ_RHO1, SQ_RR, SQ_VV, SQ_ALPHA, SQ_TAU, SQ_THETA0, SQ_CD, SQ_CQ,
+  SQ_BB = 0, SQ_RHO0, SQ_RHO1, SQ_VV, SQ_ALPHA, SQ_TAU, SQ_THETA0, SQ_CD, SQ_CQ,
   SQ_BETA, SQ_ITER, SQ_ITMAX, SQ_TOL, SQ_INFO, SQ_EXIT, SQ_TRUE, SQ_COUNT = 20
 };
 
@@ -47,23 +48,16 @@ __global__ void k_sq_init(double *sc, double itmax, double tol) {
   sc[SQ_EXIT] = 0.0;
 }
 
-// r -= alpha v with alpha = rho0 / sigma, ||r||^2; a vanishing sigma (info 10)
-// leaves r as it is.
-struct FinSqResidual {
-  double *sc;
-  double alpha;
-  bool broke;
-  __device__ void operator()(const double *t) const {
-    sc[SQ_RR] = t[0];
-    sc[SQ_ALPHA] = alpha;
-    if (broke) sc[SQ_INFO] = 10.0;
-  }
-};
+// r -= alpha v with alpha = rho0 / sigma, and the partials of ||r||^2; sigma from
+// the operator's partials; a vanishing one (info 10) leaves r as it is.
 __global__ void __launch_bounds__(256)
-k_sq_residual(int n, const double *__restrict__ v, double *__restrict__ r, double *part,
-              unsigned *ticket, double *sc) {
+k_sq_residual(int n, const double *__restrict__ v, double *__restrict__ r,
+              const double *__restrict__ sigma_part, int slots, double *rr_part, double *sc) {
   pdl_begin();
-  const double sigma = sc[SQ_SIGMA], rho0 = sc[SQ_RHO0];
+  const double rho0 = sc[SQ_RHO0];
+  double t[1];
+  sum_partials<1>(sigma_part, slots, t);
+  const double sigma = t[0];
   const bool broke = fabs(sigma) < 1e-20 * rho0;
   const double alpha = rho0 / sigma;
   double s = 0.0;
@@ -72,8 +66,12 @@ k_sq_residual(int n, const double *__restrict__ v, double *__restrict__ r, doubl
     r[i] = x;
     s += x * x;
   }
-  double t[1] = {s};
-  grid_reduce<1>(t, part, ticket, FinSqResidual{sc, alpha, broke});
+  t[0] = s;
+  block_partials<1>(t, rr_part);
+  if (blockIdx.x == 0 && threadIdx.x == 0) {
+    sc[SQ_ALPHA] = alpha;
+    if (broke) sc[SQ_INFO] = 10.0;
+  }
 }
 
 // ||u||^2 and the step's scalars: theta, gamma, tau, the coefficients of d, the
@@ -85,7 +83,7 @@ struct FinSqStep {
   double bb, tau, theta0, alpha, rr, rho0, rho1, it, itmax, tol, info0;
   __device__ void load() {
     bb = sc[SQ_BB]; tau = sc[SQ_TAU]; theta0 = sc[SQ_THETA0]; alpha = sc[SQ_ALPHA];
-    rr = sc[SQ_RR]; rho0 = sc[SQ_RHO0]; rho1 = sc[SQ_RHO1]; it = sc[SQ_ITER];
+    rho0 = sc[SQ_RHO0]; it = sc[SQ_ITER];
     itmax = sc[SQ_ITMAX]; tol = sc[SQ_TOL]; info0 = sc[SQ_INFO];
   }
   __device__ void operator()(const double *t) const {
@@ -115,11 +113,18 @@ struct FinSqStep {
   }
 };
 __global__ void __launch_bounds__(256)
-k_sq_step(int n, const double *__restrict__ u, double *part, unsigned *ticket, double *sc,
-          cudaGraphConditionalHandle handle, int use_cond) {
+k_sq_step(int n, const double *__restrict__ u, const double *__restrict__ rr_part,
+          const double *__restrict__ rho_part, int slots, double *part, unsigned *ticket,
+          double *sc, cudaGraphConditionalHandle handle, int use_cond) {
   pdl_begin();
   FinSqStep fin{sc, handle, use_cond};
   fin.load();
+  double rr[1], rho1[1];
+  sum_partials<1>(rr_part, slots, rr);
+  __syncthreads();                             // the sums share their staging
+  sum_partials<1>(rho_part, slots, rho1);
+  fin.rr = rr[0];
+  fin.rho1 = rho1[0];
   double s = 0.0;
   for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x)
     s += u[i] * u[i];
@@ -168,7 +173,7 @@ struct SqmrState {
   double *b = nullptr, *x = nullptr, *r = nullptr, *q = nullptr, *d = nullptr, *v = nullptr;
   cudaGraph_t graph = nullptr;
   cudaGraphExec_t exec = nullptr;
-  explicit SqmrState(int rows) : n(rows), vec(6 * (size_t)rows), sc(SQ_COUNT), part(3 * 2048),
+  explicit SqmrState(int rows) : n(rows), vec(6 * (size_t)rows), sc(SQ_COUNT), part(5 * 2048),
                                  tickets(4) {
     b = vec.get();
     x = b + n; r = x + n; q = r + n; d = q + n; v = d + n;
@@ -185,10 +190,15 @@ static void capture_sqmr(Hier &h, SqmrState &s, const DMat &A, cudaGraphConditio
   const int n = s.n, nb = std::max(1, std::min(num_sms() * 8, (int)ceil_div(n, 256)));
   double *sc = s.sc.get(), *part = s.part.get();
   unsigned *tk = s.tickets.get();
-  operator_apply<MODE_PLAIN, true>(st, A, s.q, nullptr, s.v, s.q, part, tk, sc + SQ_SIGMA);
-  launch_pdl(k_sq_residual, nb, 256, st, n, (const double *)s.v, s.r, part, tk, sc);
-  h.vcycle(s.r, s.v, s.r, sc + SQ_RHO1);
-  launch_pdl(k_sq_step, nb, 256, st, n, (const double *)s.v, part, tk, sc, handle, use_cond);
+  // (three of the four dots stay partials, added by the kernels that use them)
+  double *sigma_part = part + 3 * 2048, *rr_part = part + 4 * 2048;
+  const int slots = num_sms() * 8;               // no producer's grid is larger
+  operator_apply<MODE_PLAIN, true>(st, A, s.q, nullptr, s.v, s.q, sigma_part, tk, nullptr);
+  launch_pdl(k_sq_residual, nb, 256, st, n, (const double *)s.v, s.r, (const double *)sigma_part,
+             slots, rr_part, sc);
+  h.vcycle(s.r, s.v, s.r, nullptr);
+  launch_pdl(k_sq_step, nb, 256, st, n, (const double *)s.v, (const double *)rr_part,
+             vcycle_dot_partials(h), slots, part, tk, sc, handle, use_cond);
   launch_pdl(k_sq_update, nb, 256, st, n, (const double *)s.v, s.d, s.q, s.x,
              (const double *)sc);
 }
@@ -237,6 +247,9 @@ void sqmr_solve(Hier &h, const DMat *op, const double *b_h, double *x_h, int itm
   double *sc = s.sc.get(), *part = s.part.get();
   unsigned *tk = s.tickets.get();
   s.tickets.zero(st);
+  // partials past the producers' grids are zero
+  s.part.zero(st);
+  zero_vcycle_partials(h);
   CHRONOS_CUDA(cudaMemcpyAsync(s.b, b_h, sizeof(double) * n, cudaMemcpyHostToDevice, st));
   CHRONOS_CUDA(cudaMemcpyAsync(s.x, x_h, sizeof(double) * n, cudaMemcpyHostToDevice, st));
   CHRONOS_CUDA(cudaMemsetAsync(s.d, 0, sizeof(double) * n, st));
