@@ -100,7 +100,7 @@ __device__ __forceinline__ void group_reduce(double (&v)[K], int p, int b0, int 
 
 // Per-problem scalars: sc[p * GS_COUNT + GS_*].
 enum GroupScalar {
-  GS_BNORM = 0, GS_RR, GS_PTAP, GS_ALPHA, GS_PRES_AXP, GS_RESITER, GS_ITER, GS_ACTIVE,
+  GS_BNORM = 0, GS_RR, GS_PTAP, GS_RESITER, GS_ITER, GS_ACTIVE,
   GS_BREAKDOWN, GS_COUNT = 10
 };
 // Global words: g[0] problems active at the start of the current x/res update,
@@ -163,56 +163,44 @@ __global__ void k_group_init(int np, double *sc, unsigned *g, double tol, double
   }
 }
 
-// pres'axp per problem (beta of PCG_CJ.m:40).
-struct FinStore {
-  double *sc;
-  int which;
-  __device__ void operator()(int p, const double *t) const { sc[p * GS_COUNT + which] = t[0]; }
-};
-
+// The partials of pres'axp (beta of PCG_CJ.m:40), added by k_group_p_update: a
+// problem's finished sum ended the kernel with a fence, a ticket and a round of
+// loads behind its last block.  With these and the outer product's sums left to
+// their consumers: 6 problems of 11^3-20^3 1.025 -> 0.98 ms, 12 of 11^3-40^3 4.00 ->
+// 3.92 ms, 24 of 20^3-48^3 the same.
 __global__ void __launch_bounds__(256)
 k_group_dot(int np, const int *__restrict__ bstart, const int *__restrict__ rstart,
             const double *__restrict__ a, const double *__restrict__ c, double *part,
-            unsigned *tickets, double *sc) {
+            const double *__restrict__ sc) {
   pdl_begin();
   GROUP_BLOCK_SETUP
   if (sc[p * GS_COUNT + GS_ACTIVE] == 0.0) return;
   double v[1] = {0.0};
   for (int i = r0 + lb * blockDim.x + threadIdx.x; i < r1; i += nbp * blockDim.x)
     v[0] += a[i] * c[i];
-  group_reduce<1>(v, p, b0, nbp, part, tickets, FinStore{sc, GS_PRES_AXP});
+  block_partials<1>(v, part);
 }
 
 // p = pres (first iteration) or pres + beta p, beta = -(pres'axp)/ptap.
 __global__ void __launch_bounds__(256)
 k_group_p_update(int np, const int *__restrict__ bstart, const int *__restrict__ rstart,
                  const double *__restrict__ pres, double *__restrict__ pv,
-                 const double *__restrict__ sc) {
+                 const double *__restrict__ part, const double *__restrict__ sc) {
   pdl_begin();
   GROUP_BLOCK_SETUP
   const double *s = sc + p * GS_COUNT;
   if (s[GS_ACTIVE] == 0.0) return;
   const bool first = s[GS_ITER] < 0.5;
-  const double beta = first ? 0.0 : -s[GS_PRES_AXP] / s[GS_PTAP];
+  const double ptap = s[GS_PTAP];
+  double t[1];
+  sum_partials<1>(part + b0, nbp, t);
+  const double beta = first ? 0.0 : -t[0] / ptap;
   for (int i = r0 + lb * blockDim.x + threadIdx.x; i < r1; i += nbp * blockDim.x)
     pv[i] = first ? pres[i] : pres[i] + beta * pv[i];
 }
 
-struct FinAlphaGroup {
-  double *sc;
-  __device__ void operator()(int p, const double *t) const {
-    double *s = sc + p * GS_COUNT;
-    s[GS_PTAP] = t[0];
-    if (!(t[0] > 0.0) || !isfinite(t[1])) {
-      s[GS_BREAKDOWN] = 1.0;
-      s[GS_ALPHA] = 0.0;
-    } else {
-      s[GS_ALPHA] = t[1] / t[0];
-    }
-  }
-};
-
-// axp = A p on the problem's rows of the stacked FP64 operator, p'axp, p'res.
+// axp = A p on the problem's rows of the stacked FP64 operator, the partials of
+// p'axp and p'res.
 template <int L, bool I16>
 __global__ void __launch_bounds__(256)
 k_group_spmv(int np, const int *__restrict__ bstart, const int *__restrict__ rstart,
@@ -220,7 +208,7 @@ k_group_spmv(int np, const int *__restrict__ bstart, const int *__restrict__ rst
              const int *__restrict__ cbase, const uint16_t *__restrict__ c16,
              const double *__restrict__ v, const double *__restrict__ pv,
              const double *__restrict__ res, double *__restrict__ axp, double *part,
-             unsigned *tickets, double *sc) {
+             const double *__restrict__ sc) {
   pdl_begin();
   GROUP_BLOCK_SETUP
   if (sc[p * GS_COUNT + GS_ACTIVE] == 0.0) return;
@@ -245,7 +233,7 @@ k_group_spmv(int np, const int *__restrict__ bstart, const int *__restrict__ rst
       d[1] += pi * res[row];
     }
   }
-  group_reduce<2>(d, p, b0, nbp, part, tickets, FinAlphaGroup{sc});
+  block_partials<2>(d, part);
 }
 
 // x += alpha p; res -= alpha axp; ||res||^2; stop test per problem, and the
@@ -256,15 +244,16 @@ struct FinResidualGroup {
   GroupCtl c;
   cudaGraphConditionalHandle handle;
   int use_cond;
+  bool broke;
   __device__ void operator()(int p, const double *t) const {
     double *s = c.sc + p * GS_COUNT;
     // problems active when this update began; only the last of their
     // finalisers changes it, after every one of them has taken a ticket
     const unsigned nact = *(volatile unsigned *)c.g;
-    const double bnorm = s[GS_BNORM], it0 = s[GS_ITER], broke = s[GS_BREAKDOWN];
+    const double bnorm = s[GS_BNORM], it0 = s[GS_ITER];
     const double resiter = sqrt(t[0]) / bnorm;
     const double it = it0 + 1.0;
-    const bool stop = resiter < c.tol || it >= c.itmax || broke != 0.0 || !isfinite(resiter);
+    const bool stop = resiter < c.tol || it >= c.itmax || broke || !isfinite(resiter);
     s[GS_ITER] = it;
     s[GS_RESITER] = resiter;
     if (stop) {
@@ -285,14 +274,21 @@ struct FinResidualGroup {
 __global__ void __launch_bounds__(256)
 k_group_xr_update(int np, const int *__restrict__ bstart, const int *__restrict__ rstart,
                   double *__restrict__ x, double *__restrict__ res,
-                  const double *__restrict__ pv, const double *__restrict__ axp, double *part,
-                  unsigned *tickets, GroupCtl c, cudaGraphConditionalHandle handle,
+                  const double *__restrict__ pv, const double *__restrict__ axp,
+                  const double *__restrict__ spmv_part, double *part, unsigned *tickets, GroupCtl c, cudaGraphConditionalHandle handle,
                   int use_cond) {
   pdl_begin();
   GROUP_BLOCK_SETUP
-  const double *s = c.sc + p * GS_COUNT;
+  double *s = c.sc + p * GS_COUNT;
   if (s[GS_ACTIVE] == 0.0) return;
-  const double alpha = s[GS_ALPHA];
+  double t[2];
+  sum_partials<2>(spmv_part + 2 * (size_t)b0, nbp, t);
+  const bool broke = !(t[0] > 0.0) || !isfinite(t[1]);     // p'Ap <= 0 or NaN
+  const double alpha = broke ? 0.0 : t[1] / t[0];
+  if (lb == 0 && threadIdx.x == 0) {
+    s[GS_PTAP] = t[0];
+    if (broke) s[GS_BREAKDOWN] = 1.0;
+  }
   double v[1] = {0.0};
   for (int i = r0 + lb * blockDim.x + threadIdx.x; i < r1; i += nbp * blockDim.x) {
     x[i] += alpha * pv[i];
@@ -300,7 +296,7 @@ k_group_xr_update(int np, const int *__restrict__ bstart, const int *__restrict_
     res[i] = ri;
     v[0] += ri * ri;
   }
-  group_reduce<1>(v, p, b0, nbp, part, tickets, FinResidualGroup{c, handle, use_cond});
+  group_reduce<1>(v, p, b0, nbp, part, tickets, FinResidualGroup{c, handle, use_cond, broke});
 }
 
 // Batched coarsest solves x = W b: a warp per row of every problem whose
@@ -523,7 +519,7 @@ static std::unique_ptr<GroupSolve> build_stack(const std::vector<std::unique_ptr
   const size_t n0 = (size_t)g.nrows;
   g.x.alloc(n0); g.res.alloc(n0); g.p.alloc(n0); g.axp.alloc(n0); g.pres.alloc(n0); g.b.alloc(n0);
   g.sc.alloc((size_t)np * GS_COUNT);
-  g.part.alloc((size_t)g.nblocks * 2);
+  g.part.alloc((size_t)g.nblocks * 4);        // the product's two sums, the dot, the norm
   g.tickets.alloc(np);
   g.tickets.zero(st);
   g.ctl.alloc(4);
@@ -668,14 +664,14 @@ static void group_spmv(GroupSolve &g, const double *pv, const double *res, doubl
       launch_pdl(k_group_spmv<LL, true>, grid, 256, g.st, g.np, (const int *)g.bstart.get(),  \
                  (const int *)g.rstart.get(), (const int *)A.rp.get(), (const int *)A.ci.get(),\
                  (const int *)A.cbase.get(), (const uint16_t *)A.c16.get(),                   \
-                 (const double *)A.v64.get(), pv, res, axp, g.part.get(), g.tickets.get(),    \
-                 g.sc.get());                                                                 \
+                 (const double *)A.v64.get(), pv, res, axp, g.part.get(),                     \
+                 (const double *)g.sc.get());                                                 \
     else                                                                                      \
       launch_pdl(k_group_spmv<LL, false>, grid, 256, g.st, g.np, (const int *)g.bstart.get(), \
                  (const int *)g.rstart.get(), (const int *)A.rp.get(), (const int *)A.ci.get(),\
                  (const int *)A.cbase.get(), (const uint16_t *)A.c16.get(),                   \
-                 (const double *)A.v64.get(), pv, res, axp, g.part.get(), g.tickets.get(),    \
-                 g.sc.get());                                                                 \
+                 (const double *)A.v64.get(), pv, res, axp, g.part.get(),                     \
+                 (const double *)g.sc.get());                                                 \
     break;
   switch (A.lanes) {
     CHRONOS_GS_CASE(1)
@@ -696,15 +692,16 @@ static void group_capture_iteration(GroupSolve &g, cudaGraphConditionalHandle ha
   else group_vcycle<double>(g);
   const int grid = g.nblocks;
   const int *bs = g.bstart.get(), *rs = g.rstart.get();
+  double *dot_part = g.part.get() + 2 * (size_t)g.nblocks;
   launch_pdl(k_group_dot, grid, 256, st, g.np, bs, rs, (const double *)g.pres.get(),
-             (const double *)g.axp.get(), g.part.get(), g.tickets.get(), g.sc.get());
+             (const double *)g.axp.get(), dot_part, (const double *)g.sc.get());
   launch_pdl(k_group_p_update, grid, 256, st, g.np, bs, rs, (const double *)g.pres.get(),
-             g.p.get(), (const double *)g.sc.get());
+             g.p.get(), (const double *)dot_part, (const double *)g.sc.get());
   group_spmv(g, g.p.get(), g.res.get(), g.axp.get());
   GroupCtl c{g.sc.get(), g.ctl.get(), tol, (double)itmax};
   launch_pdl(k_group_xr_update, grid, 256, st, g.np, bs, rs, g.x.get(), g.res.get(),
-             (const double *)g.p.get(), (const double *)g.axp.get(), g.part.get(),
-             g.tickets.get(), c, handle, use_cond);
+             (const double *)g.p.get(), (const double *)g.axp.get(), (const double *)g.part.get(),
+             g.part.get() + 3 * (size_t)g.nblocks, g.tickets.get(), c, handle, use_cond);
 }
 
 void group_solve(GroupSolve &g, const std::vector<const double *> &b_h,
