@@ -358,6 +358,19 @@ __device__ __forceinline__ double block_sum(double v, double *smem32) {
 // GPU (release before, acquire after a ticket).
 __device__ __forceinline__ void fence_gpu() { asm volatile("fence.acq_rel.gpu;" ::: "memory"); }
 
+// Lets a kernel's blocks have as much dynamic shared memory as the device gives a
+// block.  The limit belongs to the process: set to each call's own size,
+// concurrent setups lowered it under one another's launches.
+template <typename Kernel> inline void allow_dynamic_smem(Kernel kern) {
+  int dev = 0, most = 0;
+  cudaFuncAttributes fa{};
+  CHRONOS_CUDA(cudaGetDevice(&dev));
+  CHRONOS_CUDA(cudaDeviceGetAttribute(&most, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev));
+  CHRONOS_CUDA(cudaFuncGetAttributes(&fa, kern));
+  CHRONOS_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                    most - (int)fa.sharedSizeBytes));
+}
+
 // ---- programmatic dependent launch ------------------------------------------
 // Kernels of the solve loop begin with pdl_begin(): griddepcontrol.wait
 // returns once the preceding kernel of the stream has completed and its

@@ -941,14 +941,12 @@ void emin_pattern_device(int kpow, int n, int nc, const EminStrength &str, const
     const int grid = (int)std::max<int64_t>(
         1, std::min<int64_t>(ceil_div(n, wpb), (int64_t)num_sms() * 16));
     if (from_a) {
-      CHRONOS_CUDA(cudaFuncSetAttribute(k_emin_pattern<true>,
-                                        cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+      allow_dynamic_smem(k_emin_pattern<true>);
       k_emin_pattern<true><<<grid, 32 * wpb, smem, st>>>(
           n, srp_d, sci_d, sv_d, diag.get(), str.tau, crp, cci, cv, p0rp.get(), p0ci.get(),
           fcd.get(), nnzr, last ? 1 : 0, table, ooff.get(), ocid.get(), ov.get(), olen.get());
     } else {
-      CHRONOS_CUDA(cudaFuncSetAttribute(k_emin_pattern<false>,
-                                        cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+      allow_dynamic_smem(k_emin_pattern<false>);
       k_emin_pattern<false><<<grid, 32 * wpb, smem, st>>>(
           n, srp_d, sci_d, sv_d, nullptr, 0.0, crp, cci, cv, p0rp.get(), p0ci.get(), fcd.get(),
           nnzr, last ? 1 : 0, table, ooff.get(), ocid.get(), ov.get(), olen.get());
@@ -1145,8 +1143,7 @@ HostCSR emin_device(const EminParams &prm, int n, int nc, const int *arp, const 
   const size_t kp_warp = (size_t)std::max(mmax, 1) * 8 + (size_t)hslots * 8;
   const int kp_wpb = (int)std::max<size_t>(1, std::min<size_t>(kEminWarps, (200u << 10) / kp_warp));
   const size_t kp_smem = kp_warp * kp_wpb;
-  CHRONOS_CUDA(cudaFuncSetAttribute(k_emin_kp, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                    (int)kp_smem));
+  allow_dynamic_smem(k_emin_kp);
   const int kp_grid = (int)std::max<int64_t>(
       1, std::min<int64_t>(ceil_div(n, kp_wpb), (int64_t)num_sms() * 16));
   const int wg = warp_grid(n);
