@@ -1379,12 +1379,11 @@ void dense_inverse_from_chol(int n, const double *L, double *W, cudaStream_t st)
   CHRONOS_CUDA(cudaStreamSynchronize(st));
 }
 
-// x = W b: NT threads a row, at most eight loads of W each up
-// to 8 NT columns and all of them in flight.  With a warp a row and four in
-// flight the product was a chain of batches on 8 warps an SM: 1216 rows of the
-// folded tail of elasticity 45^3 (11.8 MB, from L2) 11.5 us, now 6.1; 208 rows 3.6
-// and 2.5 us.  (Rows of
-// many small systems at once, k_group_dense, fill the GPU with a warp each.)
+// x = W b: NT threads a row, at most eight loads of W each up to 8 NT columns and
+// all of them in flight.  With a warp a row and four in flight the product was a
+// chain of batches on 8 warps an SM: 1212 rows of the folded tail of elasticity
+// 45^3 (11.8 MB, from L2) 11.5 us, now 6.1; 208 rows 3.6 and 2.5 us.  (Rows of many
+// small systems at once, k_group_dense, fill the GPU with a warp each.)
 template <int NT, typename TI, typename TO>
 __global__ void __launch_bounds__(NT < 128 ? 128 : NT)
 k_dense_matvec(int n, const double *__restrict__ W, const TI *__restrict__ b,

@@ -537,7 +537,9 @@ k_csrh_apply(int n, const int *__restrict__ rp, const int *__restrict__ ci,
 // A block of W threads per row (DMat::wide): the levels that end a hierarchy, and
 // their folded restrictions, have a few thousand rows or less of hundreds to
 // thousands of entries; with a warp per row a level's time is one row's chain of
-// batches.  The partial sums meet in warp order.
+// batches.  The partial sums meet in warp order.  With it and the
+// measured choice: PCG elasticity 24^3 FP64 (its folded restriction: 205 rows, 4.9 us a
+// launch) 2990 -> 2890 us, elasticity 33^3 FP32 88.0 -> 85.5 us per iteration.
 template <typename VT, typename XT, typename ZT, typename YT, int W, int MODE, bool DOT, bool I16>
 __global__ void __launch_bounds__(W)
 k_csr_wide(int n, const int *__restrict__ rp, const int *__restrict__ ci,
