@@ -100,6 +100,46 @@ inline bool wait_lib_streams(int device) {
   return all;
 }
 
+// Waits for everything queued on a device, the work of streams that are not the
+// library's too, and beside a capture (where cudaDeviceSynchronize is not allowed):
+// cudaFree of memory from cudaMalloc is that wait.  The word is taken when the
+// need for the wait arises, so that a full device cannot prevent it.
+class DeviceWait {
+ public:
+  DeviceWait() = default;
+  ~DeviceWait() { wait(); }
+  DeviceWait(const DeviceWait &) = delete;
+  DeviceWait &operator=(const DeviceWait &) = delete;
+  bool armed() const { return armed_; }
+  void arm() {
+    if (armed_) return;
+    armed_ = true;
+    Relaxed mode;
+    if (cudaMalloc(&word_, sizeof(int)) != cudaSuccess) {
+      cudaGetLastError();
+      word_ = nullptr;
+    }
+  }
+  void wait() {
+    if (!armed_) return;
+    Relaxed mode;
+    const cudaError_t e = word_ ? cudaFree(word_) : cudaDeviceSynchronize();
+    if (e != cudaSuccess) cudaGetLastError();
+    word_ = nullptr;
+    armed_ = false;
+  }
+
+ private:
+  // cudaMalloc and cudaFree allowed on this thread whatever is being captured
+  struct Relaxed {
+    cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+    Relaxed() { cudaThreadExchangeStreamCaptureMode(&mode); }
+    ~Relaxed() { cudaThreadExchangeStreamCaptureMode(&mode); }
+  };
+  void *word_ = nullptr;
+  bool armed_ = false;
+};
+
 // Device memory comes from one memory pool per device, owned by the library
 // (the default pool's settings are the host program's).  A setup makes and
 // drops hundreds of buffers, and mapping and unmapping their pages was most of
@@ -110,7 +150,9 @@ inline bool wait_lib_streams(int device) {
 // at once, all of it before an allocation is given up (and at exit).
 // Allocations and frees are ordered on a stream of the pool's own.  A free
 // waits for the library's streams first (cudaFree waits for the device), so
-// memory never returns to the pool while queued work may still use it.
+// memory never returns to the pool while work that the library queued may still
+// use it; a handle that a caller's capture took in waits for the device before
+// it frees, since replays run on the caller's streams (Hier::replays).
 constexpr int64_t kPoolKeepBytes = (int64_t)512 << 20;
 struct DevicePool {
   int device = -1;

@@ -67,6 +67,7 @@ PcgState::~PcgState() {
 
 Hier::~Hier() {
   if (st) cudaStreamSynchronize(st);
+  replays.wait();
   levels.clear();
   drop_pcg_graph(pcg);
   if (ev_in) cudaEventDestroy(ev_in);
@@ -84,7 +85,10 @@ CallerStream::CallerStream(Hier &h, void *stream)
   std::unique_lock<std::mutex> lk(lib_streams().mu, std::defer_lock);
   cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
   if (cudaStreamIsCapturing(caller_, &cap) != cudaSuccess) cudaGetLastError();
-  if (cap != cudaStreamCaptureStatusNone) lk.lock();
+  if (cap != cudaStreamCaptureStatusNone) {
+    h_.replays.arm();
+    lk.lock();
+  }
   CHRONOS_CUDA(cudaStreamWaitEvent(h_.st, h_.ev_in, 0));
 }
 

@@ -134,6 +134,9 @@ struct Hier {
   bool use_user_op = false;
   // events that order st after a caller's stream and the caller's stream after st
   cudaEvent_t ev_in = nullptr, ev_out = nullptr;
+  // armed once a caller's capture took st in: its replays use the levels' buffers
+  // on the caller's streams, so the handle's end waits for the device
+  DeviceWait replays;
   ~Hier();
 
   const DMat &outer_A() const { return use_user_op ? user_op : levels[0].A; }

@@ -455,7 +455,9 @@ int chronos_vcycle(chronos_hier *h, const double *b_h, double *x_h, int nrhs, vo
  * CHRONOS_FP64 (double) or CHRONOS_FP32 (float).  An FP32 hierarchy reads and
  * writes float vectors directly (AMG_Vcycle.m:1-54 in FP32 end to end, the
  * coarsest solve in FP64 as always); an FP64 hierarchy runs on FP64 copies.
- * Work is ordered on stream with no host synchronisation. */
+ * Work is ordered on stream with no host synchronisation; the call may be part of
+ * a capture on stream.  chronos_hier_free then waits for the device, so replays
+ * queued before it run on the handle's memory; none may be queued after it. */
 int chronos_vcycle_dev(chronos_hier *h, int io_precision, const void *b_d, void *x_d, int nrhs,
                        void *stream);
 
