@@ -85,7 +85,8 @@ int chronos_batch_setup(const chronos_params *prm, int nprob, const int *n,
     // chronos_amg_setup builds; lane counts are tuned afterwards on a quiet
     // GPU: the grouped solve's stacked operators, or each problem's own for
     // the per-problem path.
-    DeferFrees defer_frees;          // no thread's free waits on the others' queued work
+    // no thread's free waits on the others' queued work
+    auto defer_frees = std::make_unique<DeferFrees>();
     bt->b.h.resize(nprob);
     const int hw = std::max(1, (int)std::thread::hardware_concurrency());
     const int nworkers = std::max(1, std::min({nprob, 8, std::max(1, hw / 2)}));
@@ -179,6 +180,9 @@ int chronos_batch_setup(const chronos_params *prm, int nprob, const int *n,
       bt->b.h[p] = b.finish(false);
       builders[p].reset();
     });
+    // what follows runs on this thread alone, and makes and drops the largest
+    // temporaries (stacks, folds)
+    defer_frees.reset();
     const double t3 = now_seconds();
     wall[0] = t1 - t0;
     wall[1] = t2 - t1;

@@ -234,8 +234,8 @@ class OnDevice {
 // queued kernels; and nothing can be waited for while a caller's capture holds a
 // handle's stream: such a buffer is kept until a later free.
 // Inside a DeferFrees scope (any thread) the buffers a DBuf
-// lets go of are kept -- never reused -- and freed when the outermost scope
-// ends, after one wait for the streams.  They stay counted in
+// lets go of are kept -- never reused -- and freed, after one wait for the
+// streams, when the outermost scope ends or an allocation would be refused.  They stay counted in
 // device_bytes_live() until then.
 struct DeferredFrees {
   struct Entry { void *p; int64_t bytes; DevicePool *pool; };
@@ -305,12 +305,19 @@ class DBuf {
     release();
     if (n == 0) return;
     const int64_t bytes = (int64_t)(n * sizeof(T)), cap = device_alloc_cap();
-    if (cap > 0 && device_bytes_live().load() + bytes > cap)
+    auto beyond_cap = [&] { return cap > 0 && device_bytes_live().load() + bytes > cap; };
+    // what was let go of and is still kept is given back before a refusal
+    if (beyond_cap()) flush_deferred_frees();
+    if (beyond_cap())
       throw Error(CHRONOS_ENOMEM, "allocation of " + std::to_string(bytes) +
                                       " bytes beyond CHRONOS_DEVICE_ALLOC_CAP");
     DevicePool &pool = device_pool();
     void *p = nullptr;
-    const cudaError_t e = pool.alloc(&p, n * sizeof(T));
+    cudaError_t e = pool.alloc(&p, n * sizeof(T));
+    if (e == cudaErrorMemoryAllocation) {
+      flush_deferred_frees();
+      e = pool.alloc(&p, n * sizeof(T));
+    }
     if (e != cudaSuccess) {
       cudaGetLastError();
       throw Error(CHRONOS_ENOMEM, "device allocation of " + std::to_string(n * sizeof(T)) +

@@ -60,3 +60,52 @@ def test_free_waits_for_replays(lib, beside_capture):
         torch.cuda.synchronize()
         assert torch.equal(y, want)
     other.close()
+
+
+def _child(tmp_path, code, cap=0):
+    """The last numbers that `code` prints in a process under a memory cap, None
+    where it ends with CHRONOS_ENOMEM."""
+    import os
+    import subprocess
+    import sys
+    root = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+    head = (f"import sys; sys.path.insert(0, {root!r})\n"
+            "import numpy as np\nimport chronoslab_b200 as cb\n"
+            "from chronoslab_b200 import problems as PB\n")
+    env = dict(os.environ, CHRONOS_TUNE_CACHE=str(tmp_path / "tune.txt"))
+    if cap:
+        env["CHRONOS_DEVICE_ALLOC_CAP"] = str(int(cap))
+    r = subprocess.run([sys.executable, "-c", head + code], env=env, timeout=600,
+                       capture_output=True, text=True)
+    if r.returncode:
+        assert cap and "ENOMEM" in r.stderr, r.stderr
+        return None
+    return [float(v) for v in r.stdout.split()]
+
+
+@pytest.mark.parametrize("grouped", [1])
+def test_batch_folding_gives_way_to_the_memory_cap(lib, tmp_path, grouped):
+    """Under the smallest CHRONOS_DEVICE_ALLOC_CAP (to 8 MB) at which a batch whose
+    levels are never folded (two presmoothing steps) sets up and solves, the
+    foldable batch does too."""
+    code = ("As = [PB.poisson7(k) for k in (20, 28, 36, 44)]\n"
+            "b = [np.ones(A.shape[0]) for A in As]\n"
+            "with cb.Batch(As, cb.params(precision=cb.CHRONOS_FP64, ntv=1, batch_grouped=%d,"
+            " nupre=%%d)) as h:\n"
+            "    held = cb.device_bytes()\n"
+            "    x, its, flags, _ = h.solve(b, 200, 1e-8)\n"
+            "res = max(np.linalg.norm(v - A @ y) / np.linalg.norm(v)"
+            " for A, v, y in zip(As, b, x))\n"
+            "print(held, res)\n") % grouped
+    full, lean = _child(tmp_path, code % 1)[0], _child(tmp_path, code % 2)[0]
+    assert full > lean
+    low, high = lean, lean + (320 << 20)
+    assert _child(tmp_path, code % 2, high)
+    while high - low > 8 << 20:
+        mid = (low + high) // 2
+        if _child(tmp_path, code % 2, mid):
+            high = mid
+        else:
+            low = mid
+    held, res = _child(tmp_path, code % 1, high)
+    assert res <= 1e-8
