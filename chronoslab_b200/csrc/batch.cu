@@ -197,8 +197,24 @@ int chronos_batch_setup(const chronos_params *prm, int nprob, const int *n,
                     "these problems need the per-problem batch path, which needs use_graph = 1");
     // the grouped solve tunes its stacked operators itself; the per-problem
     // path runs each problem's own operators
-    if (!bt->b.group)
-      for (auto &h : bt->b.h) tune_hierarchy(*h);
+    if (!bt->b.group) {
+      // folded if all of them can be and leave room for their solves (PCG's six
+      // vectors, its partials and two staged ones a problem)
+      int64_t solves = 0;
+      for (const auto &h : bt->b.h) solves += 64 * (int64_t)h->levels[0].n + (1 << 20);
+      bool folded = false;
+      try {
+        for (auto &h : bt->b.h) tune_hierarchy(*h);
+        folded = device_room(solves);
+      } catch (const Error &e) {
+        if (e.code != CHRONOS_ENOMEM) throw;
+      }
+      if (!folded) {
+        for (auto &h : bt->b.h)
+          for (auto &L : h->levels) L.fold.reset();
+        for (auto &h : bt->b.h) tune_hierarchy(*h, false);
+      }
+    }
     bt->b.wall[3] = now_seconds() - t3;
     bt->b.wall[4] = now_seconds() - t0;
     *out = bt.release();

@@ -3,6 +3,7 @@
 #pragma once
 
 #include <cuda_runtime.h>
+#include <algorithm>
 #include <atomic>
 #include <cstdint>
 #include <cstdio>
@@ -272,6 +273,19 @@ inline void flush_deferred_frees() {
     OnDevice on(synced->device);
     synced->trim();
   }
+}
+// Whether the device (and CHRONOS_DEVICE_ALLOC_CAP) has room for so many bytes more.
+inline bool device_room(int64_t bytes) {
+  flush_deferred_frees();
+  const int64_t cap = device_alloc_cap();
+  if (cap > 0 && device_bytes_live().load() + bytes > cap) return false;
+  size_t avail = 0, total = 0;
+  uint64_t held = 0, used = 0;
+  DevicePool &pool = device_pool();
+  CHRONOS_CUDA(cudaMemGetInfo(&avail, &total));
+  CHRONOS_CUDA(cudaMemPoolGetAttribute(pool.pool, cudaMemPoolAttrReservedMemCurrent, &held));
+  CHRONOS_CUDA(cudaMemPoolGetAttribute(pool.pool, cudaMemPoolAttrUsedMemCurrent, &used));
+  return (int64_t)avail + (int64_t)(held - std::min(used, held)) >= bytes;
 }
 class DeferFrees {
  public:

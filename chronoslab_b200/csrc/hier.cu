@@ -1428,14 +1428,26 @@ std::unique_ptr<Hier> build_hierarchy(const chronos_params &prm, HostCSR A0, int
 
 static void tune_operators(Hier &h);
 
-void tune_hierarchy(Hier &h) {
-  // folded where the memory for it is there
-  try {
-    build_folds(h);
-    tune_operators(h);
-    return;
-  } catch (const Error &e) {
-    if (e.code != CHRONOS_ENOMEM) throw;
+// Bytes that the solves take beside the hierarchy: a block of 16 columns, the
+// largest of them, has six FP64 vectors a column and four of the hierarchy's
+// precision on every level; PCG's six vectors and partials are less.
+static int64_t solve_bytes(const Hier &h) {
+  int64_t rows = 0;
+  for (const auto &L : h.levels) rows += L.n;
+  return 16 * (48 * (int64_t)h.levels[0].n + (h.precision == CHRONOS_FP32 ? 16 : 32) * rows) +
+         (8 << 20);
+}
+
+void tune_hierarchy(Hier &h, bool fold) {
+  // folded where the memory for it is there and still leaves the solves theirs
+  if (fold) {
+    try {
+      build_folds(h);
+      tune_operators(h);
+      if (device_room(solve_bytes(h))) return;
+    } catch (const Error &e) {
+      if (e.code != CHRONOS_ENOMEM) throw;
+    }
   }
   CHRONOS_CUDA(cudaStreamSynchronize(h.st));
   for (auto &L : h.levels) {

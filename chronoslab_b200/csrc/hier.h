@@ -278,7 +278,7 @@ class CallerStream {
 std::unique_ptr<Hier> build_hierarchy(const chronos_params &prm, HostCSR A,
                                       int ntv0, const double *TV0, bool tune = true,
                                       const ProlongFn *prolong = nullptr);
-void tune_hierarchy(Hier &h);
+void tune_hierarchy(Hier &h, bool fold = true);
 // Folds the levels for which that is the faster form (fold.cu); part of
 // tune_hierarchy.
 void build_folds(Hier &h);

@@ -83,7 +83,7 @@ def _child(tmp_path, code, cap=0):
     return [float(v) for v in r.stdout.split()]
 
 
-@pytest.mark.parametrize("grouped", [1])
+@pytest.mark.parametrize("grouped", [1, 0])
 def test_batch_folding_gives_way_to_the_memory_cap(lib, tmp_path, grouped):
     """Under the smallest CHRONOS_DEVICE_ALLOC_CAP (to 8 MB) at which a batch whose
     levels are never folded (two presmoothing steps) sets up and solves, the
@@ -109,3 +109,31 @@ def test_batch_folding_gives_way_to_the_memory_cap(lib, tmp_path, grouped):
             low = mid
     held, res = _child(tmp_path, code % 1, high)
     assert res <= 1e-8
+
+
+def test_folding_leaves_room_for_the_solves(lib, tmp_path):
+    """A cap that holds the folded hierarchy or a block solve, not both: both the
+    block solve and PCG run, as they do on the same operators never folded (two
+    presmoothing steps)."""
+    files = [str(tmp_path / f"pre{k}.chh") for k in (1, 2)]
+    full, lean = _child(tmp_path, (
+        "A = PB.poisson7(60)\nn = A.shape[0]\nout = []\n"
+        f"for k, f in zip((1, 2), {files!r}):\n"
+        "    with cb.Hierarchy(A, np.ones((n, 1)), cb.params(ntv=1, nupre=k,"
+        " precision=cb.CHRONOS_FP64)) as h: h.save(f)\n"
+        "    with cb.Hierarchy.load(f) as h: out.append(cb.device_bytes())\n"
+        "print(*out)\n"))
+    block = 8 * 216000 * (6 * 48 // 6 + 4 * 12)        # columns x (vectors of FP64 bytes)
+    fold = full - lean
+    assert 0 < fold < block
+    solve = ("A = PB.poisson7(60)\nn = A.shape[0]\n"
+             "with cb.Hierarchy.load(%r) as h:\n"
+             "    B = PB.uniform_rhs(n, 3, 8)\n"
+             "    X, its, flags, _ = h.pcg_block(B, tol=1e-8)\n"
+             "    x, it, _, flag, _ = h.pcg(B[:, 0].copy(), tol=1e-8)\n"
+             "print(max(flags), flag)\n")
+    # halfway into the room that the block solve shares with the folds; the lean
+    # hierarchy needs its load's own temporaries as well
+    cap = lean + block + fold // 2
+    assert _child(tmp_path, solve % files[1], cap) == [0, 0]
+    assert _child(tmp_path, solve % files[0], cap) == [0, 0]
