@@ -1166,14 +1166,18 @@ __device__ __forceinline__ void tile_gemm(int i0, int j0, int k0, int k1, LA la,
 
 // Panel [k0, k0 + nb): D receives the diagonal block's factor (32 x 32, column
 // by column; the other blocks of the grid still read A's), A the rows below it.
-// *info: the 1-based index of the first non-positive pivot.
+// info[0]: what the panels before it found; info[1], read by later launches only:
+// that, or the 1-based index of this panel's first non-positive pivot.
 __global__ void __launch_bounds__(256)
 k_chol_panel(int n, int k0, int nb, double *A, double *D, int *info) {
   constexpr unsigned FULL = 0xffffffffu;
   __shared__ double Ls[kCholNb][kCholNb + 1], Xs[kCholNb][65];
   __shared__ int bad;
   const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
-  if (*info) return;
+  if (*info) {
+    if (blockIdx.x == 0 && tid == 0) info[1] = *info;
+    return;
+  }
   const int r0 = k0 + nb + blockIdx.x * 64;
   for (int e = tid; e < nb * 64; e += 256) {
     const int i = e & 63, j = e >> 6;
@@ -1205,7 +1209,7 @@ k_chol_panel(int n, int k0, int nb, double *A, double *D, int *info) {
   __syncthreads();
   if (blockIdx.x == 0) {
     for (int e = tid; e < kCholNb * kCholNb; e += 256) D[e] = Ls[e & 31][e >> 5];
-    if (tid == 0 && bad) *info = bad;
+    if (tid == 0) info[1] = bad;
   }
   if (bad) return;
   // row x of the panel: x L' = a, lane j its entry j; a warp's eight rows together
@@ -1269,16 +1273,16 @@ int dense_cholesky_device(int n, double *A, cudaStream_t st) {
   if (n <= 0) return 0;
   const int np = ceil_div(n, kCholNb);
   DBuf<double> D((size_t)np * kCholNb * kCholNb);
-  DBuf<int> info(1);
+  DBuf<int> info((size_t)np + 1);               // before each panel, and after the last
   info.zero(st);
   for (int p = 0; p < np; ++p) {
     const int k0 = p * kCholNb, nb = std::min(kCholNb, n - k0), rest = n - k0 - nb;
     k_chol_panel<<<std::max(1u, ceil_div(rest, 64)), 256, 0, st>>>(
-        n, k0, nb, A, D.get() + (size_t)p * kCholNb * kCholNb, info.get());
+        n, k0, nb, A, D.get() + (size_t)p * kCholNb * kCholNb, info.get() + p);
     CHRONOS_CHECK_LAUNCH();
     if (rest > 0) {
       const unsigned t = ceil_div(rest, 64);
-      k_chol_update<<<dim3(t, t), 256, 0, st>>>(n, k0, k0 + nb, A, info.get());
+      k_chol_update<<<dim3(t, t), 256, 0, st>>>(n, k0, k0 + nb, A, info.get() + p + 1);
       CHRONOS_CHECK_LAUNCH();
     }
   }
@@ -1286,7 +1290,7 @@ int dense_cholesky_device(int n, double *A, cudaStream_t st) {
                   st>>>(n, A, D.get());
   CHRONOS_CHECK_LAUNCH();
   int h = 0;
-  CHRONOS_CUDA(cudaMemcpyAsync(&h, info.get(), sizeof(int), cudaMemcpyDeviceToHost, st));
+  CHRONOS_CUDA(cudaMemcpyAsync(&h, info.get() + np, sizeof(int), cudaMemcpyDeviceToHost, st));
   CHRONOS_CUDA(cudaStreamSynchronize(st));
   return h;
 }

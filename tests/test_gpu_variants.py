@@ -424,3 +424,22 @@ def test_folding_gives_way_to_the_memory_cap(lib, tmp_path):
             low = mid
     held, rel = child(solve % files[1], high)
     assert held < full and rel <= 1e-8
+
+
+@pytest.mark.parametrize("first", [1, 31, 32, 33, 64, 65, 1000, 2430, 2500])
+def test_dense_cholesky_names_the_first_bad_pivot(lib, first):
+    """A matrix of many panel blocks with two non-positive pivots: refused with the
+    first one's number (every block of a launch sees the same flag), and the next
+    factorisation is untouched."""
+    n = 2500
+    rng = np.random.default_rng(first)
+    A = np.diag(rng.uniform(1.0, 2.0, n))
+    A[1:, 0] = A[0, 1:] = 0.01                       # diagonally dominant, L one full column
+    bad = A.copy()
+    for k in {first, min(first + 40, n)}:
+        bad[k - 1, k - 1] = -1.0
+    with pytest.raises(cb.ChronosError, match=f"pivot {first}$") as e:
+        cb.dense_chol(bad)
+    assert e.value.code == -4
+    L = cb.dense_chol(A)
+    assert np.abs(L @ L.T - A).max() <= 4 * n * 2.2e-16 * np.abs(A).max()
