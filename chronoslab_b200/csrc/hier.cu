@@ -923,6 +923,7 @@ static void alloc_vectors(Level &L, int precision, cudaStream_t st) {
   if (precision == CHRONOS_FP32) {
     L.b32.alloc(n); L.x32.alloc(n); L.r32.alloc(n); L.t32.alloc(n);
     L.b32.zero(st); L.x32.zero(st); L.r32.zero(st); L.t32.zero(st);
+    if (L.coarsest) L.t64.alloc(n);      // a caller's FP64 vector, see vcycle_level
   } else {
     L.b64.alloc(n); L.x64.alloc(n); L.r64.alloc(n); L.t64.alloc(n);
     L.b64.zero(st); L.x64.zero(st); L.r64.zero(st); L.t64.zero(st);
@@ -1710,6 +1711,12 @@ static void vcycle_level(Hier &h, int l, const BT *b, OT *out, const double *dw,
   if (dw && !dot_out) part += kDotPartials;
   unsigned *tick = h.pcg.tickets.get();
   if (L.coarsest) {
+    // every row of the product reads all of b: in place, or overlapping, from a copy
+    if (TOP && overlap(b, out, n)) {
+      BT *copy = reinterpret_cast<BT *>(L.t64.get());
+      CHRONOS_CUDA(cudaMemcpyAsync(copy, b, sizeof(BT) * n, cudaMemcpyDeviceToDevice, st));
+      b = copy;
+    }
     dense_matvec<BT, OT>(n, L.W.get(), b, out, st);
     if (TOP && dw) {
       launch_pdl(k_dot_store, std::min(num_sms() * 4, (int)ceil_div(n, 256)), 256, st, n,

@@ -137,3 +137,32 @@ def test_folding_leaves_room_for_the_solves(lib, tmp_path):
     cap = lean + block + fold // 2
     assert _child(tmp_path, solve % files[1], cap) == [0, 0]
     assert _child(tmp_path, solve % files[0], cap) == [0, 0]
+
+
+@pytest.mark.parametrize("prec,io", [("fp64", "float64"), ("fp32", "float64"),
+                                     ("fp32", "float32"), ("fp64", "float32")])
+@pytest.mark.parametrize("nx", [5, 9, 12])
+@pytest.mark.parametrize("shift", [0, 1, 16, -16])
+def test_single_level_vcycle_in_place(lib, prec, io, nx, shift):
+    """b and x the same device vector, or overlapping, where the cycle is one dense
+    product: the bits of separate vectors."""
+    import torch
+    A = PB.poisson7(nx)
+    n = A.shape[0]
+    ip = cb.CHRONOS_FP64 if io == "float64" else cb.CHRONOS_FP32
+    with cb.Hierarchy(A, np.ones((n, 1)), cb.params(
+            precision=cb.CHRONOS_FP64 if prec == "fp64" else cb.CHRONOS_FP32, ntv=1,
+            nLevMax=1)) as h:
+        assert h.nlevels == 1
+        b = torch.from_numpy(np.random.default_rng(3).standard_normal(n)).to(
+            "cuda", getattr(torch, io))
+        x = torch.empty_like(b)
+        h.vcycle_dev(b.data_ptr(), x.data_ptr(), ip)
+        both = torch.zeros(n + abs(shift), dtype=b.dtype, device="cuda")
+        at, to = max(0, -shift), max(0, shift)
+        both[at:at + n] = b
+        torch.cuda.synchronize()
+        h.vcycle_dev(both.data_ptr() + at * both.element_size(),
+                     both.data_ptr() + to * both.element_size(), ip)
+        torch.cuda.synchronize()
+        assert torch.equal(both[to:to + n], x)
