@@ -252,7 +252,7 @@ constexpr int kSellLongRow = 32;
 
 // Builds the sliced ELL form (DMat::use_sell) from the matrix's final values.
 // Returns false (nothing attached) when the slot count does not fit int32.
-static bool build_sell(DMat &m, bool fp32, cudaStream_t st) {
+static bool build_sell(DMat &m, cudaStream_t st) {
   const int n = m.nrows;
   const std::vector<int> ci = m.ci.to_host(st);
   const std::vector<double> v = m.v64.to_host(st);
@@ -312,7 +312,7 @@ static bool build_sell(DMat &m, bool fp32, cudaStream_t st) {
   if (fits16) { m.s_c16.upload(s16, st); m.s_ci.release(); }
   else { m.s_ci.upload(sci, st); m.s_c16.release(); }
   m.s_v64.upload(sv, st);
-  if (fp32) {
+  if (m.v32.size() > 0) {                  // in every precision that the matrix holds
     m.s_v32.alloc(sv.size());
     convert_f64_to_f32((int64_t)sv.size(), m.s_v64.get(), m.s_v32.get(), st);
   }
@@ -388,6 +388,11 @@ void tune_store_locked(const TuneKey &k, int L) {
 
 void autotune_lanes(DMat &m, bool fp32, cudaStream_t st, int format) {
   if (m.nrows <= 0) return;
+  // a matrix tuned before (level 1's, again in FP64) starts from its rows: what an
+  // earlier decision built would be timed in place of the candidates, and would
+  // leave out the long rows of its own threshold
+  drop_sell(m);
+  m.wide = false;
   // 'H': the hybrid CSR kernel (k_csrh_apply); the index width is part of the
   // shape.  A cached value is lanes + 100 * form (decoded at the end).
   int maxrow = 0;
@@ -450,7 +455,7 @@ void autotune_lanes(DMat &m, bool fp32, cudaStream_t st, int format) {
                        m.ncols, (long long)m.nnz, cand, t / 4);
         if (t < best) { best = t; L = cand; }
       }
-      if (format == 0 && (double)m.nnz <= 16.0 * m.nrows && build_sell(m, fp32, st)) {
+      if (format == 0 && (double)m.nnz <= 16.0 * m.nrows && build_sell(m, st)) {
         m.use_sell = true;
         set_long_rows(m, kSellLongRow, st);
         const float t = time_it();
@@ -480,7 +485,7 @@ void autotune_lanes(DMat &m, bool fp32, cudaStream_t st, int format) {
   const int lanes = L % 100;
   if (format == 1) form = 0;
   if (format == 2 && form == 0 && (double)m.nnz <= 16.0 * m.nrows) form = 1;
-  if (form == 1 && build_sell(m, fp32, st)) {
+  if (form == 1 && build_sell(m, st)) {
     m.use_sell = true;
     m.lanes = lanes;
     set_long_rows(m, kSellLongRow, st);
@@ -1483,7 +1488,7 @@ static void tune_operators(Hier &h) {
     if (F) tune_fold(*F, fp32, h.st);
   }
   // the level-1 FP64 operator of the outer PCG
-  if (fp32 && h.prm.exact_outer) autotune_lanes(h.levels[0].A, false, h.st);
+  if (fp32 && h.prm.exact_outer) autotune_lanes(h.levels[0].A, false, h.st, fmt);
   CHRONOS_CUDA(cudaStreamSynchronize(h.st));
 }
 

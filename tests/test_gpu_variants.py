@@ -443,3 +443,57 @@ def test_dense_cholesky_names_the_first_bad_pivot(lib, first):
     assert e.value.code == -4
     L = cb.dense_chol(A)
     assert np.abs(L @ L.T - A).max() <= 4 * n * 2.2e-16 * np.abs(A).max()
+
+
+@pytest.mark.parametrize("first", [8, 101, 108])
+@pytest.mark.parametrize("second", [1, 8, 108])
+def test_second_tuning_of_the_finest_operator(lib, tmp_path, first, second):
+    """FP32 hierarchy with the exact outer product: the finest operator's storage is
+    chosen twice, for FP32 and for FP64 (the decisions set here: lanes, + 100 for
+    sliced ELL, which leaves rows above 32 entries to whole warps).  Whatever is
+    chosen, the cycle is the FP64 hierarchy's to FP32 rounding and the solve
+    converges."""
+    import os
+    import subprocess
+    import sys
+    root = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+    A = _poisson_with_long_rows()
+    longest = int(np.diff(A.indptr).max())
+    assert longest > 32 and A.nnz <= 16 * A.shape[0]
+    tune = tmp_path / "tune.txt"
+    tune.write_text("".join(
+        f"v2 {kind} {A.shape[0]} {A.nnz} {A.shape[1]} {fp32} {longest} {first if fp32 else second}\n"
+        for kind in "hH" for fp32 in (0, 1)))
+    sp.save_npz(tmp_path / "A.npz", A)
+    code = (f"import sys; sys.path.insert(0, {root!r})\n"
+            "import numpy as np, scipy.sparse as sp\nimport chronoslab_b200 as cb\n"
+            f"A = sp.csr_matrix(sp.load_npz({str(tmp_path / 'A.npz')!r}))\nn = A.shape[0]\n"
+            "b = np.random.default_rng(1).standard_normal(n)\n"
+            "prm = dict(ntv=1, nupre=2, maxCoarseSZ=200)\n"
+            "with cb.Hierarchy(A, np.ones((n, 1)), cb.params(precision=cb.CHRONOS_FP32,"
+            " exact_outer=1, **prm)) as h, cb.Hierarchy(A, np.ones((n, 1)),"
+            " cb.params(precision=cb.CHRONOS_FP64, spmv_format=1, **prm)) as h64:\n"
+            "    x, y = h.vcycle(b), h64.vcycle(b)\n"
+            "    z, it, _, flag, _ = h.pcg(b, tol=1e-8)\n"
+            "print(np.linalg.norm(x - y) / np.linalg.norm(y),"
+            " np.linalg.norm(b - A @ z) / np.linalg.norm(b), flag)\n")
+    r = subprocess.run([sys.executable, "-c", code], env=dict(os.environ, CHRONOS_TUNE_CACHE=str(tune)),
+                       timeout=600, capture_output=True, text=True)
+    assert r.returncode == 0, r.stderr
+    err, res, flag = [float(v) for v in r.stdout.split()]
+    assert err <= 2e-5 and res <= 1e-8 and flag == 0
+
+
+def _poisson_with_long_rows():
+    """poisson7(14) with five rows of 60 further weak couplings."""
+    from chronoslab_b200 import problems as PB
+    A = sp.lil_matrix(PB.poisson7(14))
+    rng = np.random.default_rng(8)
+    for i in (3, 700, 1301, 2000, 2743):
+        for j in rng.choice(2744, 60, replace=False):
+            if i != j:
+                A[i, j] = A[j, i] = -0.01
+    A = sp.csr_matrix(A)
+    A = sp.csr_matrix(A + sp.identity(2744))
+    A.sort_indices()
+    return A
