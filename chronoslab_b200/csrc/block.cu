@@ -586,8 +586,9 @@ static void block_solve(Hier &h, int m, const BlockIn &B, const double *X0_h, do
   cudaStream_t st = h.st;
   auto &sp = h.block;
   if (!sp || sp->K != K) {
-    sp = std::make_shared<BlockState>();
-    BlockState &s = *sp;
+    sp.reset();
+    auto made = std::make_shared<BlockState>();    // the handle's once it is complete
+    BlockState &s = *made;
     s.K = K;
     s.n = h.levels[0].n;
     const bool fp32 = h.precision == CHRONOS_FP32;
@@ -608,6 +609,7 @@ static void block_solve(Hier &h, int m, const BlockIn &B, const double *X0_h, do
     s.part.alloc((size_t)6 * K * 2048);
     s.tickets.alloc(4 * kReduceTickets);
     s.tickets.zero(st);
+    sp = std::move(made);
   }
   BlockState &s = *sp;
   const int n = s.n;

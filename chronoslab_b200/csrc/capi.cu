@@ -932,7 +932,7 @@ int chronos_vcycle(chronos_hier *hh, const double *b_h, double *x_h, int nrhs, v
     CHRONOS_REQUIRE(hh && b_h && x_h && nrhs >= 1, CHRONOS_EINVAL, "bad argument");
     Hier &h = *hh->h;
     const int n = h.levels[0].n;
-    if (h.stage_b.size() < (size_t)n) { h.stage_b.alloc(n); h.stage_x.alloc(n); }
+    h.ensure_staging();
     CallerStream order(h, stream);
     for (int c = 0; c < nrhs; ++c) {
       h.stage_b.upload(b_h + (size_t)c * n, n, h.st);
@@ -1005,7 +1005,7 @@ int chronos_pcg(chronos_hier *hh, const int *iat_h, const int *ja_h, const doubl
       h.set_outer_operator(&op);
     }
     // staging buffers live with the handle: no allocation per call
-    if (h.stage_b.size() < (size_t)n) { h.stage_b.alloc(n); h.stage_x.alloc(n); }
+    h.ensure_staging();
     CallerStream order(h, stream);
     DBuf<double> &b = h.stage_b, &x = h.stage_x;
     b.upload(b_h, n, h.st);

@@ -1840,15 +1840,19 @@ void Hier::vcycle_f32(const float *b, float *out) {
   }
   // FP64 hierarchy: FP64 copies of the vectors around the cycle
   const int n = levels[0].n;
-  if (stage_b.size() < (size_t)n) {
-    stage_b.alloc(n);
-    stage_x.alloc(n);
-  }
+  ensure_staging();
   k_f32_to_f64<<<std::min<int64_t>(ceil_div(n, 256), (int64_t)num_sms() * 8), 256, 0, st>>>(
       n, b, stage_b.get());
   CHRONOS_CHECK_LAUNCH();
   vcycle(stage_b.get(), stage_x.get(), nullptr, nullptr);
   convert_f64_to_f32(n, stage_x.get(), out, st);
+}
+
+void Hier::ensure_staging() {
+  const size_t n = levels[0].n;
+  if (stage_x.size() >= n) return;       // stage_x is there only if stage_b is
+  stage_b.alloc(n);
+  stage_x.alloc(n);
 }
 
 void Hier::apply_A(const double *x, double *y) {
@@ -2363,7 +2367,6 @@ static void ensure_pcg_state(Hier &h, int itmax) {
   PcgState &s = h.pcg;
   const int n = h.levels[0].n;
   if (s.n != n) {
-    s.n = n;
     s.x.alloc(n); s.res.alloc(n); s.p.alloc(n); s.axp.alloc(n); s.pres.alloc(n); s.b.alloc(n);
     s.sc.alloc(SC_COUNT);
     s.part.alloc((size_t)12 * 3 * 2048);
@@ -2371,12 +2374,14 @@ static void ensure_pcg_state(Hier &h, int itmax) {
     s.tickets.zero(h.st);
     s.axp.zero(h.st);
     s.p.zero(h.st);
+    s.n = n;                  // last: what a refused allocation leaves is made again
   }
   if (s.resvec_cap < itmax + 1) {
     // resvec is baked into the graph: rebuild it when the buffer moves
+    drop_pcg_graph(s);
+    s.resvec_cap = 0;
     s.resvec.alloc((size_t)itmax + 1);
     s.resvec_cap = itmax + 1;
-    drop_pcg_graph(s);
   }
 }
 

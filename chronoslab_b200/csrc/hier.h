@@ -168,6 +168,7 @@ struct Hier {
   std::shared_ptr<BlockState> block;
   std::shared_ptr<SqmrState> sqmr;
   DBuf<double> stage_b, stage_x;    // host-buffer entry points' device staging
+  void ensure_staging();
 };
 
 // SQMR (sqmr.cu) from host vectors b and x (x0 on entry, the solution on

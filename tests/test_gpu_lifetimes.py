@@ -166,3 +166,37 @@ def test_single_level_vcycle_in_place(lib, prec, io, nx, shift):
                      both.data_ptr() + to * both.element_size(), ip)
         torch.cuda.synchronize()
         assert torch.equal(both[to:to + n], x)
+
+
+@pytest.mark.parametrize("call,vectors", [
+    ("h.vcycle(b)", 1.5), ("h.pcg(b, tol=1e-8)[0]", 5.5),
+    ("h.pcg_block(np.stack([b, b], 1), tol=1e-8)[0][:, 1]", 15.0),
+    ("(cb.SQMR(h, b, 1e-8, 200))[0]", 4.5)])
+def test_call_after_a_refused_allocation(lib, tmp_path, call, vectors):
+    """A call whose state does not fit (so many vectors of it do) is refused with
+    CHRONOS_ENOMEM; once there is room the same call gives its usual result, and so
+    do solves after one with more iterations than there is room to record."""
+    f = str(tmp_path / "h.chh")
+    load = f"A = PB.poisson7(40)\nn = A.shape[0]\nb = PB.uniform_rhs(n, 3)[:n].ravel()\n"
+    held, = _child(tmp_path, load + (
+        "with cb.Hierarchy(A, np.ones((n, 1)), cb.params(ntv=1, nupre=2,"
+        f" precision=cb.CHRONOS_FP64)) as h: h.save({f!r})\n"
+        f"with cb.Hierarchy.load({f!r}) as h, cb.Hierarchy.load({f!r}) as h2:"
+        " print(cb.device_bytes())\n"))
+    n = 40 ** 3
+    room = 600000 if "vcycle" not in call else 0          # the reductions' partials
+    got = _child(tmp_path, load + (
+        f"h, h2 = cb.Hierarchy.load({f!r}), cb.Hierarchy.load({f!r})\n"
+        "refused = 0\n"
+        f"try: {call}\n"
+        "except cb.ChronosError as e: refused = int('ENOMEM' in str(e))\n"
+        "h2.close()\n"
+        f"x = {call}\n"
+        "h.pcg(b, itmax=12, tol=0.0)\n"
+        "try: h.pcg(b, itmax=100000000, tol=1e-8)\n"
+        "except cb.ChronosError as e: refused += int('ENOMEM' in str(e))\n"
+        "z, it, rv, flag, _ = h.pcg(b, itmax=100, tol=1e-8)\n"
+        "print(refused, int(it == len(rv) - 1), np.linalg.norm(b - A @ z) / np.linalg.norm(b),\n"
+        "      np.linalg.norm(b - A @ x) / np.linalg.norm(b))\n"), held + room + vectors * 8 * n)
+    assert got[:2] == [2, 1] and got[2] <= 1e-8
+    assert got[3] <= (1.0 if "vcycle" in call else 1e-7)
