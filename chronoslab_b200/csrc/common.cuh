@@ -8,6 +8,7 @@
 #include <cstdint>
 #include <cstdio>
 #include <cstdlib>
+#include <memory>
 #include <mutex>
 #include <stdexcept>
 #include <string>
@@ -274,9 +275,46 @@ inline void flush_deferred_frees() {
     synced->trim();
   }
 }
+// State that an owner keeps between its calls only to spare the next one making it
+// again.  A call takes it, and parks it again, idle, when it is done; parked states
+// of every owner are given up before an allocation is refused.
+struct IdleStates {
+  std::mutex mu;
+  std::vector<std::pair<const void *, std::shared_ptr<void>>> list;
+  std::shared_ptr<void> take(const void *owner) {
+    std::shared_ptr<void> s;
+    std::lock_guard<std::mutex> lk(mu);
+    for (size_t k = 0; k < list.size() && !s; ++k)
+      if (list[k].first == owner) {
+        s = std::move(list[k].second);
+        list.erase(list.begin() + k);
+      }
+    return s;
+  }
+  void park(const void *owner, std::shared_ptr<void> s) {
+    std::lock_guard<std::mutex> lk(mu);
+    list.emplace_back(owner, std::move(s));
+  }
+  void give_up() {
+    decltype(list) all;
+    std::lock_guard<std::mutex> lk(mu);
+    all.swap(list);
+    for (auto &e : all) e.second.reset();
+  }
+};
+inline IdleStates &idle_states() {
+  static IdleStates *s = new IdleStates;                // outlives static handles
+  return *s;
+}
+// Gives back what the library holds without need.
+inline void give_back() {
+  idle_states().give_up();
+  flush_deferred_frees();
+}
+
 // Whether the device (and CHRONOS_DEVICE_ALLOC_CAP) has room for so many bytes more.
 inline bool device_room(int64_t bytes) {
-  flush_deferred_frees();
+  give_back();
   const int64_t cap = device_alloc_cap();
   if (cap > 0 && device_bytes_live().load() + bytes > cap) return false;
   size_t avail = 0, total = 0;
@@ -320,8 +358,8 @@ class DBuf {
     if (n == 0) return;
     const int64_t bytes = (int64_t)(n * sizeof(T)), cap = device_alloc_cap();
     auto beyond_cap = [&] { return cap > 0 && device_bytes_live().load() + bytes > cap; };
-    // what was let go of and is still kept is given back before a refusal
-    if (beyond_cap()) flush_deferred_frees();
+    // what is kept without need is given back before a refusal
+    if (beyond_cap()) give_back();
     if (beyond_cap())
       throw Error(CHRONOS_ENOMEM, "allocation of " + std::to_string(bytes) +
                                       " bytes beyond CHRONOS_DEVICE_ALLOC_CAP");
@@ -329,7 +367,7 @@ class DBuf {
     void *p = nullptr;
     cudaError_t e = pool.alloc(&p, n * sizeof(T));
     if (e == cudaErrorMemoryAllocation) {
-      flush_deferred_frees();
+      give_back();
       e = pool.alloc(&p, n * sizeof(T));
     }
     if (e != cudaSuccess) {

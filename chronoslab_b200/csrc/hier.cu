@@ -68,6 +68,7 @@ PcgState::~PcgState() {
 Hier::~Hier() {
   if (st) cudaStreamSynchronize(st);
   replays.wait();
+  idle_states().take(this);
   levels.clear();
   drop_pcg_graph(pcg);
   if (ev_in) cudaEventDestroy(ev_in);
@@ -2363,15 +2364,21 @@ static void capture_iteration(Hier &h, cudaGraphConditionalHandle handle, int us
                        use_cond, far);
 }
 
+void ensure_reduction_state(Hier &h) {
+  PcgState &s = h.pcg;
+  if (s.tickets.size() > 0) return;
+  s.part.alloc((size_t)12 * 3 * 2048);
+  s.tickets.alloc(8);
+  s.tickets.zero(h.st);
+}
+
 static void ensure_pcg_state(Hier &h, int itmax) {
   PcgState &s = h.pcg;
   const int n = h.levels[0].n;
+  ensure_reduction_state(h);
   if (s.n != n) {
     s.x.alloc(n); s.res.alloc(n); s.p.alloc(n); s.axp.alloc(n); s.pres.alloc(n); s.b.alloc(n);
     s.sc.alloc(SC_COUNT);
-    s.part.alloc((size_t)12 * 3 * 2048);
-    s.tickets.alloc(8);
-    s.tickets.zero(h.st);
     s.axp.zero(h.st);
     s.p.zero(h.st);
     s.n = n;                  // last: what a refused allocation leaves is made again
@@ -2432,8 +2439,6 @@ void zero_vcycle_partials(Hier &h) {
   CHRONOS_CUDA(cudaMemsetAsync(h.pcg.part.get() + kSpmvPartials, 0, sizeof(double) * 3 * 2048,
                                h.st));
 }
-
-void ensure_reduction_state(Hier &h) { ensure_pcg_state(h, std::max(h.pcg.resvec_cap - 1, 1)); }
 
 static void build_pcg_graph(Hier &h) {
   PcgState &s = h.pcg;

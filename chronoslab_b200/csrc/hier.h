@@ -108,7 +108,6 @@ struct PcgState {
 };
 
 struct BlockState;   // block-of-right-hand-sides solve state (block.cu)
-struct SqmrState;    // SQMR vectors and graph (sqmr.cu)
 
 // A host block of right-hand sides: column-major with n rows (ld = 0), or
 // row-major with rows ld elements apart.
@@ -166,7 +165,6 @@ struct Hier {
   void pcg_block(int nrhs, const BlockIn &B, const double *X0_h, double *X_h, int itmax,
                  double tol, int *iters, int *flags, double *seconds);
   std::shared_ptr<BlockState> block;
-  std::shared_ptr<SqmrState> sqmr;
   DBuf<double> stage_b, stage_x;    // host-buffer entry points' device staging
   void ensure_staging();
 };

@@ -164,8 +164,11 @@ void operator_apply(cudaStream_t st, const DMat &A, const double *x, const doubl
 
 }  // namespace
 
-// Vectors, scalars and the loop's graph; a handle keeps one for its own
-// level-1 operator.
+// Vectors, scalars and the loop's graph.  For the handle's own operator they are
+// parked between calls (IdleStates), up to kSqmrParkBytes: making the graph anew takes
+// 0.33 ms, a quarter of a call at 17^3 (1.26 and 1.60 ms), 7 % of one at 32^3
+// (104,544 rows: 4.18 and 4.48 ms).
+constexpr size_t kSqmrParkBytes = (size_t)32 << 20;
 struct SqmrState {
   int n = 0;
   DBuf<double> vec, sc, part;
@@ -239,10 +242,9 @@ void sqmr_solve(Hier &h, const DMat *op, const double *b_h, double *x_h, int itm
   const int n = h.levels[0].n;
   ensure_reduction_state(h);                    // the V-cycle's dot
   const DMat &A = op ? *op : h.levels[0].A;
-  std::shared_ptr<SqmrState> own;
-  if (op) own = std::make_shared<SqmrState>(n);
-  else if (!h.sqmr) h.sqmr = std::make_shared<SqmrState>(n);
-  SqmrState &s = op ? *own : *h.sqmr;
+  auto state = op ? nullptr : std::static_pointer_cast<SqmrState>(idle_states().take(&h));
+  if (!state) state = std::make_shared<SqmrState>(n);
+  SqmrState &s = *state;
   const int nb = std::max(1, std::min(num_sms() * 8, (int)ceil_div(n, 256)));
   double *sc = s.sc.get(), *part = s.part.get();
   unsigned *tk = s.tickets.get();
@@ -285,6 +287,8 @@ void sqmr_solve(Hier &h, const DMat *op, const double *b_h, double *x_h, int itm
   *iters = (int)(got[SQ_ITER] + 0.5);
   *info = *iters >= itmax ? 1 : (int)(got[SQ_INFO] + 0.5);
   *relres = std::sqrt(got[SQ_TRUE]) / std::sqrt(got[SQ_BB]);
+  if (!op && sizeof(double) * s.vec.size() <= kSqmrParkBytes)
+    idle_states().park(&h, std::move(state));
 }
 
 }  // namespace chronos

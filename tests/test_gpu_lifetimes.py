@@ -200,3 +200,27 @@ def test_call_after_a_refused_allocation(lib, tmp_path, call, vectors):
         "      np.linalg.norm(b - A @ x) / np.linalg.norm(b))\n"), held + room + vectors * 8 * n)
     assert got[:2] == [2, 1] and got[2] <= 1e-8
     assert got[3] <= (1.0 if "vcycle" in call else 1e-7)
+
+
+def test_sqmr_state_is_no_reason_to_refuse(lib, tmp_path):
+    """What SQMR keeps on its handle between calls is given up before an allocation
+    is refused, and made again by the next call: under a cap that holds one state
+    beside two handles, both handles solve in turn with the same results."""
+    f = str(tmp_path / "h.chh")
+    load = "A = PB.poisson7(40)\nn = A.shape[0]\nb = PB.uniform_rhs(n, 3).ravel()\n"
+    held, = _child(tmp_path, load + (
+        "with cb.Hierarchy(A, np.ones((n, 1)), cb.params(ntv=1, nupre=2,"
+        f" precision=cb.CHRONOS_FP64)) as h: h.save({f!r})\n"
+        f"with cb.Hierarchy.load({f!r}) as h, cb.Hierarchy.load({f!r}) as h2:"
+        " print(cb.device_bytes())\n"))
+    n = 40 ** 3
+    got = _child(tmp_path, load + (
+        f"h, h2 = cb.Hierarchy.load({f!r}), cb.Hierarchy.load({f!r})\n"
+        "r = [cb.SQMR(k, b, 1e-8, 200) for k in (h, h2, h, h2, h2)]\n"
+        "two = cb.device_bytes()\n"
+        "h.close(); h2.close()\n"
+        "print(min(np.array_equal(r[0][0], q[0]) for q in r) + 0,"
+        " np.linalg.norm(b - A @ r[0][0]) / np.linalg.norm(b), two, cb.device_bytes())\n"),
+        held + 2 * 700000 + 9 * 8 * n)
+    assert got[0] == 1 and got[1] <= 1.1e-8 and got[3] == 0
+    assert got[2] <= held + 2 * 700000 + 7 * 8 * n
