@@ -223,12 +223,7 @@ struct BlockState {
   DBuf<double> sc;              // per-column scalars, see BS_* below
   DBuf<double> part;
   DBuf<unsigned> tickets;
-  cudaGraphExec_t exec = nullptr;
-  cudaGraph_t graph = nullptr;
-  ~BlockState() {
-    if (exec) cudaGraphExecDestroy(exec);
-    if (graph) cudaGraphDestroy(graph);
-  }
+  LoopGraph loop;
 };
 
 // per-column scalar arrays (each K wide) inside sc
@@ -656,19 +651,9 @@ static void block_solve(Hier &h, int m, const BlockIn &B, const double *X0_h, do
   if (itmax > 0 && !h.prm.use_graph) {
     // one iteration per graph launch from a host loop (profilers cannot see
     // the kernel nodes of a graph holding a conditional node); same kernels
-    if (!s.exec) {
-      std::lock_guard<std::mutex> capturing(lib_streams().mu);
-      CHRONOS_CUDA(cudaStreamBeginCapture(st, cudaStreamCaptureModeThreadLocal));
-      try {
-        capture_block_iteration<K>(h, s, 0, 0);
-      } catch (...) {
-        cudaGraph_t dummy;
-        cudaStreamEndCapture(st, &dummy);
-        throw;
-      }
-      CHRONOS_CUDA(cudaStreamEndCapture(st, &s.graph));
-      CHRONOS_CUDA(cudaGraphInstantiate(&s.exec, s.graph, 0));
-    }
+    if (!s.loop.ready())
+      s.loop.build(st, false,
+                   [&](cudaGraphConditionalHandle) { capture_block_iteration<K>(h, s, 0, 0); });
     double act_h[K];
     for (int k = 0; k < itmax; ++k) {
       CHRONOS_CUDA(cudaMemcpyAsync(act_h, s.sc.get() + bs_off(BS_ACTIVE, K), sizeof(act_h),
@@ -677,34 +662,13 @@ static void block_solve(Hier &h, int m, const BlockIn &B, const double *X0_h, do
       bool any = false;
       for (int j = 0; j < K; ++j) any |= act_h[j] != 0.0;
       if (!any) break;
-      CHRONOS_CUDA(cudaGraphLaunch(s.exec, st));
+      s.loop.launch(st);
     }
   } else if (itmax > 0) {
-    if (!s.exec) {
-      CHRONOS_CUDA(cudaGraphCreate(&s.graph, 0));
-      cudaGraphConditionalHandle handle;
-      CHRONOS_CUDA(cudaGraphConditionalHandleCreate(&handle, s.graph, 1, cudaGraphCondAssignDefault));
-      cudaGraphNodeParams np{};
-      np.type = cudaGraphNodeTypeConditional;
-      np.conditional.handle = handle;
-      np.conditional.type = cudaGraphCondTypeWhile;
-      np.conditional.size = 1;
-      cudaGraphNode_t node;
-      CHRONOS_CUDA(cudaGraphAddNode(&node, s.graph, nullptr, 0, &np));
-      cudaGraph_t body = np.conditional.phGraph_out[0];
-      std::lock_guard<std::mutex> capturing(lib_streams().mu);
-      CHRONOS_CUDA(cudaStreamBeginCaptureToGraph(st, body, nullptr, nullptr, 0,
-                                                 cudaStreamCaptureModeThreadLocal));
-      try {
+    if (!s.loop.ready())
+      s.loop.build(st, true, [&](cudaGraphConditionalHandle handle) {
         capture_block_iteration<K>(h, s, handle, 1);
-      } catch (...) {
-        cudaGraph_t dummy;
-        cudaStreamEndCapture(st, &dummy);
-        throw;
-      }
-      CHRONOS_CUDA(cudaStreamEndCapture(st, &body));
-      CHRONOS_CUDA(cudaGraphInstantiate(&s.exec, s.graph, 0));
-    }
+      });
     // the while loop runs its body once before testing: skip it when no
     // column is active (all b = 0)
     double act_h[K];
@@ -713,7 +677,7 @@ static void block_solve(Hier &h, int m, const BlockIn &B, const double *X0_h, do
     CHRONOS_CUDA(cudaStreamSynchronize(st));
     bool any = false;
     for (int j = 0; j < K; ++j) any |= act_h[j] != 0.0;
-    if (any) CHRONOS_CUDA(cudaGraphLaunch(s.exec, st));
+    if (any) s.loop.launch(st);
   }
   k_zero_null_columns<K><<<nb, 256, 0, st>>>(n, s.x.get(), s.sc.get());
   CHRONOS_CHECK_LAUNCH();

@@ -385,8 +385,6 @@ template <> float *gvec<float>(DBuf<float> &f, DBuf<double> &) { return f.get();
 template <> double *gvec<double>(DBuf<float> &, DBuf<double> &d) { return d.get(); }
 
 GroupSolve::~GroupSolve() {
-  if (exec) cudaGraphExecDestroy(exec);
-  if (graph) cudaGraphDestroy(graph);
   if (st) {
     stream_destroy(st);
   }
@@ -718,12 +716,7 @@ void group_solve(GroupSolve &g, const std::vector<const double *> &b_h,
                                  cudaMemcpyHostToDevice, st));
   }
   // the loop's scalars (tol, itmax) are baked into the graph: rebuild on change
-  if (g.exec && (g.g_tol != tol || g.g_itmax != itmax)) {
-    cudaGraphExecDestroy(g.exec);
-    cudaGraphDestroy(g.graph);
-    g.exec = nullptr;
-    g.graph = nullptr;
-  }
+  if (g.g_tol != tol || g.g_itmax != itmax) g.loop.reset();
   cudaEvent_t e0, e1;
   CHRONOS_CUDA(cudaEventCreate(&e0));
   CHRONOS_CUDA(cudaEventCreate(&e1));
@@ -742,60 +735,27 @@ void group_solve(GroupSolve &g, const std::vector<const double *> &b_h,
   CHRONOS_CUDA(cudaMemcpyAsync(&active, g.ctl.get(), sizeof(unsigned), cudaMemcpyDeviceToHost,
                                st));
   CHRONOS_CUDA(cudaStreamSynchronize(st));
+  auto build = [&](bool loop) {
+    if (g.loop.ready()) return;
+    g.loop.build(st, loop, [&](cudaGraphConditionalHandle handle) {
+      group_capture_iteration(g, handle, loop ? 1 : 0, tol, itmax);
+    });
+    g.g_tol = tol;
+    g.g_itmax = itmax;
+  };
   if (active > 0 && !g.prm.use_graph) {
     // one iteration per graph launch from a host loop (profilers cannot see
     // the kernel nodes of a graph holding a conditional node); same kernels
-    if (!g.exec) {
-      std::lock_guard<std::mutex> capturing(lib_streams().mu);
-      CHRONOS_CUDA(cudaStreamBeginCapture(st, cudaStreamCaptureModeThreadLocal));
-      try {
-        group_capture_iteration(g, 0, 0, tol, itmax);
-      } catch (...) {
-        cudaGraph_t dummy;
-        cudaStreamEndCapture(st, &dummy);
-        throw;
-      }
-      CHRONOS_CUDA(cudaStreamEndCapture(st, &g.graph));
-      CHRONOS_CUDA(cudaGraphInstantiate(&g.exec, g.graph, 0));
-      g.g_tol = tol;
-      g.g_itmax = itmax;
-    }
+    build(false);
     for (int k = 0; k < itmax && active > 0; ++k) {
-      CHRONOS_CUDA(cudaGraphLaunch(g.exec, st));
+      g.loop.launch(st);
       CHRONOS_CUDA(cudaMemcpyAsync(&active, g.ctl.get(), sizeof(unsigned),
                                    cudaMemcpyDeviceToHost, st));
       CHRONOS_CUDA(cudaStreamSynchronize(st));
     }
   } else if (active > 0) {
-    if (!g.exec) {
-      CHRONOS_CUDA(cudaGraphCreate(&g.graph, 0));
-      cudaGraphConditionalHandle handle;
-      CHRONOS_CUDA(
-          cudaGraphConditionalHandleCreate(&handle, g.graph, 1, cudaGraphCondAssignDefault));
-      cudaGraphNodeParams np_{};
-      np_.type = cudaGraphNodeTypeConditional;
-      np_.conditional.handle = handle;
-      np_.conditional.type = cudaGraphCondTypeWhile;
-      np_.conditional.size = 1;
-      cudaGraphNode_t node;
-      CHRONOS_CUDA(cudaGraphAddNode(&node, g.graph, nullptr, 0, &np_));
-      cudaGraph_t body = np_.conditional.phGraph_out[0];
-      std::lock_guard<std::mutex> capturing(lib_streams().mu);
-      CHRONOS_CUDA(cudaStreamBeginCaptureToGraph(st, body, nullptr, nullptr, 0,
-                                                 cudaStreamCaptureModeThreadLocal));
-      try {
-        group_capture_iteration(g, handle, 1, tol, itmax);
-      } catch (...) {
-        cudaGraph_t dummy;
-        cudaStreamEndCapture(st, &dummy);
-        throw;
-      }
-      CHRONOS_CUDA(cudaStreamEndCapture(st, &body));
-      CHRONOS_CUDA(cudaGraphInstantiate(&g.exec, g.graph, 0));
-      g.g_tol = tol;
-      g.g_itmax = itmax;
-    }
-    CHRONOS_CUDA(cudaGraphLaunch(g.exec, st));
+    build(true);
+    g.loop.launch(st);
   }
   CHRONOS_CUDA(cudaEventRecord(e1, st));
   std::vector<double> sc((size_t)np * GS_COUNT);

@@ -44,8 +44,7 @@ struct GroupSolve {
   DBuf<double> x, res, p, axp, pres, b, sc, part;
   DBuf<unsigned> tickets, ctl;
   cudaStream_t st = nullptr;
-  cudaGraph_t graph = nullptr;
-  cudaGraphExec_t exec = nullptr;
+  LoopGraph loop;
   double g_tol = -1.0;
   int g_itmax = -1;
   ~GroupSolve();

@@ -57,12 +57,57 @@ class SetupPhase {
   double *acc_;
 };
 
-static void drop_pcg_graph(PcgState &s);
+void LoopGraph::reset() {
+  if (exec_) cudaGraphExecDestroy(exec_);
+  if (graph_) cudaGraphDestroy(graph_);
+  exec_ = nullptr;
+  graph_ = nullptr;
+}
+
+void LoopGraph::build(cudaStream_t st, bool loop,
+                      const std::function<void(cudaGraphConditionalHandle)> &queue) {
+  reset();
+  try {
+    CHRONOS_CUDA(cudaGraphCreate(&graph_, 0));
+    cudaGraph_t body = graph_;
+    cudaGraphConditionalHandle handle = 0;
+    if (loop) {
+      CHRONOS_CUDA(cudaGraphConditionalHandleCreate(&handle, graph_, 1, cudaGraphCondAssignDefault));
+      cudaGraphNodeParams np{};
+      np.type = cudaGraphNodeTypeConditional;
+      np.conditional.handle = handle;
+      np.conditional.type = cudaGraphCondTypeWhile;
+      np.conditional.size = 1;
+      cudaGraphNode_t node;
+      CHRONOS_CUDA(cudaGraphAddNode(&node, graph_, nullptr, 0, &np));
+      body = np.conditional.phGraph_out[0];
+    }
+    std::lock_guard<std::mutex> capturing(lib_streams().mu);
+    CHRONOS_CUDA(cudaStreamBeginCaptureToGraph(st, body, nullptr, nullptr, 0,
+                                               cudaStreamCaptureModeThreadLocal));
+    try {
+      queue(handle);
+    } catch (...) {
+      cudaGraph_t dropped;
+      cudaStreamEndCapture(st, &dropped);
+      throw;
+    }
+    CHRONOS_CUDA(cudaStreamEndCapture(st, &body));
+    CHRONOS_CUDA(cudaGraphInstantiate(&exec_, graph_, 0));
+  } catch (...) {
+    exec_ = nullptr;
+    reset();
+    throw;
+  }
+}
 
 PcgState::~PcgState() {
-  for (auto e : {exec, far_exec}) if (e) cudaGraphExecDestroy(e);
-  for (auto g : {graph, far_graph}) if (g) cudaGraphDestroy(g);
   if (sc_pinned) cudaFreeHost(sc_pinned);
+}
+
+static void drop_pcg_graphs(PcgState &s) {
+  s.near.reset();
+  s.far.reset();
 }
 
 Hier::~Hier() {
@@ -70,7 +115,7 @@ Hier::~Hier() {
   replays.wait();
   idle_states().take(this);
   levels.clear();
-  drop_pcg_graph(pcg);
+  drop_pcg_graphs(pcg);
   if (ev_in) cudaEventDestroy(ev_in);
   if (ev_out) cudaEventDestroy(ev_out);
   stream_destroy(st);
@@ -2054,7 +2099,7 @@ static void launch_pcg_spmv(cudaStream_t st, const DMat &A, bool fp32vals, const
 // tolerance, and at itmax; the stop is then decided on the true residual.
 // The scalars are read before the first store (and by the kernels before their
 // loop): in the order of use they were a chain of L2 round trips behind the
-// reduction.  far > 0 (the unrolled loop of far_exec): go on only while the
+// reduction.  far > 0 (the unrolled loop, PcgState::far): go on only while the
 // residual is above far times the tolerance.
 struct FinResidual {
   double *sc, *resvec;
@@ -2306,17 +2351,6 @@ static bool mixed_outer(const Hier &h) {
   return h.precision == CHRONOS_FP32 && !h.prm.exact_outer && !h.use_user_op;
 }
 
-static void drop_pcg_graph(PcgState &s) {
-  for (auto *e : {&s.exec, &s.far_exec}) {
-    if (*e) cudaGraphExecDestroy(*e);
-    *e = nullptr;
-  }
-  for (auto *g : {&s.graph, &s.far_graph}) {
-    if (*g) cudaGraphDestroy(*g);
-    *g = nullptr;
-  }
-}
-
 void Hier::set_outer_operator(const HostCSR *A) {
   if (A) {
     CHRONOS_REQUIRE(A->nrows == levels[0].n && A->ncols == levels[0].n, CHRONOS_EINVAL,
@@ -2325,11 +2359,11 @@ void Hier::set_outer_operator(const HostCSR *A) {
     user_op = DMat();
     upload_csr(*A, user_op, false, st);
     autotune_lanes(user_op, false, st);
-    drop_pcg_graph(pcg);                       // the graph holds the operator's pointers
+    drop_pcg_graphs(pcg);                       // the graph holds the operator's pointers
     use_user_op = true;
   } else if (use_user_op) {
     CHRONOS_CUDA(cudaStreamSynchronize(st));
-    drop_pcg_graph(pcg);
+    drop_pcg_graphs(pcg);
     use_user_op = false;
     user_op = DMat();
   }
@@ -2385,7 +2419,7 @@ static void ensure_pcg_state(Hier &h, int itmax) {
   }
   if (s.resvec_cap < itmax + 1) {
     // resvec is baked into the graph: rebuild it when the buffer moves
-    drop_pcg_graph(s);
+    drop_pcg_graphs(s);
     s.resvec_cap = 0;
     s.resvec.alloc((size_t)itmax + 1);
     s.resvec_cap = itmax + 1;
@@ -2405,32 +2439,10 @@ constexpr int kFarUnroll = 4;
 constexpr double kFarFactor = 30.0;
 
 // One while loop over `unroll` iterations per pass.
-static void build_while_graph(Hier &h, int unroll, double far, cudaGraph_t *graph,
-                              cudaGraphExec_t *exec) {
-  cudaStream_t st = h.st;
-  CHRONOS_CUDA(cudaGraphCreate(graph, 0));
-  cudaGraphConditionalHandle handle;
-  CHRONOS_CUDA(cudaGraphConditionalHandleCreate(&handle, *graph, 1, cudaGraphCondAssignDefault));
-  cudaGraphNodeParams np{};
-  np.type = cudaGraphNodeTypeConditional;
-  np.conditional.handle = handle;
-  np.conditional.type = cudaGraphCondTypeWhile;
-  np.conditional.size = 1;
-  cudaGraphNode_t node;
-  CHRONOS_CUDA(cudaGraphAddNode(&node, *graph, nullptr, 0, &np));
-  cudaGraph_t body = np.conditional.phGraph_out[0];
-  std::lock_guard<std::mutex> capturing(lib_streams().mu);
-  CHRONOS_CUDA(cudaStreamBeginCaptureToGraph(st, body, nullptr, nullptr, 0,
-                                             cudaStreamCaptureModeThreadLocal));
-  try {
+static void build_while_graph(Hier &h, int unroll, double far, LoopGraph &g) {
+  g.build(h.st, true, [&](cudaGraphConditionalHandle handle) {
     for (int k = 0; k < unroll; ++k) capture_iteration(h, handle, k + 1 == unroll, far);
-  } catch (...) {
-    cudaGraph_t dummy;
-    cudaStreamEndCapture(st, &dummy);
-    throw;
-  }
-  CHRONOS_CUDA(cudaStreamEndCapture(st, &body));
-  CHRONOS_CUDA(cudaGraphInstantiate(exec, *graph, 0));
+  });
 }
 
 const double *vcycle_dot_partials(Hier &h) { return h.pcg.part.get() + kDotPartials; }
@@ -2442,25 +2454,9 @@ void zero_vcycle_partials(Hier &h) {
 
 static void build_pcg_graph(Hier &h) {
   PcgState &s = h.pcg;
-  cudaStream_t st = h.st;
-  if (s.exec) return;
-  if (h.prm.use_graph) {
-    build_while_graph(h, 1, 0.0, &s.graph, &s.exec);
-    s.conditional = true;
-  } else {
-    std::lock_guard<std::mutex> capturing(lib_streams().mu);
-    CHRONOS_CUDA(cudaStreamBeginCapture(st, cudaStreamCaptureModeThreadLocal));
-    try {
-      capture_iteration(h, 0, 0);
-    } catch (...) {
-      cudaGraph_t dummy;
-      cudaStreamEndCapture(st, &dummy);
-      throw;
-    }
-    CHRONOS_CUDA(cudaStreamEndCapture(st, &s.graph));
-    CHRONOS_CUDA(cudaGraphInstantiate(&s.exec, s.graph, 0));
-    s.conditional = false;
-  }
+  if (s.near.ready()) return;
+  if (h.prm.use_graph) build_while_graph(h, 1, 0.0, s.near);
+  else s.near.build(h.st, false, [&](cudaGraphConditionalHandle) { capture_iteration(h, 0, 0); });
 }
 
 static double replace_ratio(const Hier &h) {
@@ -2528,20 +2524,19 @@ void Hier::pcg_solve(const double *b, double *x, int itmax, double tol, int *ite
   }
   if (itmax > 0) {
     build_pcg_graph(*this);
-    if (s.conditional) {
+    if (prm.use_graph) {
       // the unrolled loop leaves the last iterations (one at least, a no-op if
       // it stopped the solve) to the plain one
       if (itmax > kFarUnroll && sc_h[SC_RESITER] > kFarFactor * tol) {
-        if (!s.far_exec)
-          build_while_graph(*this, kFarUnroll, kFarFactor, &s.far_graph, &s.far_exec);
-        CHRONOS_CUDA(cudaGraphLaunch(s.far_exec, st));
+        if (!s.far.ready()) build_while_graph(*this, kFarUnroll, kFarFactor, s.far);
+        s.far.launch(st);
       }
-      CHRONOS_CUDA(cudaGraphLaunch(s.exec, st));
+      s.near.launch(st);
     } else {
       double *pinned = nullptr;
       CHRONOS_CUDA(cudaMallocHost(&pinned, sizeof(double) * SC_COUNT));
       for (int k = 0; k < itmax; ++k) {
-        CHRONOS_CUDA(cudaGraphLaunch(s.exec, st));
+        s.near.launch(st);
         CHRONOS_CUDA(cudaMemcpyAsync(pinned, s.sc.get(), sizeof(double) * SC_COUNT,
                                      cudaMemcpyDeviceToHost, st));
         CHRONOS_CUDA(cudaStreamSynchronize(st));
@@ -2605,7 +2600,7 @@ void Hier::pcg_enqueue(const double *b, double *x, int itmax, double tol) {
   k_pcg_init<<<1, 1, 0, st>>>(s.sc.get(), s.resvec.get(), tol, (double)itmax,
                               replace_ratio(*this));
   CHRONOS_CHECK_LAUNCH();
-  if (itmax > 0) CHRONOS_CUDA(cudaGraphLaunch(s.exec, st));
+  if (itmax > 0) s.near.launch(st);
   CHRONOS_CUDA(cudaMemcpyAsync(x, s.x.get(), sizeof(double) * n, cudaMemcpyDeviceToDevice, st));
   CHRONOS_CUDA(cudaMemcpyAsync(s.sc_pinned, s.sc.get(), sizeof(double) * SC_COUNT,
                                cudaMemcpyDeviceToHost, st));

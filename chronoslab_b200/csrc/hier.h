@@ -84,6 +84,26 @@ template <typename T> inline const T *vals(const DMat &m);
 template <> inline const float *vals<float>(const DMat &m) { return m.v32.get(); }
 template <> inline const double *vals<double>(const DMat &m) { return m.v64.get(); }
 
+// An iteration's launches as a CUDA graph: the body of a while loop on the device
+// (a conditional node, left when a kernel clears the handle), or once per launch.
+class LoopGraph {
+ public:
+  LoopGraph() = default;
+  ~LoopGraph() { reset(); }
+  LoopGraph(const LoopGraph &) = delete;
+  LoopGraph &operator=(const LoopGraph &) = delete;
+  bool ready() const { return exec_ != nullptr; }
+  // captures what queue(handle) launches into st; nothing is kept if that fails
+  void build(cudaStream_t st, bool loop,
+             const std::function<void(cudaGraphConditionalHandle)> &queue);
+  void launch(cudaStream_t st) const { CHRONOS_CUDA(cudaGraphLaunch(exec_, st)); }
+  void reset();
+
+ private:
+  cudaGraph_t graph_ = nullptr;
+  cudaGraphExec_t exec_ = nullptr;
+};
+
 // Device scalars of the PCG recurrence.
 enum PcgScalar {
   SC_BNORM = 0, SC_PTAP, SC_PRES_AXP, SC_RR, SC_RESITER, SC_ITER, SC_TOL, SC_ITMAX,
@@ -97,11 +117,8 @@ struct PcgState {
   DBuf<double> sc;                  // SC_COUNT scalars
   DBuf<double> part;                // block partials (3 per block, several slots)
   DBuf<unsigned> tickets;           // one ticket per reducing kernel
-  cudaGraphExec_t exec = nullptr;   // the whole solve (device-side loop) or one iteration
-  cudaGraph_t graph = nullptr;
-  cudaGraphExec_t far_exec = nullptr;   // kFarUnroll iterations per pass, far from the tolerance
-  cudaGraph_t far_graph = nullptr;
-  bool conditional = false;
+  LoopGraph near;                   // one iteration per pass (or per launch)
+  LoopGraph far;                    // kFarUnroll iterations per pass, far from the tolerance
   int resvec_cap = 0;
   double *sc_pinned = nullptr;      // pinned copy of the scalars for queued solves
   ~PcgState();

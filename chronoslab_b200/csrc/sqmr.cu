@@ -174,16 +174,11 @@ struct SqmrState {
   DBuf<double> vec, sc, part;
   DBuf<unsigned> tickets;
   double *b = nullptr, *x = nullptr, *r = nullptr, *q = nullptr, *d = nullptr, *v = nullptr;
-  cudaGraph_t graph = nullptr;
-  cudaGraphExec_t exec = nullptr;
+  LoopGraph loop;
   explicit SqmrState(int rows) : n(rows), vec(6 * (size_t)rows), sc(SQ_COUNT), part(5 * 2048),
                                  tickets(4) {
     b = vec.get();
     x = b + n; r = x + n; q = r + n; d = q + n; v = d + n;
-  }
-  ~SqmrState() {
-    if (exec) cudaGraphExecDestroy(exec);
-    if (graph) cudaGraphDestroy(graph);
   }
 };
 
@@ -204,36 +199,6 @@ static void capture_sqmr(Hier &h, SqmrState &s, const DMat &A, cudaGraphConditio
              vcycle_dot_partials(h), slots, part, tk, sc, handle, use_cond);
   launch_pdl(k_sq_update, nb, 256, st, n, (const double *)s.v, s.d, s.q, s.x,
              (const double *)sc);
-}
-
-static void build_sqmr_graph(Hier &h, SqmrState &s, const DMat &A) {
-  cudaStream_t st = h.st;
-  CHRONOS_CUDA(cudaGraphCreate(&s.graph, 0));
-  cudaGraph_t body = s.graph;
-  cudaGraphConditionalHandle handle = 0;
-  if (h.prm.use_graph) {
-    CHRONOS_CUDA(cudaGraphConditionalHandleCreate(&handle, s.graph, 1, cudaGraphCondAssignDefault));
-    cudaGraphNodeParams np{};
-    np.type = cudaGraphNodeTypeConditional;
-    np.conditional.handle = handle;
-    np.conditional.type = cudaGraphCondTypeWhile;
-    np.conditional.size = 1;
-    cudaGraphNode_t node;
-    CHRONOS_CUDA(cudaGraphAddNode(&node, s.graph, nullptr, 0, &np));
-    body = np.conditional.phGraph_out[0];
-  }
-  std::lock_guard<std::mutex> capturing(lib_streams().mu);
-  CHRONOS_CUDA(cudaStreamBeginCaptureToGraph(st, body, nullptr, nullptr, 0,
-                                             cudaStreamCaptureModeThreadLocal));
-  try {
-    capture_sqmr(h, s, A, handle, h.prm.use_graph ? 1 : 0);
-  } catch (...) {
-    cudaGraph_t dummy;
-    cudaStreamEndCapture(st, &dummy);
-    throw;
-  }
-  CHRONOS_CUDA(cudaStreamEndCapture(st, &body));
-  CHRONOS_CUDA(cudaGraphInstantiate(&s.exec, s.graph, 0));
 }
 
 void sqmr_solve(Hier &h, const DMat *op, const double *b_h, double *x_h, int itmax, double tol,
@@ -265,12 +230,15 @@ void sqmr_solve(Hier &h, const DMat *op, const double *b_h, double *x_h, int itm
   launch_pdl(k_sq_init, 1, 1, st, sc, (double)itmax, tol);
   double got[SQ_COUNT] = {};
   if (itmax > 0) {
-    if (!s.exec) build_sqmr_graph(h, s, A);
+    if (!s.loop.ready())
+      s.loop.build(st, h.prm.use_graph, [&](cudaGraphConditionalHandle handle) {
+        capture_sqmr(h, s, A, handle, h.prm.use_graph ? 1 : 0);
+      });
     if (h.prm.use_graph) {
-      CHRONOS_CUDA(cudaGraphLaunch(s.exec, st));
+      s.loop.launch(st);
     } else {
       for (int k = 0; k < itmax; ++k) {
-        CHRONOS_CUDA(cudaGraphLaunch(s.exec, st));
+        s.loop.launch(st);
         CHRONOS_CUDA(cudaMemcpyAsync(got, sc, sizeof(got), cudaMemcpyDeviceToHost, st));
         CHRONOS_CUDA(cudaStreamSynchronize(st));
         if (got[SQ_EXIT] != 0.0 || got[SQ_INFO] != 0.0) break;
