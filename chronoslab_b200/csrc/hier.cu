@@ -2101,6 +2101,9 @@ static void launch_pcg_spmv(cudaStream_t st, const DMat &A, bool fp32vals, const
 // loop): in the order of use they were a chain of L2 round trips behind the
 // reduction.  far > 0 (the unrolled loop, PcgState::far): go on only while the
 // residual is above far times the tolerance.
+__device__ __forceinline__ bool go_on(double far, double resiter, double tol) {
+  return far == 0.0 || resiter > far * tol;   // (the plain loop: whatever they are)
+}
 struct FinResidual {
   double *sc, *resvec;
   cudaGraphConditionalHandle handle;
@@ -2136,7 +2139,7 @@ struct FinResidual {
     sc[SC_RESITER] = resiter;
     sc[SC_DONE] = stop ? 1.0 : 0.0;
     resvec[(int)now] = resiter;
-    if (use_cond) cudaGraphSetConditional(handle, !stop && resiter > far * tol ? 1u : 0u);
+    if (use_cond) cudaGraphSetConditional(handle, !stop && go_on(far, resiter, tol) ? 1u : 0u);
   }
 };
 
@@ -2191,7 +2194,7 @@ struct FinReplace {
     sc[SC_RMAX] = rn;
     sc[SC_DONE] = stop ? 1.0 : 0.0;
     resvec[(int)it] = resiter;
-    if (use_cond) cudaGraphSetConditional(handle, !stop && resiter > far * tol ? 1u : 0u);
+    if (use_cond) cudaGraphSetConditional(handle, !stop && go_on(far, resiter, tol) ? 1u : 0u);
   }
 };
 

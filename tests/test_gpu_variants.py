@@ -497,3 +497,27 @@ def _poisson_with_long_rows():
     A = sp.csr_matrix(A + sp.identity(2744))
     A.sort_indices()
     return A
+
+
+@pytest.mark.parametrize("prec", [cb.CHRONOS_FP64, cb.CHRONOS_FP32])
+@pytest.mark.parametrize("problem", ["identity", "poisson"])
+@pytest.mark.parametrize("tol", [0.0, -1.0, np.nan, np.inf])
+def test_loops_agree_at_odd_tolerances(lib, prec, problem, tol):
+    """A tolerance that no residual meets, or every one, and a residual that becomes
+    exactly zero (a multiple of the identity, whose inverse is exact): the device-side
+    loop ends where the one-iteration host loop ends, in the same way."""
+    from chronoslab_b200 import problems as PB
+    A = PB.poisson7(8) if problem == "poisson" else sp.csr_matrix(2.0 * sp.identity(64))
+    n = A.shape[0]
+    b = np.arange(1.0, n + 1.0)
+    out = []
+    for use_graph in (1, 0):
+        with cb.Hierarchy(A, np.ones((n, 1)), cb.params(
+                precision=prec, ntv=1, use_graph=use_graph, maxCoarseSZ=100)) as h:
+            for itmax in (1, 3, 9):
+                try:
+                    x, it, rv, flag, _ = h.pcg(b, itmax=itmax, tol=tol)
+                    out.append((x.tobytes(), it, rv.tobytes(), flag))
+                except cb.ChronosError as e:
+                    out.append(str(e))
+    assert out[:3] == out[3:]
