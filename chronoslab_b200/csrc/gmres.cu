@@ -71,11 +71,12 @@ __global__ void k_basis_combine(int n, int k, const double *__restrict__ V, int6
   }
 }
 
-// v = w / sqrt(*n2), nothing where the norm is zero.
+// v = w / sqrt(*n2), nothing where the norm is zero (a NaN norm passes into v, where
+// the next step's test finds it).
 __global__ void k_normalise(int n, const double *__restrict__ w, const double *__restrict__ n2,
                             double *__restrict__ v) {
   const double t = *n2;
-  if (!(t > 0.0)) return;
+  if (t == 0.0) return;
   const double s = 1.0 / sqrt(t);
   for (int r = blockIdx.x * blockDim.x + threadIdx.x; r < n; r += gridDim.x * blockDim.x)
     v[r] = s * w[r];

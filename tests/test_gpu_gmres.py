@@ -98,3 +98,17 @@ def test_reference_named_wrapper(lib):
         assert r1[1] == r2[1] == 0 and r1[3] == r2[3] and np.array_equal(r1[0], r2[0])
         x, flag, rel, it, rv = cb.gmres_RIGHT(h, b, None, 1e-8, 40)
         assert flag == 0 and it[0] == 1 and rel <= 1e-8
+
+
+def test_overflow_in_the_operator_stops_at_the_next_step(lib):
+    """An operator whose product overflows: the step's basis vector is not finite,
+    and the next application of the preconditioner ends the solve with flag 2, one
+    residual beyond the first recorded and the start vector returned."""
+    A = 1e-3 * PB.poisson7(10)
+    n = A.shape[0]
+    b = PB.uniform_rhs(n, seed=6)
+    huge = 1.7e308 * PB.poisson7(10).sign()
+    with cb.Hierarchy(A, np.ones((n, 1)), cb.params(precision=cb.CHRONOS_FP64)) as h:
+        x, flag, _, it, rv = h.gmres(b, restart=6, tol=1e-8, maxit=3, A=huge)
+    assert flag == 2 and tuple(it) == (0, 0) and not x.any()
+    assert rv.size == 2 and rv[0] == pytest.approx(np.linalg.norm(b), rel=1e-12) and np.isnan(rv[1])
