@@ -91,13 +91,15 @@ struct Prod {
   DBuf<double> v;
 };
 
+// p = x y; false, and p empty, where that is more work than a fold is worth.
 template <typename X, typename Y>
-Prod multiply(int m, int ncols, const X &x, const Y &y, cudaStream_t st) {
-  Prod p;
+bool multiply(int m, int ncols, const X &x, const Y &y, Prod &p, cudaStream_t st,
+              int64_t max_products) {
+  p = Prod();
   p.rows = m;
   p.cols = ncols;
-  spgemm_device(m, ncols, x.rp, x.ci, x.v, y.rp, y.ci, y.v, p.rp, p.ci, p.v, &p.nnz, st);
-  return p;
+  return spgemm_device(m, ncols, x.rp, x.ci, x.v, y.rp, y.ci, y.v, p.rp, p.ci, p.v, &p.nnz, st,
+                       max_products);
 }
 
 struct View {
@@ -124,6 +126,17 @@ bool add_identity(Prod &p, double sign, double add, cudaStream_t st) {
 // 0.65M entries) 53 / 49 / 43 / 35; poisson 48^3 FP32 (1.8M, 9.5M) 81 / 73 / 66 /
 // 101; poisson 64^3 FP32 (4.2M, 23M) 109 / 98 / 105 / 185.
 constexpr int64_t kFoldEntries = 2 << 20;
+// Products of two entries that any of the folds' sparse products may take: twice what
+// the largest kept one does (diffusion 64^3, level 2, S U: 15M; A S 9M at most), some
+// 6 ms.
+constexpr int64_t kFoldProducts = 16 * kFoldEntries;
+// Longest row of a factor of the products: a row that long is a chain of its entries
+// in one warp.  39,305 rows of which one couples to all others (a constraint) spent
+// 148 ms on the products and 98 on the rest of the setup, for 0.23 of 0.58 ms an
+// iteration; where the smoother's row is as long, A S fills as well.
+// Also the longest row of the two-matrix apply (32 lanes: 16 batches of four entries),
+// which has no other path for long rows, as the one-matrix applies do.
+constexpr int kFoldLongest = 2048;
 // A dense tail has at most kFoldDenseRows rows (FP64: 34 MB a product), where
 // the level's operator is dense enough (n^2 <= kFoldDenseRatio entries of A)
 // for the folded rows to be nearly full anyway.  Elasticity 17^3, FP64, 1629
@@ -144,13 +157,22 @@ int64_t smoother_bound(const DMat &G) {
 
 // Lanes per row of a two-matrix apply: one batch of four entries a lane covers
 // an average row, and as many more lanes, up to one an entry, as the GPU has
-// threads idle (the longest rows' batches are then shorter chains).
-int fold_lanes(int64_t entries, int rows) {
+// threads idle (the longest rows' batches are then shorter chains); a longest row far
+// above the average takes eight batches a lane at most.
+int fold_lanes(int64_t entries, int rows, int longest) {
   const double avg = (double)entries / std::max(rows, 1);
   const int64_t resident = (int64_t)num_sms() * 2048;
   int L = 1;
-  while (L < 32 && (4 * L < avg || (L < avg && (int64_t)rows * 2 * L <= resident / 4))) L *= 2;
+  while (L < 32 && (4 * L < avg || (L < avg && (int64_t)rows * 2 * L <= resident / 4) ||
+                    longest > 32 * L))
+    L *= 2;
   return L;
+}
+
+int longest_row(const DMat &M) {
+  int t = 0;
+  for (int i = 0; i < M.nrows; ++i) t = std::max(t, M.rp_h[i + 1] - M.rp_h[i]);
+  return t;
 }
 
 void adopt(Prod &p, DMat &d, bool fp32, cudaStream_t st) {
@@ -168,13 +190,17 @@ std::unique_ptr<Fold> fold_operators(const DMat &A, const DMat &G, const DMat &G
   // S replaces G and G' in both smoothing steps and spares a vector between
   // them; a factor with long rows fills up when it is squared
   const int64_t worth = 2 * G.nnz + 2 * (int64_t)n + kFoldEntries / 2;
-  if (!dense && smoother_bound(G) > 4 * worth) return nullptr;
-  Prod S = multiply(n, n, View(Gt), View(G), st);
+  // (a bound of 2^31 could also be a product that the row pointers cannot hold)
+  const int64_t most = std::min<int64_t>(4 * worth, INT32_MAX - 1);
+  if ((!dense && smoother_bound(G) > most) || longest_row(Gt) > kFoldLongest) return nullptr;
+  Prod S, U, R, Q, E, X;
+  if (!multiply(n, n, View(Gt), View(G), S, st, most)) return nullptr;
   if (!dense && S.nnz > worth) return nullptr;
   k_scale_values<<<std::max<int>(1, std::min<int64_t>(ceil_div(S.nnz, 256), num_sms() * 8)), 256,
                    0, st>>>(S.nnz, omega, S.v.get());
   CHRONOS_CHECK_LAUNCH();
-  auto smooth_only = [&] {
+  auto smooth_only = [&]() -> std::unique_ptr<Fold> {
+    if (S.nnz > worth) return nullptr;
     adopt(S, f->S, fp32, st);
     f->form = FOLD_SMOOTH;
     return std::move(f);
@@ -182,55 +208,61 @@ std::unique_ptr<Fold> fold_operators(const DMat &A, const DMat &G, const DMat &G
   // R has at least about as many entries as A, Q and E four times R's
   // (twice and more where its rows are short): no product that would be dropped
   if (!dense && (A.nnz < (int64_t)16 * n ? 2 : 1) * A.nnz > kFoldEntries) return smooth_only();
-  Prod U = multiply(n, n, View(A), S, st);
-  if (!add_identity(U, -1.0, 1.0, st)) return smooth_only();        // U = I - A S
-  Prod R = multiply(nc, n, View(Pt), U, st);
-  if (!dense && R.nnz > kFoldEntries) return smooth_only();
-  Prod Q, E;
-  bool all = dense || (3 * A.nnz <= kFoldEntries && 4 * R.nnz <= kFoldEntries);
-  if (all && add_identity(U, 1.0, 1.0, st)) {                       // I + U
-    Q = multiply(n, n, S, U, st);
-    U = Prod();
-    all = dense || Q.nnz <= kFoldEntries;
-    if (all) {
-      Prod X = multiply(n, n, S, View(A), st);
-      all = add_identity(X, -1.0, 1.0, st);                         // I - S A
-      if (all) E = multiply(n, nc, X, View(P), st);
-      all = all && (dense || Q.nnz + E.nnz <= kFoldEntries);
+  if (std::max(longest_row(A), longest_row(Pt)) > kFoldLongest) return smooth_only();
+  if (!multiply(n, n, View(A), S, U, st, kFoldProducts) || !add_identity(U, -1.0, 1.0, st) ||
+      !multiply(nc, n, View(Pt), U, R, st, kFoldProducts) ||        // U = I - A S
+      (!dense && R.nnz > kFoldEntries))
+    return smooth_only();
+  const bool all =
+      (dense || (3 * A.nnz <= kFoldEntries && 4 * R.nnz <= kFoldEntries)) &&
+      add_identity(U, 1.0, 1.0, st) &&                              // I + U
+      multiply(n, n, S, U, Q, st, kFoldProducts) && (dense || Q.nnz <= kFoldEntries) &&
+      multiply(n, n, S, View(A), X, st, kFoldProducts) &&
+      add_identity(X, -1.0, 1.0, st) &&                             // I - S A
+      multiply(n, nc, X, View(P), E, st, kFoldProducts) &&
+      (dense || Q.nnz + E.nnz <= kFoldEntries);
+  U = Prod();
+  X = Prod();
+  if (all && !dense) {
+    adopt(Q, f->Q, fp32, st);
+    adopt(E, f->E, fp32, st);
+    const int longest = std::max(longest_row(f->Q), longest_row(f->E));
+    if (longest <= kFoldLongest) {
+      adopt(S, f->S, fp32, st);
+      adopt(R, f->R, fp32, st);
+      f->lanes = fold_lanes(f->Q.nnz, n, longest);
+      f->R.wide = wide_rows(f->R, kWideTake);
+      f->form = FOLD_ALL;
+      return f;
     }
-  } else {
-    all = false;
+    f->Q = DMat();
+    f->E = DMat();
   }
-  if (!all) {
+  if (!all || !dense) {
+    if (S.nnz > worth || R.nnz > kFoldEntries) return smooth_only();
     adopt(S, f->S, fp32, st);
-    adopt(R, f->R, fp32, st);
-    f->lanes = fold_lanes(f->S.nnz + P.nnz, n);
-    f->form = FOLD_DOWN;
+    const int longest = std::max(longest_row(f->S), longest_row(P));
+    f->form = FOLD_SMOOTH;
+    if (longest <= kFoldLongest) {
+      adopt(R, f->R, fp32, st);
+      f->lanes = fold_lanes(f->S.nnz + P.nnz, n, longest);
+      f->form = FOLD_DOWN;
+    }
     return f;
   }
-  if (dense) {
-    f->D.alloc((size_t)n * n);
-    DBuf<double> Y((size_t)n * nc), tv;
-    DBuf<int> trp, tci;
-    csr_transpose_device(nc, n, R.nnz, R.rp, R.ci, R.v, trp, tci, tv, st);
-    k_sparse_dense<<<n, 256, 0, st>>>(nc, E.rp.get(), E.ci.get(), E.v.get(), B,
-                                      Y.get());
-    CHRONOS_CHECK_LAUNCH();
-    k_dense_tail<<<n, 256, sizeof(double) * nc, st>>>(n, nc, Y.get(), trp.get(), tci.get(),
-                                                      tv.get(), Q.rp.get(), Q.ci.get(),
-                                                      Q.v.get(), f->D.get());
-    CHRONOS_CHECK_LAUNCH();
-    CHRONOS_CUDA(cudaStreamSynchronize(st));
-    f->form = FOLD_DENSE;
-    return f;
-  }
-  adopt(S, f->S, fp32, st);
-  adopt(Q, f->Q, fp32, st);
-  adopt(E, f->E, fp32, st);
-  adopt(R, f->R, fp32, st);
-  f->lanes = fold_lanes(f->Q.nnz, n);
-  f->R.wide = wide_rows(f->R, kWideTake);
-  f->form = FOLD_ALL;
+  f->D.alloc((size_t)n * n);
+  DBuf<double> Y((size_t)n * nc), tv;
+  DBuf<int> trp, tci;
+  csr_transpose_device(nc, n, R.nnz, R.rp, R.ci, R.v, trp, tci, tv, st);
+  k_sparse_dense<<<n, 256, 0, st>>>(nc, E.rp.get(), E.ci.get(), E.v.get(), B,
+                                    Y.get());
+  CHRONOS_CHECK_LAUNCH();
+  k_dense_tail<<<n, 256, sizeof(double) * nc, st>>>(n, nc, Y.get(), trp.get(), tci.get(),
+                                                    tv.get(), Q.rp.get(), Q.ci.get(),
+                                                    Q.v.get(), f->D.get());
+  CHRONOS_CHECK_LAUNCH();
+  CHRONOS_CUDA(cudaStreamSynchronize(st));
+  f->form = FOLD_DENSE;
   return f;
 }
 

@@ -91,10 +91,12 @@ int fsai_bucket_set_count();
 
 // ---- Galerkin (setup_kernels.cu) ---------------------------------------------
 // C = X * Y (X: m x k, Y: k x ncols), Gustavson accumulation order, exact
-// zeros dropped, columns sorted.  Output arrays allocated here.
-void spgemm_device(int m, int ncols, const int *xrp, const int *xci, const double *xv,
+// zeros dropped, columns sorted.  Output arrays allocated here.  max_products > 0:
+// false, and nothing formed, where the sum takes more products than that.
+bool spgemm_device(int m, int ncols, const int *xrp, const int *xci, const double *xv,
                    const int *yrp, const int *yci, const double *yv, DBuf<int> &crp,
-                   DBuf<int> &cci, DBuf<double> &cv, int64_t *nnz_c, cudaStream_t st);
+                   DBuf<int> &cci, DBuf<double> &cv, int64_t *nnz_c, cudaStream_t st,
+                   int64_t max_products = 0);
 
 // ---- dense coarse level (setup_kernels.cu) ----------------------------------
 // In-place lower Cholesky of the n x n column-major A (device); returns 0 or

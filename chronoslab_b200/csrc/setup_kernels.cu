@@ -574,16 +574,22 @@ std::vector<int> fsai_numeric_batched(const std::vector<FsaiJob> &jobs, cudaStre
 // Sparse product C = X * Y with per-row hash tables in global memory
 // =============================================================================
 
+// prod[i]: the products of row i; their sum added to *sum unless that is null.
 __global__ void k_spgemm_products(int m, const int *xrp, const int *xci, const int *yrp,
-                                  int64_t *prod) {
+                                  int64_t *prod, int64_t *sum) {
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= m) return;
   int64_t s = 0;
-  for (int k = xrp[i]; k < xrp[i + 1]; ++k) {
-    const int j = xci[k];
-    s += yrp[j + 1] - yrp[j];
+  if (i < m) {
+    for (int k = xrp[i]; k < xrp[i + 1]; ++k) {
+      const int j = xci[k];
+      s += yrp[j + 1] - yrp[j];
+    }
+    prod[i] = s;
   }
-  prod[i] = s;
+  if (!sum) return;
+  s = warp_sum(s);
+  if ((threadIdx.x & 31) == 0 && s > 0)
+    atomicAdd(reinterpret_cast<unsigned long long *>(sum), (unsigned long long)s);
 }
 
 __device__ __forceinline__ unsigned hash_slot(int key, unsigned mask) {
@@ -747,7 +753,9 @@ __global__ void __launch_bounds__(32 * SpgemmClass<SLOTS>::warps)
 k_spgemm_symbolic_sm(int m, int ncols, int lo, const int *__restrict__ xrp,
                      const int *__restrict__ xci, const int *__restrict__ yrp,
                      const int *__restrict__ yci, const int64_t *__restrict__ prod,
-                     int *__restrict__ cnt, int *nbig) {
+                     int *__restrict__ cnt, int *nbig, const int64_t *__restrict__ sum,
+                     int64_t max_products) {
+  if (sum && *sum > max_products) return;
   constexpr int W = SpgemmClass<SLOTS>::warps;
   constexpr bool TOP = SLOTS == kSpgemmSmSlots;
   extern __shared__ int spg_keys[];
@@ -891,14 +899,16 @@ k_spgemm_numeric_sm(int m, int lo, const int *__restrict__ xrp, const int *__res
 template <int SLOTS>
 static void spgemm_symbolic(int m, int ncols, int lo, const int *xrp, const int *xci,
                             const int *yrp, const int *yci, const int64_t *prod, int *cnt,
-                            int *nbig, cudaStream_t st) {
+                            int *nbig, const int64_t *sum, int64_t max_products,
+                            cudaStream_t st) {
   using C = SpgemmClass<SLOTS>;
   const int grid = std::max(1, std::min<int>(ceil_div(m, C::warps), num_sms() * 16));
   const size_t smem = (size_t)C::warps * SLOTS * sizeof(int);
   CHRONOS_CUDA(cudaFuncSetAttribute(k_spgemm_symbolic_sm<SLOTS>,
                                     cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
   k_spgemm_symbolic_sm<SLOTS><<<grid, 32 * C::warps, smem, st>>>(m, ncols, lo, xrp, xci, yrp, yci,
-                                                                 prod, cnt, nbig);
+                                                                 prod, cnt, nbig, sum,
+                                                                 max_products);
   CHRONOS_CHECK_LAUNCH();
 }
 
@@ -965,18 +975,23 @@ static unsigned next_pow2(uint64_t v) {
   return (unsigned)p;
 }
 
-void spgemm_device(int m, int ncols, const int *xrp, const int *xci, const double *xv,
+bool spgemm_device(int m, int ncols, const int *xrp, const int *xci, const double *xv,
                    const int *yrp, const int *yci, const double *yv, DBuf<int> &crp,
-                   DBuf<int> &cci, DBuf<double> &cv, int64_t *nnz_c, cudaStream_t st) {
+                   DBuf<int> &cci, DBuf<double> &cv, int64_t *nnz_c, cudaStream_t st,
+                   int64_t max_products) {
   crp.alloc((size_t)m + 1);
   if (m == 0) {
     crp.zero(st);
     *nnz_c = 0;
-    return;
+    return true;
   }
   DBuf<int64_t> dprod((size_t)m + 1), drps((size_t)m + 1);
   DBuf<unsigned char> tmp;
-  k_spgemm_products<<<ceil_div(m, 256), 256, 0, st>>>(m, xrp, xci, yrp, dprod.get());
+  // the products' sum behind the row counts; the symbolic kernels do nothing where
+  // it is too large
+  int64_t *sum = max_products > 0 ? dprod.get() + m : nullptr;
+  if (sum) CHRONOS_CUDA(cudaMemsetAsync(sum, 0, sizeof(int64_t), st));
+  k_spgemm_products<<<ceil_div(m, 256), 256, 0, st>>>(m, xrp, xci, yrp, dprod.get(), sum);
   CHRONOS_CHECK_LAUNCH();
   // symbolic: in each warp's shared table; rows whose distinct columns outgrow
   // the largest (cnt = -1) again in global tables sized from their products.
@@ -984,15 +999,22 @@ void spgemm_device(int m, int ncols, const int *xrp, const int *xci, const doubl
   DBuf<int> counts(2 * ((size_t)m + 1) + 1);
   int *cnt = counts.get(), *cnt2 = cnt + m + 1, *dnbig = cnt2 + m + 1;
   counts.zero(st);
-  spgemm_symbolic<256>(m, ncols, 0, xrp, xci, yrp, yci, dprod.get(), cnt, dnbig, st);
-  spgemm_symbolic<1024>(m, ncols, 128, xrp, xci, yrp, yci, dprod.get(), cnt, dnbig, st);
-  spgemm_symbolic<kSpgemmSmSlots>(m, ncols, 512, xrp, xci, yrp, yci, dprod.get(), cnt, dnbig, st);
+  spgemm_symbolic<256>(m, ncols, 0, xrp, xci, yrp, yci, dprod.get(), cnt, dnbig, sum,
+                       max_products, st);
+  spgemm_symbolic<1024>(m, ncols, 128, xrp, xci, yrp, yci, dprod.get(), cnt, dnbig, sum,
+                        max_products, st);
+  spgemm_symbolic<kSpgemmSmSlots>(m, ncols, 512, xrp, xci, yrp, yci, dprod.get(), cnt, dnbig, sum,
+                                  max_products, st);
   scan_counts(m, cnt, drps.get(), tmp, st);
   int64_t total = 0;
   int nbig = 0;
   CHRONOS_CUDA(cudaMemcpyAsync(&total, drps.get() + m, sizeof(total), cudaMemcpyDeviceToHost, st));
   CHRONOS_CUDA(cudaMemcpyAsync(&nbig, dnbig, sizeof(nbig), cudaMemcpyDeviceToHost, st));
+  int64_t products = 0;
+  if (sum)
+    CHRONOS_CUDA(cudaMemcpyAsync(&products, sum, sizeof(products), cudaMemcpyDeviceToHost, st));
   CHRONOS_CUDA(cudaStreamSynchronize(st));
+  if (products > max_products) return false;
   std::vector<int> cnt_h;
   if (nbig > 0) {
     cnt_h.resize(m);
@@ -1112,6 +1134,7 @@ void spgemm_device(int m, int ncols, const int *xrp, const int *xci, const doubl
   }
   CHRONOS_CUDA(cudaStreamSynchronize(st));
   *nnz_c = nnz;
+  return true;
 }
 
 // =============================================================================

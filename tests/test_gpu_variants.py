@@ -521,3 +521,46 @@ def test_loops_agree_at_odd_tolerances(lib, prec, problem, tol):
                 except cb.ChronosError as e:
                     out.append(str(e))
     assert out[:3] == out[3:]
+
+
+def _with_hub(nx, reach):
+    """poisson7(nx) and one node before it, coupled to the first `reach` nodes."""
+    from chronoslab_b200 import problems as PB
+    m = nx ** 3
+    c = np.zeros(m)
+    c[:reach] = -0.5
+    A = sp.bmat([[sp.csr_matrix([[0.5 * reach + 2.0]]), sp.csr_matrix(c)],
+                 [sp.csr_matrix(c[:, None]), PB.poisson7(nx) + sp.identity(m)]], format="csr")
+    A.sort_indices()
+    return A
+
+
+@pytest.mark.parametrize("prec,tol", [(cb.CHRONOS_FP64, 1e-12), (cb.CHRONOS_FP32, 2e-5)])
+@pytest.mark.parametrize("nx,reach", [(11, 1331), (13, 2197), (20, 500), (20, 2040), (20, 2050),
+                                      (30, 27000), (40, 1500)])
+def test_folded_levels_with_a_hub_row(lib, nx, reach, prec, tol):
+    """One row of the smoother with up to all columns (below, at and above what the
+    two-matrix apply takes): the operator form's cycle, and the same iterations."""
+    A = _with_hub(nx, reach)
+    n = A.shape[0]
+    b = np.random.default_rng(nx).standard_normal(n)
+    prm = dict(precision=prec, ntv=1, maxCoarseSZ=400)
+    with cb.Hierarchy(A, np.ones((n, 1)), cb.params(**prm)) as hf, \
+            cb.Hierarchy(A, np.ones((n, 1)), cb.params(spmv_format=1, **prm)) as hp:
+        xf, xp = hf.vcycle(b), hp.vcycle(b)
+        assert np.linalg.norm(xf - xp) <= tol * np.linalg.norm(xp)
+        r1, r2 = hf.pcg(b, tol=1e-8), hp.pcg(b, tol=1e-8)
+        assert r1[3] == r2[3] == 0 and abs(r1[1] - r2[1]) <= 1
+
+
+def test_hub_row_does_not_fill_the_setup(lib):
+    """39,305 rows, one coupled to all others: A S would have 1.5e9 entries, which no
+    fold keeps.  Folding and tuning take no longer than the rest of the setup."""
+    A = _with_hub(34, 34 ** 3)
+    with cb.Hierarchy(A, np.ones((A.shape[0], 1)), cb.params(
+            precision=cb.CHRONOS_FP64, ntv=1)) as h:
+        t = h.setup_times()
+    with cb.Hierarchy(A, np.ones((A.shape[0], 1)), cb.params(
+            precision=cb.CHRONOS_FP64, ntv=1)) as h:
+        t = h.setup_times()
+    assert t["autotune"] <= t["total"] - t["autotune"]
