@@ -11,6 +11,7 @@
 // deterministic grid reductions.
 #include <algorithm>
 #include <cmath>
+#include <type_traits>
 
 #include "hier.h"
 #include "spmv.cuh"
@@ -232,6 +233,21 @@ enum { BS_BNORM = 0, BS_PTAP, BS_ALPHA, BS_PRES_AXP, BS_RESITER, BS_ITER, BS_ACT
 // after the K-wide arrays: tol, itmax
 __host__ __device__ constexpr int bs_off(int which, int K) { return which * K; }
 
+// dst[j] = A(:,j)'B(:,j)
+template <int K>
+__global__ void __launch_bounds__(256)
+k_bdot(int n, const double *__restrict__ A, const double *__restrict__ B, double *part,
+       unsigned *ticket, double *dst) {
+  pdl_begin();
+  double s = 0.0;
+  const size_t total = (size_t)n * K;
+  for (size_t o = blockIdx.x * (size_t)blockDim.x + threadIdx.x; o < total;
+       o += (size_t)gridDim.x * blockDim.x)
+    s += A[o] * B[o];
+  double vals[1][1] = {{s}};
+  grid_reduce_cols<K, 1, 1>(vals, part, ticket, StoreK<K>{dst});
+}
+
 template <typename T, typename BT, typename OT, int K>
 static void vcycle_block(Hier &h, BlockState &s, int l, const BT *b, OT *out, const double *dw,
                          double *dot_out);
@@ -251,6 +267,10 @@ static void vcycle_block(Hier &h, BlockState &s, int l, const BT *b, OT *out, co
   if (L.coarsest) {
     launch_pdl(k_dense_matmat<BT, OT, K>, n, 256, st, n, (const double *)L.W.get(), b, out);
     CHRONOS_CHECK_LAUNCH();
+    if constexpr (std::is_same_v<OT, double>)
+      if (dw)                                   // a single-level hierarchy
+        launch_pdl(k_bdot<K>, std::min(num_sms() * 4, (int)ceil_div((int64_t)n * K, 256)), 256,
+                   st, n, (const double *)out, dw, part, tick, dot_out);
     return;
   }
   T *x = blk<T>(s.x32, s.x64, l), *r = blk<T>(s.r32, s.r64, l), *t = blk<T>(s.t32, s.t64, l);
@@ -478,19 +498,6 @@ k_bpcg_xr_update(int n, double *__restrict__ x, double *__restrict__ res,
 
 // ||B(:,j)||^2 and ||R(:,j)||^2 into sc (BNORM, RESITER hold squares until init)
 template <int K>
-__global__ void __launch_bounds__(256)
-k_bnorm2(int n, const double *__restrict__ B, double *part, unsigned *ticket, double *dst) {
-  pdl_begin();
-  double s = 0.0;
-  const size_t total = (size_t)n * K;
-  for (size_t o = blockIdx.x * (size_t)blockDim.x + threadIdx.x; o < total;
-       o += (size_t)gridDim.x * blockDim.x)
-    s += B[o] * B[o];
-  double vals[1][1] = {{s}};
-  grid_reduce_cols<K, 1, 1>(vals, part, ticket, StoreK<K>{dst});
-}
-
-template <int K>
 __global__ void k_bpcg_init(double *sc, const double *b2, const double *r2, double tol,
                             double itmax) {
   pdl_begin();
@@ -642,9 +649,10 @@ static void block_solve(Hier &h, int m, const BlockIn &B, const double *X0_h, do
   spmm<double, double, double, double, K, MODE_RESID, false>(st, A, A.v64.get(), s.x.get(), b,
                                                              s.res.get(), 1.0);
   const int nb = std::max(1, std::min(num_sms() * 8, (int)ceil_div((int64_t)n * K, 256)));
-  launch_pdl(k_bnorm2<K>, nb, 256, st, n, (const double *)b, s.part.get(),
+  launch_pdl(k_bdot<K>, nb, 256, st, n, (const double *)b, (const double *)b, s.part.get(),
              s.tickets.get() + 3 * kReduceTickets, b2);
-  launch_pdl(k_bnorm2<K>, nb, 256, st, n, (const double *)s.res.get(), s.part.get(),
+  launch_pdl(k_bdot<K>, nb, 256, st, n, (const double *)s.res.get(), (const double *)s.res.get(),
+             s.part.get(),
              s.tickets.get() + 3 * kReduceTickets, r2);
   launch_pdl(k_bpcg_init<K>, 1, K, st, s.sc.get(), (const double *)b2, (const double *)r2, tol,
              (double)itmax);

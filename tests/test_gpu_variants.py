@@ -564,3 +564,27 @@ def test_hub_row_does_not_fill_the_setup(lib):
             precision=cb.CHRONOS_FP64, ntv=1)) as h:
         t = h.setup_times()
     assert t["autotune"] <= t["total"] - t["autotune"]
+
+
+@pytest.mark.parametrize("nrhs", [1, 2, 5, 16])
+@pytest.mark.parametrize("prec", [cb.CHRONOS_FP64, cb.CHRONOS_FP32])
+def test_single_level_block(lib, nrhs, prec):
+    """A problem that is its own coarsest level, with a condition of 1e12: the inverse
+    is good to a few digits and a solve takes several steps.  Each column takes the
+    steps of its own solve, whatever the memory of the block's scalars held before
+    (not-a-numbers here)."""
+    n = 120
+    Q, _ = np.linalg.qr(np.random.default_rng(2).standard_normal((n, n)))
+    D = (Q * np.logspace(-12, 0, n)) @ Q.T
+    A = sp.csr_matrix(0.5 * (D + D.T))
+    B = A @ np.random.default_rng(3).standard_normal((n, nrhs))
+    with cb.Hierarchy(A, np.ones((n, 1)), cb.params(precision=prec, ntv=1, exact_outer=1)) as h:
+        assert h.nlevels == 1
+        single = [h.pcg(np.ascontiguousarray(B[:, j]), itmax=40, tol=1e-14) for j in range(nrhs)]
+        for k in 3 * list(range(3, 40)):
+            with pytest.raises(cb.ChronosError):
+                cb.dense_chol(np.full((k, k), np.nan))
+        X, its, flags, _ = h.pcg_block(B, itmax=40, tol=1e-14)
+        for j in range(nrhs):
+            _, it, rv, flag, _ = single[j]
+            assert flag == flags[j] == 0 and it >= 2 and abs(int(its[j]) - it) <= 1, (it, its[j])
