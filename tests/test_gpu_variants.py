@@ -588,3 +588,34 @@ def test_single_level_block(lib, nrhs, prec):
         for j in range(nrhs):
             _, it, rv, flag, _ = single[j]
             assert flag == flags[j] == 0 and it >= 2 and abs(int(its[j]) - it) <= 1, (it, its[j])
+
+
+@pytest.mark.parametrize("nrhs", [3, 16, 17, 35])
+def test_row_major_blocks_of_any_width(lib, nrhs):
+    """chronos_pcg_block_rows on row-major right-hand sides, wider than one solve's 16
+    columns too (rows then lie apart), with and without start vectors: the bits of the
+    column-major call."""
+    import ctypes as C
+    from chronoslab_b200 import problems as PB
+    A = PB.poisson7(11)
+    n = A.shape[0]
+    rng = np.random.default_rng(nrhs)
+    B, X0 = rng.standard_normal((n, nrhs)), rng.standard_normal((nrhs, n))
+    pd, pi = C.POINTER(C.c_double), C.POINTER(C.c_int)
+
+    def solve(h, b, rows, x0):
+        x, its, fl = np.full((nrhs, n), 7.0), np.zeros(nrhs, np.int32), np.ones(nrhs, np.int32)
+        cb.check(lib.chronos_pcg_block_rows(
+            h._h, nrhs, b.ctypes.data_as(pd), rows, None if x0 is None else x0.ctypes.data_as(pd),
+            x.ctypes.data_as(pd), 200, 1e-8, its.ctypes.data_as(pi), fl.ctypes.data_as(pi), None,
+            None))
+        assert not fl.any()
+        return x, its
+
+    with cb.Hierarchy(A, np.ones((n, 1)), cb.params(ntv=1, maxCoarseSZ=100)) as h:
+        for x0 in (None, X0):
+            by_rows = solve(h, np.ascontiguousarray(B), 1, x0)
+            by_cols = solve(h, np.ascontiguousarray(B.T), 0, x0)
+            assert np.array_equal(by_rows[0], by_cols[0]) and np.array_equal(by_rows[1], by_cols[1])
+            assert np.all(np.linalg.norm(B - A @ by_rows[0].T, axis=0)
+                          <= 1e-8 * np.linalg.norm(B, axis=0))
