@@ -233,6 +233,7 @@ int chronos_batch_solve(chronos_batch *bt, const double *const *b_h, double *con
       group_solve(*B.group, bb, xx, itmax, tol, iters, flags, seconds);
       return;
     }
+    DeferFrees together(false);
     std::vector<DBuf<double>> bd(np), xd(np);
     std::vector<char> zero(np, 0);
     for (int p = 0; p < np; ++p) {
@@ -281,6 +282,7 @@ int chronos_batch_solve(chronos_batch *bt, const double *const *b_h, double *con
     cudaEventDestroy(start);
     for (auto &e : done) cudaEventDestroy(e);
     stream_destroy(fork);
+    together.start();
     if (seconds) *seconds = ms * 1e-3;
   });
 }
@@ -311,7 +313,10 @@ int chronos_batch_info(const chronos_batch *bt, int p, int *nlev, int *n0) {
 }
 
 int chronos_batch_free(chronos_batch *bt) {
-  return batch_guard([&] { delete bt; });
+  return batch_guard([&] {
+    DeferFrees together;                 // a wait for every stream once, not once a buffer
+    delete bt;
+  });
 }
 
 }  // extern "C"

@@ -790,7 +790,10 @@ int chronos_amg_setup_prolong(const chronos_params *prm, int n, const int *iat_h
 }
 
 int chronos_hier_free(chronos_hier *h) {
-  return guard([&] { delete h; });
+  return guard([&] {
+    DeferFrees together;                 // a wait for every stream once, not once a buffer
+    delete h;
+  });
 }
 
 int chronos_device_bytes(int64_t *bytes) {
@@ -1090,6 +1093,7 @@ int chronos_gmres(chronos_hier *hh, const int *iat_h, const int *ja_h, const dou
       csr_apply<double, double, double, double, MODE_PLAIN, false>(st, op.lanes, n, op.rp, op.ci,
                                                                   op.v64, x, nullptr, y, 1.0);
     };
+    DeferFrees together(false);
     DBuf<double> b, x;
     b.upload(b_h, n, st);
     x.upload(x_h, n, st);
@@ -1103,6 +1107,7 @@ int chronos_gmres(chronos_hier *hh, const int *iat_h, const int *ja_h, const dou
     *flag = r.flag;
     if (nresvec) *nresvec = (int)r.resvec.size();
     if (resvec_h) std::memcpy(resvec_h, r.resvec.data(), sizeof(double) * r.resvec.size());
+    together.start();
   });
 }
 
@@ -1114,6 +1119,7 @@ int chronos_adjoint_grad(chronos_hier *hh, const double *u_h, const double *g_h,
     Hier &h = *hh->h;
     const int n = h.levels[0].n;
     const DMat &A = h.levels[0].A;
+    DeferFrees together(false);
     DBuf<double> u, g, lam(n), grad(std::max<int64_t>(A.nnz, 1));
     u.upload(u_h, n, h.st);
     g.upload(g_h, n, h.st);
@@ -1125,6 +1131,7 @@ int chronos_adjoint_grad(chronos_hier *hh, const double *u_h, const double *g_h,
     grad.download(grad_h, A.nnz, h.st);
     CHRONOS_CUDA(cudaStreamSynchronize(h.st));
     *iters = it;
+    together.start();
     CHRONOS_REQUIRE(fl == 0, CHRONOS_EBREAKDOWN, "adjoint solve did not converge");
   });
 }

@@ -234,11 +234,13 @@ class OnDevice {
 // while a batch setup builds hierarchies on several host threads, one
 // thread's free of a setup temporary would wait for every other thread's
 // queued kernels; and nothing can be waited for while a caller's capture holds a
-// handle's stream: such a buffer is kept until a later free.
+// handle's stream: such a buffer is kept until a later free.  A free of many
+// buffers also takes one wait this way: 64 problems with a stream each took 590 ms
+// to free with a wait a buffer (335 with cudaFree), 36 ms with one.
 // Inside a DeferFrees scope (any thread) the buffers a DBuf
 // lets go of are kept -- never reused -- and freed, after one wait for the
-// streams, when the outermost scope ends or an allocation would be refused.  They stay counted in
-// device_bytes_live() until then.
+// streams, when the outermost scope ends or an allocation would be refused.
+// They stay counted in device_bytes_live() until then.
 struct DeferredFrees {
   struct Entry { void *p; int64_t bytes; DevicePool *pool; };
   std::mutex mu;
@@ -327,12 +329,21 @@ inline bool device_room(int64_t bytes) {
 }
 class DeferFrees {
  public:
-  DeferFrees() { deferred_frees().depth++; }
+  explicit DeferFrees(bool from_here = true) { if (from_here) start(); }
+  // (a function that lets go of several buffers at its end makes one such object in
+  // front of them and starts it there: one wait for them all)
+  void start() {
+    if (!on_) deferred_frees().depth++;
+    on_ = true;
+  }
   ~DeferFrees() {
-    if (--deferred_frees().depth == 0) flush_deferred_frees();
+    if (on_ && --deferred_frees().depth == 0) flush_deferred_frees();
   }
   DeferFrees(const DeferFrees &) = delete;
   DeferFrees &operator=(const DeferFrees &) = delete;
+
+ private:
+  bool on_ = false;
 };
 
 // Owning device allocation (from the device's pool), movable, typed.

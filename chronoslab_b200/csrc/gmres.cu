@@ -123,6 +123,7 @@ void gmres_right_device(Hier &h, const std::function<void(const double *, double
     return;
   }
   const int64_t ld = n;
+  DeferFrees together(false);
   DBuf<double> V((size_t)(inner + 1) * n), r(n), w(n), z(n), xm(n), xmin(n), part;
   // projections of the two passes and the norm's square, read together
   DBuf<double> hd(2 * (size_t)inner + 3);
@@ -360,6 +361,7 @@ void gmres_right_device(Hier &h, const std::function<void(const double *, double
   if (flag == 2 && initer != 0 && !resvec.empty()) resvec.pop_back();
   res.resvec = std::move(resvec);
   CHRONOS_CUDA(cudaStreamSynchronize(st));
+  together.start();
 }
 
 }  // namespace chronos

@@ -224,3 +224,23 @@ def test_sqmr_state_is_no_reason_to_refuse(lib, tmp_path):
         held + 2 * 700000 + 9 * 8 * n)
     assert got[0] == 1 and got[1] <= 1.1e-8 and got[3] == 0
     assert got[2] <= held + 2 * 700000 + 7 * 8 * n
+
+
+def test_freeing_a_batch_takes_one_wait(lib):
+    """Freeing 48 problems, each with a stream of its own, takes per problem no more
+    than three times what freeing 6 takes (a wait for every stream at each buffer made
+    it ten times)."""
+    import time
+
+    def close_time(count):
+        As = [PB.poisson7(10) for _ in range(count)]
+        best = np.inf
+        for _ in range(3):
+            h = cb.Batch(As, cb.params(ntv=1, maxCoarseSZ=100, batch_grouped=0))
+            t = time.perf_counter()
+            h.close()
+            best = min(best, time.perf_counter() - t)
+        return best / count
+
+    few = close_time(6)
+    assert close_time(48) <= 3.0 * few
