@@ -6,8 +6,9 @@
 // column index is fetched once (a broadcast) and reused K times, and the
 // gathers X[c*K + 0..K-1] are K-wide coalesced loads.  Each column keeps its
 // own scalars, iteration count and stopping test; a converged column is frozen
-// (its x, res and p no longer change), so every column returns exactly what a
-// single-column PCG_CJ returns.  The block dot products are K-wide
+// (its x, res and p no longer change), so every column takes the steps of its own
+// PCG_CJ, to rounding: a block cycle folds fewer levels, and sums its rows in
+// another order, than a single vector's.  The block dot products are K-wide
 // deterministic grid reductions.
 #include <algorithm>
 #include <cmath>
@@ -229,7 +230,7 @@ struct BlockState {
 
 // per-column scalar arrays (each K wide) inside sc
 enum { BS_BNORM = 0, BS_PTAP, BS_ALPHA, BS_PRES_AXP, BS_RESITER, BS_ITER, BS_ACTIVE, BS_FLAG,
-       BS_PRES, BS_COUNT };
+       BS_COUNT };
 // after the K-wide arrays: tol, itmax
 __host__ __device__ constexpr int bs_off(int which, int K) { return which * K; }
 

@@ -423,8 +423,9 @@ int fsai_numeric_device(int n, const int *arp, const int *aci, const double *av,
 
 // -----------------------------------------------------------------------------
 // FSAI numeric phase of many problems at once (a batch's level): every row of
-// every problem goes to the smallest shared-memory tile (MMAX) that holds its
-// local system, and each tile size is one launch over all problems' rows.
+// every problem goes to the smallest tile (MMAX: lanes and registers up to 32
+// unknowns, shared memory above) that holds its local system, and each tile size is
+// one launch over all problems' rows.
 // Which tile sizes exist -- the bucket edges -- is chosen per batch shape by
 // timing the candidate sets below on the batch's own rows (CUDA events); a
 // row's arithmetic does not depend on its tile, so every set gives the same
@@ -702,11 +703,9 @@ __global__ void k_spgemm_numeric(int r0, int r1, const int *rows, const int *xrp
 // sort; now 1.5 ms together.
 constexpr int kSpgemmSmSlots = 4096;
 
-// One class of rows: table slots, the largest count that may use it, warps per
-// block.
+// One class of rows, of at most SLOTS / 2 distinct columns: warps per block.
 template <int SLOTS> struct SpgemmClass {
   static constexpr int warps = SLOTS <= 1024 ? 8 : 4;
-  static constexpr int max_count = SLOTS / 2;
 };
 
 // Entries [k0, k0 + 32) of row X: lane l holds entry k0 + l's value, the offset
@@ -1387,8 +1386,8 @@ k_gram(int n, const double *__restrict__ X, double *__restrict__ W) {
 }
 
 void dense_inverse_from_chol(int n, const double *L, double *W, cudaStream_t st) {
-  CHRONOS_REQUIRE((size_t)n * sizeof(double) <= 200 * 1024, CHRONOS_ENOTSUP,
-                  "coarsest level too large for the dense solve");
+  // (beyond 25,600 rows an array of the dense solve takes 5.2 GB)
+  CHRONOS_REQUIRE(n <= 25600, CHRONOS_ENOTSUP, "coarsest level too large for the dense solve");
   DBuf<double> X((size_t)n * n);
   X.zero(st);
   k_tri_inverse_diag<<<ceil_div(n, kCholNb), 32, 0, st>>>(n, L, X.get());
@@ -1406,8 +1405,9 @@ void dense_inverse_from_chol(int n, const double *L, double *W, cudaStream_t st)
   CHRONOS_CUDA(cudaStreamSynchronize(st));
 }
 
-// x = W b: NT threads a row, at most eight loads of W each up to 8 NT columns and
-// all of them in flight.  With a warp a row and four in flight the product was a
+// x = W b: NT threads a row, each with eight loads of W in flight: the whole row up
+// to 2048 columns, longer rows (a single level or one that stopped coarsening) in
+// rounds of 2048.  With a warp a row and four in flight the product was a
 // chain of batches on 8 warps an SM: 1212 rows of the folded tail of elasticity
 // 45^3 (11.8 MB, from L2) 11.5 us, now 6.1; 208 rows 3.6 and 2.5 us.  (Rows of many
 // small systems at once, k_group_dense, fill the GPU with a warp each.)
