@@ -319,13 +319,15 @@ inline bool device_room(int64_t bytes) {
   give_back();
   const int64_t cap = device_alloc_cap();
   if (cap > 0 && device_bytes_live().load() + bytes > cap) return false;
-  size_t avail = 0, total = 0;
   uint64_t held = 0, used = 0;
   DevicePool &pool = device_pool();
-  CHRONOS_CUDA(cudaMemGetInfo(&avail, &total));
   CHRONOS_CUDA(cudaMemPoolGetAttribute(pool.pool, cudaMemPoolAttrReservedMemCurrent, &held));
   CHRONOS_CUDA(cudaMemPoolGetAttribute(pool.pool, cudaMemPoolAttrUsedMemCurrent, &used));
-  return (int64_t)avail + (int64_t)(held - std::min(used, held)) >= bytes;
+  const int64_t idle = (int64_t)(held - std::min(used, held));
+  if (idle >= bytes) return true;
+  size_t avail = 0, total = 0;
+  CHRONOS_CUDA(cudaMemGetInfo(&avail, &total));
+  return (int64_t)avail + idle >= bytes;
 }
 class DeferFrees {
  public:

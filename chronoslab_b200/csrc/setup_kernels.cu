@@ -575,9 +575,10 @@ std::vector<int> fsai_numeric_batched(const std::vector<FsaiJob> &jobs, cudaStre
 // Sparse product C = X * Y with per-row hash tables in global memory
 // =============================================================================
 
-// prod[i]: the products of row i; their sum added to *sum unless that is null.
-__global__ void k_spgemm_products(int m, const int *xrp, const int *xci, const int *yrp,
-                                  int64_t *prod, int64_t *sum) {
+// prod[i]: the products of row i; their sum added to *sum.
+__global__ void __launch_bounds__(256)
+k_spgemm_products(int m, const int *xrp, const int *xci, const int *yrp, int64_t *prod, int64_t *sum) {
+  __shared__ int64_t warp[8];
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   int64_t s = 0;
   if (i < m) {
@@ -587,10 +588,14 @@ __global__ void k_spgemm_products(int m, const int *xrp, const int *xci, const i
     }
     prod[i] = s;
   }
-  if (!sum) return;
   s = warp_sum(s);
-  if ((threadIdx.x & 31) == 0 && s > 0)
+  if ((threadIdx.x & 31) == 0) warp[threadIdx.x >> 5] = s;
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    s = 0;
+    for (int w = 0; w < 8; ++w) s += warp[w];
     atomicAdd(reinterpret_cast<unsigned long long *>(sum), (unsigned long long)s);
+  }
 }
 
 __device__ __forceinline__ unsigned hash_slot(int key, unsigned mask) {
@@ -754,7 +759,7 @@ k_spgemm_symbolic_sm(int m, int ncols, int lo, const int *__restrict__ xrp,
                      const int *__restrict__ yci, const int64_t *__restrict__ prod,
                      int *__restrict__ cnt, int *nbig, const int64_t *__restrict__ sum,
                      int64_t max_products) {
-  if (sum && *sum > max_products) return;
+  if (*sum > max_products) return;            // more than the caller wants formed
   constexpr int W = SpgemmClass<SLOTS>::warps;
   constexpr bool TOP = SLOTS == kSpgemmSmSlots;
   extern __shared__ int spg_keys[];
@@ -984,36 +989,35 @@ bool spgemm_device(int m, int ncols, const int *xrp, const int *xci, const doubl
     *nnz_c = 0;
     return true;
   }
-  DBuf<int64_t> dprod((size_t)m + 1), drps((size_t)m + 1);
+  const int64_t most = max_products > 0 ? max_products : INT64_MAX;
+  // behind the row offsets: the products' sum and the rows beyond the tables, read
+  // with the offsets' last in one copy
+  DBuf<int64_t> dprod((size_t)m + 1), drps((size_t)m + 3);
+  int64_t *sum = drps.get() + m + 1;
+  int *dnbig = reinterpret_cast<int *>(sum + 1);
+  CHRONOS_CUDA(cudaMemsetAsync(sum, 0, 2 * sizeof(int64_t), st));
   DBuf<unsigned char> tmp;
-  // the products' sum behind the row counts; the symbolic kernels do nothing where
-  // it is too large
-  int64_t *sum = max_products > 0 ? dprod.get() + m : nullptr;
-  if (sum) CHRONOS_CUDA(cudaMemsetAsync(sum, 0, sizeof(int64_t), st));
   k_spgemm_products<<<ceil_div(m, 256), 256, 0, st>>>(m, xrp, xci, yrp, dprod.get(), sum);
   CHRONOS_CHECK_LAUNCH();
   // symbolic: in each warp's shared table; rows whose distinct columns outgrow
   // the largest (cnt = -1) again in global tables sized from their products.
-  // counts: cnt (m + 1), emitted (m + 1), rows beyond the tables
-  DBuf<int> counts(2 * ((size_t)m + 1) + 1);
-  int *cnt = counts.get(), *cnt2 = cnt + m + 1, *dnbig = cnt2 + m + 1;
+  // counts: cnt (m + 1), emitted (m + 1)
+  DBuf<int> counts(2 * ((size_t)m + 1));
+  int *cnt = counts.get(), *cnt2 = cnt + m + 1;
   counts.zero(st);
   spgemm_symbolic<256>(m, ncols, 0, xrp, xci, yrp, yci, dprod.get(), cnt, dnbig, sum,
-                       max_products, st);
+                       most, st);
   spgemm_symbolic<1024>(m, ncols, 128, xrp, xci, yrp, yci, dprod.get(), cnt, dnbig, sum,
-                        max_products, st);
+                        most, st);
   spgemm_symbolic<kSpgemmSmSlots>(m, ncols, 512, xrp, xci, yrp, yci, dprod.get(), cnt, dnbig, sum,
-                                  max_products, st);
+                                  most, st);
   scan_counts(m, cnt, drps.get(), tmp, st);
-  int64_t total = 0;
-  int nbig = 0;
-  CHRONOS_CUDA(cudaMemcpyAsync(&total, drps.get() + m, sizeof(total), cudaMemcpyDeviceToHost, st));
-  CHRONOS_CUDA(cudaMemcpyAsync(&nbig, dnbig, sizeof(nbig), cudaMemcpyDeviceToHost, st));
-  int64_t products = 0;
-  if (sum)
-    CHRONOS_CUDA(cudaMemcpyAsync(&products, sum, sizeof(products), cudaMemcpyDeviceToHost, st));
+  int64_t heads[3] = {};
+  CHRONOS_CUDA(cudaMemcpyAsync(heads, drps.get() + m, sizeof(heads), cudaMemcpyDeviceToHost, st));
   CHRONOS_CUDA(cudaStreamSynchronize(st));
-  if (products > max_products) return false;
+  int64_t total = heads[0];
+  const int nbig = (int)heads[2];
+  if (heads[1] > most) return false;
   std::vector<int> cnt_h;
   if (nbig > 0) {
     cnt_h.resize(m);
