@@ -394,13 +394,19 @@ int chronos_hier_free(chronos_hier *h);
  * the MATLAB workspace): save writes every level's operator, smoother factor
  * and prolongation (FP64), omega, lambda_max, the coarsest inverse and the
  * parameters; load rebuilds a handle from such a file without the setup --
- * same V-cycle bit for bit -- or returns CHRONOS_EIO for a file it cannot
+ * same V-cycle bit for bit where the device has the same room for its folded
+ * levels and the autotuner the same decisions -- or returns CHRONOS_EIO for a file it cannot
  * use (wrong magic, version, parameter layout, truncated or inconsistent). */
 int chronos_hier_save(const chronos_hier *h, const char *path);
 /* Device memory the library holds in this process (bytes; no counterpart in
  * the reference).  The environment variable CHRONOS_DEVICE_ALLOC_CAP (bytes)
  * caps it: an allocation beyond the cap fails with CHRONOS_ENOMEM as a failed
- * cudaMalloc does, and the call that met it frees what it had allocated. */
+ * cudaMalloc does, and the call that met it frees what it had allocated.
+ * Device memory comes from a pool of the library's own, one per device, which
+ * keeps up to 512 MiB beyond what is counted here for later calls, also after
+ * the last handle is freed and until the process ends: other allocators of the
+ * process do not get that part.  All of it is given back to the driver before
+ * one of the library's allocations is refused. */
 int chronos_device_bytes(int64_t *bytes);
 int chronos_hier_load(const char *path, chronos_hier **out);
 int chronos_hier_nlevels(const chronos_hier *h, int *nlev);
