@@ -315,8 +315,7 @@ inline void give_back() {
 }
 
 // Whether the device (and CHRONOS_DEVICE_ALLOC_CAP) has room for so many bytes more.
-inline bool device_room(int64_t bytes) {
-  give_back();
+inline bool device_room_now(int64_t bytes) {
   const int64_t cap = device_alloc_cap();
   if (cap > 0 && device_bytes_live().load() + bytes > cap) return false;
   uint64_t held = 0, used = 0;
@@ -328,6 +327,11 @@ inline bool device_room(int64_t bytes) {
   size_t avail = 0, total = 0;
   CHRONOS_CUDA(cudaMemGetInfo(&avail, &total));
   return (int64_t)avail + idle >= bytes;
+}
+inline bool device_room(int64_t bytes) {
+  if (device_room_now(bytes)) return true;
+  give_back();
+  return device_room_now(bytes);
 }
 class DeferFrees {
  public:
