@@ -220,7 +220,7 @@ struct BlockState {
   int K = 0, n = 0;
   std::vector<DBuf<float>> b32, x32, r32, t32;
   std::vector<DBuf<double>> b64, x64, r64, t64;
-  DBuf<double> x, res, p, axp, pres, b;
+  DBuf<double> x, res, p, axp, pres;
   DBuf<double> norms;           // ||b||^2 and ||r0||^2 per column
   DBuf<double> sc;              // per-column scalars, see BS_* below
   DBuf<double> part;
@@ -605,7 +605,7 @@ static void block_solve(Hier &h, int m, const BlockIn &B, const double *X0_h, do
     }
     const size_t m0 = (size_t)s.n * K;
     s.x.alloc(m0); s.res.alloc(m0); s.p.alloc(m0); s.axp.alloc(m0); s.pres.alloc(m0);
-    s.b.alloc(m0); s.norms.alloc(2 * K);
+    s.norms.alloc(2 * K);
     s.p.zero(st);
     s.axp.zero(st);
     s.sc.alloc((size_t)BS_COUNT * K + 8);
@@ -616,8 +616,9 @@ static void block_solve(Hier &h, int m, const BlockIn &B, const double *X0_h, do
   }
   BlockState &s = *sp;
   const int n = s.n;
-  // (A p is not formed yet when the host blocks come in, nor needed when x goes out)
-  double *staged = s.axp.get(), *b = s.b.get(), *b2 = s.norms.get(), *r2 = s.norms.get() + K;
+  // (A p is not formed yet when the host blocks come in, nor needed when x goes out;
+  // b has served once res is formed, before the first M^-1 res)
+  double *staged = s.axp.get(), *b = s.pres.get(), *b2 = s.norms.get(), *r2 = s.norms.get() + K;
   // host blocks -> row-major device blocks; a row-major host block of exactly
   // K columns is already in the solve's layout
   const int lb = std::max(1, std::min(num_sms() * 8, (int)ceil_div(n, 32)));

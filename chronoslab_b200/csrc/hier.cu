@@ -1481,12 +1481,12 @@ std::unique_ptr<Hier> build_hierarchy(const chronos_params &prm, HostCSR A0, int
 static void tune_operators(Hier &h);
 
 // Bytes that the solves take beside the hierarchy: a block of 16 columns, the
-// largest of them, has six FP64 vectors a column and four of the hierarchy's
+// largest of them, has five FP64 vectors a column and four of the hierarchy's
 // precision on every level; PCG's six vectors and partials are less.
 static int64_t solve_bytes(const Hier &h) {
   int64_t rows = 0;
   for (const auto &L : h.levels) rows += L.n;
-  return 16 * (48 * (int64_t)h.levels[0].n + (h.precision == CHRONOS_FP32 ? 16 : 32) * rows) +
+  return 16 * (40 * (int64_t)h.levels[0].n + (h.precision == CHRONOS_FP32 ? 16 : 32) * rows) +
          (8 << 20);
 }
 

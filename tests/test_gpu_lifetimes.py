@@ -246,3 +246,21 @@ def test_freeing_a_batch_takes_one_wait(lib):
 
     few = close_time(6)
     assert close_time(48) <= max(3.0 * few, 2e-3)
+
+
+@pytest.mark.parametrize("prec,size", [(cb.CHRONOS_FP64, 8), (cb.CHRONOS_FP32, 4)])
+def test_block_solve_holds_five_vectors(lib, prec, size):
+    """What a block solve leaves on its handle: x, r, p, A p and M^-1 r in FP64 and four
+    vectors of the hierarchy's precision a level, for each of its columns, and the
+    partials of its reductions."""
+    A = PB.poisson7(40)
+    n = A.shape[0]
+    with cb.Hierarchy(A, np.ones((n, 1)), cb.params(precision=prec, ntv=1)) as h:
+        rows = sum(h.level_info(l)["n"] for l in range(h.nlevels))
+        before = cb.device_bytes()
+        B = PB.uniform_rhs(n, 3, 16)
+        X, _, flags, _ = h.pcg_block(B, tol=1e-8)
+        held = cb.device_bytes() - before
+    assert not flags.any()
+    assert np.all(np.linalg.norm(B - A @ X, axis=0) <= 1e-8 * np.linalg.norm(B, axis=0))
+    assert held <= 16 * (5 * 8 * n + 4 * size * rows) + (2 << 20)
